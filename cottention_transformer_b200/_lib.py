@@ -37,6 +37,8 @@ _SIGNATURES = {
     "cott_cos_attn_bwd_train": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "cott_cos_attn_wide_fwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "cott_cos_attn_wide_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "cott_cos_attn_f32_fwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "cott_cos_attn_f32_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "cott_cos_attn_prefill_state": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "cott_decode_step": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, ctypes.c_longlong, _P, _P],
     "cott_decode_steps": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, ctypes.c_longlong, _P, _P],
@@ -53,7 +55,7 @@ _SIGNATURES = {
 }
 _STR = {"cott_version": [], "cott_last_error": [], "cott_status_string": [_I]}
 _SIZE = {"cott_bidir_scratch_bytes": [_I, _I, _I, _I, _I, _I], "cott_cos_attn_saved_bytes": [_I, _I, _I],
-         "cott_cos_attn_wide_workspace_bytes": [_I, _I, _I], "cott_cos_attn_seg_workspace_bytes": [_I, _I, _I, _I]}
+         "cott_cos_attn_wide_workspace_bytes": [_I, _I, _I], "cott_cos_attn_f32_workspace_bytes": [_I, _I, _I, _I], "cott_cos_attn_seg_workspace_bytes": [_I, _I, _I, _I]}
 
 class CottRotaryTables(ctypes.Structure):
     """``cott_rotary_tables``: fp32 sin / cos tables, the rotary dim and the element stride between batch entries."""

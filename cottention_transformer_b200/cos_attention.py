@@ -13,7 +13,8 @@ Two modes, chosen by dtype (not a fallback chain -- each mode is a CUDA path of 
 * float16 / bfloat16, head dim 128: the fused head-dim-128 kernels (``cott_cos_attn_wide_fwd`` / ``_bwd``);
 * float16 / bfloat16, head dim 192 / 256: the row factors pulled out of the scan, tensor-core scans on
   64-wide slices of the head dimension, closed-form backward (``_WideCausal``);
-* float32 / float64 (and any other shape): the reference's own structure --
+* float32, head dims 32 / 64: the same math in fused fp32 kernels (``cott_cos_attn_f32_fwd`` / ``_bwd``);
+* float64 (and any other shape): the reference's own structure --
   elementwise torch ops around ``CustomAttention`` (the exact-mode scan kernel), gradients of
   ``norm_const`` by autograd exactly as in the reference.
 """
@@ -359,6 +360,72 @@ class _WideCausal(torch.autograd.Function):
         return dq, dk, dv, dnc, None
 
 
+def f32_supported(q, k, v, norm_const, keep=None) -> bool:
+    """What the fused fp32 kernels take: dense-able fp32 [B, H, N, 32 | 64] tensors with an fp32 ``norm_const`` and a bool
+    mask.  Under autocast the module math runs in 16 bits around the scan (``CustomAttention``'s dtype rule), and a float
+    mask may hold fractions: both stay with ``_exact_causal``, like every other dtype and head dim."""
+    return (
+        q.dtype == torch.float32 and k.dtype == torch.float32 and v.dtype == torch.float32
+        and q.dim() == 4 and q.shape[-1] in (32, 64) and k.shape == q.shape and v.shape == q.shape and q.numel() > 0
+        and k.device == q.device and v.device == q.device
+        and norm_const.dtype == torch.float32 and norm_const.device == q.device and norm_const.numel() == q.shape[1]
+        and (keep is None or (keep.dtype == torch.bool and keep.device == q.device and tuple(keep.shape) == (q.shape[0], q.shape[2])))
+        and not torch.is_autocast_enabled()
+    )
+
+
+def _dense16(t):
+    """``t`` contiguous with a 16-byte aligned base (a contiguous view at an odd offset is copied)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _FusedF32(torch.autograd.Function):
+    """fp32, head dims 32 / 64: ``cott_cos_attn_f32_fwd`` / ``_bwd`` -- the whole module math in three launches forward and
+    four backward, in place of some fifty elementwise passes around four scans with one CTA per sequence."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, norm_const, keep):
+        ctx.save_for_backward(q, k, v, norm_const)
+        ctx.keep = keep
+        q, k, v = _dense16(q), _dense16(k), _dense16(v)
+        nc = norm_const.detach().contiguous()
+        kp = None if keep is None else keep.contiguous()
+        B, H, N, D = q.shape
+        L = _lib.lib()
+        out = torch.empty(B, H, N, D, dtype=q.dtype, device=q.device)
+        with torch.cuda.device(q.device):
+            ws = torch.empty(L.cott_cos_attn_f32_workspace_bytes(B, H, N, D), dtype=torch.uint8, device=q.device)
+            st = L.cott_cos_attn_f32_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(ws),
+                                         B, H, N, D, _lib.stream_ptr(q.device))
+        _lib.check(st, "cott_cos_attn_f32_fwd")
+        ctx.ws = ws
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        q, k, v, norm_const = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: gradients that can be differentiated again come from the module math
+            x = [t.view_as(t) for t in (q, k, v, norm_const)]  # (one name per argument: the same tensor may be several of them)
+            wanted = [t for t in x if t.requires_grad]
+            g = iter(torch.autograd.grad(_exact_causal(*x, ctx.keep), wanted, dout, create_graph=True, allow_unused=True))
+            return (*(next(g) if t.requires_grad else None for t in x), None)
+        q, k, v, dout = _dense16(q), _dense16(k), _dense16(v), _dense16(dout)
+        nc = norm_const.contiguous()
+        kp = None if ctx.keep is None else ctx.keep.contiguous()
+        B, H, N, D = q.shape
+        L = _lib.lib()
+        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+        dnc = torch.empty_like(nc)
+        with torch.cuda.device(q.device):
+            ws = torch.empty(L.cott_cos_attn_f32_workspace_bytes(B, H, N, D), dtype=torch.uint8, device=q.device)
+            st = L.cott_cos_attn_f32_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(dout), _lib.ptr(ctx.ws),
+                                         _lib.ptr(ws), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dnc), B, H, N, D,
+                                         _lib.stream_ptr(q.device))
+        _lib.check(st, "cott_cos_attn_f32_bwd")
+        return dq, dk, dv, dnc, None
+
+
 def _exact_causal(q, k, v, norm_const, keep):
     """The reference's structure (GPTCosAttention.py:229-248,282) around the exact-mode scan."""
     B, H, N, _ = q.shape
@@ -397,6 +464,8 @@ def cos_attn_causal(q, k, v, norm_const, keep=None, segments=None, one_pass_back
         if q.shape[-1] == 128:
             return _FusedWide128.apply(q, k, v, norm_const, keep)
         return _WideCausal.apply(q, k, v, norm_const, keep)
+    if f32_supported(q, k, v, norm_const, keep):
+        return _FusedF32.apply(q, k, v, norm_const, keep)
     return _exact_causal(q, k, v, norm_const, keep)
 
 

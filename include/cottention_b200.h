@@ -207,6 +207,21 @@ int cott_cos_attn_wide_bwd(const void* q, const void* k, const void* v, const un
                            void* stream);
 
 /*
+ * The same module math in fp32 (q, k, v, out, dout and the gradients float32, dense [B, H, N, D], D = 32 or 64), on CUDA
+ * cores with fp32 products and sums: the mode that is used to check a model (GPT_Trainer/GPTCosAttention.py:229-248,282
+ * around FastAttention2.kernel.float32).  Every 64-position chunk of every sequence is a CTA of its own, started from the
+ * state before (after) it.  `keep`: as in cott_cos_attn_fwd_seg, or NULL; no running count is needed.
+ * Both workspaces: cott_cos_attn_f32_workspace_bytes(B, H, N, D) bytes, 16-byte aligned; the forward leaves the states
+ * before the chunks in its one, pass it, untouched, to the backward as `fwd_workspace`.
+ */
+size_t cott_cos_attn_f32_workspace_bytes(int B, int H, int N, int D);
+int cott_cos_attn_f32_fwd(const float* q, const float* k, const float* v, const unsigned char* keep,
+                          const float* norm_const, float* out, void* workspace, int B, int H, int N, int D, void* stream);
+int cott_cos_attn_f32_bwd(const float* q, const float* k, const float* v, const unsigned char* keep,
+                          const float* norm_const, const float* dout, const void* fwd_workspace, void* workspace,
+                          float* dq, float* dk, float* dv, float* dnorm_const, int B, int H, int N, int D, void* stream);
+
+/*
  * Prefill -> decode hand-off: the decode state (cott_decode_step layout, float32 [B,H,Dv,Dk]) that a prompt of N
  * tokens at positions 1..N leaves behind, state[b,h,j,i] = sum_s v'_s[j] k^_s[i], computed with the segment-state
  * kernels instead of N recurrent steps (the reference absorbs a prompt token by token, GPTCosAttention.py:253-272).

@@ -1,0 +1,99 @@
+"""The fused fp32 causal kernels (head dims 32 and 64) against the fp64 math and against the unfused fp32 path."""
+import pytest
+import torch
+
+from oracle import cott_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# fp32 sums of up to D + 64 products per step with random signs: a relative error of a few times 2^-24 * sqrt(128) = 7e-7
+REL32 = 4e-6
+
+
+def _inputs(B, H, N, D, masked, seed):
+    g = torch.Generator().manual_seed(seed)
+    q, k, v, do = (torch.randn(B, H, N, D, generator=g) for _ in range(4))
+    nc = 0.5 + 0.2 * torch.randn(1, H, 1, 1, generator=g)
+    keep = None
+    if masked:
+        keep = torch.rand(B, N, generator=g) < 0.7
+        keep[0, : N // 3] = False  # positions before the first kept one: n_s = 0
+    return q, k, v, do, nc, keep
+
+
+def _truth(q, k, v, do, nc, keep):
+    q, k, v, nc = (t.double().requires_grad_() for t in (q, k, v, nc))
+    out = O.cos_attn_causal(q, k, v, nc, keep=keep)
+    return out.detach(), *torch.autograd.grad(out, (q, k, v, nc), do.double())
+
+
+def _rel(a, b):
+    return ((a.double().cpu() - b.double().cpu()).norm() / b.double().norm().clamp(min=1e-30)).item()
+
+
+def _run(fn, q, k, v, do, nc, keep):
+    leaf = [t.detach().requires_grad_() for t in (q, k, v, nc)]
+    out = fn(*leaf, keep)
+    return out.detach(), *torch.autograd.grad(out, leaf, do)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 64), (2, 3, 63, 32), (1, 2, 64, 64), (2, 2, 65, 64), (1, 3, 129, 32), (2, 4, 1000, 64),
+                                   (1, 2, 64 * 9, 32)])  # (nine chunks: one more than the prefix kernel loads at a time)
+def test_fused_f32_matches_fp64(shape, masked):
+    from cottention_transformer_b200 import cos_attn_causal
+    q, k, v, do, nc, keep = _inputs(*shape, masked, seed=sum(shape))
+    if masked and not keep.any():
+        keep[0, -1] = True
+    truth = _truth(q, k, v, do, nc, keep)
+    got = _run(cos_attn_causal, *(t.cuda() for t in (q, k, v, do, nc)), None if keep is None else keep.cuda())
+    for name, a, b in zip(("out", "dq", "dk", "dv", "dnorm"), got, truth):
+        # the gradient of norm_const is a signed sum that may cancel: measured against the size of its terms
+        scale = 20 if name == "dnorm" else 1
+        if b.norm() == 0:
+            assert a.norm() == 0, name
+        else:
+            assert _rel(a, b) <= scale * REL32, (name, _rel(a, b))
+
+
+def test_fused_f32_agrees_with_the_unfused_path_over_the_forms_it_accepts():
+    """Strided, offset and expanded inputs, zero and tiny rows, infinities in a masked row, and create_graph."""
+    from cottention_transformer_b200 import cos_attn_causal
+    from cottention_transformer_b200.cos_attention import _exact_causal, f32_supported
+    B, H, N, D = 2, 3, 150, 64
+    q, k, v, do, nc, keep = (t.cuda() for t in _inputs(B, H, N, D, True, seed=5))
+    q[0, 0, 7] = 0          # normalised to zero
+    k[1, 2, 9] = 1e-20      # |k| below the epsilon (1e-20^2 underflows to a zero norm)
+    flat = torch.empty(B * H * N * D + 1, device="cuda")
+    off = flat[1:].view(B, H, N, D)
+    off.copy_(k)            # contiguous, 4 bytes off a 16-byte boundary
+    strided = q.transpose(1, 2).contiguous().transpose(1, 2)
+    wide = do[:, :1].expand(B, H, N, D)
+    for args in ((strided, off, v, wide, nc, keep), (q, k, v, do, nc.reshape(H), None)):
+        assert f32_supported(*args[:3], args[4], args[5])
+        for name, a, b in zip(("out", "dq", "dk", "dv", "dnorm"), _run(cos_attn_causal, *args), _run(_exact_causal, *args)):
+            assert a.shape == b.shape and a.isfinite().all()
+            assert _rel(a, b) <= 5 * REL32, name
+    # a row that is masked by padding may hold anything finite; an infinity reaches the same outputs on both paths
+    q[0, 1, N - 1, 3] = float("inf")
+    a, b = cos_attn_causal(q, k, v, nc), _exact_causal(q, k, v, nc, None)
+    assert torch.equal(a.isnan(), b.isnan())
+    # second derivatives keep going through the module math
+    leaf = v.detach().requires_grad_()
+    (g,) = torch.autograd.grad(cos_attn_causal(k, k, leaf, nc.requires_grad_()).sum(), nc, create_graph=True)
+    assert g.requires_grad
+
+
+def test_f32_forms_that_stay_with_the_unfused_path():
+    from cottention_transformer_b200.cos_attention import f32_supported
+    q = torch.randn(1, 2, 5, 64, device="cuda")
+    nc = torch.zeros(2, device="cuda")
+    assert f32_supported(q, q, q, nc)
+    assert not f32_supported(q, q, q.double(), nc)
+    assert not f32_supported(q, q, q[..., :32], nc)
+    assert not f32_supported(q[..., :16], q[..., :16], q[..., :16], nc)
+    assert not f32_supported(q, q, q, nc.double())
+    assert not f32_supported(q, q, q, nc, torch.ones(1, 5, device="cuda"))
+    assert not f32_supported(q[:, :, :0], q[:, :, :0], q[:, :, :0], nc)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert not f32_supported(q, q, q, nc)
