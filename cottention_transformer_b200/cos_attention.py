@@ -256,8 +256,8 @@ def rotary_packed_(qkv, sin, cos, heads=None):
 
 class _FusedWide128(torch.autograd.Function):
     """Head dim 128 in bf16 / fp16: ``cott_cos_attn_wide_fwd`` / ``_bwd`` -- one tensor-core pass forward (row norms,
-    length factor and output scaling inside the kernel), and a row-dot pass plus three tensor-core passes backward with
-    the normalisation terms in their epilogues.  The forward's row factors travel to the backward in ``ws``."""
+    length factor and output scaling inside the kernel) and three tensor-core passes backward with the normalisation
+    terms in their epilogues.  The forward's row factors and segment states travel to the backward in ``ws``."""
 
     @staticmethod
     def forward(ctx, q, k, v, norm_const, keep):
@@ -274,21 +274,21 @@ class _FusedWide128(torch.autograd.Function):
             st = L.cott_cos_attn_wide_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out),
                                           _lib.ptr(ws), B, H, N, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
         _lib.check(st, "cott_cos_attn_wide_fwd")
-        ctx.save_for_backward(q, k, v, out, nc, ws)
+        ctx.save_for_backward(q, k, v, nc, ws)
         ctx.kp = kp
         ctx.nc_shape, ctx.nc_dtype = norm_const.shape, norm_const.dtype
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, nc, ws = ctx.saved_tensors
+        q, k, v, nc, ws = ctx.saved_tensors
         B, H, N, D = q.shape
         dout = dout.contiguous().to(q.dtype)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dnc = torch.empty(H, dtype=torch.float32, device=q.device)
         with torch.cuda.device(q.device):
             st = _lib.lib().cott_cos_attn_wide_bwd(
-                _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ctx.kp), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(ws),
+                _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ctx.kp), _lib.ptr(nc), None, _lib.ptr(dout), _lib.ptr(ws),
                 _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dnc), B, H, N, D, D, _lib.DTYPE_CODE[q.dtype],
                 _lib.stream_ptr(q.device))
         _lib.check(st, "cott_cos_attn_wide_bwd")

@@ -3,56 +3,75 @@
 //
 // The reference runs kernel_mod_4<T, 32> for D_attn >= 128 (Cuda_Kernel/combined_kernel_general.cu:173-251, selected at
 // :281-284): one warp per output column, four state elements per lane, N serial steps.  Here a CTA owns one
-// (batch, head) sequence and one 64-column slice of the value / output dimension, walks the sequence in chunks of
+// (batch, head) sequence and one W-column slice of the value / output dimension, walks the sequence in chunks of
 // 128 positions, and the whole head dimension of Q and K goes into the SAME score and state accumulators:
 //   P   = mask(X Y^T)            128 x 128, contraction over 128 = two 64-column panels, 8 k-steps   (tcgen05, TMEM)
-//   Acc = P Zs + X S             128 x 64                                                            (A = P from TMEM)
-//   S  += Y^T Zs                 128 x 64 with M = 128: the natural tcgen05 shape, every TMEM lane holds a state row
-// X, Y are [128 x 128] tiles (two swizzled 64-column panels each), Zs the [128 x 64] slice of Z with its rows scaled.
+//   Acc = P Zs + X S             128 x W                                                             (A = P from TMEM)
+//   S  += Y^T Zs                 128 x W with M = 128: the natural tcgen05 shape, every TMEM lane holds a state row
+// X, Y are [128 x 128] tiles (two swizzled 64-column panels each), Zs the [128 x W] slice of Z with its rows scaled.
 // Nothing goes through a scratch buffer and the products are rounded to 16 bits once.
 //
+// W = 128 wherever the value dimension is a multiple of 128, else 64.  A chunk is a chain of hand-offs (load -> row pass
+// -> scores -> mask -> products -> output rows) of 3-4.5 us whatever W is, so the width sets the rate: with W = 64 two
+// CTAs computed the same scores and re-read the same X and Y.  Measured at B 1, H 16, N 16384 (bf16): a pass 104 -> 65-75 us,
+// a state-only pass 45 -> 31 us, forward + backward 563 -> 392 us (a row-dot pass, two transposes and the eps pass went too).
+//
 // The module math around the scan (GPT_Trainer/GPTCosAttention.py:229-248 and its backward) is row scalings, which
-// enter through hooks rather than through extra passes over the tensors:
+// enter through hooks rather than through extra passes over the tensors (the hooks that use a whole row need W = 128 =
+// the head dim):
 //   NORMS   (forward): 1/|x_t|, 1/|y_s| from the tiles themselves, Zs = diag(keep a_s / |y_s|) Z, out rows / |x_t|;
 //           the three row vectors are also written out for the backward
 //   yscale, zscale, oscale: per-position fp32 vectors that scale the rows of Y (in shared memory), of Z (likewise)
 //           and of the output
-//   C, ccoef: out_row += ccoef[pos] * C_row for a fourth tile C (the normalisation terms of the backward: -q (q^.dq^) / |q|^2 ...)
-//   eps:    eps[pos] += oscale[pos] * (C_row . Acc_row)   (v'_s . dv'_s, summed over the two column slices by atomics)
+//   C: a fourth tensor whose rows enter the output rows, o = oscale:
+//           kWdRowAdd   out = o acc + ccoef[pos] C                       (dk: ccoef = -eps / |k|^2)
+//           kWdRowNorm  out = o acc - o^3 (C . acc) C                    (dq through the normalisation of q)
+//           kWdRowEps   out = o acc, and with eps = o (C . acc) = v' . dv': ck_out = -rk^2 eps and the gradient of
+//                       norm_const, -sigma (1 - sigma) sum ln(n) eps     (dv)
 // REV walks the sequence backwards with the mask flipped (the reversed scans of Custom_Kernel.py:107-108).
 // STATE_ONLY keeps only the state chain and writes the segment's own S to global memory (segment-parallel launches).
 //
-// Shared memory (all dynamic): two stages of (X 32 KB, Y 32 KB, Z 16 KB), the double-buffered 16-bit state operand
-// 2 x 16 KB and a two-slot output staging ring 2 x 16 KB = 224 KB, then the row scalars and the barriers.  A stage is
-// refilled as soon as the MMAs of its chunk have completed: output rows are staged in the ring (C rows are copied
-// there straight from global memory by the thread that owns the row), so no store has to drain first.
-// TMEM: P 2 x 128 | Acc 2 x 64 | S 64.
+// Shared memory (all dynamic, W = 128): two stages of (X 32 KB, Y 32 KB, Z 32 KB) and the 16-bit state operand 32 KB =
+// 224 KB, then the barriers.  Output rows are staged over the X tile, whose readers are done when the accumulator is
+// complete; Y and Z of a stage are refilled at that moment (they have a barrier of their own, so the row pass of the next
+// use runs while X is still being stored and reloaded), X once its store has read it.
+// TMEM: P 2 x 128 | Acc W | S W.
 #pragma once
 
 #include "causal_tc.cuh"
 
 namespace cott {
 
-constexpr int kWdThreads = 640;  // 3 issuing warps, 1 TMA warp, 4 groups of 4 warps
+constexpr int kWdThreads = 768;  // 3 issuing warps, 1 TMA warp, 5 groups of 4 warps
 constexpr int kWdStages = 2;
-constexpr int kWdStageBytes = 5 * kTileBytes;
-constexpr int kWdStateBytes = kTcChunk * 128;  // one 16-bit [128 x 64] state operand
+template <int W, bool STATE_ONLY> struct WdCfg {
+  static constexpr int kPanels = W / 64;                                        // 64-column panels of Z, S and the output
+  static constexpr int kStages = STATE_ONLY ? 3 : kWdStages;                    // (the state chain has no X tile)
+  static constexpr int kStageBytes = ((STATE_ONLY ? 2 : 4) + kPanels) * kTileBytes;
+  static constexpr int kStateBytes = STATE_ONLY ? 0 : kPanels * kTileBytes;     // the 16-bit [128 x W] state operand
+  static constexpr size_t kSmemBytes = kStages * kStageBytes + kStateBytes + 2 * 2 * kTcChunk * sizeof(float) + 40 * sizeof(uint64_t);
+};
+enum { kWdRowPlain = 0, kWdRowAdd = 1, kWdRowNorm = 2, kWdRowEps = 3 };
 
 struct WideArgs {
   const float* yscale;  // [B*H*N] or null
   const float* zscale;
   const float* oscale;
-  const float* ccoef;
-  float* eps;           // [B*H*N], accumulated by atomics (zero it first), or null
-  const float* norm_const;  // NORMS only: [H]
+  const float* ccoef;       // kWdRowAdd
+  const float* norm_const;  // NORMS and kWdRowEps: [H]
   float* rq_out;        // NORMS only (may be null): 1/|x_t|, 1/|y_s|, keep a_s/|y_s|
   float* rk_out;
   float* w_out;
-  const float* init_state;  // [B*H][slices][nseg][128 x 64] fp32, the state before each segment in scan order, or null
-  float* state_out;         // STATE_ONLY: [B*H][slices][nseg][128 x 64]
-  const unsigned char* keep;  // NORMS only: padding ([B, N], with its inclusive running count) or both null
+  const float* rk;      // kWdRowEps: 1/|k|
+  float* ck_out;        // kWdRowEps
+  float* dnorm;         // kWdRowEps: [H], accumulated by atomics (zero it first)
+  const float* init_state;  // [B*H][slices][nseg][128 x W] fp32, the state before each segment in scan order, or null
+  int init_transposed;      // W = 128: the matrices of init_state are the transposes of this pass's states
+  float* state_out;         // STATE_ONLY: [B*H][slices][nseg][128 x W]
+  const unsigned char* keep;  // NORMS only: padding ([B, N]) or null; with it `count`, its inclusive running count (also kWdRowEps)
   const int* count;
   const void* c;        // the C tensor [B,H,N,dz] (dense), or null
+  int row_mode;
   int dz;               // row length of Z / C / out in elements
   int chunks_per_seg;
   int H, N;
@@ -66,25 +85,27 @@ __device__ __forceinline__ float row_sumsq2(unsigned char* tile, int row) {
   return row_sumsq_rolled<T>(tile, row) + row_sumsq_rolled<T>(tile + kTileBytes, row);
 }
 
-template <typename T, bool REV, bool NORMS, bool STATE_ONLY>
+template <typename T, int W, bool REV, bool NORMS, bool STATE_ONLY>
 __global__ void __launch_bounds__(kWdThreads, 1)
 wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapY,
             const __grid_constant__ CUtensorMap mapZ, const __grid_constant__ CUtensorMap mapOut, const WideArgs a) {
   using namespace ptx;
-  constexpr int NS = kWdStages;
+  using Cfg = WdCfg<W, STATE_ONLY>;
+  constexpr int NS = Cfg::kStages, NP = Cfg::kPanels;
   constexpr bool BF = Pack2<T>::kBf16;
+  static_assert(!NORMS || W == 128, "the row norm of x is shared by the two output groups: head dim = W = 128");
 
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sS = smem + NS * kWdStageBytes;  // 2 x [128 x 64] 16-bit state operand (rows = columns of Y)
-  unsigned char* sO = sS + 2 * kWdStateBytes;     // 2 x [128 x 64] output staging ring
-  float* s_rq = reinterpret_cast<float*>(sO + 2 * kTileBytes);  // [NS][128] output row scale of a stage (NORMS)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_rq + NS * kTcChunk);
-  uint64_t *bar_full = bars, *bar_free_in = bars + 2, *bar_out = bars + 4, *bar_prep = bars + 6, *bar_p_full = bars + 8,
-           *bar_p_ready = bars + 10, *bar_acc_full = bars + 12, *bar_acc_free = bars + 14, *bar_state = bars + 16;
-  uint64_t &bar_s_full = bars[18], &bar_state2 = bars[19], &bar_init = bars[20];
-  uint64_t* bar_stg_free = bars + 21;  // [2]: the store of the chunk that used the slot has read it
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 23);
-  int& abort_flag_s = *(reinterpret_cast<int*>(bars + 23) + 1);
+  unsigned char* sS = smem + NS * Cfg::kStageBytes;  // [128 x W] 16-bit state operand (rows = columns of Y)
+  float* s_x = reinterpret_cast<float*>(sS + Cfg::kStateBytes);  // [2 chunk parities][2 panels][128]: half-row sums the output groups exchange
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_x + 2 * 2 * kTcChunk);
+  uint64_t *bar_full_x = bars, *bar_full = bars + 3, *bar_free_in = bars + 6, *bar_out = bars + 9, *bar_prep = bars + 12,
+           *bar_p_full = bars + 15, *bar_p_ready = bars + 17, *bar_acc_full = bars + 19;
+  uint64_t &bar_acc_free = bars[21], &bar_xs = bars[22], &bar_state = bars[23], &bar_s_full = bars[24], &bar_state2 = bars[25],
+           &bar_init = bars[26];
+  uint64_t* bar_pair = bars + 28;  // [4]: the two output warps that share rows 32 wq .. exchange their half-row sums
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 27);
+  int& abort_flag_s = *(reinterpret_cast<int*>(bars + 27) + 1);
   volatile int* abort_flag = &abort_flag_s;
 
   const int tid = threadIdx.x, lane = tid & 31;
@@ -99,36 +120,39 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   const size_t state_index = (static_cast<size_t>(bh) * gridDim.y + slice) * gridDim.z + seg;
   const size_t row_base = static_cast<size_t>(bh) * N;  // the per-position vectors are [B*H, N]
   const unsigned char* keep_b = (NORMS && a.keep) ? a.keep + static_cast<size_t>(bb) * N : nullptr;
-  const int* count_b = (NORMS && a.count) ? a.count + static_cast<size_t>(bb) * N : nullptr;
+  const int* count_b = a.count ? a.count + static_cast<size_t>(bb) * N : nullptr;
   // first row of local chunk c (the reversed scan numbers chunks and segments from the end of the sequence)
   auto row0_of = [&](int c) { return (REV ? total_chunks - 1 - (chunk0 + c) : chunk0 + c) * kTcChunk; };
-  auto st_x = [&](int c) { return smem + (c % NS) * kWdStageBytes; };
-  auto st_y = [&](int c) { return smem + (c % NS) * kWdStageBytes + 2 * kTileBytes; };
-  auto st_z = [&](int c) { return smem + (c % NS) * kWdStageBytes + 4 * kTileBytes; };
-  auto st_o = [&](int c) { return sO + (c & 1) * kTileBytes; };
+  // tiles of a stage: Y (2 panels), Z (NP panels), X (2 panels, the first NP of which receive the output rows)
+  auto st_y = [&](int c) { return smem + (c % NS) * Cfg::kStageBytes; };
+  auto st_z = [&](int c) { return st_y(c) + 2 * kTileBytes; };
+  auto st_x = [&](int c) { return st_z(c) + NP * kTileBytes; };
 
   if (smem_u32(smem) & 1023u) {  // the swizzle atoms need the 1024-byte alignment the declaration asks for
     if (tid == 0) atomicCAS(&g_cott_status, 0, (15 << 16));
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < NS; ++s) {
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&bar_full_x[s], 1);
       mbar_init(&bar_full[s], 1);
-      // state group (state MMAs done) + in NORMS mode the output group (it reads the X tile for the row norm);
-      // the TMA thread itself waits for the accumulator MMAs
-      mbar_init(&bar_free_in[s], (NORMS && !STATE_ONLY) ? 8 : 4);
-      mbar_init(&bar_out[s], 4);
+      // state group (STATE_ONLY: the MMA commit itself): state MMAs done; the TMA thread waits for the accumulator MMAs
+      mbar_init(&bar_free_in[s], STATE_ONLY ? 1 : 4);
+      mbar_init(&bar_out[s], 4 * NP);
       mbar_init(&bar_prep[s], 4);
-      mbar_init(&bar_p_full[s], 1);
-      mbar_init(&bar_p_ready[s], 4);
-      mbar_init(&bar_acc_full[s], 1);
-      mbar_init(&bar_acc_free[s], 4);
-      mbar_init(&bar_state[s], 4);
-      mbar_init(&bar_stg_free[s], 1);
     }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bar_p_full[b], 1);
+      mbar_init(&bar_p_ready[b], 4);
+      mbar_init(&bar_acc_full[b], 1);
+    }
+    mbar_init(&bar_acc_free, 4 * NP);
+    mbar_init(&bar_xs, 1);
+    mbar_init(&bar_state, 4);
     mbar_init(&bar_s_full, 1);
     mbar_init(&bar_state2, 4);
     mbar_init(&bar_init, 4);
+    for (int w = 0; w < 4; ++w) mbar_init(&bar_pair[w], 2);
     mbar_fence_init();
     abort_flag_s = 0;
     tma_prefetch_desc(&mapX);
@@ -143,34 +167,39 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const uint32_t tP0 = tmem, tAcc0 = tmem + 256, tS = tmem + 384;  // P 2 x 128 | Acc 2 x 64 | S 64
+  const uint32_t tP0 = tmem, tAcc = tmem + 256, tS = tmem + 384;  // P 2 x 128 | Acc W | S W
 
   // Roles:
   //   warp 0, lane 0:   scores P(c+1) = X Y^T
   //   warp 1, lane 0:   accumulators Acc(c) = X S + P Zs
   //   warp 19, lane 0:  state S += Y^T Zs (c)
   //   warps 2-5:        mask group: mask + convert P in TMEM
-  //   warps 6-9:        output group: accumulator -> output rows
+  //   warps 6-9, 20-23: output groups (panel 0 / panel 1 of the slice): accumulator -> output rows
   //   warps 10-13:      state group: fp32 state -> 16-bit operand
   //   warp 14, lane 0:  TMA loads and stores
   //   warps 15-18:      operand group: row norms / row scalings of Y and Z in place
   constexpr uint32_t kIdescP = make_idesc(128, 128, BF, false, false);
-  constexpr uint32_t kIdescAcc = make_idesc(128, 64, BF, false, true);
-  constexpr uint32_t kIdescS = make_idesc(128, 64, BF, true, true);
+  constexpr uint32_t kIdescAcc = make_idesc(128, W, BF, false, true);
+  constexpr uint32_t kIdescS = make_idesc(128, W, BF, true, true);
+  constexpr uint64_t kPanel = kTileBytes >> 4;
+  // an MN-major operand of one or two 64-column panels, kTileBytes apart
+  auto pdesc = [](unsigned char* p) { return make_smem_desc(smem_u32(p), kTileBytes, 1024); };
   if (warp == 14) {
     // ---------------------------------------------------------------- TMA loads and stores
     if (lane == 0) {
-      const int xz = 64 * slice;  // column offset of the Z / C / output slice
-      auto issue_loads = [&](int c) {
+      const int xz = W * slice;  // column offset of the Z / C / output slice
+      auto load_yz = [&](int c) {
         const int s = c % NS, y = row0_of(c);
-        mbar_expect_tx(&bar_full[s], (STATE_ONLY ? 3 : 5) * kTileBytes);
-        if (!STATE_ONLY) {
-          tma_load_tile_x(st_x(c), &mapX, &bar_full[s], 0, y, h, bb);
-          tma_load_tile_x(st_x(c) + kTileBytes, &mapX, &bar_full[s], 64, y, h, bb);
-        }
+        mbar_expect_tx(&bar_full[s], (2 + NP) * kTileBytes);
         tma_load_tile_x(st_y(c), &mapY, &bar_full[s], 0, y, h, bb);
         tma_load_tile_x(st_y(c) + kTileBytes, &mapY, &bar_full[s], 64, y, h, bb);
-        tma_load_tile_x(st_z(c), &mapZ, &bar_full[s], xz, y, h, bb);
+        for (int p = 0; p < NP; ++p) tma_load_tile_x(st_z(c) + p * kTileBytes, &mapZ, &bar_full[s], xz + 64 * p, y, h, bb);
+      };
+      auto load_x = [&](int c) {
+        const int s = c % NS, y = row0_of(c);
+        mbar_expect_tx(&bar_full_x[s], 2 * kTileBytes);
+        tma_load_tile_x(st_x(c), &mapX, &bar_full_x[s], 0, y, h, bb);
+        tma_load_tile_x(st_x(c) + kTileBytes, &mapX, &bar_full_x[s], 64, y, h, bb);
       };
       auto prefetch = [&](int c) {  // pull a chunk further ahead into L2: with two stages a refill should be an L2 hit
         if (c >= nchunks) return;
@@ -181,28 +210,30 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
         }
         tma_prefetch_tile_x(&mapY, 0, y, h, bb);
         tma_prefetch_tile_x(&mapY, 64, y, h, bb);
-        tma_prefetch_tile_x(&mapZ, xz, y, h, bb);
+        for (int p = 0; p < NP; ++p) tma_prefetch_tile_x(&mapZ, xz + 64 * p, y, h, bb);
       };
-      for (int c = 0; c < NS && c < nchunks; ++c) issue_loads(c);
+      for (int c = 0; c < NS && c < nchunks; ++c) {
+        load_yz(c);
+        if (!STATE_ONLY) load_x(c);
+      }
       prefetch(NS);
       for (int c = 0; c < nchunks; ++c) {
         const int s = c % NS;
-        if (c + NS < nchunks) {
-          // every MMA of chunk c has completed and nothing else reads its tiles: refill the stage.  (The output
-          // group may be running late -- its rows of the previous chunk, a C row still on its way from HBM -- so the
-          // accumulator MMAs are waited for here, not reported by it.)
+        const bool refill = c + NS < nchunks;
+        if (refill) {
+          // every MMA of chunk c has completed: Y and Z have no reader left
           if (!STATE_ONLY && !wait_bar(&bar_acc_full[c & 1], (c >> 1) & 1, abort_flag, kWaitAcc, c)) break;
           if (!wait_bar(&bar_free_in[s], (c / NS) & 1, abort_flag, kWaitStageFree, c)) break;
-          issue_loads(c + NS);
+          load_yz(c + NS);
           prefetch(c + NS + 1);
         }
         if (STATE_ONLY) continue;
         if (!wait_bar(&bar_out[s], (c / NS) & 1, abort_flag, kWaitStageFree, c)) break;
-        tma_store_tile_x(&mapOut, st_o(c), xz, row0_of(c), h, bb);
+        for (int p = 0; p < NP; ++p) tma_store_tile_x(&mapOut, st_x(c) + p * kTileBytes, xz + 64 * p, row0_of(c), h, bb);
         tma_store_commit();
-        if (c >= 1) {  // the store of chunk c-1 has read its staging slot
-          tma_store_wait_read<1>();
-          mbar_arrive(&bar_stg_free[(c - 1) & 1]);
+        if (refill) {
+          tma_store_wait_read<0>();
+          load_x(c + NS);
         }
       }
       tma_store_wait<0>();
@@ -213,7 +244,6 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
       auto issue_scores = [&](int c) {  // caller has waited for the prepared tiles of chunk c and for the buffer
         const uint64_t dX = kdesc(smem_u32(st_x(c))), dY = kdesc(smem_u32(st_y(c)));
         const uint32_t tP = tP0 + 128 * (c & 1);
-        constexpr uint64_t kPanel = kTileBytes >> 4;
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           mma_ss(tP, dX + (k >> 2) * kPanel + 2 * (k & 3), dY + (k >> 2) * kPanel + 2 * (k & 3), kIdescP, k > 0);
@@ -222,7 +252,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
       // The scores read X and Y only: they can go as soon as the TMA has landed, without waiting for the row pass
       // of the operand group -- unless that pass rewrites Y (yscale).
       uint64_t* gate = a.yscale ? bar_prep : bar_full;
-      bool ok = wait_bar1(&gate[0], 0, abort_flag, kWaitPrepped, 0);
+      bool ok = wait_bar2(&gate[0], 0, &bar_full_x[0], 0, abort_flag, kWaitPrepped, 0);
       if (ok) {
         tc_fence_after_sync();
         issue_scores(0);
@@ -230,8 +260,8 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
       for (int c = 0; ok && c + 1 < nchunks; ++c) {
         // scores of chunk c+1: its tiles, and (buffer reuse) the accumulator MMAs of chunk c-1 done
         const int s1 = (c + 1) % NS;
-        ok = wait_bar2(&gate[s1], ((c + 1) / NS) & 1, c >= 1 ? &bar_acc_full[(c + 1) & 1] : &gate[s1],
-                       c >= 1 ? (((c - 1) >> 1) & 1) : (((c + 1) / NS) & 1), abort_flag, kWaitTma, c);
+        ok = wait_bar4(&gate[s1], ((c + 1) / NS) & 1, &bar_full_x[s1], ((c + 1) / NS) & 1, c >= 1 ? &bar_acc_full[(c + 1) & 1] : nullptr,
+                       ((c - 1) >> 1) & 1, nullptr, 0, abort_flag, kWaitTma, c);
         if (!ok) break;
         tc_fence_after_sync();
         issue_scores(c + 1);
@@ -247,35 +277,38 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
                        c > 0 ? ((c - 1) & 1) : 0, nullptr, 0, nullptr, 0, abort_flag, kWaitPrepped, c))
           break;
         tc_fence_after_sync();
-        // A = Y^T: MN-major, M = 128 = the two panels of Y (one panel apart), K = the 128 positions
-        const uint64_t dYm = make_smem_desc(smem_u32(st_y(c)), kTileBytes, 1024), dZm = mdesc(smem_u32(st_z(c)));
+        // A = Y^T: MN-major, M = 128 = the two panels of Y, K = the 128 positions
+        const uint64_t dYm = pdesc(st_y(c)), dZm = pdesc(st_z(c));
         mma_ss(tS, dYm, dZm, kIdescS, (c > 0 || has_init) ? 1u : 0u);
 #pragma unroll
         for (int k = 1; k < 8; ++k) mma_ss(tS, dYm + 128 * k, dZm + 128 * k, kIdescS, 1u);
-        mma_commit(&bar_s_full);
+        if (STATE_ONLY) mma_commit(&bar_free_in[c % NS]);
+        if (!STATE_ONLY || c + 1 == last) mma_commit(&bar_s_full);
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- accumulators
     if (lane == 0 && !STATE_ONLY) {
+      const uint64_t dS = pdesc(sS);
       for (int c = 0; c < nchunks; ++c) {
         const int s = c % NS, b = c & 1;
-        const uint64_t dX = kdesc(smem_u32(st_x(c))), dZm = mdesc(smem_u32(st_z(c)));
-        const uint32_t tP = tP0 + 128 * b, tAcc = tAcc0 + 64 * b;
-        // masked scores of chunk c, the 16-bit state after chunk c-1, the accumulator buffer read out, the prepared Z
-        if (!wait_bar4(&bar_p_ready[b], (c >> 1) & 1, c > 0 ? &bar_state[(c - 1) & 1] : (has_init ? &bar_init : nullptr),
-                       c > 0 ? (((c - 1) >> 1) & 1) : 0, c >= 2 ? &bar_acc_free[b] : nullptr, ((c >> 1) - 1) & 1, &bar_prep[s],
-                       (c / NS) & 1, abort_flag, kWaitScoreReady, c))
+        const uint64_t dX = kdesc(smem_u32(st_x(c))), dZm = pdesc(st_z(c));
+        const uint32_t tP = tP0 + 128 * b;
+        const bool with_s = c > 0 || has_init;
+        // the state term: the 16-bit state after chunk c-1 and the accumulator read out
+        if (!wait_bar4(&bar_full_x[s], (c / NS) & 1, c > 0 ? &bar_state : (has_init ? &bar_init : nullptr), c > 0 ? ((c - 1) & 1) : 0,
+                       c > 0 ? &bar_acc_free : nullptr, (c - 1) & 1, nullptr, 0, abort_flag, kWaitState, c))
           break;
         tc_fence_after_sync();
-        const bool with_s = c > 0 || has_init;
         if (with_s) {
-          // Acc = X S: A = X K-major over both panels, B = the 16-bit state [K = 128 rows, N = 64], MN-major
-          const uint64_t dS = mdesc(smem_u32(sS + b * kWdStateBytes));
-          constexpr uint64_t kPanel = kTileBytes >> 4;
+          // Acc = X S: A = X K-major over both panels, B = the 16-bit state [K = 128 rows, N = W], MN-major
 #pragma unroll
           for (int k = 0; k < 8; ++k) mma_ss(tAcc, dX + (k >> 2) * kPanel + 2 * (k & 3), dS + 128 * k, kIdescAcc, k > 0);
         }
+        mma_commit(&bar_xs);  // the 16-bit state has been read: it may be rewritten
+        // masked scores of chunk c, the prepared Z
+        if (!wait_bar2(&bar_p_ready[b], (c >> 1) & 1, &bar_prep[s], (c / NS) & 1, abort_flag, kWaitScoreReady, c)) break;
+        tc_fence_after_sync();
         mma_ts(tAcc, tP, dZm, kIdescAcc, with_s ? 1u : 0u);  // Acc += P Zs   (P from TMEM, Zs MN-major)
 #pragma unroll
         for (int k = 1; k < 8; ++k) mma_ts(tAcc, tP + 8 * k, dZm + 128 * k, kIdescAcc, 1u);
@@ -300,26 +333,37 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     // ---------------------------------------------------------------- state group (thread = state row = TMEM lane)
     const int wq = warp & 3, row = 32 * wq + lane;
     const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
+    // 32 fp32 columns 32 blk .. of this thread's row -> the 16-bit operand
+    auto to_operand = [&](const uint32_t* r, int blk) {
+      unsigned char* dst = sS + (blk >> 1) * kTileBytes;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *tile_piece(dst, row, 4 * (blk & 1) + j) =
+            make_uint4(Pack2<T>::pack(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])),
+                       Pack2<T>::pack(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
+                       Pack2<T>::pack(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
+                       Pack2<T>::pack(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])));
+    };
     if (has_init) {
-      // the state before this segment: fp32 into TMEM, 16-bit into the operand buffer of chunk 0
-      const float* src = a.init_state + state_index * (kTcChunk * kTcD) + row * kTcD;
+      // the state before this segment: fp32 into TMEM, 16-bit into the operand buffer.  (Transposed: this thread's row
+      // is a column of the stored matrix, and consecutive threads read consecutive elements.)
+      const float* src = a.init_state + state_index * (kTcChunk * W);
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
+      for (int blk = 0; blk < 2 * NP; ++blk) {
         uint32_t r[32];
+        if (a.init_transposed) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float4 f = *reinterpret_cast<const float4*>(src + 32 * half + 4 * j);
-          r[4 * j] = __float_as_uint(f.x), r[4 * j + 1] = __float_as_uint(f.y);
-          r[4 * j + 2] = __float_as_uint(f.z), r[4 * j + 3] = __float_as_uint(f.w);
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(src[(32 * blk + j) * W + row]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 f = *reinterpret_cast<const float4*>(src + row * W + 32 * blk + 4 * j);
+            r[4 * j] = __float_as_uint(f.x), r[4 * j + 1] = __float_as_uint(f.y);
+            r[4 * j + 2] = __float_as_uint(f.z), r[4 * j + 3] = __float_as_uint(f.w);
+          }
         }
-        tmem_st_x32(tS + lane_base + 32 * half, r);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          *tile_piece(sS, row, 4 * half + j) =
-              make_uint4(Pack2<T>::pack(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])),
-                         Pack2<T>::pack(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
-                         Pack2<T>::pack(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
-                         Pack2<T>::pack(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])));
+        tmem_st_x32(tS + lane_base + 32 * blk, r);
+        to_operand(r, blk);
       }
       tmem_st_wait();
       fence_proxy_async_smem();
@@ -327,17 +371,12 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
       warp_arrive(&bar_init, lane);
     }
     if (STATE_ONLY) {
-      // every state MMA frees its stage; after the last one the segment's own state goes to global memory
-      bool ok = true;
-      for (int c = 0; ok && c < nchunks; ++c) {
-        if (!(ok = wait_bar_warp(&bar_s_full, c & 1, abort_flag, kWaitState, c))) break;
-        if (lane == 0) mbar_arrive(&bar_free_in[c % NS]);
-      }
-      if (ok) {
+      // after the last state MMA the segment's own state goes to global memory
+      if (wait_bar_warp(&bar_s_full, 0, abort_flag, kWaitState, 0)) {
         tc_fence_after_sync();
-        float* dst = a.state_out + state_index * (kTcChunk * kTcD) + row * kTcD;
+        float* dst = a.state_out + state_index * (kTcChunk * W) + row * W;
 #pragma unroll 1
-        for (int blk = 0; blk < 4; ++blk) {
+        for (int blk = 0; blk < 4 * NP; ++blk) {
           uint32_t r[16];
           tmem_ld_x16(tS + lane_base + 16 * blk, r);
           tmem_ld_wait();
@@ -350,28 +389,22 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
       }
     } else {
       for (int c = 0; c + 1 < nchunks; ++c) {
-        // S after chunk c -> 16-bit operand for chunk c+1 (buffer (c+1)&1)
+        // S after chunk c -> 16-bit operand for chunk c+1, once the state term of chunk c has read the operand
         if (!wait_bar_warp(&bar_s_full, c & 1, abort_flag, kWaitState, c)) break;
-        tc_fence_after_sync();
         if (lane == 0) mbar_arrive(&bar_free_in[c % NS]);  // the state MMAs of chunk c have read its tiles
-        uint32_t r[32], pk[32];
-        tmem_ld_x32(tS + lane_base, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) pk[j] = Pack2<T>::pack(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-        tmem_ld_x32(tS + lane_base + 32, r);
-        tmem_ld_wait();
+        if (!wait_bar_warp(&bar_xs, c & 1, abort_flag, kWaitAccFree, c)) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int blk = 0; blk < 2 * NP; ++blk) {
+          uint32_t r[32];
+          tmem_ld_x32(tS + lane_base + 32 * blk, r);
+          tmem_ld_wait();
+          to_operand(r, blk);
+        }
         tc_fence_before_sync();
-        warp_arrive(&bar_state2, lane);  // the fp32 state has been read: the next state MMAs may run
-#pragma unroll
-        for (int j = 0; j < 16; ++j) pk[16 + j] = Pack2<T>::pack(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-        // the 16-bit buffer written now was last read by the accumulator MMAs of chunk c-1
-        if (c > 0 && !wait_bar_warp(&bar_acc_full[(c - 1) & 1], ((c - 1) >> 1) & 1, abort_flag, kWaitAccFree, c)) break;
-        unsigned char* dst = sS + ((c + 1) & 1) * kWdStateBytes;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) *tile_piece(dst, row, j) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
         fence_proxy_async_smem();
-        warp_arrive(&bar_state[c & 1], lane);
+        warp_arrive(&bar_state2, lane);  // the fp32 state has been read: the next state MMAs may run
+        if (lane == 0) mbar_arrive(&bar_state);
       }
     }
   } else if (warp >= 15 && warp < 19) {
@@ -380,81 +413,117 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     const float sigma = NORMS ? 1.0f / (1.0f + __expf(-a.norm_const[h])) : 0.f;
     for (int c = 0; c < nchunks; ++c) {
       const int s = c % NS;
-      if (!wait_bar_warp(&bar_full[s], (c / NS) & 1, abort_flag, kWaitTma, c)) break;
       const int pos = row0_of(c) + row;
+      float ys = 1.f, zs = 1.f;
+      if constexpr (!NORMS) {  // (read before the wait: they travel with the tiles)
+        if (a.yscale) ys = pos < N ? a.yscale[row_base + pos] : 0.f;
+        if (a.zscale) zs = pos < N ? a.zscale[row_base + pos] : 0.f;
+      }
+      if (!wait_bar_warp(&bar_full[s], (c / NS) & 1, abort_flag, kWaitTma, c)) break;
       if constexpr (NORMS) {
         const RowMask m = row_mask(keep_b, count_b, pos, N);
         const float rk = m.kp ? inv_norm(row_sumsq2<T>(st_y(c), row)) : 0.f;
         const float w = rk * length_factor(m.n, sigma);
-        scale_row_rolled<T>(st_z(c), row, w);
+        for (int p = 0; p < NP; ++p) scale_row_rolled<T>(st_z(c) + p * kTileBytes, row, w);
         if (!STATE_ONLY && slice == 0 && pos < N && a.rk_out) {
           a.rk_out[row_base + pos] = rk;
           a.w_out[row_base + pos] = w;
         }
       } else {
         if (a.yscale) {
-          const float f = pos < N ? a.yscale[row_base + pos] : 0.f;
-          scale_row_rolled<T>(st_y(c), row, f);
-          scale_row_rolled<T>(st_y(c) + kTileBytes, row, f);
+          scale_row_rolled<T>(st_y(c), row, ys);
+          scale_row_rolled<T>(st_y(c) + kTileBytes, row, ys);
         }
-        if (a.zscale) scale_row_rolled<T>(st_z(c), row, pos < N ? a.zscale[row_base + pos] : 0.f);
+        if (a.zscale)
+          for (int p = 0; p < NP; ++p) scale_row_rolled<T>(st_z(c) + p * kTileBytes, row, zs);
       }
       fence_proxy_async_smem();
       warp_arrive(&bar_prep[s], lane);
     }
-  } else if (warp >= 6 && warp < 10) {
-    // ---------------------------------------------------------------- output group
-    if (!STATE_ONLY) {
+  } else if ((warp >= 6 && warp < 10) || warp >= 20) {
+    // ---------------------------------------------------------------- output groups (panel 0, panel 1)
+    const int panel = warp >= 20 ? 1 : 0;
+    if (!STATE_ONLY && panel < NP) {
       const int wq = warp & 3, row = 32 * wq + lane;
       const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
       const bool has_c = a.c != nullptr;
+      // sum of this thread's half-row value and its partner's (the warp of the other panel that owns the same rows).
+      // Two buffers by chunk parity: a buffer is written again two chunks later, past the pair's next barrier.
+      // (One exchange per chunk, so the barrier's phase is the chunk's parity.)
+      auto pair_sum = [&](float& x, int c) -> bool {
+        if constexpr (NP == 2) {
+          float* buf = s_x + (c & 1) * 2 * kTcChunk;
+          buf[panel * kTcChunk + row] = x;
+          warp_arrive(&bar_pair[wq], lane);
+          if (!wait_bar_warp(&bar_pair[wq], c & 1, abort_flag, kWaitPrepped, c)) return false;
+          x += buf[(panel ^ 1) * kTcChunk + row];
+        }
+        return true;
+      };
+      const float sigma = a.row_mode == kWdRowEps ? 1.0f / (1.0f + __expf(-a.norm_const[h])) : 0.f;
+      float gsum = 0.f;  // sum of ln(n_s) eps_s over this thread's rows
       for (int c = 0; c < nchunks; ++c) {
         const int s = c % NS, b = c & 1;
         const int pos = row0_of(c) + row;
-        unsigned char* dst = st_o(c);
-        // (every phase of `full` is observed)
-        if (!wait_bar_warp(&bar_full[s], (c / NS) & 1, abort_flag, kWaitTma, c)) break;
-        float beta = 1.f, alpha = 0.f;
+        unsigned char* dst = st_x(c) + panel * kTileBytes;
+        float beta = 1.f, alpha = 0.f, rk = 0.f;
         if constexpr (NORMS) {
-          // the row norm of x only needs the TMA data: taken while the MMAs run (the stage cannot be refilled before
-          // this group reports the accumulator MMAs)
-          beta = row_mask(keep_b, count_b, pos, N).kp ? inv_norm(row_sumsq2<T>(st_x(c), row)) : 0.f;
-          if (slice == 0 && pos < N && a.rq_out) a.rq_out[row_base + pos] = beta;
-          if (lane == 0) mbar_arrive(&bar_free_in[s]);  // (warp-converged) this warp is done with the X tile
+          // the row norm of x only needs the TMA data: taken while the MMAs run
+          if (!wait_bar_warp(&bar_full_x[s], (c / NS) & 1, abort_flag, kWaitTma, c)) break;
+          float ss = row_sumsq_rolled<T>(dst, row);
+          if (!pair_sum(ss, c)) break;
+          beta = row_mask(keep_b, count_b, pos, N).kp ? inv_norm(ss) : 0.f;
+          if (panel == 0 && pos < N && a.rq_out) a.rq_out[row_base + pos] = beta;
         } else {
           if (a.oscale) beta = pos < N ? a.oscale[row_base + pos] : 0.f;
-          if (has_c && a.ccoef) alpha = pos < N ? a.ccoef[row_base + pos] : 0.f;
+          if (a.row_mode == kWdRowAdd) alpha = pos < N ? a.ccoef[row_base + pos] : 0.f;
+          if (a.row_mode == kWdRowEps) rk = pos < N ? a.rk[row_base + pos] : 0.f;
         }
-        // this thread's C row, straight from global memory: issued now, so that the loads have the waits below to land
+        // the warp's C rows, straight from global memory and issued now, so that the loads have the wait below to land:
+        // lane l takes piece l % 8 of rows 4 j + l / 8 (four whole 128-byte rows per instruction)
         uint4 u[8];
         if (has_c) {
-          const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(a.c) + (row_base + min(pos, N - 1)) * a.dz + 64 * slice);
+          const int r0 = row0_of(c) + 32 * wq + (lane >> 3);
+          const T* src = static_cast<const T*>(a.c) + 64 * (NP * slice + panel) + 8 * (lane & 7);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) u[j] = pos < N ? src[j] : make_uint4(0, 0, 0, 0);
-        }
-        // the staging slot was last stored from two chunks ago
-        if (c >= 2 && !wait_bar_warp(&bar_stg_free[b], ((c - 2) >> 1) & 1, abort_flag, kWaitStageFree, c)) break;
-        if (has_c) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) *tile_piece(dst, row, j) = u[j];
+          for (int j = 0; j < 8; ++j)
+            u[j] = r0 + 4 * j < N ? *reinterpret_cast<const uint4*>(src + (row_base + r0 + 4 * j) * a.dz) : make_uint4(0, 0, 0, 0);
         }
         if (!wait_bar_warp(&bar_acc_full[b], (c >> 1) & 1, abort_flag, kWaitAcc, c)) break;
         tc_fence_after_sync();
-        const uint32_t tAcc = tAcc0 + 64 * b + lane_base;
-        if (has_c) {
-          if (a.eps) {  // eps += beta (C_row . Acc_row), then the row itself
-            const float e = beta * row_from_acc_dot<T>(dst, row, tAcc, beta);
-            if (pos < N) atomicAdd(a.eps + row_base + pos, e);
+        const uint32_t t = tAcc + 64 * panel + lane_base;
+        if (has_c) {  // the X tile has no reader left: the C rows go there, and are replaced by the output rows
+#pragma unroll
+          for (int j = 0; j < 8; ++j) *tile_piece(dst, 32 * wq + 4 * j + (lane >> 3), lane & 7) = u[j];
+          __syncwarp();
+          if (a.row_mode == kWdRowEps) {
+            float eps = beta * row_from_acc_dot<T>(dst, row, t, beta);
+            if (!pair_sum(eps, c)) break;
+            if (panel == 0 && pos < N) {
+              a.ck_out[row_base + pos] = -rk * rk * eps;
+              const float n = count_b ? fmaxf(static_cast<float>(count_b[pos]), 1.f) : static_cast<float>(pos + 1);
+              if (n > 1.f) gsum += logf(n) * eps;
+            }
           } else {
-            row_from_acc<T, true>(dst, row, tAcc, beta, alpha);
+            if (a.row_mode == kWdRowNorm) {
+              float dot = row_dot_acc<T>(dst, row, t);
+              if (!pair_sum(dot, c)) break;
+              alpha = -beta * beta * beta * dot;
+            }
+            row_from_acc<T, true>(dst, row, t, beta, alpha);
           }
         } else {
-          row_from_acc<T, false>(dst, row, tAcc, beta, 0.f);
+          row_from_acc<T, false>(dst, row, t, beta, 0.f);
         }
         tc_fence_before_sync();
-        warp_arrive(&bar_acc_free[b], lane);
+        warp_arrive(&bar_acc_free, lane);
         fence_proxy_async_smem();
         warp_arrive(&bar_out[s], lane);
+      }
+      if (a.row_mode == kWdRowEps && panel == 0) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) gsum += __shfl_down_sync(0xffffffffu, gsum, off);
+        if (lane == 0) atomicAdd(a.dnorm + h, -sigma * (1.0f - sigma) * gsum);
       }
     }
   }
@@ -464,113 +533,58 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   tc_fence_before_sync();
   __syncthreads();
   if (tid == 0 && *abort_flag) {
-    for (int c = (nchunks > NS ? nchunks - NS : 0); c < nchunks; ++c) mbar_wait(&bar_full[c % NS], (c / NS) & 1, 64);
+    for (int c = (nchunks > NS ? nchunks - NS : 0); c < nchunks; ++c) {
+      mbar_wait(&bar_full[c % NS], (c / NS) & 1, 64);
+      if (!STATE_ONLY) mbar_wait(&bar_full_x[c % NS], (c / NS) & 1, 64);
+    }
   }
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 // Decode state of a whole prompt from the segment states of a head-dim-128 state pass:
-// state[bh][j][i] (+)= sum_seg seg_state[bh][j / 64][seg][i][j % 64]   (the decode kernel keeps the value index first,
-// GPTCosAttention.py:264).  grid = (B*H, 2 slices), any block size.
-__global__ void wide_seg_to_decode_state_kernel(const float* __restrict__ seg_state, float* __restrict__ state, int nseg,
-                                                int accumulate) {
-  const int slice = blockIdx.y;
-  const size_t base = (static_cast<size_t>(blockIdx.x) * gridDim.y + slice) * nseg * (kTcChunk * kTcD);
+// state[bh][j][i] (+)= sum_seg seg_state[bh][seg][i][j]   (the decode kernel keeps the value index first,
+// GPTCosAttention.py:264).  grid = (B*H, any), block 256: a block takes 32 x 32 tiles through shared memory, so that
+// both sides are read and written in whole lines.
+__global__ void __launch_bounds__(256)
+wide_seg_to_decode_state_kernel(const float* __restrict__ seg_state, float* __restrict__ state, int nseg, int accumulate) {
+  __shared__ float tile[32][33];
+  const size_t base = static_cast<size_t>(blockIdx.x) * nseg * (128 * 128);
   float* dst = state + static_cast<size_t>(blockIdx.x) * (128 * 128);
-  for (int e = threadIdx.x; e < 64 * 128; e += blockDim.x) {
-    const int jj = e / 128, i = e % 128;  // output element [64 slice + jj][i] = input element [i][jj]
-    float sum = accumulate ? dst[(64 * slice + jj) * 128 + i] : 0.f;
-    for (int s = 0; s < nseg; ++s) sum += seg_state[base + static_cast<size_t>(s) * (kTcChunk * kTcD) + i * kTcD + jj];
-    dst[(64 * slice + jj) * 128 + i] = sum;
-  }
-}
-
-inline size_t wide_smem_bytes() {
-  return static_cast<size_t>(kWdStages * kWdStageBytes + 2 * kWdStateBytes + 2 * kTileBytes + kWdStages * kTcChunk * sizeof(float) +
-                             32 * sizeof(uint64_t));
-}
-
-// Exclusive prefix over the segments of each (b, h, slice), in scan order: prefix[u][seg] = sum_{s' < seg} state[u][s'].
-// grid = (B*H*slices, any), any block size; `elems` floats per matrix (the elements are split over gridDim.y blocks).
-__global__ void seg_prefix_kernel(const float* __restrict__ state, float* __restrict__ prefix, int nseg, int elems) {
-  const size_t base = static_cast<size_t>(blockIdx.x) * nseg * elems;
-  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < elems; e += gridDim.y * blockDim.x) {
-    float run = 0.f;
-    for (int s = 0; s < nseg; ++s) {
-      prefix[base + static_cast<size_t>(s) * elems + e] = run;
-      run += state[base + static_cast<size_t>(s) * elems + e];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int tl = blockIdx.y; tl < 16; tl += gridDim.y) {
+    const int i0 = 32 * (tl >> 2), j0 = 32 * (tl & 3);
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) {
+      float sum = 0.f;
+      for (int s = 0; s < nseg; ++s) sum += seg_state[base + static_cast<size_t>(s) * (128 * 128) + (i0 + y + r) * 128 + j0 + x];
+      tile[y + r][x] = sum;
     }
-  }
-}
-
-// The segment states of a pass whose roles of Y and Z are swapped are the transposes of these: with the full state
-// M[r][c] (128 x 128, r over the columns of Y, c over the columns of Z) stored as two [128 x 64] column slices,
-//   dst[u][I][seg][r][c] = src[u][r / 64][seg][64 I + c][r % 64]          (u = batch * heads + head, I = 0, 1)
-// (dq's prefix states from the forward's, dk's from dv's: two state-only launches less per backward).
-// grid = (B*H, nseg, any), any block size.
-__global__ void seg_transpose_kernel(const float* __restrict__ src, float* __restrict__ dst, int nseg) {
-  const int u = blockIdx.x, seg = blockIdx.y;
-  constexpr int E = kTcChunk * kTcD;  // 128 x 64
-  for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < 2 * E; e += gridDim.z * blockDim.x) {
-    const int I = e / E, r = (e % E) / kTcD, c = e % kTcD;
-    dst[((static_cast<size_t>(u) * 2 + I) * nseg + seg) * E + r * kTcD + c] =
-        src[((static_cast<size_t>(u) * 2 + r / 64) * nseg + seg) * E + (64 * I + c) * kTcD + r % 64];
-  }
-}
-
-// coef[r] = -scale[r]^2 * (a[r, :] . b[r, :]) for rows of 128 16-bit elements: sixteen threads per row, one 16-byte piece
-// each.  (-q^.dq^ / |q|^2 of the normalisation backward, from q^_t . dq^_t = dO_t . O_t.)
-template <typename T>
-__global__ void rowdot_coef_kernel(const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ scale,
-                                   float* __restrict__ coef, long rows) {
-  const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const long r = i >> 4;
-  float s = 0.f;
-  if (r < rows) {
-    const uint4 u = *reinterpret_cast<const uint4*>(a + r * 128 + (i & 15) * 8);
-    const uint4 w = *reinterpret_cast<const uint4*>(b + r * 128 + (i & 15) * 8);
-    const uint32_t* x = reinterpret_cast<const uint32_t*>(&u);
-    const uint32_t* y = reinterpret_cast<const uint32_t*>(&w);
+    __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = Pack2<T>::unpack(x[e]), g = Pack2<T>::unpack(y[e]);
-      s = fmaf(f.x, g.x, fmaf(f.y, g.y, s));
+    for (int r = 0; r < 32; r += 8) {
+      float* d = dst + (j0 + y + r) * 128 + i0 + x;
+      *d = (accumulate ? *d : 0.f) + tile[x][y + r];
     }
-  }
-#pragma unroll
-  for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off, 16);
-  if (r < rows && (i & 15) == 0) {
-    const float q = scale[r];
-    coef[r] = -q * q * s;
+    __syncthreads();
   }
 }
 
-// After the dV pass: ck[r] = -rk[r]^2 eps[r], and d norm_const[h] += -sigma (1 - sigma) sum_s ln(n_s) eps_s
-// (GPTCosAttention.py:241 by the chain rule; n_s = the running count of kept positions, s + 1 without padding).
-// grid = (B*H, ceil(N / 1024)), block = 256.
-__global__ void eps_coef_kernel(const float* __restrict__ eps, const float* __restrict__ rk, float* __restrict__ ck,
-                                const float* __restrict__ norm_const, float* __restrict__ dnorm, const int* __restrict__ count,
-                                int H, int N) {
-  const int bh = blockIdx.x, h = bh % H, b = bh / H;
-  const size_t base = static_cast<size_t>(bh) * N;
-  float g = 0.f;
-  for (int s = blockIdx.y * 1024 + threadIdx.x; s < min(N, (static_cast<int>(blockIdx.y) + 1) * 1024); s += blockDim.x) {
-    const float e = eps[base + s], r = rk[base + s];
-    ck[base + s] = -r * r * e;
-    const float n = count ? fmaxf(static_cast<float>(count[static_cast<size_t>(b) * N + s]), 1.f) : static_cast<float>(s + 1);
-    if (n > 1.f) g += logf(n) * e;
-  }
-  __shared__ float red[8];
+// Exclusive prefix over the segments of each sequence (and slice), in scan order and in place:
+// state[u][seg] <- sum_{s' < seg} state[u][s'].  grid = (B*H*slices, elems / 256), block = 256: a thread owns one element
+// and loads eight segments at a time (one block per sequence and one load at a time took 31 us for 16 x 9 matrices of 16 KB).
+__global__ void __launch_bounds__(256) seg_prefix_kernel(float* __restrict__ state, int nseg, int elems) {
+  float* p = state + static_cast<size_t>(blockIdx.x) * nseg * elems + blockIdx.y * 256 + threadIdx.x;
+  float run = 0.f;
+  for (int s = 0; s < nseg; s += 8) {
+    float x[8];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) g += __shfl_down_sync(0xffffffffu, g, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = g;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += red[w];
-    const float sigma = 1.0f / (1.0f + __expf(-norm_const[h]));
-    atomicAdd(dnorm + h, -sigma * (1.0f - sigma) * t);
+    for (int i = 0; i < 8; ++i) x[i] = s + i < nseg ? p[static_cast<size_t>(s + i) * elems] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (s + i < nseg) p[static_cast<size_t>(s + i) * elems] = run;
+      run += x[i];
+    }
   }
 }
 

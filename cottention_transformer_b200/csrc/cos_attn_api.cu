@@ -288,8 +288,8 @@ struct WideTensors {  // X, Y: [B,H,N,128]; Z, C, out: [B,H,N,dz] (dz a multiple
 };
 inline TileStrides dense_rows(long H, long N, long D) { return TileStrides{H * N * D, N * D, D}; }
 
-template <typename T, bool REV, bool NORMS, bool STATE_ONLY>
-int launch_wide_t(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, int nseg, cudaStream_t stream) {
+template <typename T, int W, bool REV, bool NORMS, bool STATE_ONLY>
+int launch_wide_w(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, int nseg, cudaStream_t stream) {
   CUtensorMap mx, my, mz, mo;
   const int bf = dtype == COTT_BF16;
   int r;
@@ -303,19 +303,27 @@ int launch_wide_t(const WideTensors& t, WideArgs a, int B, int H, int N, int dty
   a.dz = t.dz;
   a.H = H;
   a.N = N;
-  auto kern = wide_kernel<T, REV, NORMS, STATE_ONLY>;
-  const size_t smem = wide_smem_bytes();
+  auto kern = wide_kernel<T, W, REV, NORMS, STATE_ONLY>;
+  constexpr size_t smem = WdCfg<W, STATE_ONLY>::kSmemBytes;
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3((unsigned)((long)B * H), t.dz / 64, nseg), kWdThreads, smem, stream>>>(mx, my, mz, mo, a);
+  kern<<<dim3((unsigned)((long)B * H), t.dz / W, nseg), kWdThreads, smem, stream>>>(mx, my, mz, mo, a);
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
+// columns of V (and of the state) that one CTA owns: the whole head where the value dimension allows it
+inline int wide_width(int dz) { return dz % 128 == 0 ? 128 : 64; }
+template <typename T, bool REV, bool NORMS, bool STATE_ONLY>
+int launch_wide_t(const WideTensors& t, const WideArgs& a, int B, int H, int N, int dtype, int nseg, cudaStream_t stream) {
+  if (wide_width(t.dz) == 128) return launch_wide_w<T, 128, REV, NORMS, STATE_ONLY>(t, a, B, H, N, dtype, nseg, stream);
+  if constexpr (!NORMS) return launch_wide_w<T, 64, REV, false, STATE_ONLY>(t, a, B, H, N, dtype, nseg, stream);
+  return fail(COTT_ERR_UNSUPPORTED, "the fused head-dim-128 path takes a value dim of 128 (got %d)", t.dz);
+}
 
 // One scan-type pass over head-dim-128 tensors, cut into `nseg` segments per sequence when nseg > 1: the segments'
-// own states (STATE_ONLY launch), their exclusive prefix in scan order, then the pass itself.  `ws`: 2 x B*H*(dz/64)*nseg
-// fp32 [128 x 64] matrices (only touched when nseg > 1).
-// `given_prefix`: the prefix states are already there (a transposed copy of another pass's), skip the state-only launch.
-// After the call ws + A holds the prefix states this pass ran with (A = units * nseg matrices).
+// own states (STATE_ONLY launch), their exclusive prefix in scan order, then the pass itself.  `ws`: wide_ws_floats fp32
+// (only touched when nseg > 1); after the call it holds the prefix states this pass ran with.
+// `given_prefix`: the states are already there, as the transposes of this pass's (the pass with Y and Z swapped left
+// them: sum y (x) z is the transpose of sum z (x) y); skip the state-only launch.
 template <typename T, bool REV, bool NORMS>
 int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, int nseg_requested, float* ws, cudaStream_t stream,
              const float* given_prefix = nullptr) {
@@ -325,30 +333,27 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
   a.state_out = nullptr;
   if (plan.nseg > 1 && given_prefix) {
     a.init_state = given_prefix;
+    a.init_transposed = 1;
   } else if (plan.nseg > 1) {
-    const size_t units = (size_t)B * H * (t.dz / 64);
-    const size_t A = units * plan.nseg * (size_t)(kTcChunk * kTcD);
+    const int W = wide_width(t.dz);
     WideArgs sa = a;
     sa.state_out = ws;
-    sa.eps = nullptr;
     sa.rq_out = sa.rk_out = sa.w_out = nullptr;
     WideTensors st = t;
     st.x = nullptr, st.c = nullptr, st.out = nullptr;
     int r = launch_wide_t<T, REV, NORMS, true>(st, sa, B, H, N, dtype, plan.nseg, stream);
     if (r) return r;
-    seg_prefix_kernel<<<dim3((unsigned)units, 8), 256, 0, stream>>>(ws, ws + A, plan.nseg, kTcChunk * kTcD);
+    seg_prefix_kernel<<<dim3((unsigned)((long)B * H * (t.dz / W)), kTcChunk * W / 256), 256, 0, stream>>>(ws, plan.nseg, kTcChunk * W);
     COTT_CUDA_TRY(cudaGetLastError());
-    a.init_state = ws + A;
+    a.init_state = ws;
   }
   return launch_wide_t<T, REV, NORMS, false>(t, a, B, H, N, dtype, plan.nseg, stream);
 }
 
-size_t wide_ws_floats(int B, int H, int N, int dz, int nseg) {
-  return 2 * (size_t)B * H * (dz / 64) * plan_segments(N, nseg).nseg * (size_t)(kTcChunk * kTcD);
-}
+size_t wide_ws_floats(int B, int H, int N, int dz, int nseg) { return (size_t)B * H * plan_segments(N, nseg).nseg * (size_t)(kTcChunk * dz); }
 
 int wide_seg_count(int B, int H, int N, int dz) {
-  const long units = (long)B * H * (dz / 64);
+  const long units = (long)B * H * (dz / wide_width(dz));
   const int total = (N + kTcChunk - 1) / kTcChunk;
   if (units <= 0 || total < 4) return 1;
   int sm = 148, dev = 0;
@@ -358,25 +363,19 @@ int wide_seg_count(int B, int H, int N, int dz) {
   return nseg < 2 ? 1 : (int)nseg;
 }
 
-// workspace of the fused head-dim-128 pair: six fp32 vectors [B*H*N] (1/|q|, 1/|k|, keep a/|k|, -q^.dq^/|q|^2, eps,
-// -eps/|k|^2), the running keep count [B*N], then the segment states
+// workspace of the fused head-dim-128 pair: the prefix states of the forward-direction passes and those of the reversed
+// ones (first: they are read as 16-byte words), then four fp32 vectors [B*H*N] (1/|q|, 1/|k|, keep a/|k|, -eps/|k|^2) and
+// the running keep count [B*N]
 struct WideWs {
-  float *rq, *rk, *w, *cq, *eps, *ck;
+  float *seg_fwd, *seg_rev;
+  float *rq, *rk, *w, *ck;
   int* count;
-  float* seg;      // 2 x A floats: the segments' own states and their prefix, of the pass that is running
-  float* seg_fwd;  // A floats: the forward's prefix states (the backward transposes them for dq)
-  float* seg_t;    // A floats: a transposed prefix for the pass that is running
 };
 WideWs wide_ws(void* workspace, int B, int H, int N) {
-  const size_t V = (size_t)B * H * N;
+  const size_t V = (size_t)B * H * N, A = wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128));
   float* f = static_cast<float*>(workspace);
-  WideWs s{f, f + V, f + 2 * V, f + 3 * V, f + 4 * V, f + 5 * V, reinterpret_cast<int*>(f + 6 * V), nullptr, nullptr, nullptr};
-  const size_t cnt = ((size_t)B * N + 3) & ~(size_t)3;
-  const size_t A = wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128)) / 2;
-  s.seg = f + 6 * V + cnt;
-  s.seg_fwd = s.seg + 2 * A;
-  s.seg_t = s.seg_fwd + A;
-  return s;
+  float* v = f + 2 * A;
+  return WideWs{f, f + A, v, v + V, v + 2 * V, v + 3 * V, reinterpret_cast<int*>(v + 4 * V)};
 }
 
 template <typename T>
@@ -392,58 +391,34 @@ int run_wide_fwd(const void* q, const void* k, const void* v, const unsigned cha
     a.keep = keep, a.count = ws.count;
   }
   WideTensors t{q, k, v, nullptr, out, 128};
-  const int nseg = plan_segments(N, wide_seg_count(B, H, N, 128)).nseg;
-  int st = run_wide<T, false, true>(t, a, B, H, N, dtype, nseg, ws.seg, stream);
-  if (st == COTT_OK && nseg > 1) {  // the backward's dq pass starts its segments from the transposes of these
-    const size_t A = wide_ws_floats(B, H, N, 128, nseg) / 2;
-    COTT_CUDA_TRY(cudaMemcpyAsync(ws.seg_fwd, ws.seg + A, A * sizeof(float), cudaMemcpyDeviceToDevice, stream));
-  }
-  return st;
+  return run_wide<T, false, true>(t, a, B, H, N, dtype, wide_seg_count(B, H, N, 128), ws.seg_fwd, stream);
 }
 
 template <typename T>
-int run_wide_bwd(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, const void* out, const void* dout,
+int run_wide_bwd(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, const void* dout,
                  void* workspace, void* dq, void* dk, void* dv, float* dnorm, int B, int H, int N, int dtype, cudaStream_t stream) {
   WideWs ws = wide_ws(workspace, B, H, N);
-  const long rows = (long)B * H * N;
-  const int nseg = plan_segments(N, wide_seg_count(B, H, N, 128)).nseg;
-  const size_t A = wide_ws_floats(B, H, N, 128, nseg) / 2;
-  const dim3 tgrid((unsigned)((long)B * H), (unsigned)nseg, 8);
-  // -q^.dq^ / |q|^2 from q^_t . dq^_t = dO_t . O_t
-  rowdot_coef_kernel<T><<<(unsigned)((rows * 16 + 255) / 256), 256, 0, stream>>>(static_cast<const T*>(dout), static_cast<const T*>(out), ws.rq,
-                                                                                ws.cq, rows);
-  COTT_CUDA_TRY(cudaGetLastError());
+  const int nseg = wide_seg_count(B, H, N, 128);
   int st;
-  {  // dq = rq scan(dO, V, diag(w) K) + cq q                      (Custom_Kernel.py:106 with the module math around it)
+  {  // dq = rq scan(dO, V, diag(w) K), through the normalisation      (Custom_Kernel.py:106 with the module math around it)
     WideArgs a = {};
-    a.zscale = ws.w, a.oscale = ws.rq, a.ccoef = ws.cq;
+    a.zscale = ws.w, a.oscale = ws.rq, a.row_mode = kWdRowNorm;
     WideTensors t{dout, v, k, q, dq, 128};
-    if (nseg > 1) {  // sum_s v_s (x) w_s k_s is the transpose of the forward's sum_s k_s (x) w_s v_s
-      seg_transpose_kernel<<<tgrid, 256, 0, stream>>>(ws.seg_fwd, ws.seg_t, nseg);
-      COTT_CUDA_TRY(cudaGetLastError());
-    }
-    if ((st = run_wide<T, false, false>(t, a, B, H, N, dtype, nseg, ws.seg, stream, nseg > 1 ? ws.seg_t : nullptr))) return st;
+    if ((st = run_wide<T, false, false>(t, a, B, H, N, dtype, nseg, nullptr, stream, ws.seg_fwd))) return st;
   }
-  COTT_CUDA_TRY(cudaMemsetAsync(ws.eps, 0, sizeof(float) * rows, stream));
   COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
   {  // dv = w scan_rev(K, diag(rq) Q, dO);  eps = v' . dv'          (:108)
     WideArgs a = {};
-    a.yscale = ws.rq, a.oscale = ws.w, a.eps = ws.eps;
+    a.yscale = ws.rq, a.oscale = ws.w, a.row_mode = kWdRowEps;
+    a.rk = ws.rk, a.ck_out = ws.ck, a.dnorm = dnorm, a.norm_const = nc, a.count = keep ? ws.count : nullptr;
     WideTensors t{k, q, dout, v, dv, 128};
-    if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, ws.seg, stream))) return st;
+    if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, ws.seg_rev, stream))) return st;
   }
-  eps_coef_kernel<<<dim3((unsigned)((long)B * H), (unsigned)((N + 1023) / 1024)), 256, 0, stream>>>(ws.eps, ws.rk, ws.ck, nc, dnorm,
-                                                                                                 keep ? ws.count : nullptr, H, N);
-  COTT_CUDA_TRY(cudaGetLastError());
   {  // dk = w scan_rev(V, dO, diag(rq) Q) + ck k                    (:107)
     WideArgs a = {};
-    a.zscale = ws.rq, a.oscale = ws.w, a.ccoef = ws.ck;
+    a.zscale = ws.rq, a.oscale = ws.w, a.row_mode = kWdRowAdd, a.ccoef = ws.ck;
     WideTensors t{v, dout, q, k, dk, 128};
-    if (nseg > 1) {  // sum_t dO_t (x) q^_t is the transpose of the dv pass's sum_t q^_t (x) dO_t (its prefix is still in ws.seg + A)
-      seg_transpose_kernel<<<tgrid, 256, 0, stream>>>(ws.seg + A, ws.seg_t, nseg);
-      COTT_CUDA_TRY(cudaGetLastError());
-    }
-    if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, ws.seg, stream, nseg > 1 ? ws.seg_t : nullptr))) return st;
+    if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, nullptr, stream, ws.seg_rev))) return st;
   }
   return COTT_OK;
 }
@@ -946,7 +921,7 @@ int cott_cos_attn_bwd_train(const void* q, const void* k, const void* v, const u
 size_t cott_cos_attn_wide_workspace_bytes(int B, int H, int N) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
   const size_t V = (size_t)B * H * N, cnt = ((size_t)B * N + 3) & ~(size_t)3;
-  return (6 * V + cnt + 2 * wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128))) * sizeof(float);
+  return (4 * V + cnt + 2 * wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128))) * sizeof(float);
 }
 
 static int check_wide_args(int B, int H, int N, int Dk, int Dv, int dtype) {
@@ -982,16 +957,16 @@ int cott_cos_attn_wide_bwd(const void* q, const void* k, const void* v, const un
     if (H > 0) COTT_CUDA_TRY(cudaMemsetAsync(dnorm_const, 0, sizeof(float) * H, static_cast<cudaStream_t>(stream)));
     return COTT_OK;
   }
-  if ((st = check_ptrs16({{q, "q"}, {k, "k"}, {v, "v"}, {out, "out"}, {dout, "dout"}, {dq, "dq"}, {dk, "dk"}, {dv, "dv"},
-                          {workspace, "workspace"}})))
+  (void)out;  // (the backward of the row norm of q is taken from its own accumulator)
+  if ((st = check_ptrs16({{q, "q"}, {k, "k"}, {v, "v"}, {dout, "dout"}, {dq, "dq"}, {dk, "dk"}, {dv, "dv"}, {workspace, "workspace"}})))
     return st;
   if (!norm_const) return fail(COTT_ERR_NULL, "null pointer: norm_const");
   DeviceScope scope(q);
   COTT_CUDA_TRY(scope.status());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return dtype == COTT_BF16
-             ? run_wide_bwd<__nv_bfloat16>(q, k, v, keep, norm_const, out, dout, workspace, dq, dk, dv, dnorm_const, B, H, N, dtype, s)
-             : run_wide_bwd<__half>(q, k, v, keep, norm_const, out, dout, workspace, dq, dk, dv, dnorm_const, B, H, N, dtype, s);
+             ? run_wide_bwd<__nv_bfloat16>(q, k, v, keep, norm_const, dout, workspace, dq, dk, dv, dnorm_const, B, H, N, dtype, s)
+             : run_wide_bwd<__half>(q, k, v, keep, norm_const, dout, workspace, dq, dk, dv, dnorm_const, B, H, N, dtype, s);
 }
 
 }  // extern "C"
@@ -1007,11 +982,11 @@ int run_wide_prefill_state(const void* k, const void* v, const float* nc, float*
   WideArgs a = {};
   a.norm_const = nc;
   a.chunks_per_seg = plan.cps;
-  a.state_out = ws.seg;
+  a.state_out = ws.seg_fwd;
   WideTensors t{nullptr, k, v, nullptr, nullptr, 128};
   int st = launch_wide_t<T, false, true, true>(t, a, B, H, N, dtype, plan.nseg, stream);
   if (st) return st;
-  wide_seg_to_decode_state_kernel<<<dim3((unsigned)((long)B * H), 2), 256, 0, stream>>>(ws.seg, state, plan.nseg, accumulate != 0);
+  wide_seg_to_decode_state_kernel<<<dim3((unsigned)((long)B * H), 16), 256, 0, stream>>>(ws.seg_fwd, state, plan.nseg, accumulate != 0);
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
