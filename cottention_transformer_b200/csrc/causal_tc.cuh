@@ -1093,12 +1093,14 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                        dDm = mdesc(q0 + 3 * kTileBytes);
         const uint32_t acc0 = (ci > 0 || has_init) ? 1u : 0u;
         if (ci > 0 || has_init) {
-          // the state terms need the 16-bit state after chunk ci-1 and the accumulators read out, not the
-          // masked scores: they are issued while the score tiles are still being masked
-          // (rotary in the kernel: they read the rotated K tile, which the score group reports with Qw)
-          if (ci > 0 ? !wait_bar4(&bar_state, (ci - 1) & 1, &bar_acc_free, (ci - 1) & 1, ROT ? &bar_prep[s] : nullptr,
-                                  (ci / NS) & 1, nullptr, 0, abort_flag, kWaitState, ci)
-                     : !wait_bar1(&bar_init, 0, abort_flag, kWaitState, ci))
+          // the state terms need the K and V tiles, the 16-bit state after chunk ci-1 and the accumulators read out, not
+          // the masked scores: they are issued while the score tiles are still being masked
+          // (rotary in the kernel: they read the rotated K tile, which the score group reports with Qw; that report
+          // implies the load, but the load has to be waited for here in any case -- the starting state of a segment may
+          // well arrive before the first tiles do)
+          if (!wait_bar4(&bar_full[s], (ci / NS) & 1, ci > 0 ? &bar_state : &bar_init, ci > 0 ? ((ci - 1) & 1) : 0,
+                         ci > 0 ? &bar_acc_free : nullptr, (ci - 1) & 1, ROT ? &bar_prep[s] : nullptr, (ci / NS) & 1, abort_flag,
+                         kWaitState, ci))
             break;
           tc_fence_after_sync();
           const uint32_t rb = r0 + (ci & 1) * (kTcD * 128);
