@@ -102,7 +102,7 @@ bidir_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
   constexpr uint32_t kIdescAcc = make_idesc(128, 64, BF, false, true);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int c = 0; c < 2 && c < nchunks; ++c) {  // the first two Q tiles travel while the state is built
         mbar_expect_tx(&bar_fullq[c], kTileBytes);
@@ -130,7 +130,7 @@ bidir_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
       tma_store_wait<0>();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int c = 0; ok && c < nchunks; ++c) {  // S += K^T Zw
         const int s = c % kBtcKv;
@@ -311,7 +311,7 @@ bidir_bwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
   constexpr uint32_t kIdescMN = make_idesc(128, 64, BF, false, true);   // B MN-major
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       uint32_t ph_free1 = 0, ph_out = 0;  // phase bit per stage
       // hand back the stage of slot g: a first-pass chunk that does not stay is released by its MMAs, every other
@@ -351,7 +351,7 @@ bidir_bwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
       tma_store_wait<0>();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       uint32_t ph_prep1 = 0;
       int p2 = 0;  // second-pass items issued so far (they take the two accumulator sets in turn, across sequences too)

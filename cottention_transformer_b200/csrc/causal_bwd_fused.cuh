@@ -197,7 +197,7 @@ causal_bwd_fused_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
   constexpr uint32_t kIdescMM = make_idesc(128, 64, BF, true, true);    // A MN-major, B MN-major
   constexpr uint32_t kIdescR = make_idesc(64, 64, BF, true, true);
   if (warp == 14) {
-    if (lane == 0) {
+    if (elect_one()) {
       // dO of a stage is free as soon as every MMA of its item has completed; q, K, V as soon as the output
       // groups have read their rows.  All four land on the same `full` barrier; the single S tile has its own.
       auto load_early = [&](int ci) {
@@ -258,7 +258,7 @@ causal_bwd_fused_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
       tma_store_wait<0>();
     }
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_scores = [&](int ci) {  // caller has waited for Qw(ci), Vw(ci) (hence the TMA) and for tE, tF, sE
         const uint64_t dQ = kdesc(smem_u32(st_q(ci))), dK = kdesc(smem_u32(st_k(ci))), dV = kdesc(smem_u32(st_v(ci))),
                        dD = kdesc(smem_u32(st_d(ci)));
@@ -295,7 +295,7 @@ causal_bwd_fused_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t r0 = smem_u32(sR), e0 = smem_u32(sE);
       const uint64_t dEk0 = kdesc(e0), dEk1 = kdesc(e0 + kTileBytes);        // E as a K-major A operand (two panels)
       const uint64_t dEm = make_smem_desc(e0, kTileBytes, 1024)   ;     // E^T: MN-major A, M blocks one panel apart

@@ -68,7 +68,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
   constexpr uint32_t kIdescS = make_idesc(64, 64, BF, true, true);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int c = 0; c < nchunks; ++c) {
         const int s = c & 1;
         if (c >= 2 && !wait_bar(&bar_free[s], ((c >> 1) - 1) & 1, abort_flag, kWaitStageFree, c)) break;
@@ -80,7 +80,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int c = 0; ok && c < nchunks; ++c) {
         const int s = c & 1;

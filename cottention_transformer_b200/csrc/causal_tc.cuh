@@ -630,7 +630,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
   constexpr uint32_t kIdescS = make_idesc(64, 64, BF, true, true);
   if (warp == 0) {
     // ---------------------------------------------------------------- scores
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_scores = [&](int c) {  // caller has waited for the TMA of chunk c and for the buffer
         const uint64_t dX = kdesc(smem_u32(tile_x(c))), dY = kdesc(smem_u32(stage_of(c) + kIdxY * kTileBytes));
         const uint32_t tP = tP0 + 128 * (c & 1);
@@ -663,7 +663,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     // ---------------------------------------------------------------- state
     // state MMA -> conversion -> next state MMA is the loop that sets the chunk period: its issuing thread
     // does nothing else
-    if (lane == 0) {
+    if (elect_one()) {
       for (int c = 0; c + 1 < nchunks; ++c) {
         {
           // state update of chunk c: Zw(c), and the conversion of S after chunk c-1
@@ -684,7 +684,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     // ---------------------------------------------------------------- TMA loads and stores
     // A thread of its own.  The output rows of a chunk are staged over the ring tile of the chunk (forward:
     // the X tile, dQ: the q tile -- the tile whose rows the output group reads last) and stored from there.
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_loads = [&](int c) {
         const int s = c % NS;
         unsigned char* st = stage_of(c);
@@ -712,7 +712,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- accumulators
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t dS0 = mdesc(smem_u32(sS));
       for (int c = 0; c < nchunks; ++c) {
         const int s = c % NS, b = c & 1;
@@ -1003,7 +1003,7 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // TMA loads and stores (a thread of its own, see causal_tc_kernel).  dK and dV are staged in the K and
     // V tiles of the chunk's own stage: q and dO are refilled as soon as every MMA of the chunk has
     // completed, K and V once the output stores have read them.
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_inputs = [&](int ci) {
         const int s = ci % NS;
         const int y = (last_chunk - ci) * kTcChunk;
@@ -1043,7 +1043,7 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       tma_store_wait<0>();
     }
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_scores = [&](int ci) {  // caller has waited for TMA(ci), Qw(ci) and for the tiles to be free
         const uint32_t q0 = smem_u32(smem + (ci % NS) * STAGE);
         const uint64_t dQ = kdesc(q0), dK = kdesc(q0 + kTileBytes), dV = kdesc(q0 + 2 * kTileBytes),
@@ -1084,7 +1084,7 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t r0 = smem_u32(sR);
       for (int ci = 0; ci < nchunks; ++ci) {
         const int s = ci % NS;

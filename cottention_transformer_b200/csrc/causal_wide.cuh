@@ -186,7 +186,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   auto pdesc = [](unsigned char* p) { return make_smem_desc(smem_u32(p), kTileBytes, 1024); };
   if (warp == 14) {
     // ---------------------------------------------------------------- TMA loads and stores
-    if (lane == 0) {
+    if (elect_one()) {
       const int xz = W * slice;  // column offset of the Z / C / output slice
       auto load_yz = [&](int c) {
         const int s = c % NS, y = row0_of(c);
@@ -240,7 +240,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     }
   } else if (warp == 0) {
     // ---------------------------------------------------------------- scores
-    if (lane == 0 && !STATE_ONLY) {
+    if (!STATE_ONLY && elect_one()) {
       auto issue_scores = [&](int c) {  // caller has waited for the prepared tiles of chunk c and for the buffer
         const uint64_t dX = kdesc(smem_u32(st_x(c))), dY = kdesc(smem_u32(st_y(c)));
         const uint32_t tP = tP0 + 128 * (c & 1);
@@ -269,7 +269,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     }
   } else if (warp == 19) {
     // ---------------------------------------------------------------- state
-    if (lane == 0) {
+    if (elect_one()) {
       const int last = STATE_ONLY ? nchunks : nchunks - 1;  // the state after the last chunk is only needed by STATE_ONLY
       for (int c = 0; c < last; ++c) {
         // state update of chunk c: its prepared tiles, and the conversion of S after chunk c-1 (it reads the fp32 state)
@@ -288,7 +288,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- accumulators
-    if (lane == 0 && !STATE_ONLY) {
+    if (!STATE_ONLY && elect_one()) {
       const uint64_t dS = pdesc(sS);
       for (int c = 0; c < nchunks; ++c) {
         const int s = c % NS, b = c & 1;
