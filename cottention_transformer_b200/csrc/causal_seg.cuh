@@ -5,7 +5,7 @@
 // boundary only needs the state accumulated over everything before it (forward, dQ) or after it (dK/dV):
 //   1. seg_state_kernel   one CTA per (b, h, segment): the segment's own contribution  sum_s y_s (x) z_s
 //                         (forward state: y = k^, z = v';  reverse state: y = q^, z = dO), tcgen05 M = 64 MMAs
-//   2. seg_scan_kernel    exclusive prefix (or suffix) sums over the segments of each (b, h), fp32
+//   2. seg_prefix_kernel  exclusive prefix (or suffix) sums over the segments of each (b, h), fp32
 //   3. causal_tc_kernel / causal_bwd_kv_kernel with gridDim.y = number of segments and `init_state`
 // Step 1 re-reads two of the tensors, i.e. the forward moves 6 instead of 4 tensor passes.
 #pragma once
@@ -147,31 +147,27 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
 
 inline size_t seg_state_smem_bytes() { return static_cast<size_t>(4 * kTileBytes + 1024); }
 
-// Exclusive scans over the segments of each (b, h):  grid = B*H, any block size.
-//   prefix[seg]   = sum_{s' < seg} state[s']          (forward state before the segment)
-//   prefix_t[seg] = prefix[seg] transposed            (the dQ pass uses the state with rows d_v)
-//   suffix[seg]   = sum_{s' > seg} state[s']          (reverse state after the segment)
-// Null outputs are skipped.
-__global__ void seg_scan_kernel(const float* __restrict__ state, float* __restrict__ prefix, float* __restrict__ prefix_t,
-                                float* __restrict__ suffix, int nseg) {
-  const size_t base = static_cast<size_t>(blockIdx.x) * nseg * (kTcD * kTcD);
-  for (int e = threadIdx.x; e < kTcD * kTcD; e += blockDim.x) {
-    const int et = (e % kTcD) * kTcD + e / kTcD;
-    if (prefix || prefix_t) {
-      float run = 0.f;
-      for (int s = 0; s < nseg; ++s) {
-        if (prefix) prefix[base + static_cast<size_t>(s) * (kTcD * kTcD) + e] = run;
-        if (prefix_t) prefix_t[base + static_cast<size_t>(s) * (kTcD * kTcD) + et] = run;
-        run += state[base + static_cast<size_t>(s) * (kTcD * kTcD) + e];
+// Exclusive prefix (REV: suffix) over the segments of a sequence, in place: state[u][seg] <- sum over the segments before
+// (after) it.  grid = (sequences, ceil(elems / 4 / 64)), block = 64: a thread owns four neighbouring elements and has
+// eight segments in flight, so that the chain is additions and not memory round trips.
+// Measured: 16 x 9 matrices of 16 KB in 6 us (one block per sequence, one load at a time and a transposed copy: 31 us).
+template <bool REV>
+__global__ void __launch_bounds__(64) seg_prefix_kernel(float4* __restrict__ state, int nseg, int quads) {
+  const int e = blockIdx.y * 64 + threadIdx.x;
+  if (e >= quads) return;
+  float4* p = state + static_cast<size_t>(blockIdx.x) * nseg * quads + e;
+  float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < nseg; s += 8) {
+    float4 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (s + i < nseg) x[i] = p[static_cast<size_t>(REV ? nseg - 1 - s - i : s + i) * quads];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (s + i < nseg) {
+        p[static_cast<size_t>(REV ? nseg - 1 - s - i : s + i) * quads] = run;
+        run.x += x[i].x, run.y += x[i].y, run.z += x[i].z, run.w += x[i].w;
       }
-    }
-    if (suffix) {
-      float run = 0.f;
-      for (int s = nseg - 1; s >= 0; --s) {
-        suffix[base + static_cast<size_t>(s) * (kTcD * kTcD) + e] = run;
-        run += state[base + static_cast<size_t>(s) * (kTcD * kTcD) + e];
-      }
-    }
   }
 }
 

@@ -458,17 +458,23 @@ __device__ __forceinline__ void state_to_smem_rolled(uint32_t tS_lane, unsigned 
 // A segment's starting state (fp32 [64 x 64], row-major) -> TMEM in the M=64 accumulator layout (lanes 16-31
 // of the warp belong to no row of that layout and receive a copy of lanes 0-15) and, as 16 bits, into the
 // swizzled smem operand.  The caller waits for the TMEM stores (tcgen05.wait::st) and fences.
-template <typename T>
+// TR: `state` holds the transpose (consecutive threads then read consecutive elements).
+template <typename T, bool TR = false>
 __device__ __noinline__ void load_init_state(const float* state, uint32_t tS_lane, unsigned char* sS, int wq, int lane) {
-  const float* src = state + (16 * wq + (lane & 15)) * kTcD;
+  const float* src = state + (16 * wq + (lane & 15)) * (TR ? 1 : kTcD);
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
     uint32_t r[32];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float4 f = *reinterpret_cast<const float4*>(src + 32 * half + 4 * j);
-      r[4 * j] = __float_as_uint(f.x), r[4 * j + 1] = __float_as_uint(f.y);
-      r[4 * j + 2] = __float_as_uint(f.z), r[4 * j + 3] = __float_as_uint(f.w);
+      if constexpr (TR) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[4 * j + e] = __float_as_uint(src[(32 * half + 4 * j + e) * kTcD]);
+      } else {
+        const float4 f = *reinterpret_cast<const float4*>(src + 32 * half + 4 * j);
+        r[4 * j] = __float_as_uint(f.x), r[4 * j + 1] = __float_as_uint(f.y);
+        r[4 * j + 2] = __float_as_uint(f.z), r[4 * j + 3] = __float_as_uint(f.w);
+      }
     }
     ptx::tmem_st_x32(tS_lane + 32 * half, r);
     if (lane < 16) {
@@ -510,6 +516,8 @@ constexpr int kTcStagesFwd = 4;  // the forward kernel has the shared memory for
 // sensitive to every instruction added to their loops, and the common case needs neither.
 // SAVE (forward only): the 16-bit state operand of every chunk -- the state BEFORE the chunk, [64 x 64], rows d_k --
 // is also written to `saved` ([B*H][chunks of the sequence][64][64], row-major), for the one-pass backward.
+// decode_state (forward, EXT): the state after the whole sequence also goes to [B*H][64][64] with the value index first
+// (the layout of the decode step, GPTCosAttention.py:264): the last segment runs one more state update and stores it.
 // ROT (forward and dQ, EXT only, one segment): q and k are rotated by the rotary embedding inside the kernel -- the
 // Q and K tiles are rewritten in shared memory before any MMA reads them, and the dQ rows are rotated back before
 // they are stored -- so the tensors in HBM stay un-rotated and no separate pass over q, k, dq, dk is needed.
@@ -520,7 +528,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
                  const __grid_constant__ CUtensorMap mapOut, const float* __restrict__ norm_const, int H, int N,
                  const float* __restrict__ init_state_arg, int chunks_per_seg_arg,
                  const unsigned char* __restrict__ keep_arg, const int* __restrict__ count_arg,
-                 uint4* __restrict__ saved, const RotArgs rot) {
+                 uint4* __restrict__ saved, const RotArgs rot, float* __restrict__ decode_state) {
   using namespace ptx;
   static_assert(!ROT || (EXT && !SAVE && (MODE == kModeFwd || MODE == kModeDq)), "rotary: forward / dQ, EXT, no saved states");
   // Shared memory: NS stages of the tiles that are only read (forward: Y, Z; dQ: X, Y, Z), a ring of
@@ -566,6 +574,9 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
   const int chunk0 = seg * chunks_per_seg;
   const int nchunks = EXT ? min(chunks_per_seg, total_chunks - chunk0) : total_chunks;
   const bool has_init = EXT && init_state != nullptr && seg > 0;
+  // state updates of this CTA: the one after its last chunk is only needed as the decode state
+  const bool final_state = EXT && MODE == kModeFwd && decode_state != nullptr && seg + 1 == static_cast<int>(gridDim.y);
+  const int nstates = nchunks - 1 + (final_state ? 1 : 0);
   const unsigned char* keep_b = (EXT && keep_arg) ? keep_arg + static_cast<size_t>(bh / H) * N : nullptr;
   const int* count_b = (EXT && count_arg) ? count_arg + static_cast<size_t>(bh / H) * N : nullptr;
   // first row of local chunk c (the reversed scan numbers chunks and segments from the end of the sequence)
@@ -664,7 +675,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     // state MMA -> conversion -> next state MMA is the loop that sets the chunk period: its issuing thread
     // does nothing else
     if (elect_one()) {
-      for (int c = 0; c + 1 < nchunks; ++c) {
+      for (int c = 0; c < nstates; ++c) {
         {
           // state update of chunk c: Zw(c), and the conversion of S after chunk c-1
           if (!wait_bar4(&bar_prep[c % NS], (c / NS) & 1, c > 0 ? &bar_state2 : (has_init ? &bar_init : nullptr),
@@ -754,8 +765,10 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     const int wq = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
     if (has_init) {
-      // the state before this segment: fp32 into TMEM, 16-bit into the operand buffer of chunk 0
-      load_init_state<T>(init_state + (static_cast<size_t>(bh) * gridDim.y + seg) * (kTcD * kTcD), tS + lane_base, sS, wq, lane);
+      // the state before this segment: fp32 into TMEM, 16-bit into the operand buffer of chunk 0 (dQ: its state is the
+      // transpose of the forward's, sum v (x) w k against sum k (x) w v)
+      load_init_state<T, MODE == kModeDq>(init_state + (static_cast<size_t>(bh) * gridDim.y + seg) * (kTcD * kTcD), tS + lane_base, sS,
+                                          wq, lane);
       tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before_sync();
@@ -766,10 +779,24 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
         for (int j = 0; j < 8; ++j) dst[j] = *tile_piece(sS, 16 * wq + lane, j);
       }
     }
-    for (int c = 0; c + 1 < nchunks; ++c) {
+    for (int c = 0; c < nstates; ++c) {
       // S after chunk c -> 16-bit operand for chunk c+1 (buffer (c+1)&1)
       if (!wait_bar_warp(&bar_s_full, c & 1, abort_flag, kWaitState, c)) break;
       tc_fence_after_sync();
+      if (EXT && MODE == kModeFwd && c + 1 == nchunks) {  // the last one: to the decode state [value][key], row i = key index
+        float* dst = decode_state + static_cast<size_t>(bh) * (kTcD * kTcD) + 16 * wq + lane;
+#pragma unroll 1
+        for (int blk = 0; blk < 4; ++blk) {
+          uint32_t r[16];
+          tmem_ld_x16(tS + lane_base + 16 * blk, r);
+          tmem_ld_wait();
+          if (lane < 16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[(16 * blk + j) * kTcD] = __uint_as_float(r[j]);
+          }
+        }
+        break;
+      }
       if (lane == 0) mbar_arrive(&bar_free_in[c % NS]);  // the state MMAs of chunk c have read its tiles
       // The state MMA of chunk c+1 waits for this read of the fp32 state (and the accumulator MMAs of
       // chunk c+1 for the 16-bit copy): that loop sets the chunk period.  So the read is reported as soon

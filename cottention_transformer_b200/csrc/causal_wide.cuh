@@ -68,6 +68,7 @@ struct WideArgs {
   const float* init_state;  // [B*H][slices][nseg][128 x W] fp32, the state before each segment in scan order, or null
   int init_transposed;      // W = 128: the matrices of init_state are the transposes of this pass's states
   float* state_out;         // STATE_ONLY: [B*H][slices][nseg][128 x W]
+  float* decode_state;      // NORMS: the state after the whole sequence, [B*H][128][128] with the value index first, or null
   const unsigned char* keep;  // NORMS only: padding ([B, N]) or null; with it `count`, its inclusive running count (also kWdRowEps)
   const int* count;
   const void* c;        // the C tensor [B,H,N,dz] (dense), or null
@@ -117,6 +118,9 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   const int chunk0 = seg * a.chunks_per_seg;
   const int nchunks = min(a.chunks_per_seg, total_chunks - chunk0);
   const bool has_init = !STATE_ONLY && a.init_state != nullptr && seg > 0;
+  // state updates of this CTA: the one after its last chunk is only needed by STATE_ONLY and as the decode state
+  const bool final_state = NORMS && !STATE_ONLY && a.decode_state != nullptr && seg + 1 == static_cast<int>(gridDim.z);
+  const int nstates = STATE_ONLY || final_state ? nchunks : nchunks - 1;
   const size_t state_index = (static_cast<size_t>(bh) * gridDim.y + slice) * gridDim.z + seg;
   const size_t row_base = static_cast<size_t>(bh) * N;  // the per-position vectors are [B*H, N]
   const unsigned char* keep_b = (NORMS && a.keep) ? a.keep + static_cast<size_t>(bb) * N : nullptr;
@@ -270,8 +274,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   } else if (warp == 19) {
     // ---------------------------------------------------------------- state
     if (elect_one()) {
-      const int last = STATE_ONLY ? nchunks : nchunks - 1;  // the state after the last chunk is only needed by STATE_ONLY
-      for (int c = 0; c < last; ++c) {
+      for (int c = 0; c < nstates; ++c) {
         // state update of chunk c: its prepared tiles, and the conversion of S after chunk c-1 (it reads the fp32 state)
         if (!wait_bar4(&bar_prep[c % NS], (c / NS) & 1, (!STATE_ONLY && c > 0) ? &bar_state2 : (has_init ? &bar_init : nullptr),
                        c > 0 ? ((c - 1) & 1) : 0, nullptr, 0, nullptr, 0, abort_flag, kWaitPrepped, c))
@@ -283,7 +286,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
 #pragma unroll
         for (int k = 1; k < 8; ++k) mma_ss(tS, dYm + 128 * k, dZm + 128 * k, kIdescS, 1u);
         if (STATE_ONLY) mma_commit(&bar_free_in[c % NS]);
-        if (!STATE_ONLY || c + 1 == last) mma_commit(&bar_s_full);
+        if (!STATE_ONLY || c + 1 == nstates) mma_commit(&bar_s_full);
       }
     }
   } else if (warp == 1) {
@@ -388,9 +391,22 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
         }
       }
     } else {
-      for (int c = 0; c + 1 < nchunks; ++c) {
+      for (int c = 0; c < nstates; ++c) {
         // S after chunk c -> 16-bit operand for chunk c+1, once the state term of chunk c has read the operand
         if (!wait_bar_warp(&bar_s_full, c & 1, abort_flag, kWaitState, c)) break;
+        if (NORMS && c + 1 == nchunks) {  // the last one: to the decode state [value][key], row = key index
+          tc_fence_after_sync();
+          float* dst = a.decode_state + static_cast<size_t>(bh) * (128 * 128) + row;
+#pragma unroll 1
+          for (int blk = 0; blk < 8; ++blk) {
+            uint32_t r[16];
+            tmem_ld_x16(tS + lane_base + 16 * blk, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[(16 * blk + j) * 128] = __uint_as_float(r[j]);
+          }
+          break;
+        }
         if (lane == 0) mbar_arrive(&bar_free_in[c % NS]);  // the state MMAs of chunk c have read its tiles
         if (!wait_bar_warp(&bar_xs, c & 1, abort_flag, kWaitAccFree, c)) break;
         tc_fence_after_sync();
@@ -567,24 +583,6 @@ wide_seg_to_decode_state_kernel(const float* __restrict__ seg_state, float* __re
       *d = (accumulate ? *d : 0.f) + tile[x][y + r];
     }
     __syncthreads();
-  }
-}
-
-// Exclusive prefix over the segments of each sequence (and slice), in scan order and in place:
-// state[u][seg] <- sum_{s' < seg} state[u][s'].  grid = (B*H*slices, elems / 256), block = 256: a thread owns one element
-// and loads eight segments at a time (one block per sequence and one load at a time took 31 us for 16 x 9 matrices of 16 KB).
-__global__ void __launch_bounds__(256) seg_prefix_kernel(float* __restrict__ state, int nseg, int elems) {
-  float* p = state + static_cast<size_t>(blockIdx.x) * nseg * elems + blockIdx.y * 256 + threadIdx.x;
-  float run = 0.f;
-  for (int s = 0; s < nseg; s += 8) {
-    float x[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = s + i < nseg ? p[static_cast<size_t>(s + i) * elems] : 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (s + i < nseg) p[static_cast<size_t>(s + i) * elems] = run;
-      run += x[i];
-    }
   }
 }
 

@@ -65,16 +65,34 @@ SegPlan plan_segments(int N, int nseg_requested) {
   return p;
 }
 
+// Segments per sequence for `units` independent sequences of N positions: one CTA per SM, at least two chunks each, and
+// only where it pays.  A pass over c chunks takes about c chunk periods; cut into segments of cps chunks it takes cps of
+// them, about half as long again for the segments' own states, and the launches and the prefix in between, which cost
+// `overhead` chunk periods.  (Measured, forward + backward, head dim 64: B 2, H 16, N 1024 in 4 segments of 2 chunks 75 us
+// against 51 us in one; B 4, H 8, N 2048 in 4 segments of 4 chunks 66 us against 90 us; B 1, H 16, N 8192 in 9 of 8 97 against 310.)
+int seg_count(long units, int N, int overhead) {
+  const int total = (N + kTcChunk - 1) / kTcChunk;
+  if (units <= 0 || total < 4) return 1;
+  int sm = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  long nseg = sm / units;
+  if (nseg > total / 2) nseg = total / 2;
+  if (nseg < 2) return 1;
+  const long cps = (total + nseg - 1) / nseg;
+  return 2 * total > 3 * cps + 2 * overhead ? (int)nseg : 1;
+}
+
 template <typename T>
 int launch_fwd(const void* q, const void* k, const void* v, const float* nc, void* out, int B, int H, int N,
-               int dtype, cudaStream_t stream, const float* init = nullptr, SegPlan plan = SegPlan(), void* saved = nullptr) {
+               int dtype, cudaStream_t stream, const float* init = nullptr, SegPlan plan = SegPlan(), void* saved = nullptr,
+               float* decode_state = nullptr) {
   const long BH = (long)B * H;
   CUtensorMap mq, mk, mv, mo;
   int st;
   if ((st = tmap(&mq, q, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) ||
       (st = tmap(&mo, out, dtype, B, H, N, out_strides(plan, H, N))))
     return st;
-  const bool ext = plan.nseg > 1 || init || plan.keep;
+  const bool ext = plan.nseg > 1 || init || plan.keep || decode_state;
   auto kern = plan.rot.sin ? causal_tc_kernel<T, kModeFwd, true, false, true>
               : saved      ? (ext ? causal_tc_kernel<T, kModeFwd, true, true> : causal_tc_kernel<T, kModeFwd, false, true>)
                            : (ext ? causal_tc_kernel<T, kModeFwd, true, false> : causal_tc_kernel<T, kModeFwd, false, false>);
@@ -82,7 +100,7 @@ int launch_fwd(const void* q, const void* k, const void* v, const float* nc, voi
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (plan.cps == 0) plan.cps = plan_segments(N, 1).cps;
   COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)BH, plan.nseg), kTcThreads, smem, stream, mq, mk, mv, mq, mo, nc, H, N, init, plan.cps,
-                           plan.keep, plan.count, static_cast<uint4*>(saved), plan.rot));
+                           plan.keep, plan.count, static_cast<uint4*>(saved), plan.rot, decode_state));
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
@@ -104,7 +122,7 @@ int launch_bwd_dq(const void* q, const void* k, const void* v, const float* nc, 
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (plan.cps == 0) plan.cps = plan_segments(N, 1).cps;
   COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)BH, plan.nseg), kTcThreads, smem, stream, md, mv, mk, mq, mo, nc, H, N, init, plan.cps,
-                           plan.keep, plan.count, static_cast<uint4*>(nullptr), plan.rot));
+                           plan.keep, plan.count, static_cast<uint4*>(nullptr), plan.rot, static_cast<float*>(nullptr)));
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
@@ -177,10 +195,15 @@ int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides s
   return COTT_OK;
 }
 
-// workspace of the segment-parallel path: five arrays of B*H*nseg fp32 [64 x 64] matrices
-//   0 forward segment states | 1 their exclusive prefix | 2 the prefix transposed | 3 reverse segment states |
-//   4 their exclusive suffix
+// workspace of the segment-parallel path: two arrays of B*H*nseg fp32 [64 x 64] matrices, then the running keep count
+//   0 forward segment states, then their exclusive prefix | 1 reverse segment states, then their exclusive suffix
 size_t seg_array_floats(int B, int H, int nseg) { return (size_t)B * H * nseg * kTcD * kTcD; }
+int launch_seg_prefix(float* state, long sequences, int nseg, int elems, bool reverse, cudaStream_t stream) {
+  auto kern = reverse ? seg_prefix_kernel<true> : seg_prefix_kernel<false>;
+  kern<<<dim3((unsigned)sequences, (unsigned)((elems / 4 + 63) / 64)), 64, 0, stream>>>(reinterpret_cast<float4*>(state), nseg, elems / 4);
+  COTT_CUDA_TRY(cudaGetLastError());
+  return COTT_OK;
+}
 
 void apply_layout(SegPlan& plan, const cott_layout* l) {
   if (!l) return;
@@ -191,24 +214,22 @@ void apply_layout(SegPlan& plan, const cott_layout* l) {
 template <typename T>
 int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, void* out,
                 float* ws, int nseg, const cott_layout* layout, int B, int H, int N, int dtype, cudaStream_t stream,
-                void* saved = nullptr, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0}) {
+                void* saved = nullptr, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0}, float* decode_state = nullptr) {
   SegPlan plan = plan_segments(N, nseg);
   apply_layout(plan, layout);
   plan.rot = rot;
   const size_t A = seg_array_floats(B, H, plan.nseg);
-  if (keep) {  // running count of the kept positions, behind the five state arrays
-    int* count = reinterpret_cast<int*>(ws + 5 * A);
+  if (keep) {  // running count of the kept positions, behind the state arrays
+    int* count = reinterpret_cast<int*>(ws + 2 * A);
     keep_count_kernel<<<(unsigned)B, 256, 0, stream>>>(keep, count, N);
     COTT_CUDA_TRY(cudaGetLastError());
     plan.keep = keep;
     plan.count = count;
   }
-  if (plan.nseg == 1) return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, nullptr, plan, saved);
+  if (plan.nseg == 1) return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, nullptr, plan, saved, decode_state);
   int st = launch_seg_state<T, kSegFwdState>(k, v, in_strides(plan, H, N), in_strides(plan, H, N), nc, ws, B, H, N, dtype, plan, stream);
-  if (st) return st;
-  seg_scan_kernel<<<(unsigned)((long)B * H), 256, 0, stream>>>(ws, ws + A, ws + 2 * A, nullptr, plan.nseg);
-  COTT_CUDA_TRY(cudaGetLastError());
-  return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, ws + A, plan, saved);
+  if (st || (st = launch_seg_prefix(ws, (long)B * H, plan.nseg, kTcD * kTcD, false, stream))) return st;
+  return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, ws, plan, saved, decode_state);
 }
 
 template <typename T>
@@ -221,7 +242,7 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // the forward call left the running count in the workspace
     plan.keep = keep;
-    plan.count = reinterpret_cast<const int*>(ws + 5 * A);
+    plan.count = reinterpret_cast<const int*>(ws + 2 * A);
   }
   if (plan.nseg == 1) {
     COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
@@ -229,15 +250,15 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
     int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, nullptr, plan);
     return st ? st : launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   }
-  // dQ: the forward prefix states, transposed (written by the forward call into the same workspace)
-  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws + 2 * A, plan);
+  // dQ: the forward prefix states (left in the workspace by the forward call), read transposed
+  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws, plan);
   if (st) return st;
   // dK, dV: reverse states of the segments, their exclusive suffix
-  if ((st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + 3 * A, B, H, N, dtype, plan,
-                                              stream))) return st;
-  seg_scan_kernel<<<(unsigned)((long)B * H), 256, 0, stream>>>(ws + 3 * A, nullptr, nullptr, ws + 4 * A, plan.nseg);
-  COTT_CUDA_TRY(cudaGetLastError());
-  return launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, ws + 4 * A, plan);
+  if ((st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + A, B, H, N, dtype, plan,
+                                              stream)) ||
+      (st = launch_seg_prefix(ws + A, (long)B * H, plan.nseg, kTcD * kTcD, true, stream)))
+    return st;
+  return launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, ws + A, plan);
 }
 
 // The time-out path of the tensor-core kernels on its own: one CTA sets up what those kernels set up (an
@@ -338,13 +359,12 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
     const int W = wide_width(t.dz);
     WideArgs sa = a;
     sa.state_out = ws;
-    sa.rq_out = sa.rk_out = sa.w_out = nullptr;
+    sa.rq_out = sa.rk_out = sa.w_out = sa.decode_state = nullptr;
     WideTensors st = t;
     st.x = nullptr, st.c = nullptr, st.out = nullptr;
     int r = launch_wide_t<T, REV, NORMS, true>(st, sa, B, H, N, dtype, plan.nseg, stream);
     if (r) return r;
-    seg_prefix_kernel<<<dim3((unsigned)((long)B * H * (t.dz / W)), kTcChunk * W / 256), 256, 0, stream>>>(ws, plan.nseg, kTcChunk * W);
-    COTT_CUDA_TRY(cudaGetLastError());
+    if ((r = launch_seg_prefix(ws, (long)B * H * (t.dz / W), plan.nseg, kTcChunk * W, false, stream))) return r;
     a.init_state = ws;
   }
   return launch_wide_t<T, REV, NORMS, false>(t, a, B, H, N, dtype, plan.nseg, stream);
@@ -352,16 +372,7 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
 
 size_t wide_ws_floats(int B, int H, int N, int dz, int nseg) { return (size_t)B * H * plan_segments(N, nseg).nseg * (size_t)(kTcChunk * dz); }
 
-int wide_seg_count(int B, int H, int N, int dz) {
-  const long units = (long)B * H * (dz / wide_width(dz));
-  const int total = (N + kTcChunk - 1) / kTcChunk;
-  if (units <= 0 || total < 4) return 1;
-  int sm = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-  long nseg = sm / units;
-  if (nseg > total / 2) nseg = total / 2;
-  return nseg < 2 ? 1 : (int)nseg;
-}
+int wide_seg_count(int B, int H, int N, int dz) { return seg_count((long)B * H * (dz / wide_width(dz)), N, 3); }
 
 // workspace of the fused head-dim-128 pair: the prefix states of the forward-direction passes and those of the reversed
 // ones (first: they are read as 16-byte words), then four fp32 vectors [B*H*N] (1/|q|, 1/|k|, keep a/|k|, -eps/|k|^2) and
@@ -380,11 +391,12 @@ WideWs wide_ws(void* workspace, int B, int H, int N) {
 
 template <typename T>
 int run_wide_fwd(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, void* out, void* workspace,
-                 int B, int H, int N, int dtype, cudaStream_t stream) {
+                 int B, int H, int N, int dtype, cudaStream_t stream, float* decode_state = nullptr) {
   WideWs ws = wide_ws(workspace, B, H, N);
   WideArgs a = {};
   a.norm_const = nc;
-  a.rq_out = ws.rq, a.rk_out = ws.rk, a.w_out = ws.w;
+  if (!decode_state) a.rq_out = ws.rq, a.rk_out = ws.rk, a.w_out = ws.w;  // (a prompt has no backward)
+  a.decode_state = decode_state;
   if (keep) {
     keep_count_kernel<<<(unsigned)B, 256, 0, stream>>>(keep, ws.count, N);
     COTT_CUDA_TRY(cudaGetLastError());
@@ -432,16 +444,14 @@ int run_bwd_train(const void* q, const void* k, const void* v, const unsigned ch
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // the forward call left the running count in the workspace
     plan.keep = keep;
-    plan.count = reinterpret_cast<const int*>(ws + 5 * A);
+    plan.count = reinterpret_cast<const int*>(ws + 2 * A);
   }
   if (plan.nseg == 1) return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   // reverse states of the segments and their exclusive suffix; the prefix states come from `saved`
-  int st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + 3 * A, B, H, N, dtype, plan,
+  int st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + A, B, H, N, dtype, plan,
                                              stream);
-  if (st) return st;
-  seg_scan_kernel<<<(unsigned)((long)B * H), 256, 0, stream>>>(ws + 3 * A, nullptr, nullptr, ws + 4 * A, plan.nseg);
-  COTT_CUDA_TRY(cudaGetLastError());
-  return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 4 * A, plan);
+  if (st || (st = launch_seg_prefix(ws + A, (long)B * H, plan.nseg, kTcD * kTcD, true, stream))) return st;
+  return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + A, plan);
 }
 
 int check_ptrs16(std::initializer_list<std::pair<const void*, const char*>> ps) {
@@ -511,7 +521,7 @@ int launch_bidir_bwd_tc(const void* q, const void* k, const void* v, const unsig
 // The bare scan of cott_scan on the tensor cores (head dim 64, 16-bit dtypes): the forward kernel without its row
 // scalings, walking the sequence backwards when `reversed`.  `out` may be one of the inputs: a chunk's rows are
 // stored after every load of that chunk has completed, and no other chunk reads them.
-// `ws` (2 x B*H*nseg fp32 [64 x 64] matrices) is only used when plan.nseg > 1: the segments' own states and their
+// `ws` (B*H*nseg fp32 [64 x 64] matrices) is only used when plan.nseg > 1: the segments' own states, then their
 // exclusive prefix in scan order.
 template <typename T>
 int launch_scan_tc_t(const void* q, const void* k, const void* v, void* out, int B, int H, int N, int dtype, int reversed,
@@ -523,13 +533,11 @@ int launch_scan_tc_t(const void* q, const void* k, const void* v, void* out, int
     return st;
   const float* init = nullptr;
   if (plan.nseg > 1) {
-    const size_t A = seg_array_floats(B, H, plan.nseg);
     st = reversed ? launch_seg_state<T, kSegRawStateRev>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, stream)
                   : launch_seg_state<T, kSegRawState>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, stream);
     if (st) return st;
-    seg_scan_kernel<<<(unsigned)((long)B * H), 256, 0, stream>>>(ws, ws + A, nullptr, nullptr, plan.nseg);
-    COTT_CUDA_TRY(cudaGetLastError());
-    init = ws + A;
+    if ((st = launch_seg_prefix(ws, (long)B * H, plan.nseg, kTcD * kTcD, false, stream))) return st;
+    init = ws;
   }
   auto kern = plan.nseg > 1 ? (reversed ? causal_tc_kernel<T, kModeScanRev, true> : causal_tc_kernel<T, kModeScan, true>)
                             : (reversed ? causal_tc_kernel<T, kModeScanRev, false> : causal_tc_kernel<T, kModeScan, false>);
@@ -537,7 +545,8 @@ int launch_scan_tc_t(const void* q, const void* k, const void* v, void* out, int
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)((long)B * H), plan.nseg), kTcThreads, smem, stream, mq, mk, mv, mq, mo,
                            static_cast<const float*>(nullptr), H, N, init, plan.cps, static_cast<const unsigned char*>(nullptr),
-                           static_cast<const int*>(nullptr), static_cast<uint4*>(nullptr), RotArgs{nullptr, nullptr, 0, 0}));
+                           static_cast<const int*>(nullptr), static_cast<uint4*>(nullptr), RotArgs{nullptr, nullptr, 0, 0},
+                           static_cast<float*>(nullptr)));
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
@@ -621,7 +630,7 @@ int launch_scan_tc_wide(const void* q, const void* k, const void* v, void* out, 
   T* oo = static_cast<T*>(out);
   // few (batch, head) pairs and a long sequence: several CTAs per sequence, as in the fused path
   const SegPlan plan = plan_segments(N, cott_cos_attn_seg_count(B, H, N));
-  const size_t ws_bytes = plan.nseg > 1 ? 2 * seg_array_floats(B, H, plan.nseg) * sizeof(float) : 0;
+  const size_t ws_bytes = plan.nseg > 1 ? seg_array_floats(B, H, plan.nseg) * sizeof(float) : 0;
   const size_t tmp_bytes = Dk > kTcD ? sizeof(T) * rows * kTcD : 0;
   char* scratch = nullptr;  // stream-ordered: segment states, then the partial result of the slices I > 0
   if (ws_bytes + tmp_bytes) {
@@ -756,21 +765,11 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
   return st ? st : launch_bwd_dkdv<__half>(q, k, v, norm_const, dout, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, plan);
 }
 
-int cott_cos_attn_seg_count(int B, int H, int N) {
-  const long BH = (long)B * H;
-  const int total = (N + kTcChunk - 1) / kTcChunk;
-  if (BH <= 0 || total < 4) return 1;
-  int sm = 148;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-  long nseg = sm / BH;              // one CTA per SM; more sequences than half the SMs: no gain
-  if (nseg > total / 2) nseg = total / 2;  // at least two chunks per segment
-  return nseg < 2 ? 1 : (int)nseg;
-}
+int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N, 6); }
 
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
-  return 5 * seg_array_floats(B, H, plan_segments(N, nseg).nseg) * sizeof(float) + (size_t)B * N * sizeof(int);
+  return 2 * seg_array_floats(B, H, plan_segments(N, nseg).nseg) * sizeof(float) + (size_t)B * N * sizeof(int);
 }
 
 int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
@@ -993,6 +992,32 @@ int run_wide_prefill_state(const void* k, const void* v, const float* nc, float*
 }  // namespace
 
 extern "C" {
+
+int cott_cos_attn_prefill(const void* q, const void* k, const void* v, const float* norm_const, void* out, float* state, void* workspace,
+                          int nseg, int B, int H, int N, int Dk, int Dv, int dtype, void* stream) {
+  const bool wide = Dk == 128 && Dv == 128;
+  int st = wide ? check_wide_args(B, H, N, Dk, Dv, dtype) : check_fused_args(B, H, N, Dk, Dv, dtype);
+  if (st) return st;
+  if ((long)B * H == 0) return COTT_OK;
+  if ((st = check_ptrs16({{state, "state"}}))) return st;
+  DeviceScope scope(state);
+  COTT_CUDA_TRY(scope.status());
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (N == 0) {  // an empty prompt leaves an empty state
+    COTT_CUDA_TRY(cudaMemsetAsync(state, 0, sizeof(float) * (size_t)B * H * Dk * Dv, s));
+    return COTT_OK;
+  }
+  if ((st = check_ptrs16({{q, "q"}, {k, "k"}, {v, "v"}, {out, "out"}, {workspace, "workspace"}}))) return st;
+  if (!norm_const) return fail(COTT_ERR_NULL, "null pointer: norm_const");
+  if (wide)
+    return dtype == COTT_BF16 ? run_wide_fwd<__nv_bfloat16>(q, k, v, nullptr, norm_const, out, workspace, B, H, N, dtype, s, state)
+                              : run_wide_fwd<__half>(q, k, v, nullptr, norm_const, out, workspace, B, H, N, dtype, s, state);
+  float* ws = static_cast<float*>(workspace);
+  const RotArgs none{nullptr, nullptr, 0, 0};
+  return dtype == COTT_BF16
+             ? run_fwd_seg<__nv_bfloat16>(q, k, v, nullptr, norm_const, out, ws, nseg, nullptr, B, H, N, dtype, s, nullptr, none, state)
+             : run_fwd_seg<__half>(q, k, v, nullptr, norm_const, out, ws, nseg, nullptr, B, H, N, dtype, s, nullptr, none, state);
+}
 
 int cott_cos_attn_prefill_state(const void* k, const void* v, const float* norm_const, float* state, void* workspace,
                                 int nseg, int accumulate, int B, int H, int N, int Dk, int Dv, int dtype, void* stream) {

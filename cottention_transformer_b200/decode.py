@@ -24,26 +24,27 @@ class CosAttnDecodeState:
         self.cur_s = 1
 
     def prefill(self, q, k, v, norm_const):
-        """Absorb a whole prompt at once (fresh state only): the outputs come from the fused causal kernels and the
-        state from the segment-state kernels, instead of T recurrent steps.  bf16 / fp16, head dim 64 or 128; anything
+        """Absorb a whole prompt at once (fresh state only): outputs and state come from the fused causal kernels in one
+        call (``cott_cos_attn_prefill``) instead of T recurrent steps.  bf16 / fp16, head dim 64 or 128; anything
         else falls back to ``step``.  Returns ``[B, H, T, d_v]``."""
         from .cos_attention import cos_attn_causal, fused_supported, wide_supported
         wide = wide_supported(q, k, v) and q.shape[-1] == 128
         if self.cur_s != 1 or not (wide or fused_supported(q, k, v)):
             return self.step(q, k, v, norm_const)
         B, H, T, D = q.shape
-        k, v = k.contiguous(), v.contiguous()
-        with torch.no_grad():
-            out = cos_attn_causal(q, k, v, norm_const)
+        q, k, v = q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous()
         L = _lib.lib()
         nc = norm_const.detach().reshape(-1).to(device=q.device, dtype=torch.float32).contiguous()
+        if nc.numel() != H:
+            raise RuntimeError(f"norm_const must have one entry per head ({H}), got {nc.numel()}")
+        out = torch.empty_like(v)
         with torch.cuda.device(q.device):
             nseg = 1 if wide else L.cott_cos_attn_seg_count(B, H, T)
             nbytes = L.cott_cos_attn_wide_workspace_bytes(B, H, T) if wide else L.cott_cos_attn_seg_workspace_bytes(B, H, T, nseg)
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-            st = L.cott_cos_attn_prefill_state(_lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(self.state), _lib.ptr(ws), nseg,
-                                               0, B, H, T, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
-        _lib.check(st, "cott_cos_attn_prefill_state")
+            st = L.cott_cos_attn_prefill(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(self.state),
+                                         _lib.ptr(ws), nseg, B, H, T, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
+        _lib.check(st, "cott_cos_attn_prefill")
         self.cur_s += T
         return out
 
