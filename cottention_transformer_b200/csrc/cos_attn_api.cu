@@ -765,11 +765,12 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
   return st ? st : launch_bwd_dkdv<__half>(q, k, v, norm_const, dout, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, plan);
 }
 
-int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N, 6); }
+int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N, 4); }
 
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
-  return 2 * seg_array_floats(B, H, plan_segments(N, nseg).nseg) * sizeof(float) + (size_t)B * N * sizeof(int);
+  // (five arrays is what callers have always been asked for; two of them are used)
+  return 5 * seg_array_floats(B, H, plan_segments(N, nseg).nseg) * sizeof(float) + (size_t)B * N * sizeof(int);
 }
 
 int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
