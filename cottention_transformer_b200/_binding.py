@@ -30,6 +30,16 @@ def module():
     return _mod
 
 
+def autograd():
+    """The module whose functions carry their own autograd nodes, or None where the Python autograd functions are needed:
+    without the binding, and under tracing, compilation and functorch transforms, which look at a Python function and its
+    operators (or refuse them by name) and would not see these."""
+    import torch
+    if torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None or torch._C._functorch.peek_interpreter_stack() is not None:
+        return None
+    return module()
+
+
 def ops():
     """``torch.ops.cottention_b200`` when the binding is loaded, else None."""
     if module() is None:

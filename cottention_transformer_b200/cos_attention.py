@@ -190,18 +190,25 @@ def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None):
         raise RuntimeError("cos_attn_causal_packed needs a CUDA tensor (there is no CPU path)")
     if qkv.dim() != 5 or qkv.shape[2] != 3 or qkv.shape[-1] != 64 or qkv.dtype not in FUSED_DTYPES:
         raise RuntimeError("cos_attn_causal_packed takes a [B, N, 3, H, 64] bfloat16 / float16 tensor")
+    m = _binding.autograd()
     if rotary is None:
-        return _FusedCausalPacked.apply(qkv, norm_const, keep)
+        return m.causal_packed(qkv, norm_const, keep, None, None) if m is not None else _FusedCausalPacked.apply(qkv, norm_const, keep)
     sin, cos = rotary
     sin = sin.to(device=qkv.device, dtype=torch.float32).contiguous()
     cos = cos.to(device=qkv.device, dtype=torch.float32).contiguous()
     B, N, _, H, _ = qkv.shape
     if sin.shape != cos.shape or sin.shape[-2] != N or (sin.dim() == 3 and sin.shape[0] not in (1, B)):
         raise RuntimeError("sin / cos must be [N, rot/2] or [B, N, rot/2]")
-    with torch.cuda.device(qkv.device):
-        one_segment = _lib.lib().cott_cos_attn_seg_count(B, H, N) == 1
+    if m is not None:
+        one_segment = m.seg_count(qkv, B, H, N) == 1
+    else:
+        with torch.cuda.device(qkv.device):
+            one_segment = _lib.lib().cott_cos_attn_seg_count(B, H, N) == 1
     if (2 * sin.shape[-1]) % 16 or not one_segment:
-        return _FusedCausalPacked.apply(rotary_packed_(qkv.contiguous(), sin, cos), norm_const, keep)
+        qkv = rotary_packed_(qkv.contiguous(), sin, cos)
+        return m.causal_packed(qkv, norm_const, keep, None, None) if m is not None else _FusedCausalPacked.apply(qkv, norm_const, keep)
+    if m is not None:
+        return m.causal_packed(qkv, norm_const, keep, sin, cos)
     return _FusedCausalPacked.apply(qkv, norm_const, keep, sin, cos)
 
 
@@ -458,14 +465,23 @@ def cos_attn_causal(q, k, v, norm_const, keep=None, segments=None, one_pass_back
     """
     if not (q.is_cuda and k.is_cuda and v.is_cuda):
         raise RuntimeError("cos_attn_causal needs CUDA tensors (there is no CPU path)")
+    m = _binding.autograd()
     if fused_supported(q, k, v, keep):
+        if m is not None:
+            return m.cos_attn_causal(q, k, v, norm_const, keep, 0 if segments is None else int(segments), bool(one_pass_backward))
         return _FusedCausal.apply(q, k, v, norm_const, segments, keep, bool(one_pass_backward))
     if wide_supported(q, k, v, keep):
         if q.shape[-1] == 128:
+            if m is not None:
+                return m.cos_attn_wide(q, k, v, norm_const, keep)
             return _FusedWide128.apply(q, k, v, norm_const, keep)
         return _WideCausal.apply(q, k, v, norm_const, keep)
     if f32_supported(q, k, v, norm_const, keep):
-        return _FusedF32.apply(q, k, v, norm_const, keep)
+        # (private copies of the parameter and the mask, as the module math takes them: an update of either between the
+        # forward and the backward does not reach the backward)
+        if m is not None:
+            return m.cos_attn_f32(q, k, v, norm_const, keep)
+        return _FusedF32.apply(q, k, v, norm_const.clone(), None if keep is None else keep.clone())
     return _exact_causal(q, k, v, norm_const, keep)
 
 
@@ -566,7 +582,8 @@ def cos_attn_bidirectional_packed(qkv, norm_const, keep=None):
         raise RuntimeError("cos_attn_bidirectional_packed needs a CUDA tensor (there is no CPU path)")
     if qkv.dim() != 5 or qkv.shape[2] != 3 or qkv.shape[-1] != 64 or qkv.dtype not in FUSED_DTYPES:
         raise RuntimeError("cos_attn_bidirectional_packed takes a [B, N, 3, H, 64] bfloat16 / float16 tensor")
-    return _BidirectionalPacked.apply(qkv, norm_const, keep)
+    m = _binding.autograd()
+    return m.bidir_packed(qkv, norm_const, keep) if m is not None else _BidirectionalPacked.apply(qkv, norm_const, keep)
 
 
 def cos_attn_bidirectional(q, k, v, norm_const, keep=None):

@@ -9,6 +9,8 @@
 //    package make one dispatcher call per direction instead of a dozen Python-level tensor calls -- at BERT shapes
 //    the step is otherwise bound by the host, not by its kernels.
 //
+// 3. The autograd functions around them, and the decode and prefill calls.
+//
 // Nothing here computes: every function validates, allocates its outputs and calls one extern "C" entry point on
 // torch's current stream.  The ctypes route (cottention_transformer_b200/_lib.py) stays for non-torch hosts.
 #include <ATen/autocast_mode.h>
@@ -69,10 +71,20 @@ at::Tensor forward_(at::Tensor& Q, at::Tensor& K, at::Tensor& V, const int8_t bl
 }
 
 // ---- 2. fused operators ---------------------------------------------------------------------------------------
+// norm_const as the floats the C side reads: no copy when it already is a dense fp32 tensor on this device
+at::Tensor nc_floats(const at::Tensor& norm_const, const at::Tensor& like) {
+  at::Tensor nc = norm_const.detach();
+  if (nc.scalar_type() != at::kFloat || nc.device() != like.device()) nc = nc.to(like.device(), at::kFloat);
+  return nc.contiguous();
+}
 at::Tensor nc_f32(const at::Tensor& norm_const, const at::Tensor& like, int64_t H) {
-  at::Tensor nc = norm_const.detach().reshape({-1}).to(like.device(), at::kFloat).contiguous();
-  TORCH_CHECK(nc.numel() == H, "norm_const must have one entry per head (", H, "), got ", nc.numel());
-  return nc;
+  TORCH_CHECK(norm_const.numel() == H, "norm_const must have one entry per head (", H, "), got ", norm_const.numel());
+  return nc_floats(norm_const, like);
+}
+// (the packed and decode entry points take a longer parameter, as they always have; a shorter one would be read past its end)
+at::Tensor nc_at_least(const at::Tensor& norm_const, const at::Tensor& like, int64_t H) {
+  TORCH_CHECK(norm_const.numel() >= H, "norm_const must have one entry per head (", H, "), got ", norm_const.numel());
+  return nc_floats(norm_const, like);
 }
 
 // causal forward: returns (out, workspace, saved); workspace / saved are empty tensors when not needed
@@ -170,6 +182,335 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> bidir_bwd(const at::T
   return {dq, dk, dv, dnc};
 }
 
+// ---- 3. autograd functions --------------------------------------------------------------------------------------
+// One call from Python per direction: validation, allocation, launches and the autograd node in C++.  (A step of a small
+// model is bound by the host: two Python-level autograd functions, ctypes conversions and dispatcher calls cost more
+// than the kernels of a 200-token sequence.)  The Python autograd functions of cos_attention.py stay for hosts without
+// this module and for the cases that need them (tracing, functorch transforms); both end in the same C calls.
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<at::Tensor>;
+
+bool has(const OptTensor& t) { return t.has_value() && t->defined(); }
+OptTensor keep_u8(const OptTensor& keep, const at::Tensor& like) {
+  if (!has(keep)) return c10::nullopt;
+  // always a tensor of our own: the backward reads it again, whatever the caller has done to the mask by then.  (A bool
+  // mask is read as the bytes it is, which a plain copy gives.)
+  if (keep->scalar_type() == at::kBool && keep->device() == like.device()) return keep->clone(at::MemoryFormat::Contiguous);
+  at::Tensor k = keep->to(like.device(), at::kByte).contiguous();
+  return k.is_alias_of(*keep) ? k.clone() : k;
+}
+// the gradient of norm_const in the shape and dtype of the parameter
+at::Tensor nc_grad(const at::Tensor& dnc, at::IntArrayRef shape, at::ScalarType dtype) {
+  at::Tensor g = dnc.reshape(shape);
+  return g.scalar_type() == dtype ? g : g.to(dtype);
+}
+at::Tensor bytes_like(const at::Tensor& t, size_t n) { return at::empty({(int64_t)std::max<size_t>(n, 16)}, t.options().dtype(at::kByte)); }
+const unsigned char* u8(const OptTensor& t) { return static_cast<const unsigned char*>(ptr_or_null(t)); }
+at::Tensor dense_as(const at::Tensor& t, at::ScalarType dtype) {
+  at::Tensor c = t.contiguous();
+  return c.scalar_type() == dtype ? c : c.to(dtype);
+}
+void save_nc(AutogradContext* ctx, const at::Tensor& norm_const) {
+  ctx->saved_data["nc_shape"] = norm_const.sizes().vec();
+  ctx->saved_data["nc_dtype"] = (int64_t)norm_const.scalar_type();
+}
+at::Tensor nc_grad(AutogradContext* ctx, const at::Tensor& dnc) {
+  return nc_grad(dnc, ctx->saved_data["nc_shape"].toIntVector(), (at::ScalarType)ctx->saved_data["nc_dtype"].toInt());
+}
+void save_opt(AutogradContext* ctx, const char* key, const OptTensor& t) {
+  if (has(t)) ctx->saved_data[key] = *t;
+}
+OptTensor load_opt(AutogradContext* ctx, const char* key) {
+  const auto it = ctx->saved_data.find(key);
+  return it == ctx->saved_data.end() ? OptTensor() : OptTensor(it->second.toTensor());
+}
+
+// 16-bit, head dim 64
+struct CausalFn : torch::autograd::Function<CausalFn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
+                          const OptTensor& keep, int64_t nseg, bool one_pass) {
+    const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+    const OptTensor kp = keep_u8(keep, q);
+    auto [out, ws, saved] = causal_fwd(q, k, v, norm_const, kp, nseg, one_pass);
+    ctx->save_for_backward({q, k, v, norm_const.detach()});
+    ctx->saved_data["ws"] = ws;
+    ctx->saved_data["saved"] = saved;
+    ctx->saved_data["nseg"] = nseg;
+    save_opt(ctx, "keep", kp);
+    save_nc(ctx, norm_const);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const at::Tensor ws = ctx->saved_data["ws"].toTensor(), saved = ctx->saved_data["saved"].toTensor();
+    const int64_t nseg = ctx->saved_data["nseg"].toInt();
+    at::Tensor dq, dk, dv, dnc;
+    if (at::GradMode::is_enabled()) {  // create_graph: through the dispatcher, which says that there is no second derivative
+      static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("cottention_b200::causal_bwd", "").typed<decltype(causal_bwd)>();
+      std::tie(dq, dk, dv, dnc) = op.call(s[0], s[1], s[2], s[3], load_opt(ctx, "keep"), grads[0], ws, saved, nseg);
+    } else {
+      std::tie(dq, dk, dv, dnc) = causal_bwd(s[0], s[1], s[2], s[3], load_opt(ctx, "keep"), grads[0], ws, saved, nseg);
+    }
+    return {dq, dk, dv, nc_grad(ctx, dnc), Variable(), Variable(), Variable()};
+  }
+};
+
+// the packed [B, N, 3, H, 64] forms
+struct Packed {
+  at::Tensor qkv;
+  int64_t B, N, H, D, e;
+  cott_layout lay;
+  explicit Packed(const at::Tensor& t)
+      : qkv(t), B(t.size(0)), N(t.size(1)), H(t.size(3)), D(t.size(4)), e(t.element_size()),
+        lay{N * 3 * H * D, D, 3 * H * D, N * H * D, D, H * D} {}
+  char* part(int i) const { return static_cast<char*>(qkv.data_ptr()) + i * H * D * e; }  // q, k, v of the first token
+};
+struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& qkv_, const at::Tensor& norm_const, const OptTensor& keep,
+                          const OptTensor& sin, const OptTensor& cos) {
+    const Packed p(qkv_.contiguous());
+    const c10::cuda::CUDAGuard guard(p.qkv.device());
+    const at::Tensor nc = nc_at_least(norm_const, p.qkv, p.H);
+    const OptTensor kp = keep_u8(keep, p.qkv);
+    at::Tensor out = at::empty({p.B, p.N, p.H, p.D}, p.qkv.options());
+    const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
+    const bool rot = has(sin);
+    const int nseg = rot ? 1 : cott_cos_attn_seg_count(B, H, N);
+    at::Tensor ws = bytes_like(p.qkv, cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
+    if (rot) {
+      const cott_rotary_tables r = tables(*sin, *cos, N);
+      check(cott_cos_attn_fwd_rotary(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), out.data_ptr(), ws.data_ptr(), &p.lay, &r, B,
+                                     H, N, D, D, code, stream_of(p.qkv)),
+            "cott_cos_attn_fwd_rotary");
+    } else {
+      check(cott_cos_attn_fwd_seg(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), out.data_ptr(), ws.data_ptr(), nseg, &p.lay, B, H,
+                                  N, D, D, code, stream_of(p.qkv)),
+            "cott_cos_attn_fwd_seg");
+    }
+    ctx->save_for_backward({p.qkv, nc, rot ? *sin : at::Tensor(), rot ? *cos : at::Tensor()});
+    ctx->saved_data["ws"] = ws;
+    ctx->saved_data["nseg"] = (int64_t)nseg;
+    save_opt(ctx, "keep", kp);
+    save_nc(ctx, norm_const);
+    return out;
+  }
+  static cott_rotary_tables tables(const at::Tensor& sin, const at::Tensor& cos, int N) {
+    const int64_t half = sin.size(-1);
+    const bool per_batch = sin.dim() == 3 && sin.size(0) > 1;
+    return cott_rotary_tables{sin.data_ptr<float>(), cos.data_ptr<float>(), (int)(2 * half), per_batch ? (long long)(N * half) : 0};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Packed p(s[0]), d(at::empty_like(s[0]));
+    const c10::cuda::CUDAGuard guard(p.qkv.device());
+    const at::Tensor &nc = s[1], dout = dense_as(grads[0], p.qkv.scalar_type()), ws = ctx->saved_data["ws"].toTensor();
+    const OptTensor kp = load_opt(ctx, "keep");
+    at::Tensor dnc = at::empty({p.H}, p.qkv.options().dtype(at::kFloat));
+    const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
+    if (s[2].defined()) {
+      const cott_rotary_tables r = tables(s[2], s[3], N);
+      check(cott_cos_attn_bwd_rotary(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), dout.data_ptr(), ws.data_ptr(), &p.lay, &r,
+                                     d.part(0), d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D, D, code, stream_of(p.qkv)),
+            "cott_cos_attn_bwd_rotary");
+    } else {
+      check(cott_cos_attn_bwd_seg(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), dout.data_ptr(), ws.data_ptr(),
+                                  (int)ctx->saved_data["nseg"].toInt(), &p.lay, d.part(0), d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D,
+                                  D, code, stream_of(p.qkv)),
+            "cott_cos_attn_bwd_seg");
+    }
+    return {d.qkv, nc_grad(ctx, dnc), Variable(), Variable(), Variable()};
+  }
+};
+struct BidirPackedFn : torch::autograd::Function<BidirPackedFn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& qkv_, const at::Tensor& norm_const, const OptTensor& keep) {
+    const Packed p(qkv_.contiguous());
+    const c10::cuda::CUDAGuard guard(p.qkv.device());
+    const at::Tensor nc = nc_at_least(norm_const, p.qkv, p.H);
+    const OptTensor kp = keep_u8(keep, p.qkv);
+    at::Tensor out = at::empty({p.B, p.N, p.H, p.D}, p.qkv.options());
+    check(cott_bidir_fwd_strided(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), out.data_ptr(), &p.lay, (int)p.B, (int)p.H,
+                                 (int)p.N, (int)p.D, (int)p.D, dtype_code(p.qkv.scalar_type()), stream_of(p.qkv)),
+          "cott_bidir_fwd_strided");
+    ctx->save_for_backward({p.qkv, nc});
+    save_opt(ctx, "keep", kp);
+    save_nc(ctx, norm_const);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Packed p(s[0]), d(at::empty_like(s[0]));
+    const c10::cuda::CUDAGuard guard(p.qkv.device());
+    const at::Tensor dout = dense_as(grads[0], p.qkv.scalar_type());
+    at::Tensor dnc = at::empty({p.H}, p.qkv.options().dtype(at::kFloat));
+    check(cott_bidir_bwd_strided(p.part(0), p.part(1), p.part(2), u8(load_opt(ctx, "keep")), s[1].data_ptr<float>(), dout.data_ptr(), &p.lay,
+                                 d.part(0), d.part(1), d.part(2), dnc.data_ptr<float>(), (int)p.B, (int)p.H, (int)p.N, (int)p.D, (int)p.D,
+                                 dtype_code(p.qkv.scalar_type()), stream_of(p.qkv)),
+          "cott_bidir_bwd_strided");
+    return {d.qkv, nc_grad(ctx, dnc), Variable()};
+  }
+};
+
+// 16-bit, head dim 128
+struct WideFn : torch::autograd::Function<WideFn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
+                          const OptTensor& keep) {
+    const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+    const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+    const c10::cuda::CUDAGuard guard(q.device());
+    const at::Tensor nc = nc_f32(norm_const, q, H);
+    const OptTensor kp = keep_u8(keep, q);
+    at::Tensor out = at::empty_like(v), ws = bytes_like(q, cott_cos_attn_wide_workspace_bytes(B, H, N));
+    check(cott_cos_attn_wide_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), u8(kp), nc.data_ptr<float>(), out.data_ptr(), ws.data_ptr(), B, H, N, D,
+                                 D, dtype_code(q.scalar_type()), stream_of(q)),
+          "cott_cos_attn_wide_fwd");
+    ctx->save_for_backward({q, k, v, nc, ws});
+    save_opt(ctx, "keep", kp);
+    save_nc(ctx, norm_const);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const at::Tensor &q = s[0], dout = dense_as(grads[0], q.scalar_type());
+    const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+    const c10::cuda::CUDAGuard guard(q.device());
+    at::Tensor dq = at::empty_like(q), dk = at::empty_like(s[1]), dv = at::empty_like(s[2]), dnc = at::empty({H}, q.options().dtype(at::kFloat));
+    check(cott_cos_attn_wide_bwd(q.data_ptr(), s[1].data_ptr(), s[2].data_ptr(), u8(load_opt(ctx, "keep")), s[3].data_ptr<float>(), nullptr,
+                                 dout.data_ptr(), s[4].data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dnc.data_ptr<float>(), B, H, N, D,
+                                 D, dtype_code(q.scalar_type()), stream_of(q)),
+          "cott_cos_attn_wide_bwd");
+    return {dq, dk, dv, nc_grad(ctx, dnc), Variable()};
+  }
+};
+
+// Custom_Kernel.py's CustomAttention: forward and the three permuted scans through the entry point of Q's dtype
+at::Tensor scan_by_dtype(at::ScalarType t, at::Tensor Q, at::Tensor K, at::Tensor V, bool reversed) {
+  return t == at::kHalf ? forward_<at::kHalf>(Q, K, V, 1, false, reversed) : forward_<at::kBFloat16>(Q, K, V, 1, false, reversed);
+}
+struct CustomAttentionFn : torch::autograd::Function<CustomAttentionFn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& Q_, const at::Tensor& K_, const at::Tensor& V_) {
+    const at::Tensor Q = Q_.contiguous(), K = K_.contiguous(), V = V_.contiguous();
+    ctx->save_for_backward({Q, K, V});
+    return scan_by_dtype(Q.scalar_type(), Q, K, V, false);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const at::Tensor Q = s[0].contiguous(), K = s[1].contiguous(), V = s[2].contiguous(), g = grads[0].contiguous();
+    const at::ScalarType t = Q.scalar_type();
+    return {scan_by_dtype(t, g, V, K, false), scan_by_dtype(t, V, g, Q, true), scan_by_dtype(t, K, Q, g, true)};
+  }
+};
+
+// one decode call on a [B, H, Dv, Dk] state
+at::Tensor decode_steps(const at::Tensor& state, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
+                        int64_t pos) {
+  const at::Tensor q = q_.contiguous(), k = dense_as(k_.scalar_type() == q.scalar_type() ? k_ : k_.to(q.scalar_type()), q.scalar_type()),
+                   v = dense_as(v_.scalar_type() == q.scalar_type() ? v_ : v_.to(q.scalar_type()), q.scalar_type());
+  const c10::cuda::CUDAGuard guard(q.device());
+  const at::Tensor nc = nc_at_least(norm_const, q, q.size(1));
+  at::Tensor out = at::empty({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
+  check(cott_decode_steps(state.data_ptr<float>(), q.data_ptr(), k.data_ptr(), v.data_ptr(), nc.data_ptr<float>(), out.data_ptr(), (int)q.size(0),
+                          (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)v.size(3), dtype_code(q.scalar_type()), pos, nullptr, stream_of(q)),
+        "cott_decode_steps");
+  return out;
+}
+
+// a whole prompt: outputs and the decode state it leaves (head dim 64 or 128)
+at::Tensor prefill(const at::Tensor& state, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const) {
+  const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+  const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+  const c10::cuda::CUDAGuard guard(q.device());
+  const at::Tensor nc = nc_f32(norm_const, q, H);
+  const int nseg = D == 128 ? 1 : cott_cos_attn_seg_count(B, H, N);
+  at::Tensor out = at::empty_like(v);
+  const at::Tensor ws = bytes_like(q, D == 128 ? cott_cos_attn_wide_workspace_bytes(B, H, N) : cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
+  check(cott_cos_attn_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), nc.data_ptr<float>(), out.data_ptr(), state.data_ptr<float>(),
+                              ws.data_ptr(), nseg, B, H, N, D, D, dtype_code(q.scalar_type()), stream_of(q)),
+        "cott_cos_attn_prefill");
+  return out;
+}
+
+// fp32, head dims 32 and 64
+at::Tensor dense16(const at::Tensor& t) {
+  at::Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+// the module math in differentiable torch operators around the scan, for gradients that are differentiated again
+at::Tensor exact_causal(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& norm_const, const OptTensor& keep) {
+  const int64_t B = q.size(0), H = q.size(1), N = q.size(2);
+  at::Tensor qh = q / q.norm(2, -1, true).clamp_min(1e-12), kh = k / k.norm(2, -1, true).clamp_min(1e-12);
+  const at::Tensor n = has(keep) ? keep->to(at::kLong).cumsum(-1).to(q.scalar_type()).view({B, 1, N, 1})
+                                 : at::arange(1, N + 1, q.options()).view({1, 1, N, 1});
+  at::Tensor vp = v / n.pow(norm_const.sigmoid().reshape({1, H, 1, 1})).clamp_min(1);
+  if (has(keep)) {
+    const at::Tensor m = keep->view({B, 1, N, 1}).to(q.scalar_type());
+    qh = qh * m, kh = kh * m, vp = vp * m;
+  }
+  return CustomAttentionFn::apply(qh, kh, vp);
+}
+struct F32Fn : torch::autograd::Function<F32Fn> {
+  static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
+                          const OptTensor& keep) {
+    const at::Tensor q = dense16(q_), k = dense16(k_), v = dense16(v_), nc = norm_const.contiguous();
+    const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+    const c10::cuda::CUDAGuard guard(q.device());
+    at::Tensor out = at::empty(q.sizes(), q.options()), ws = bytes_like(q, cott_cos_attn_f32_workspace_bytes(B, H, N, D));
+    check(cott_cos_attn_f32_fwd(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), u8(keep), nc.data_ptr<float>(), out.data_ptr<float>(),
+                                ws.data_ptr(), B, H, N, D, stream_of(q)),
+          "cott_cos_attn_f32_fwd");
+    ctx->save_for_backward({q_, k_, v_, norm_const});
+    ctx->saved_data["ws"] = ws;
+    save_opt(ctx, "keep", keep);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const OptTensor keep = load_opt(ctx, "keep");
+    if (at::GradMode::is_enabled()) {  // create_graph
+      variable_list x, wanted;
+      for (const at::Tensor& t : s) x.push_back(t.view_as(t));  // (one name per argument: the same tensor may be several of them)
+      for (const at::Tensor& t : x)
+        if (t.requires_grad()) wanted.push_back(t);
+      variable_list g = torch::autograd::grad({exact_causal(x[0], x[1], x[2], x[3], keep)}, wanted, {grads[0]}, true, true, true);
+      variable_list r(5);
+      for (size_t i = 0, j = 0; i < 4; ++i)
+        if (x[i].requires_grad()) r[i] = g[j++];
+      return r;
+    }
+    const at::Tensor q = dense16(s[0]), k = dense16(s[1]), v = dense16(s[2]), nc = s[3].contiguous(), dout = dense16(grads[0]);
+    const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+    const c10::cuda::CUDAGuard guard(q.device());
+    at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dnc = at::empty_like(nc);
+    const at::Tensor ws = bytes_like(q, cott_cos_attn_f32_workspace_bytes(B, H, N, D));
+    check(cott_cos_attn_f32_bwd(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), u8(keep), nc.data_ptr<float>(),
+                                dout.data_ptr<float>(), ctx->saved_data["ws"].toTensor().data_ptr(), ws.data_ptr(), dq.data_ptr<float>(),
+                                dk.data_ptr<float>(), dv.data_ptr<float>(), dnc.data_ptr<float>(), B, H, N, D, stream_of(q)),
+          "cott_cos_attn_f32_bwd");
+    return {dq, dk, dv, dnc, Variable()};
+  }
+};
+
+// what Python calls
+at::Tensor cos_attn_causal(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& norm_const, const OptTensor& keep,
+                           int64_t nseg, bool one_pass) {
+  return CausalFn::apply(q, k, v, norm_const, keep, nseg, one_pass);
+}
+at::Tensor cos_attn_wide(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& norm_const, const OptTensor& keep) {
+  return WideFn::apply(q, k, v, norm_const, keep);
+}
+// (private copies of the parameter and of the mask: neither is read at its own address again after this call)
+at::Tensor cos_attn_f32(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& norm_const, const OptTensor& keep) {
+  return F32Fn::apply(q, k, v, norm_const.clone(), has(keep) ? OptTensor(keep->clone(at::MemoryFormat::Contiguous)) : OptTensor());
+}
+at::Tensor causal_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep, const OptTensor& sin, const OptTensor& cos) {
+  return CausalPackedFn::apply(qkv, norm_const, keep, sin, cos);
+}
+at::Tensor bidir_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep) {
+  return BidirPackedFn::apply(qkv, norm_const, keep);
+}
+at::Tensor custom_attention(const at::Tensor& Q, const at::Tensor& K, const at::Tensor& V) { return CustomAttentionFn::apply(Q, K, V); }
+
 }  // namespace
 
 TORCH_LIBRARY(cottention_b200, m) {
@@ -190,6 +531,18 @@ TORCH_LIBRARY_IMPL(cottention_b200, CUDA, m) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // how a non-zero status of the C ABI surfaces in Python: RuntimeError carrying the status text and the library's message
   m.def("_raise_for_status", [](int status) { check(status, "cottention_b200"); }, py::arg("status"));
+  m.def("seg_count", [](const at::Tensor& t, int64_t B, int64_t H, int64_t N) {
+    const c10::cuda::CUDAGuard guard(t.device());
+    return cott_cos_attn_seg_count((int)B, (int)H, (int)N);
+  });
+  m.def("cos_attn_causal", &cos_attn_causal);
+  m.def("cos_attn_wide", &cos_attn_wide);
+  m.def("cos_attn_f32", &cos_attn_f32);
+  m.def("causal_packed", &causal_packed);
+  m.def("bidir_packed", &bidir_packed);
+  m.def("custom_attention", &custom_attention);
+  m.def("decode_steps", &decode_steps);
+  m.def("prefill", &prefill);
   m.def("float32", &forward_<at::kBFloat16>, "FastAttention forward (float32 entry point)", py::arg("Q"), py::arg("K"), py::arg("V"),
         py::arg("block_size"), py::arg("inplace") = false, py::arg("reversed") = false);
   m.def("float64", &forward_<at::kBFloat16>, "FastAttention forward (float64 entry point)", py::arg("Q"), py::arg("K"), py::arg("V"),

@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _binding, _lib
 
 
 class CosAttnDecodeState:
@@ -31,6 +31,11 @@ class CosAttnDecodeState:
         wide = wide_supported(q, k, v) and q.shape[-1] == 128
         if self.cur_s != 1 or not (wide or fused_supported(q, k, v)):
             return self.step(q, k, v, norm_const)
+        m = _binding.autograd()
+        if m is not None:
+            out = m.prefill(self.state, q, k, v, norm_const)
+            self.cur_s += q.shape[2]
+            return out
         B, H, T, D = q.shape
         q, k, v = q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous()
         L = _lib.lib()
@@ -57,6 +62,11 @@ class CosAttnDecodeState:
         Dv = v.shape[-1]
         if q.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             raise RuntimeError("decode takes float32, float16 or bfloat16 tokens")
+        m = _binding.autograd()
+        if m is not None:
+            out = m.decode_steps(self.state, q, k, v, norm_const, self.cur_s)
+            self.cur_s += T
+            return out
         q, k, v = q.contiguous(), k.to(q.dtype).contiguous(), v.to(q.dtype).contiguous()
         nc = norm_const.detach().reshape(-1).to(device=q.device, dtype=torch.float32).contiguous()
         out = torch.empty(B, H, T, Dv, dtype=q.dtype, device=q.device)

@@ -1,0 +1,108 @@
+"""The compiled autograd functions against the Python ones they stand in for: same results bit for bit, and the same
+behaviour where a caller does something between the forward and the backward, or transforms the call."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _args(name, dt, seed=3, B=2, H=3, N=150):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dt)  # noqa: E731
+    nc = 0.5 + 0.2 * torch.randn(1, H, 1, 1, device="cuda", generator=g)
+    keep = torch.rand(B, N, device="cuda", generator=g) < 0.7
+    keep[:, 0] = True
+    D = {"wide": 128, "f32": 32}.get(name, 64)
+    if name in ("packed", "rotary", "bidir"):
+        x = (r(B, N, 3, H, D),)
+        do = r(B, N, H, D)
+    else:
+        x = tuple(r(B, H, N, D) for _ in range(3))
+        do = r(B, H, N, D)
+    ang = torch.rand(N, 16, device="cuda", generator=g)
+    return x, nc, keep, do, (torch.sin(ang), torch.cos(ang))
+
+
+def _call(name, x, nc, keep, rot):
+    import cottention_transformer_b200 as C
+    if name == "dropin":
+        return C.CustomAttention.apply(*x)
+    if name == "bidir":
+        return C.cos_attn_bidirectional_packed(x[0], nc, keep)
+    if name in ("packed", "rotary"):
+        return C.cos_attn_causal_packed(x[0], nc, keep, rot if name == "rotary" else None)
+    return C.cos_attn_causal(*x, nc, keep, one_pass_backward=name == "one_pass")
+
+
+PATHS = [("causal", torch.bfloat16), ("one_pass", torch.float16), ("packed", torch.bfloat16), ("rotary", torch.float16),
+         ("bidir", torch.bfloat16), ("wide", torch.float16), ("f32", torch.float32), ("dropin", torch.bfloat16), ("dropin", torch.float64)]
+
+
+@pytest.mark.parametrize("name,dt", PATHS)
+@pytest.mark.parametrize("masked", [False, True])
+def test_same_bits_as_the_python_functions(name, dt, masked, monkeypatch):
+    from cottention_transformer_b200 import _binding
+    if _binding.module() is None:
+        pytest.skip("binding not built")
+    x, nc, keep, do, rot = _args(name, dt)
+    rot_args = rot
+    res = []
+    for compiled in (True, False):
+        if not compiled:
+            monkeypatch.setattr(_binding, "autograd", lambda: None)
+        leaf = [t.clone().requires_grad_() for t in x]
+        ncl = nc.clone().requires_grad_()
+        k = keep.clone() if masked else None
+        src = [t * 1 for t in leaf] if name == "rotary" else leaf  # (few heads: the rotary embedding works in place)
+        out = _call(name, src, ncl, k, rot_args)
+        if masked:
+            k.fill_(True)  # what the caller does to its mask afterwards is not the backward's business
+        wrt = leaf if name == "dropin" else [*leaf, ncl]
+        res.append((out.detach(), *torch.autograd.grad(out, wrt, do)))
+    names = ["out", *("dx%d" % i for i in range(len(x))), "dnorm"]
+    for n, a, b in zip(names, *res):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        if n == "dnorm" and dt != torch.float32:  # sums by atomics: the order of the additions is not fixed
+            assert torch.allclose(a, b, rtol=1e-3, atol=1e-4)
+        else:
+            assert torch.equal(a, b), n
+
+
+def test_saved_tensor_hooks_and_modified_inputs():
+    from cottention_transformer_b200 import cos_attn_causal
+    x, nc, _, do, _ = _args("causal", torch.bfloat16)
+    packed = []
+    leaf = [t.clone().requires_grad_() for t in x]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.clone(), lambda t: t):
+        out = cos_attn_causal(*leaf, nc.requires_grad_())
+    assert len(packed) == 4  # q, k, v and norm_const pass through the hooks
+    a = torch.autograd.grad(out, leaf, do)
+    b = torch.autograd.grad(cos_attn_causal(*leaf, nc), leaf, do)
+    assert all(torch.equal(s, t) for s, t in zip(a, b))
+    q = x[0].clone().requires_grad_() * 1
+    out = cos_attn_causal(q, x[1], x[2], nc)
+    q.mul_(2)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(do)
+
+
+def test_transforms_are_refused_as_before():
+    from cottention_transformer_b200 import cos_attn_causal
+    x, nc, _, _, _ = _args("causal", torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda q: cos_attn_causal(q, x[1], x[2], nc).float().sum())(x[0])
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda q: cos_attn_causal(q, x[1], x[2], nc))(x[0][None])
+    with pytest.raises((RuntimeError, NotImplementedError)):
+        torch.func.jvp(lambda q: cos_attn_causal(q, x[1], x[2], nc), (x[0],), (x[0],))
+
+
+def test_short_norm_const_is_refused():
+    from cottention_transformer_b200 import CosAttnDecodeState, cos_attn_bidirectional_packed, cos_attn_causal_packed
+    x, nc, _, _, _ = _args("packed", torch.bfloat16)
+    for fn in (cos_attn_causal_packed, cos_attn_bidirectional_packed):
+        with pytest.raises(RuntimeError, match="one entry per head"):
+            fn(x[0], nc[:, :2])
+    tok = torch.randn(1, 3, 1, 64, device="cuda").bfloat16()
+    with pytest.raises(RuntimeError, match="one entry per head"):
+        CosAttnDecodeState(1, 3, 64).step(tok, tok, tok, nc[:, :2])
