@@ -6,9 +6,9 @@
 //     state[j][i] += v'[j] * k^[i]                                          (:264, layout [d_v, d_k])
 //     out[j]       = sum_i q^[i] * state[j][i]                              (:267)
 // The reference runs this on the CPU in float64 for batch 1; here the state is fp32 in HBM,
-// [B, H, d_v, d_k], updated in place.  One CTA per (b,h); a row of the state is spread over
-// d_k/4 lanes that each own one float4, so every state access is a coalesced 128-bit access and
-// the row dot product is a shuffle reduction.
+// [B, H, d_v, d_k], updated in place.  One CTA per 16 KB of a (b,h) state (64 rows, at d_k = 128 32 of them: the
+// rows are independent of each other); a row of the state is spread over d_k/4 lanes that each own one float4, so
+// every state access is a coalesced 128-bit access and the row dot product is a shuffle reduction.
 //
 // cott_decode_steps runs T consecutive positions in one launch with the state held in registers
 // between steps (it is read from and written to HBM once), which is also how a prompt is absorbed.
@@ -18,9 +18,13 @@
 
 namespace cott {
 
-// Threads per CTA: 128 for d <= 64 (8 CTAs per SM: the 1024 (b,h) states of a batch-64, 16-head step are then
-// resident in one wave of 148 x 8 CTAs, and twice the bytes are in flight per SM), 256 for d = 128.
-template <int DK> struct DecodeCfg { static constexpr int kThreads = DK <= 64 ? 128 : 256, kCtasPerSm = DK <= 64 ? 8 : 2; };
+// Bound by HBM: the state is read and written once.  128 threads with 16 KB of state in registers and eight CTAs per SM:
+// the CTAs of an SM are at different points of load -> products -> store, and the last wave is short.  (The 1024
+// (b,h) states of a batch-64, 16-head step are one wave at d = 64.  At d = 128 one CTA per state, 64 KB and two per SM, was
+// three and a half waves that loaded and stored in turn: 28.1 us for 64 x 16 states, now 24.5.)
+constexpr int kDecodeThreads = 128;
+constexpr int kDecodeCtasPerSm = 8;
+template <int DK> struct DecodeCfg { static constexpr int kRows = DK == 128 ? 32 : 64; };  // state rows of a CTA
 
 template <typename T>
 __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
@@ -29,16 +33,16 @@ __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
 // positions: optional [B] int64 array of the 1-based position of the FIRST token of this call for
 // each batch entry; if null, `pos0` is used for all.  LPR = lanes per state row = Dk/4.
 // (the kernel is latency-bound on its state loads, so resident CTAs are what hides the HBM latency)
-template <typename T, int DK, int MAX_DV>
-__global__ void __launch_bounds__(DecodeCfg<DK>::kThreads, DecodeCfg<DK>::kCtasPerSm)
+template <typename T, int DK>
+__global__ void __launch_bounds__(kDecodeThreads, kDecodeCtasPerSm)
 decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
               const float* __restrict__ norm_const, T* __restrict__ out, int H, int Dv, int Tsteps, long long pos0,
               const long long* __restrict__ positions) {
-  constexpr int kDecodeThreads = DecodeCfg<DK>::kThreads;
   constexpr int LPR = DK / 4;                    // lanes per row (4, 8, 16 or 32)
   constexpr int ROWS_PER_PASS = kDecodeThreads / LPR;
-  constexpr int MAXR = (MAX_DV + ROWS_PER_PASS - 1) / ROWS_PER_PASS;  // state rows held per thread
-  __shared__ float sq[DK], sk[DK], sv[MAX_DV];
+  constexpr int ROWS = DecodeCfg<DK>::kRows;
+  constexpr int MAXR = (ROWS + ROWS_PER_PASS - 1) / ROWS_PER_PASS;  // state rows held per thread
+  __shared__ float sq[DK], sk[DK], sv[ROWS];
   __shared__ float red[2][kDecodeThreads / 32];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -53,21 +57,23 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
   const float sigma = 1.0f / (1.0f + __expf(-norm_const[h]));
   const long long p0 = positions ? positions[b] : pos0;
   const int piece = tid % LPR;        // which float4 of the row
-  const int row0 = tid / LPR;         // first row of this thread; then += ROWS_PER_PASS
+  const int j0 = static_cast<int>(blockIdx.y) * ROWS;  // first row of this CTA
+  const int rows = min(ROWS, Dv - j0);
+  const int row0 = tid / LPR;         // first row of this thread, in the CTA; then += ROWS_PER_PASS
 
-  float* st = state + bh * static_cast<long>(Dv) * DK;
+  float* st = state + (bh * static_cast<long>(Dv) + j0) * DK;
   float4 s[MAXR];
 #pragma unroll
   for (int r = 0; r < MAXR; ++r) {
     const int j = row0 + r * ROWS_PER_PASS;
-    s[r] = (j < Dv) ? *reinterpret_cast<const float4*>(st + static_cast<long>(j) * DK + 4 * piece)
+    s[r] = (j < rows) ? *reinterpret_cast<const float4*>(st + static_cast<long>(j) * DK + 4 * piece)
                     : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
   for (int t = 0; t < Tsteps; ++t) {
     const T* qt = q + (bh * Tsteps + t) * static_cast<long>(DK);
     const T* kt = k + (bh * Tsteps + t) * static_cast<long>(DK);
-    const T* vt = v + (bh * Tsteps + t) * static_cast<long>(Dv);
+    const T* vt = v + (bh * Tsteps + t) * static_cast<long>(Dv) + j0;
     // stage q, k, v and their norms
     float x = 0.f, y = 0.f;
     if (tid < DK) {
@@ -76,7 +82,7 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
       sq[tid] = x;
       sk[tid] = y;
     }
-    if (tid < Dv) sv[tid] = ld_as_float(vt + tid);
+    if (tid < rows) sv[tid] = ld_as_float(vt + tid);
     float xx = x * x, yy = y * y;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -103,7 +109,7 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
 #pragma unroll
     for (int r = 0; r < MAXR; ++r) {
       const int j = row0 + r * ROWS_PER_PASS;
-      const bool valid = j < Dv;  // the same for all LPR lanes of a row; rows of one warp may differ
+      const bool valid = j < rows;  // the same for all LPR lanes of a row; rows of one warp may differ
       const float vj = valid ? sv[j] * ws : 0.f;
       s[r].x += vj * k4.x;
       s[r].y += vj * k4.y;
@@ -112,7 +118,7 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
       float dot = q4.x * s[r].x + q4.y * s[r].y + q4.z * s[r].z + q4.w * s[r].w;
 #pragma unroll
       for (int off = LPR / 2; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off, LPR);
-      if (valid && piece == 0) out[(bh * Tsteps + t) * static_cast<long>(Dv) + j] = from_acc<T>(dot * rq);
+      if (valid && piece == 0) out[(bh * Tsteps + t) * static_cast<long>(Dv) + j0 + j] = from_acc<T>(dot * rq);
     }
     __syncthreads();  // sq/sk/sv/red are rewritten by the next step
   }
@@ -120,7 +126,7 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
 #pragma unroll
   for (int r = 0; r < MAXR; ++r) {
     const int j = row0 + r * ROWS_PER_PASS;
-    if (j < Dv) *reinterpret_cast<float4*>(st + static_cast<long>(j) * DK + 4 * piece) = s[r];
+    if (j < rows) *reinterpret_cast<float4*>(st + static_cast<long>(j) * DK + 4 * piece) = s[r];
   }
 }
 
@@ -128,16 +134,11 @@ template <typename T>
 int launch_decode(float* state, const void* q, const void* k, const void* v, const float* nc, void* out, int B, int H,
                   int Dk, int Dv, int T_steps, long long pos0, const long long* positions, cudaStream_t stream) {
   const unsigned grid = static_cast<unsigned>(static_cast<long>(B) * H);
-#define COTT_DECODE_CASE(DK)                                                                                     \
-  case DK:                                                                                                       \
-    if (Dv <= 64)                                                                                                \
-      COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK, 64>, dim3(grid), DecodeCfg<DK>::kThreads, 0, stream, state,           \
-                               static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), nc, \
-                               static_cast<T*>(out), H, Dv, T_steps, pos0, positions));                          \
-    else                                                                                                         \
-      COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK, 128>, dim3(grid), DecodeCfg<DK>::kThreads, 0, stream, state,          \
-                               static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), nc, \
-                               static_cast<T*>(out), H, Dv, T_steps, pos0, positions));                          \
+#define COTT_DECODE_CASE(DK)                                                                                              \
+  case DK:                                                                                                                \
+    COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK>, dim3(grid, (Dv + DecodeCfg<DK>::kRows - 1) / DecodeCfg<DK>::kRows),    \
+                             kDecodeThreads, 0, stream, state, static_cast<const T*>(q), static_cast<const T*>(k),        \
+                             static_cast<const T*>(v), nc, static_cast<T*>(out), H, Dv, T_steps, pos0, positions));       \
     break;
   switch (Dk) {
     COTT_DECODE_CASE(16)
