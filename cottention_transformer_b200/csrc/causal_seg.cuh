@@ -3,7 +3,7 @@
 //
 // The sequence is cut into segments of `chunks_per_seg` chunks.  A causal kernel that starts at a segment
 // boundary only needs the state accumulated over everything before it (forward, dQ) or after it (dK/dV):
-//   1. seg_state_kernel   one CTA per (b, h, segment): the segment's own contribution  sum_s y_s (x) z_s
+//   1. seg_state_kernel   one CTA per (b, h, half segment): the segment's own contribution  sum_s y_s (x) z_s
 //                         (forward state: y = k^, z = v';  reverse state: y = q^, z = dO), tcgen05 M = 64 MMAs
 //   2. seg_prefix_kernel  exclusive prefix (or suffix) sums over the segments of each (b, h), fp32
 //   3. causal_tc_kernel / causal_bwd_kv_kernel with gridDim.y = number of segments and `init_state`
@@ -25,7 +25,7 @@ enum { kSegFwdState = 0, kSegRevState = 1, kSegRawState = 2, kSegRawStateRev = 3
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kSegThreads, 2)
 seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant__ CUtensorMap mapZ,
-                 const float* __restrict__ norm_const, float* __restrict__ state, int H, int N, int chunks_per_seg,
+                 const float* __restrict__ norm_const, float* __restrict__ state, int H, int N, int chunks_per_seg, int parts,
                  const unsigned char* __restrict__ keep, const int* __restrict__ count) {
   using namespace ptx;
   constexpr bool BF = Pack2<T>::kBf16;
@@ -40,8 +40,11 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int bh = blockIdx.x, h = bh % H, bb = bh / H, seg = blockIdx.y;
   const int total_chunks = (N + kTcChunk - 1) / kTcChunk;
-  const int chunk0 = seg * chunks_per_seg;
-  const int nchunks = min(chunks_per_seg, total_chunks - chunk0);
+  // A segment is shared by `parts` (1 or 2) CTAs, blockIdx.y = segment * parts + part, that take its halves
+  // (the last segment may be shorter than one half: its second part is then empty and its state zero)
+  const int half = (chunks_per_seg + parts - 1) / parts;
+  const int chunk0 = (seg / parts) * chunks_per_seg + (seg % parts) * half;
+  const int nchunks = max(0, min(seg % parts ? chunks_per_seg - half : half, total_chunks - chunk0));
   const unsigned char* keep_b = keep ? keep + static_cast<size_t>(bh / H) * N : nullptr;
   const int* count_b = count ? count + static_cast<size_t>(bh / H) * N : nullptr;
 
@@ -92,7 +95,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
         for (int k = 0; k < 8; ++k) mma_ss(tS, dYm + 128 * k, dZm + 128 * k, kIdescS, (c > 0 || k > 0) ? 1u : 0u);
         mma_commit(&bar_free[s]);
       }
-      if (ok) mma_commit(&bar_done);
+      if (ok) mma_commit(&bar_done);  // (without chunks: completes at once, and zeros are stored)
     }
   } else {
     const int wq = warp & 3, row = 32 * wq + lane;
@@ -123,6 +126,10 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
         uint32_t r[16];
         tmem_ld_x16(tS + lane_base + 16 * blk, r);
         tmem_ld_wait();
+        if (nchunks == 0) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = 0u;
+        }
         if (lane < 16) {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
@@ -137,7 +144,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && *abort_flag) {
+  if (tid == 0 && *abort_flag && nchunks > 0) {
     mbar_wait(&bar_full[0], 0, 64);
     mbar_wait(&bar_full[1], 0, 64);
   }
@@ -147,25 +154,29 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
 
 inline size_t seg_state_smem_bytes() { return static_cast<size_t>(4 * kTileBytes + 1024); }
 
-// Exclusive prefix (REV: suffix) over the segments of a sequence, in place: state[u][seg] <- sum over the segments before
-// (after) it.  grid = (sequences, ceil(elems / 4 / 64)), block = 64: a thread owns four neighbouring elements and has
-// eight segments in flight, so that the chain is additions and not memory round trips.
+// Exclusive prefix (REV: suffix) over the segments of a sequence: dst[u][seg] = sum over the segments before (after) it;
+// a segment's state is the sum of its `parts` (1 or 2) entries in src.  With one part dst may be src.
+// grid = (sequences, ceil(elems / 4 / 64)), block = 64: a thread owns four neighbouring elements and has eight entries in
+// flight, so that the chain is additions and not memory round trips.
 // Measured: 16 x 9 matrices of 16 KB in 6 us (one block per sequence, one load at a time and a transposed copy: 31 us).
 template <bool REV>
-__global__ void __launch_bounds__(64) seg_prefix_kernel(float4* __restrict__ state, int nseg, int quads) {
+__global__ void __launch_bounds__(64) seg_prefix_kernel(const float4* src, float4* dst, int nseg, int parts, int quads) {
   const int e = blockIdx.y * 64 + threadIdx.x;
   if (e >= quads) return;
-  float4* p = state + static_cast<size_t>(blockIdx.x) * nseg * quads + e;
+  const int n = nseg * parts;
+  const float4* p = src + static_cast<size_t>(blockIdx.x) * n * quads + e;
+  float4* o = dst + static_cast<size_t>(blockIdx.x) * nseg * quads + e;
   float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = 0; s < nseg; s += 8) {
+  for (int s = 0; s < n; s += 8) {
     float4 x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (s + i < nseg) x[i] = p[static_cast<size_t>(REV ? nseg - 1 - s - i : s + i) * quads];
+      if (s + i < n) x[i] = p[static_cast<size_t>(REV ? n - 1 - s - i : s + i) * quads];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (s + i < nseg) {
-        p[static_cast<size_t>(REV ? nseg - 1 - s - i : s + i) * quads] = run;
+      if (s + i < n) {
+        // (what a segment starts from is written before its first entry in the direction of the walk is added)
+        if ((s + i) % parts == 0) o[static_cast<size_t>(REV ? nseg - 1 - (s + i) / parts : (s + i) / parts) * quads] = run;
         run.x += x[i].x, run.y += x[i].y, run.z += x[i].z, run.w += x[i].w;
       }
   }

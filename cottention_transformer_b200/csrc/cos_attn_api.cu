@@ -180,9 +180,12 @@ int launch_bwd_fused(const void* q, const void* k, const void* v, const float* n
 }
 
 // state[bh][seg] of every segment: Y^T Z with one operand row-scaled (see seg_state_kernel)
+// Two CTAs per segment where it has the chunks for them: the kernel only streams (two stages of 32 KB and an M = 64 MMA),
+// two of its CTAs fit an SM, and one per SM left the memory half idle (B 1, H 16, N 65536: 66 -> 48 us).
+int seg_parts(const SegPlan& plan) { return plan.cps >= 4 ? 2 : 1; }
 template <typename T, int MODE>
 int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides sz, const float* nc, float* state, int B,
-                     int H, int N, int dtype, SegPlan plan, cudaStream_t stream) {
+                     int H, int N, int dtype, SegPlan plan, int parts, cudaStream_t stream) {
   const long BH = (long)B * H;
   CUtensorMap my, mz;
   int st;
@@ -190,17 +193,19 @@ int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides s
   auto kern = seg_state_kernel<T, MODE>;
   const size_t smem = seg_state_smem_bytes();
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3((unsigned)BH, plan.nseg), kSegThreads, smem, stream>>>(my, mz, nc, state, H, N, plan.cps, plan.keep, plan.count);
+  kern<<<dim3((unsigned)BH, plan.nseg * parts), kSegThreads, smem, stream>>>(my, mz, nc, state, H, N, plan.cps, parts, plan.keep, plan.count);
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
 
-// workspace of the segment-parallel path: two arrays of B*H*nseg fp32 [64 x 64] matrices, then the running keep count
-//   0 forward segment states, then their exclusive prefix | 1 reverse segment states, then their exclusive suffix
+// workspace of the segment-parallel path: five arrays of B*H*nseg fp32 [64 x 64] matrices, then the running keep count
+//   0, 1 the (half) segments' own states, of the pass that is running | 2 exclusive prefix of the forward ones |
+//   3 exclusive suffix of the reverse ones
 size_t seg_array_floats(int B, int H, int nseg) { return (size_t)B * H * nseg * kTcD * kTcD; }
-int launch_seg_prefix(float* state, long sequences, int nseg, int elems, bool reverse, cudaStream_t stream) {
+int launch_seg_prefix(const float* src, float* dst, long sequences, int nseg, int parts, int elems, bool reverse, cudaStream_t stream) {
   auto kern = reverse ? seg_prefix_kernel<true> : seg_prefix_kernel<false>;
-  kern<<<dim3((unsigned)sequences, (unsigned)((elems / 4 + 63) / 64)), 64, 0, stream>>>(reinterpret_cast<float4*>(state), nseg, elems / 4);
+  kern<<<dim3((unsigned)sequences, (unsigned)((elems / 4 + 63) / 64)), 64, 0, stream>>>(reinterpret_cast<const float4*>(src),
+                                                                                       reinterpret_cast<float4*>(dst), nseg, parts, elems / 4);
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
@@ -220,16 +225,16 @@ int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char
   plan.rot = rot;
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // running count of the kept positions, behind the state arrays
-    int* count = reinterpret_cast<int*>(ws + 2 * A);
+    int* count = reinterpret_cast<int*>(ws + 5 * A);
     keep_count_kernel<<<(unsigned)B, 256, 0, stream>>>(keep, count, N);
     COTT_CUDA_TRY(cudaGetLastError());
     plan.keep = keep;
     plan.count = count;
   }
   if (plan.nseg == 1) return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, nullptr, plan, saved, decode_state);
-  int st = launch_seg_state<T, kSegFwdState>(k, v, in_strides(plan, H, N), in_strides(plan, H, N), nc, ws, B, H, N, dtype, plan, stream);
-  if (st || (st = launch_seg_prefix(ws, (long)B * H, plan.nseg, kTcD * kTcD, false, stream))) return st;
-  return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, ws, plan, saved, decode_state);
+  int st = launch_seg_state<T, kSegFwdState>(k, v, in_strides(plan, H, N), in_strides(plan, H, N), nc, ws, B, H, N, dtype, plan, seg_parts(plan), stream);
+  if (st || (st = launch_seg_prefix(ws, ws + 2 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, false, stream))) return st;
+  return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, ws + 2 * A, plan, saved, decode_state);
 }
 
 template <typename T>
@@ -242,7 +247,7 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // the forward call left the running count in the workspace
     plan.keep = keep;
-    plan.count = reinterpret_cast<const int*>(ws + 2 * A);
+    plan.count = reinterpret_cast<const int*>(ws + 5 * A);
   }
   if (plan.nseg == 1) {
     COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
@@ -251,14 +256,14 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
     return st ? st : launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   }
   // dQ: the forward prefix states (left in the workspace by the forward call), read transposed
-  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws, plan);
+  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws + 2 * A, plan);
   if (st) return st;
   // dK, dV: reverse states of the segments, their exclusive suffix
-  if ((st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + A, B, H, N, dtype, plan,
-                                              stream)) ||
-      (st = launch_seg_prefix(ws + A, (long)B * H, plan.nseg, kTcD * kTcD, true, stream)))
+  if ((st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
+                                              seg_parts(plan), stream)) ||
+      (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream)))
     return st;
-  return launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, ws + A, plan);
+  return launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, ws + 3 * A, plan);
 }
 
 // The time-out path of the tensor-core kernels on its own: one CTA sets up what those kernels set up (an
@@ -364,7 +369,7 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
     st.x = nullptr, st.c = nullptr, st.out = nullptr;
     int r = launch_wide_t<T, REV, NORMS, true>(st, sa, B, H, N, dtype, plan.nseg, stream);
     if (r) return r;
-    if ((r = launch_seg_prefix(ws, (long)B * H * (t.dz / W), plan.nseg, kTcChunk * W, false, stream))) return r;
+    if ((r = launch_seg_prefix(ws, ws, (long)B * H * (t.dz / W), plan.nseg, 1, kTcChunk * W, false, stream))) return r;
     a.init_state = ws;
   }
   return launch_wide_t<T, REV, NORMS, false>(t, a, B, H, N, dtype, plan.nseg, stream);
@@ -444,14 +449,14 @@ int run_bwd_train(const void* q, const void* k, const void* v, const unsigned ch
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // the forward call left the running count in the workspace
     plan.keep = keep;
-    plan.count = reinterpret_cast<const int*>(ws + 2 * A);
+    plan.count = reinterpret_cast<const int*>(ws + 5 * A);
   }
   if (plan.nseg == 1) return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   // reverse states of the segments and their exclusive suffix; the prefix states come from `saved`
-  int st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws + A, B, H, N, dtype, plan,
-                                             stream);
-  if (st || (st = launch_seg_prefix(ws + A, (long)B * H, plan.nseg, kTcD * kTcD, true, stream))) return st;
-  return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + A, plan);
+  int st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
+                                             seg_parts(plan), stream);
+  if (st || (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream))) return st;
+  return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 3 * A, plan);
 }
 
 int check_ptrs16(std::initializer_list<std::pair<const void*, const char*>> ps) {
@@ -521,8 +526,8 @@ int launch_bidir_bwd_tc(const void* q, const void* k, const void* v, const unsig
 // The bare scan of cott_scan on the tensor cores (head dim 64, 16-bit dtypes): the forward kernel without its row
 // scalings, walking the sequence backwards when `reversed`.  `out` may be one of the inputs: a chunk's rows are
 // stored after every load of that chunk has completed, and no other chunk reads them.
-// `ws` (B*H*nseg fp32 [64 x 64] matrices) is only used when plan.nseg > 1: the segments' own states, then their
-// exclusive prefix in scan order.
+// `ws` (3 x B*H*nseg fp32 [64 x 64] matrices) is only used when plan.nseg > 1: the half segments' own states and the
+// exclusive prefix over the segments in scan order.
 template <typename T>
 int launch_scan_tc_t(const void* q, const void* k, const void* v, void* out, int B, int H, int N, int dtype, int reversed,
                      cudaStream_t stream, TileStrides sqk, TileStrides sv, TileStrides so, SegPlan plan, float* ws) {
@@ -533,11 +538,12 @@ int launch_scan_tc_t(const void* q, const void* k, const void* v, void* out, int
     return st;
   const float* init = nullptr;
   if (plan.nseg > 1) {
-    st = reversed ? launch_seg_state<T, kSegRawStateRev>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, stream)
-                  : launch_seg_state<T, kSegRawState>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, stream);
+    st = reversed ? launch_seg_state<T, kSegRawStateRev>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, seg_parts(plan), stream)
+                  : launch_seg_state<T, kSegRawState>(k, v, sqk, sv, nullptr, ws, B, H, N, dtype, plan, seg_parts(plan), stream);
     if (st) return st;
-    if ((st = launch_seg_prefix(ws, (long)B * H, plan.nseg, kTcD * kTcD, false, stream))) return st;
-    init = ws;
+    const size_t A = seg_array_floats(B, H, plan.nseg);
+    if ((st = launch_seg_prefix(ws, ws + 2 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, false, stream))) return st;
+    init = ws + 2 * A;
   }
   auto kern = plan.nseg > 1 ? (reversed ? causal_tc_kernel<T, kModeScanRev, true> : causal_tc_kernel<T, kModeScan, true>)
                             : (reversed ? causal_tc_kernel<T, kModeScanRev, false> : causal_tc_kernel<T, kModeScan, false>);
@@ -630,7 +636,7 @@ int launch_scan_tc_wide(const void* q, const void* k, const void* v, void* out, 
   T* oo = static_cast<T*>(out);
   // few (batch, head) pairs and a long sequence: several CTAs per sequence, as in the fused path
   const SegPlan plan = plan_segments(N, cott_cos_attn_seg_count(B, H, N));
-  const size_t ws_bytes = plan.nseg > 1 ? seg_array_floats(B, H, plan.nseg) * sizeof(float) : 0;
+  const size_t ws_bytes = plan.nseg > 1 ? 3 * seg_array_floats(B, H, plan.nseg) * sizeof(float) : 0;
   const size_t tmp_bytes = Dk > kTcD ? sizeof(T) * rows * kTcD : 0;
   char* scratch = nullptr;  // stream-ordered: segment states, then the partial result of the slices I > 0
   if (ws_bytes + tmp_bytes) {
@@ -769,7 +775,6 @@ int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H,
 
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
-  // (five arrays is what callers have always been asked for; two of them are used)
   return 5 * seg_array_floats(B, H, plan_segments(N, nseg).nseg) * sizeof(float) + (size_t)B * N * sizeof(int);
 }
 
@@ -1048,9 +1053,9 @@ int cott_cos_attn_prefill_state(const void* k, const void* v, const float* norm_
   const SegPlan plan = plan_segments(N, nseg);
   float* ws = static_cast<float*>(workspace);
   st = dtype == COTT_BF16 ? launch_seg_state<__nv_bfloat16, kSegFwdState>(k, v, contiguous_bhnd(H, N), contiguous_bhnd(H, N), norm_const, ws, B, H, N,
-                                                                        dtype, plan, s)
+                                                                        dtype, plan, 1, s)
                           : launch_seg_state<__half, kSegFwdState>(k, v, contiguous_bhnd(H, N), contiguous_bhnd(H, N), norm_const, ws, B, H, N, dtype,
-                                                                 plan, s);
+                                                                 plan, 1, s);
   if (st) return st;
   seg_to_decode_state_kernel<<<(unsigned)((long)B * H), 256, 0, s>>>(ws, state, plan.nseg, accumulate != 0);
   COTT_CUDA_TRY(cudaGetLastError());
