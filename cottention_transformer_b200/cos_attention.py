@@ -114,6 +114,11 @@ class _FusedCausal(torch.autograd.Function):
         return dq, dk, dv, dnc.reshape(ctx.nc_shape).to(ctx.nc_dtype), None, None, None
 
 
+def _table_stride(sin, N):
+    """Elements between the rotary tables of two batch entries (0: one table for all)."""
+    return N * sin.shape[-1] if sin.dim() == 3 and sin.shape[0] > 1 else 0
+
+
 class _FusedCausalPacked(torch.autograd.Function):
     """The fused causal op on the packed output of a QKV projection: ``qkv`` is ``[B, N, 3, H, 64]`` and the result
     ``[B, N, H, 64]``; q, k, v, the output and all gradients are read and written in place through strided tensor
@@ -129,49 +134,46 @@ class _FusedCausalPacked(torch.autograd.Function):
         L = _lib.lib()
         q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
         kp = None if keep is None else keep.to(device=qkv.device, dtype=torch.uint8).contiguous()
-        rot = None
-        if sin is not None:  # the rotary embedding of q, k inside the kernels (one segment per sequence)
-            per_batch = sin.dim() == 3 and sin.shape[0] > 1
-            rot = _lib.CottRotaryTables(_lib.ptr(sin), _lib.ptr(cos), 2 * sin.shape[-1], N * sin.shape[-1] if per_batch else 0)
+        code, stream = _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device)
+        rqk = qlay = None
         with torch.cuda.device(qkv.device):
-            nseg = 1 if rot is not None else L.cott_cos_attn_seg_count(B, H, N)
+            nseg = 1 if sin is not None else L.cott_cos_attn_seg_count(B, H, N)
             ws = torch.empty(L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg), dtype=torch.uint8, device=qkv.device)
-            if rot is not None:
-                st = L.cott_cos_attn_fwd_rotary(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out),
-                                                _lib.ptr(ws), ctypes.byref(lay), ctypes.byref(rot), B, H, N, D, D,
-                                                _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device))
-            else:
-                st = L.cott_cos_attn_fwd_seg(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out),
-                                             _lib.ptr(ws), nseg, ctypes.byref(lay), B, H, N, D, D, _lib.DTYPE_CODE[qkv.dtype],
-                                             _lib.stream_ptr(qkv.device))
-        _lib.check(st, "cott_cos_attn_fwd_rotary" if rot is not None else "cott_cos_attn_fwd_seg")
-        ctx.save_for_backward(qkv, nc, sin, cos)
-        ctx.ws, ctx.nseg, ctx.kp, ctx.lay, ctx.rot = ws, nseg, kp, lay, rot
+            if sin is not None:  # rotated copies of q and k, [B, N, 2, H, D]
+                rqk = torch.empty(B, N, 2, H, D, dtype=qkv.dtype, device=qkv.device)
+                qlay = _lib.CottLayout(N * 2 * H * D, D, 2 * H * D, 0, 0, 0)
+                st = L.cott_rotary_copy(_lib.ptr(q), _lib.ptr(k), _lib.ptr(rqk[:, :, 0]), _lib.ptr(rqk[:, :, 1]), _lib.ptr(sin), _lib.ptr(cos),
+                                        ctypes.byref(lay), ctypes.byref(qlay), B, H, N, D, 2 * sin.shape[-1], _table_stride(sin, N), code, stream)
+                _lib.check(st, "cott_rotary_copy")
+                q, k = rqk[:, :, 0], rqk[:, :, 1]
+            st = L.cott_cos_attn_fwd_split(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(ws), nseg,
+                                           ctypes.byref(lay), None if qlay is None else ctypes.byref(qlay), B, H, N, D, D, code, stream)
+        _lib.check(st, "cott_cos_attn_fwd_split")
+        ctx.save_for_backward(qkv, nc, sin, cos, rqk)
+        ctx.ws, ctx.nseg, ctx.kp, ctx.lay, ctx.qlay = ws, nseg, kp, lay, qlay
         ctx.nc_shape, ctx.nc_dtype = norm_const.shape, norm_const.dtype
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        qkv, nc, sin, cos = ctx.saved_tensors
+        qkv, nc, sin, cos, rqk = ctx.saved_tensors
         B, N, three, H, D = qkv.shape
         dout = dout.contiguous().to(qkv.dtype)
         dqkv = torch.empty_like(qkv)
         dnc = torch.empty(H, dtype=torch.float32, device=qkv.device)
         L = _lib.lib()
+        code, stream = _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device)
+        q, k = (qkv[:, :, 0], qkv[:, :, 1]) if rqk is None else (rqk[:, :, 0], rqk[:, :, 1])
         with torch.cuda.device(qkv.device):
-            if ctx.rot is not None:
-                st = L.cott_cos_attn_bwd_rotary(
-                    _lib.ptr(qkv[:, :, 0]), _lib.ptr(qkv[:, :, 1]), _lib.ptr(qkv[:, :, 2]), _lib.ptr(ctx.kp), _lib.ptr(nc),
-                    _lib.ptr(dout), _lib.ptr(ctx.ws), ctypes.byref(ctx.lay), ctypes.byref(ctx.rot), _lib.ptr(dqkv[:, :, 0]),
-                    _lib.ptr(dqkv[:, :, 1]), _lib.ptr(dqkv[:, :, 2]), _lib.ptr(dnc), B, H, N, D, D, _lib.DTYPE_CODE[qkv.dtype],
-                    _lib.stream_ptr(qkv.device))
-            else:
-                st = L.cott_cos_attn_bwd_seg(
-                    _lib.ptr(qkv[:, :, 0]), _lib.ptr(qkv[:, :, 1]), _lib.ptr(qkv[:, :, 2]), _lib.ptr(ctx.kp), _lib.ptr(nc),
-                    _lib.ptr(dout), _lib.ptr(ctx.ws), ctx.nseg, ctypes.byref(ctx.lay), _lib.ptr(dqkv[:, :, 0]),
-                    _lib.ptr(dqkv[:, :, 1]), _lib.ptr(dqkv[:, :, 2]), _lib.ptr(dnc), B, H, N, D, D, _lib.DTYPE_CODE[qkv.dtype],
-                    _lib.stream_ptr(qkv.device))
-        _lib.check(st, "cott_cos_attn_bwd_rotary" if ctx.rot is not None else "cott_cos_attn_bwd_seg")
+            st = L.cott_cos_attn_bwd_split(
+                _lib.ptr(q), _lib.ptr(k), _lib.ptr(qkv[:, :, 2]), _lib.ptr(ctx.kp), _lib.ptr(nc), _lib.ptr(dout), _lib.ptr(ctx.ws), ctx.nseg,
+                ctypes.byref(ctx.lay), None if rqk is None else ctypes.byref(ctx.qlay), _lib.ptr(dqkv[:, :, 0]), _lib.ptr(dqkv[:, :, 1]),
+                _lib.ptr(dqkv[:, :, 2]), _lib.ptr(dnc), B, H, N, D, D, code, stream)
+            _lib.check(st, "cott_cos_attn_bwd_split")
+            if rqk is not None:  # the gradients of the rotated q and k, back through the rotation
+                st = L.cott_rotary(_lib.ptr(dqkv[:, :, 0]), _lib.ptr(dqkv[:, :, 1]), _lib.ptr(sin), _lib.ptr(cos), ctypes.byref(ctx.lay), B, H, N, D,
+                                   2 * sin.shape[-1], _table_stride(sin, N), 1, code, stream)
+                _lib.check(st, "cott_rotary")
         return dqkv, dnc.reshape(ctx.nc_shape).to(ctx.nc_dtype), None, None, None
 
 
@@ -182,10 +184,13 @@ def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None):
 
     ``rotary=(sin, cos)`` -- fp32 ``[N, rot/2]`` or ``[B, N, rot/2]``, the two halves of the module's
     ``embed_positions`` gathered at ``position_ids`` (GPTCosAttention.py:458-476) -- applies the rotary embedding to
-    q and k **inside the kernels** (their tiles are rotated in shared memory, dq and dk are rotated back on the way
-    out): the same bits as ``rotary_packed_`` followed by this op, without that op's passes over q, k, dq, dk, and
-    ``qkv`` itself is left as the projection wrote it.  The rotary dim must be a multiple of 16; sequences that this
-    op would cut into segments (few heads, very long N) take the separate rotary pass instead."""
+    q and k: the same bits as ``rotary_packed_`` followed by this op, and ``qkv`` itself is left as the projection wrote
+    it.  The rotated q and k go to a buffer that is kept for the backward (two thirds of ``qkv``), and dq and dk are
+    rotated back in place.  (Inside the kernels, ``cott_cos_attn_fwd_rotary`` / ``_bwd_rotary``, the rotation needs neither
+    buffer nor passes but sits on the chunk chain of all three kernels: 109 us for B 8, H 16, N 1024 forward and backward against 78 us with
+    the passes.)
+    The rotary dim must be a multiple of 16; sequences that this op would cut into segments (few heads, very long N) are
+    rotated in ``qkv`` itself instead."""
     if not qkv.is_cuda:
         raise RuntimeError("cos_attn_causal_packed needs a CUDA tensor (there is no CPU path)")
     if qkv.dim() != 5 or qkv.shape[2] != 3 or qkv.shape[-1] != 64 or qkv.dtype not in FUSED_DTYPES:

@@ -48,6 +48,7 @@ struct SegPlan {
   const unsigned char* keep = nullptr;  // padding: [B, N] keep flags and their inclusive running count, or both null
   const int* count = nullptr;
   TileStrides in{0, 0, 0}, out{0, 0, 0};  // strides of q, k, v, dq, dk, dv / of out, dout; all zero = contiguous [B,H,N,64]
+  TileStrides qk{0, 0, 0};  // strides of q and k where they differ from v's (rotated copies); all zero = `in`
   RotArgs rot{nullptr, nullptr, 0, 0};    // rotary embedding of q, k inside the kernels (one segment only), or sin = null
   // The caller has already zeroed the norm_const gradient on the stream, before the dQ launch: a memset between the dQ
   // and the dK/dV launch would end the chain of programmatic dependent launches (the dK/dV kernel could not set itself
@@ -55,6 +56,7 @@ struct SegPlan {
   bool dnorm_zeroed = false;
 };
 TileStrides in_strides(const SegPlan& p, long H, long N) { return p.in.n ? p.in : contiguous_bhnd(H, N); }
+TileStrides qk_strides(const SegPlan& p, long H, long N) { return p.qk.n ? p.qk : in_strides(p, H, N); }
 TileStrides out_strides(const SegPlan& p, long H, long N) { return p.out.n ? p.out : contiguous_bhnd(H, N); }
 SegPlan plan_segments(int N, int nseg_requested) {
   const int total = (N + kTcChunk - 1) / kTcChunk;
@@ -89,7 +91,7 @@ int launch_fwd(const void* q, const void* k, const void* v, const float* nc, voi
   const long BH = (long)B * H;
   CUtensorMap mq, mk, mv, mo;
   int st;
-  if ((st = tmap(&mq, q, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) ||
+  if ((st = tmap(&mq, q, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) ||
       (st = tmap(&mo, out, dtype, B, H, N, out_strides(plan, H, N))))
     return st;
   const bool ext = plan.nseg > 1 || init || plan.keep || decode_state;
@@ -111,7 +113,7 @@ int launch_bwd_dq(const void* q, const void* k, const void* v, const float* nc, 
   const long BH = (long)B * H;
   CUtensorMap mq, mk, mv, md, mo;
   int st;
-  if ((st = tmap(&mq, q, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, in_strides(plan, H, N))) ||
+  if ((st = tmap(&mq, q, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, qk_strides(plan, H, N))) ||
       (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&md, dout, dtype, B, H, N, out_strides(plan, H, N))) ||
       (st = tmap(&mo, dq, dtype, B, H, N, in_strides(plan, H, N))))
     return st;
@@ -134,7 +136,7 @@ int launch_bwd_dkdv(const void* q, const void* k, const void* v, const float* nc
   const long BH = (long)B * H;
   CUtensorMap mq, mk, mv, md, mdk, mdv;
   int st;
-  if ((st = tmap(&mq, q, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, in_strides(plan, H, N))) ||
+  if ((st = tmap(&mq, q, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, qk_strides(plan, H, N))) ||
       (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&md, dout, dtype, B, H, N, out_strides(plan, H, N))) ||
       (st = tmap(&mdk, dk, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mdv, dv, dtype, B, H, N, in_strides(plan, H, N))))
     return st;
@@ -160,7 +162,7 @@ int launch_bwd_fused(const void* q, const void* k, const void* v, const float* n
   const long rows = (long)((N + kTcChunk - 1) / kTcChunk) * kTcD;  // state rows per (b, h)
   CUtensorMap mq, mk, mv, md, ms, mdq, mdk, mdv;
   int st;
-  if ((st = tmap(&mq, q, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, in_strides(plan, H, N))) ||
+  if ((st = tmap(&mq, q, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, qk_strides(plan, H, N))) ||
       (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&md, dout, dtype, B, H, N, out_strides(plan, H, N))) ||
       (st = tmap(&mdq, dq, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mdk, dk, dtype, B, H, N, in_strides(plan, H, N))) ||
       (st = tmap(&mdv, dv, dtype, B, H, N, in_strides(plan, H, N))))
@@ -219,9 +221,11 @@ void apply_layout(SegPlan& plan, const cott_layout* l) {
 template <typename T>
 int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, void* out,
                 float* ws, int nseg, const cott_layout* layout, int B, int H, int N, int dtype, cudaStream_t stream,
-                void* saved = nullptr, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0}, float* decode_state = nullptr) {
+                void* saved = nullptr, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0}, float* decode_state = nullptr,
+                const cott_layout* qk_layout = nullptr) {
   SegPlan plan = plan_segments(N, nseg);
   apply_layout(plan, layout);
+  if (qk_layout) plan.qk = TileStrides{qk_layout->in_b, qk_layout->in_h, qk_layout->in_n};
   plan.rot = rot;
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // running count of the kept positions, behind the state arrays
@@ -232,7 +236,7 @@ int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char
     plan.count = count;
   }
   if (plan.nseg == 1) return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, nullptr, plan, saved, decode_state);
-  int st = launch_seg_state<T, kSegFwdState>(k, v, in_strides(plan, H, N), in_strides(plan, H, N), nc, ws, B, H, N, dtype, plan, seg_parts(plan), stream);
+  int st = launch_seg_state<T, kSegFwdState>(k, v, qk_strides(plan, H, N), in_strides(plan, H, N), nc, ws, B, H, N, dtype, plan, seg_parts(plan), stream);
   if (st || (st = launch_seg_prefix(ws, ws + 2 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, false, stream))) return st;
   return launch_fwd<T>(q, k, v, nc, out, B, H, N, dtype, stream, ws + 2 * A, plan, saved, decode_state);
 }
@@ -240,9 +244,11 @@ int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char
 template <typename T>
 int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, const void* dout,
                 float* ws, int nseg, const cott_layout* layout, void* dq, void* dk, void* dv, float* dnorm, int B, int H,
-                int N, int dtype, cudaStream_t stream, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0}) {
+                int N, int dtype, cudaStream_t stream, RotArgs rot = RotArgs{nullptr, nullptr, 0, 0},
+                const cott_layout* qk_layout = nullptr) {
   SegPlan plan = plan_segments(N, nseg);
   apply_layout(plan, layout);
+  if (qk_layout) plan.qk = TileStrides{qk_layout->in_b, qk_layout->in_h, qk_layout->in_n};
   plan.rot = rot;
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // the forward call left the running count in the workspace
@@ -259,7 +265,7 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
   int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws + 2 * A, plan);
   if (st) return st;
   // dK, dV: reverse states of the segments, their exclusive suffix
-  if ((st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
+  if ((st = launch_seg_state<T, kSegRevState>(q, dout, qk_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
                                               seg_parts(plan), stream)) ||
       (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream)))
     return st;
@@ -453,7 +459,7 @@ int run_bwd_train(const void* q, const void* k, const void* v, const unsigned ch
   }
   if (plan.nseg == 1) return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   // reverse states of the segments and their exclusive suffix; the prefix states come from `saved`
-  int st = launch_seg_state<T, kSegRevState>(q, dout, in_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
+  int st = launch_seg_state<T, kSegRevState>(q, dout, qk_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
                                              seg_parts(plan), stream);
   if (st || (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream))) return st;
   return launch_bwd_fused<T>(q, k, v, nc, dout, saved, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 3 * A, plan);
@@ -781,6 +787,12 @@ size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg) {
 int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
                           const float* norm_const, void* out, void* workspace, int nseg, const cott_layout* layout,
                           int B, int H, int N, int Dk, int Dv, int dtype, void* stream) {
+  return cott_cos_attn_fwd_split(q, k, v, keep, norm_const, out, workspace, nseg, layout, nullptr, B, H, N, Dk, Dv, dtype, stream);
+}
+
+int cott_cos_attn_fwd_split(const void* q, const void* k, const void* v, const unsigned char* keep, const float* norm_const,
+                            void* out, void* workspace, int nseg, const cott_layout* layout, const cott_layout* qk_layout, int B,
+                            int H, int N, int Dk, int Dv, int dtype, void* stream) {
   int st = check_fused_args(B, H, N, Dk, Dv, dtype);
   if (st) return st;
   if ((long)B * H * N == 0) return COTT_OK;
@@ -790,14 +802,25 @@ int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const uns
   COTT_CUDA_TRY(scope.status());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* ws = static_cast<float*>(workspace);
-  return dtype == COTT_BF16 ? run_fwd_seg<__nv_bfloat16>(q, k, v, keep, norm_const, out, ws, nseg, layout, B, H, N, dtype, s)
-                            : run_fwd_seg<__half>(q, k, v, keep, norm_const, out, ws, nseg, layout, B, H, N, dtype, s);
+  const RotArgs none{nullptr, nullptr, 0, 0};
+  return dtype == COTT_BF16 ? run_fwd_seg<__nv_bfloat16>(q, k, v, keep, norm_const, out, ws, nseg, layout, B, H, N, dtype, s, nullptr, none,
+                                                         nullptr, qk_layout)
+                            : run_fwd_seg<__half>(q, k, v, keep, norm_const, out, ws, nseg, layout, B, H, N, dtype, s, nullptr, none, nullptr,
+                                                  qk_layout);
 }
 
 int cott_cos_attn_bwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
                           const float* norm_const, const void* dout, void* workspace, int nseg,
                           const cott_layout* layout, void* dq, void* dk, void* dv, float* dnorm_const, int B, int H,
                           int N, int Dk, int Dv, int dtype, void* stream) {
+  return cott_cos_attn_bwd_split(q, k, v, keep, norm_const, dout, workspace, nseg, layout, nullptr, dq, dk, dv, dnorm_const, B, H, N, Dk, Dv,
+                                 dtype, stream);
+}
+
+int cott_cos_attn_bwd_split(const void* q, const void* k, const void* v, const unsigned char* keep, const float* norm_const,
+                            const void* dout, void* workspace, int nseg, const cott_layout* layout, const cott_layout* qk_layout,
+                            void* dq, void* dk, void* dv, float* dnorm_const, int B, int H, int N, int Dk, int Dv, int dtype,
+                            void* stream) {
   int st = check_fused_args(B, H, N, Dk, Dv, dtype);
   if (st) return st;
   if (!dnorm_const && H > 0) return fail(COTT_ERR_NULL, "null pointer: dnorm_const");
@@ -814,8 +837,10 @@ int cott_cos_attn_bwd_seg(const void* q, const void* k, const void* v, const uns
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* ws = static_cast<float*>(workspace);
   return dtype == COTT_BF16
-             ? run_bwd_seg<__nv_bfloat16>(q, k, v, keep, norm_const, dout, ws, nseg, layout, dq, dk, dv, dnorm_const, B, H, N, dtype, s)
-             : run_bwd_seg<__half>(q, k, v, keep, norm_const, dout, ws, nseg, layout, dq, dk, dv, dnorm_const, B, H, N, dtype, s);
+             ? run_bwd_seg<__nv_bfloat16>(q, k, v, keep, norm_const, dout, ws, nseg, layout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, RotArgs{nullptr, nullptr, 0, 0},
+                                          qk_layout)
+             : run_bwd_seg<__half>(q, k, v, keep, norm_const, dout, ws, nseg, layout, dq, dk, dv, dnorm_const, B, H, N, dtype, s,
+                                   RotArgs{nullptr, nullptr, 0, 0}, qk_layout);
 }
 
 namespace {

@@ -279,27 +279,39 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
     const bool rot = has(sin);
     const int nseg = rot ? 1 : cott_cos_attn_seg_count(B, H, N);
     at::Tensor ws = bytes_like(p.qkv, cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
+    at::Tensor rqk;  // the rotated q and k, [B, N, 2, H, D]
     if (rot) {
-      const cott_rotary_tables r = tables(*sin, *cos, N);
-      check(cott_cos_attn_fwd_rotary(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), out.data_ptr(), ws.data_ptr(), &p.lay, &r, B,
-                                     H, N, D, D, code, stream_of(p.qkv)),
-            "cott_cos_attn_fwd_rotary");
-    } else {
-      check(cott_cos_attn_fwd_seg(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), out.data_ptr(), ws.data_ptr(), nseg, &p.lay, B, H,
-                                  N, D, D, code, stream_of(p.qkv)),
-            "cott_cos_attn_fwd_seg");
+      rqk = at::empty({p.B, p.N, 2, p.H, p.D}, p.qkv.options());
+      rotate(p, rqk, *sin, *cos, false);
     }
-    ctx->save_for_backward({p.qkv, nc, rot ? *sin : at::Tensor(), rot ? *cos : at::Tensor()});
+    const cott_layout ql = qk_layout(p);
+    check(cott_cos_attn_fwd_split(rot ? rqk.data_ptr() : p.part(0), rot ? k_of(rqk, p) : p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(),
+                                  out.data_ptr(), ws.data_ptr(), nseg, &p.lay, rot ? &ql : nullptr, B, H, N, D, D, code, stream_of(p.qkv)),
+          "cott_cos_attn_fwd_split");
+    ctx->save_for_backward({p.qkv, nc, rot ? *sin : at::Tensor(), rot ? *cos : at::Tensor(), rqk});
     ctx->saved_data["ws"] = ws;
     ctx->saved_data["nseg"] = (int64_t)nseg;
     save_opt(ctx, "keep", kp);
     save_nc(ctx, norm_const);
     return out;
   }
-  static cott_rotary_tables tables(const at::Tensor& sin, const at::Tensor& cos, int N) {
+  static cott_layout qk_layout(const Packed& p) { return cott_layout{p.N * 2 * p.H * p.D, p.D, 2 * p.H * p.D, 0, 0, 0}; }
+  static void* k_of(const at::Tensor& rqk, const Packed& p) { return static_cast<char*>(rqk.data_ptr()) + p.H * p.D * p.e; }
+  // q and k of `p` rotated into rqk, or (inverse) the gradients in `p` rotated back in place
+  static void rotate(const Packed& p, const at::Tensor& rqk, const at::Tensor& sin, const at::Tensor& cos, bool inverse) {
     const int64_t half = sin.size(-1);
-    const bool per_batch = sin.dim() == 3 && sin.size(0) > 1;
-    return cott_rotary_tables{sin.data_ptr<float>(), cos.data_ptr<float>(), (int)(2 * half), per_batch ? (long long)(N * half) : 0};
+    const long long stride = sin.dim() == 3 && sin.size(0) > 1 ? (long long)(p.N * half) : 0;
+    const int B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D, code = dtype_code(p.qkv.scalar_type());
+    if (inverse) {
+      check(cott_rotary(p.part(0), p.part(1), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, B, H, N, D, (int)(2 * half), stride, 1, code,
+                        stream_of(p.qkv)),
+            "cott_rotary");
+      return;
+    }
+    const cott_layout ql = qk_layout(p);
+    check(cott_rotary_copy(p.part(0), p.part(1), rqk.data_ptr(), k_of(rqk, p), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, &ql, B, H, N, D,
+                           (int)(2 * half), stride, code, stream_of(p.qkv)),
+          "cott_rotary_copy");
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
@@ -309,17 +321,13 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
     const OptTensor kp = load_opt(ctx, "keep");
     at::Tensor dnc = at::empty({p.H}, p.qkv.options().dtype(at::kFloat));
     const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
-    if (s[2].defined()) {
-      const cott_rotary_tables r = tables(s[2], s[3], N);
-      check(cott_cos_attn_bwd_rotary(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), dout.data_ptr(), ws.data_ptr(), &p.lay, &r,
-                                     d.part(0), d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D, D, code, stream_of(p.qkv)),
-            "cott_cos_attn_bwd_rotary");
-    } else {
-      check(cott_cos_attn_bwd_seg(p.part(0), p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(), dout.data_ptr(), ws.data_ptr(),
-                                  (int)ctx->saved_data["nseg"].toInt(), &p.lay, d.part(0), d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D,
-                                  D, code, stream_of(p.qkv)),
-            "cott_cos_attn_bwd_seg");
-    }
+    const bool rot = s[2].defined();
+    const cott_layout ql = qk_layout(p);
+    check(cott_cos_attn_bwd_split(rot ? s[4].data_ptr() : p.part(0), rot ? k_of(s[4], p) : p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(),
+                                  dout.data_ptr(), ws.data_ptr(), (int)ctx->saved_data["nseg"].toInt(), &p.lay, rot ? &ql : nullptr, d.part(0),
+                                  d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D, D, code, stream_of(p.qkv)),
+          "cott_cos_attn_bwd_split");
+    if (rot) rotate(d, at::Tensor(), s[2], s[3], true);
     return {d.qkv, nc_grad(ctx, dnc), Variable(), Variable(), Variable()};
   }
 };

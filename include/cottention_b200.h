@@ -158,6 +158,15 @@ int cott_cos_attn_bwd_seg(const void* q, const void* k, const void* v, const uns
                           const float* norm_const, const void* dout, void* workspace, int nseg,
                           const cott_layout* layout, void* dq, void* dk, void* dv, float* dnorm_const, int B,
                           int H, int N, int Dk, int Dv, int dtype, void* stream);
+/* The same with q and k in a layout of their own (`qk_layout`, its in_* fields; NULL = `layout`): rotated copies of the q and k
+ * of a packed projection (cott_rotary_copy) next to its v.  dq, dk, dv have the layout of v. */
+int cott_cos_attn_fwd_split(const void* q, const void* k, const void* v, const unsigned char* keep, const float* norm_const,
+                            void* out, void* workspace, int nseg, const cott_layout* layout, const cott_layout* qk_layout, int B,
+                            int H, int N, int Dk, int Dv, int dtype, void* stream);
+int cott_cos_attn_bwd_split(const void* q, const void* k, const void* v, const unsigned char* keep, const float* norm_const,
+                            const void* dout, void* workspace, int nseg, const cott_layout* layout, const cott_layout* qk_layout,
+                            void* dq, void* dk, void* dv, float* dnorm_const, int B, int H, int N, int Dk, int Dv, int dtype,
+                            void* stream);
 
 /*
  * Training pair: forward that keeps what a ONE-pass backward needs, and that backward.
@@ -368,6 +377,11 @@ int cott_selftest_device_wait(int polls, int code, int chunk, void* stream);
  * (table_batch_stride = N * rot_dim/2).  inverse != 0 applies the transposed rotation (the backward of the op). */
 int cott_rotary(void* q, void* k, const float* sin_table, const float* cos_table, const cott_layout* layout, int B,
                 int H, int N, int D, int rot_dim, long long table_batch_stride, int inverse, int dtype, void* stream);
+/* The rotation from (q, k) to (q_out, k_out), which get whole rows (the elements past rot_dim unchanged); the sources are
+ * left alone.  `layout` / `out_layout`: strides (in_*) of the sources / of the copies, NULL = dense [B, H, N, D]. */
+int cott_rotary_copy(const void* q, const void* k, void* q_out, void* k_out, const float* sin_table, const float* cos_table,
+                     const cott_layout* layout, const cott_layout* out_layout, int B, int H, int N, int D, int rot_dim,
+                     long long table_batch_stride, int dtype, void* stream);
 
 /*
  * The fused causal forward / backward with the rotary position embedding of the reference's GPT module folded in

@@ -106,3 +106,35 @@ def test_short_norm_const_is_refused():
     tok = torch.randn(1, 3, 1, 64, device="cuda").bfloat16()
     with pytest.raises(RuntimeError, match="one entry per head"):
         CosAttnDecodeState(1, 3, 64).step(tok, tok, tok, nc[:, :2])
+
+
+@pytest.mark.parametrize("N,rot", [(1, 64), (130, 16), (300, 48)])
+@pytest.mark.parametrize("per_batch", [False, True])
+def test_rotation_inside_the_kernels_gives_the_bits_of_the_copying_pass(N, rot, per_batch):
+    """``cott_cos_attn_fwd_rotary`` / ``_bwd_rotary`` (C callers without room for the rotated copies) against the op."""
+    import ctypes
+
+    from cottention_transformer_b200 import _lib, cos_attn_causal_packed
+    B, H, D = 3, 30, 64  # (90 sequences: one segment each)
+    g = torch.Generator(device="cuda").manual_seed(N + rot)
+    qkv = torch.randn(B, N, 3, H, D, device="cuda", generator=g).bfloat16()
+    do = torch.randn(B, N, H, D, device="cuda", generator=g).bfloat16()
+    nc = 0.5 + 0.2 * torch.randn(H, device="cuda", generator=g)
+    ang = torch.rand(*((B, N, rot // 2) if per_batch else (N, rot // 2)), device="cuda", generator=g) * 6
+    sin, cos = torch.sin(ang), torch.cos(ang)
+    leaf = qkv.clone().requires_grad_()
+    out = cos_attn_causal_packed(leaf, nc, None, (sin, cos))
+    (dx,) = torch.autograd.grad(out, leaf, do)
+    assert torch.equal(leaf, qkv)
+    L, P = _lib.lib(), (lambda t: t.data_ptr())
+    o, d, dnc = torch.empty_like(out), torch.empty_like(qkv), torch.empty(H, device="cuda")
+    ws = torch.empty(L.cott_cos_attn_seg_workspace_bytes(B, H, N, 1), dtype=torch.uint8, device="cuda")
+    lay = _lib.CottLayout(N * 3 * H * D, D, 3 * H * D, N * H * D, D, H * D)
+    tab = _lib.CottRotaryTables(P(sin), P(cos), rot, N * rot // 2 if per_batch else 0)
+    st = _lib.stream_ptr(qkv.device)
+    q, k, v = (P(qkv[:, :, i]) for i in range(3))
+    _lib.check(L.cott_cos_attn_fwd_rotary(q, k, v, None, P(nc), P(o), P(ws), ctypes.byref(lay), ctypes.byref(tab), B, H, N, D, D, 3, st), "fwd")
+    _lib.check(L.cott_cos_attn_bwd_rotary(q, k, v, None, P(nc), P(do), P(ws), ctypes.byref(lay), ctypes.byref(tab), P(d[:, :, 0]), P(d[:, :, 1]),
+                                          P(d[:, :, 2]), P(dnc), B, H, N, D, D, 3, st), "bwd")
+    _lib.check_device_status()
+    assert torch.equal(o, out) and torch.equal(d, dx)
