@@ -521,14 +521,15 @@ constexpr int kTcStagesFwd = 4;  // the forward kernel has the shared memory for
 // ROT (forward and dQ, EXT only, one segment): q and k are rotated by the rotary embedding inside the kernel -- the
 // Q and K tiles are rewritten in shared memory before any MMA reads them, and the dQ rows are rotated back before
 // they are stored -- so the tensors in HBM stay un-rotated and no separate pass over q, k, dq, dk is needed.
-template <typename T, int MODE, bool EXT, bool SAVE = false, bool ROT = false>
-__global__ void __launch_bounds__(kTcThreads, 1)
-causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapY,
-                 const __grid_constant__ CUtensorMap mapZ, const __grid_constant__ CUtensorMap mapQ,
-                 const __grid_constant__ CUtensorMap mapOut, const float* __restrict__ norm_const, int H, int N,
-                 const float* __restrict__ init_state_arg, int chunks_per_seg_arg,
-                 const unsigned char* __restrict__ keep_arg, const int* __restrict__ count_arg,
-                 uint4* __restrict__ saved, const RotArgs rot, float* __restrict__ decode_state) {
+// (`bh`, `seg_arg` of `nsegs`: what this CTA works on.  The body is a function of its own so that causal_bwd_both_kernel can
+// run it next to the dK/dV body.)
+template <typename T, int MODE, bool EXT, bool SAVE, bool ROT>
+__device__ __forceinline__ void causal_tc_body(const CUtensorMap& mapX, const CUtensorMap& mapY, const CUtensorMap& mapZ,
+                                               const CUtensorMap& mapQ, const CUtensorMap& mapOut, const float* __restrict__ norm_const,
+                                               int H, int N, const float* __restrict__ init_state_arg, int chunks_per_seg_arg,
+                                               const unsigned char* __restrict__ keep_arg, const int* __restrict__ count_arg,
+                                               uint4* __restrict__ saved, const RotArgs& rot, float* __restrict__ decode_state,
+                                               const int bh, const int seg_arg, const int nsegs) {
   using namespace ptx;
   static_assert(!ROT || (EXT && !SAVE && (MODE == kModeFwd || MODE == kModeDq)), "rotary: forward / dQ, EXT, no saved states");
   // Shared memory: NS stages of the tiles that are only read (forward: Y, Z; dQ: X, Y, Z), a ring of
@@ -561,7 +562,6 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // broadcast: provably warp-uniform
-  const int bh = blockIdx.x;
   const int h = bh % H, bb = bh / H;
   pdl_allow_next();  // the next kernel of the stream may set itself up on the SMs this one leaves free
   // Segment-parallel launches (gridDim.y > 1) give each CTA `chunks_per_seg` consecutive chunks of the
@@ -570,12 +570,12 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
   const int total_chunks = (N + kTcChunk - 1) / kTcChunk;
   const float* init_state = EXT ? init_state_arg : nullptr;
   const int chunks_per_seg = EXT ? chunks_per_seg_arg : total_chunks;
-  const int seg = EXT ? static_cast<int>(blockIdx.y) : 0;
+  const int seg = EXT ? seg_arg : 0;
   const int chunk0 = seg * chunks_per_seg;
   const int nchunks = EXT ? min(chunks_per_seg, total_chunks - chunk0) : total_chunks;
   const bool has_init = EXT && init_state != nullptr && seg > 0;
   // state updates of this CTA: the one after its last chunk is only needed as the decode state
-  const bool final_state = EXT && MODE == kModeFwd && decode_state != nullptr && seg + 1 == static_cast<int>(gridDim.y);
+  const bool final_state = EXT && MODE == kModeFwd && decode_state != nullptr && seg + 1 == nsegs;
   const int nstates = nchunks - 1 + (final_state ? 1 : 0);
   const unsigned char* keep_b = (EXT && keep_arg) ? keep_arg + static_cast<size_t>(bh / H) * N : nullptr;
   const int* count_b = (EXT && count_arg) ? count_arg + static_cast<size_t>(bh / H) * N : nullptr;
@@ -767,7 +767,7 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     if (has_init) {
       // the state before this segment: fp32 into TMEM, 16-bit into the operand buffer of chunk 0 (dQ: its state is the
       // transpose of the forward's, sum v (x) w k against sum k (x) w v)
-      load_init_state<T, MODE == kModeDq>(init_state + (static_cast<size_t>(bh) * gridDim.y + seg) * (kTcD * kTcD), tS + lane_base, sS,
+      load_init_state<T, MODE == kModeDq>(init_state + (static_cast<size_t>(bh) * nsegs + seg) * (kTcD * kTcD), tS + lane_base, sS,
                                           wq, lane);
       tmem_st_wait();
       fence_proxy_async_smem();
@@ -921,6 +921,17 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
+template <typename T, int MODE, bool EXT, bool SAVE = false, bool ROT = false>
+__global__ void __launch_bounds__(kTcThreads, 1)
+causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapY,
+                 const __grid_constant__ CUtensorMap mapZ, const __grid_constant__ CUtensorMap mapQ,
+                 const __grid_constant__ CUtensorMap mapOut, const float* __restrict__ norm_const, int H, int N,
+                 const float* __restrict__ init_state, int chunks_per_seg, const unsigned char* __restrict__ keep,
+                 const int* __restrict__ count, uint4* __restrict__ saved, const RotArgs rot, float* __restrict__ decode_state) {
+  causal_tc_body<T, MODE, EXT, SAVE, ROT>(mapX, mapY, mapZ, mapQ, mapOut, norm_const, H, N, init_state, chunks_per_seg, keep, count, saved, rot,
+                                          decode_state, blockIdx.x, blockIdx.y, gridDim.y);
+}
+
 // -------------------------------------------------------------------------------------------------
 // dK, dV and the gradient of the length-norm parameter: one reverse-direction pass.
 //
@@ -937,14 +948,13 @@ causal_tc_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
 // ROT: as in causal_tc_kernel -- the Q and K tiles are rotated in shared memory, by a warp group of their own that
 // works as soon as a stage has arrived (two chunks ahead of its use: the rotation is off the chain that sets the chunk
 // period), and the dK rows are rotated back before they are stored.
-template <typename T, bool EXT, bool ROT = false>
-__global__ void __launch_bounds__(ROT ? kKvThreadsRot : kKvThreads, 1)
-causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
-                     const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
-                     const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV, float* __restrict__ dnorm,
-                     const float* __restrict__ norm_const, int H, int N, const float* __restrict__ init_state_arg,
-                     int chunks_per_seg_arg, const unsigned char* __restrict__ keep_arg,
-                     const int* __restrict__ count_arg, const RotArgs rot) {
+template <typename T, bool EXT, bool ROT>
+__device__ __forceinline__ void causal_bwd_kv_body(const CUtensorMap& mapQ, const CUtensorMap& mapK, const CUtensorMap& mapV,
+                                                   const CUtensorMap& mapDO, const CUtensorMap& mapDK, const CUtensorMap& mapDV,
+                                                   float* __restrict__ dnorm, const float* __restrict__ norm_const, int H, int N,
+                                                   const float* __restrict__ init_state_arg, int chunks_per_seg_arg,
+                                                   const unsigned char* __restrict__ keep_arg, const int* __restrict__ count_arg,
+                                                   const RotArgs& rot, const int bh, const int seg_arg, const int nsegs) {
   using namespace ptx;
   static_assert(!ROT || EXT, "rotary: EXT only");
   constexpr int STAGE = 4 * kTileBytes;
@@ -964,7 +974,6 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // broadcast: provably warp-uniform
-  const int bh = blockIdx.x;
   const int h = bh % H, bb = bh / H;
   pdl_allow_next();
   // Segment-parallel launches (gridDim.y > 1): this CTA owns `chunks_per_seg` consecutive chunks, walks them
@@ -973,11 +982,11 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
   const int total_chunks = (N + kTcChunk - 1) / kTcChunk;
   const float* init_state = EXT ? init_state_arg : nullptr;
   const int chunks_per_seg = EXT ? chunks_per_seg_arg : total_chunks;
-  const int seg = EXT ? static_cast<int>(blockIdx.y) : 0;
+  const int seg = EXT ? seg_arg : 0;
   const int chunk0 = seg * chunks_per_seg;
   const int nchunks = EXT ? min(chunks_per_seg, total_chunks - chunk0) : total_chunks;
   const int last_chunk = chunk0 + nchunks - 1;
-  const bool has_init = EXT && init_state != nullptr && seg + 1 < static_cast<int>(gridDim.y);
+  const bool has_init = EXT && init_state != nullptr && seg + 1 < nsegs;
   const unsigned char* keep_b = (EXT && keep_arg) ? keep_arg + static_cast<size_t>(bh / H) * N : nullptr;
   const int* count_b = (EXT && count_arg) ? count_arg + static_cast<size_t>(bh / H) * N : nullptr;
   const long long rot_base = ROT ? static_cast<long long>(bb) * rot.batch_stride : 0;
@@ -1178,6 +1187,8 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       // Qw of the next chunk, while the accumulator MMAs of this one run
       if (ci + 1 < nchunks && !(ok = prepare(ci + 1))) break;
     }
+  } else if (!ROT && warp >= 15) {
+    // (causal_bwd_both_kernel launches more warps than this body has roles)
   } else if (ROT && warp >= 15) {
     // rotary group: the Q and K tiles of every stage, as soon as it has arrived
     const int wq = warp & 3;
@@ -1197,7 +1208,7 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     const int wq = warp & 3, row = 32 * wq + lane;
     const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
     if (has_init) {  // the state after this segment: fp32 into TMEM, 16-bit into the operand buffer of item 0
-      load_init_state<T>(init_state + (static_cast<size_t>(bh) * gridDim.y + seg) * (kTcD * kTcD), tR + lane_base, sR, wq, lane);
+      load_init_state<T>(init_state + (static_cast<size_t>(bh) * nsegs + seg) * (kTcD * kTcD), tR + lane_base, sR, wq, lane);
       tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before_sync();
@@ -1278,6 +1289,40 @@ causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
   }
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+template <typename T, bool EXT, bool ROT = false>
+__global__ void __launch_bounds__(ROT ? kKvThreadsRot : kKvThreads, 1)
+causal_bwd_kv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+                     const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
+                     const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV, float* __restrict__ dnorm,
+                     const float* __restrict__ norm_const, int H, int N, const float* __restrict__ init_state, int chunks_per_seg,
+                     const unsigned char* __restrict__ keep, const int* __restrict__ count, const RotArgs rot) {
+  causal_bwd_kv_body<T, EXT, ROT>(mapQ, mapK, mapV, mapDO, mapDK, mapDV, dnorm, norm_const, H, N, init_state, chunks_per_seg, keep, count, rot,
+                                  blockIdx.x, blockIdx.y, gridDim.y);
+}
+
+// Both halves of the backward in one launch: gridDim.y = 2 x segments, the dK/dV CTAs first (they take longer), then the
+// dQ CTAs, which fill the SMs that the former leave idle or finish early.  The two do not depend on each other; as two
+// launches each had its own last wave.  A CTA has the larger thread count and register budget of the two bodies.
+// Measured, backward: B 7, H 12, N 1531, masked fp16 63 -> 50 us; B 8, H 16, N 4096 137 -> 131; B 4, H 8, N 2048 70 -> 44;
+// B 1, H 4, N 200 19 -> 13.
+template <typename T, bool EXT>
+__global__ void __launch_bounds__(kTcThreads, 1)
+causal_bwd_both_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
+                       const __grid_constant__ CUtensorMap mapDQ, const __grid_constant__ CUtensorMap mapDK,
+                       const __grid_constant__ CUtensorMap mapDV, float* __restrict__ dnorm, const float* __restrict__ norm_const, int H, int N,
+                       const float* __restrict__ prefix, const float* __restrict__ suffix, int chunks_per_seg,
+                       const unsigned char* __restrict__ keep, const int* __restrict__ count) {
+  const RotArgs none{nullptr, nullptr, 0, 0};
+  const int nsegs = gridDim.y / 2, y = blockIdx.y;
+  if (y < nsegs)
+    causal_bwd_kv_body<T, EXT, false>(mapQ, mapK, mapV, mapDO, mapDK, mapDV, dnorm, norm_const, H, N, suffix, chunks_per_seg, keep, count, none,
+                                      blockIdx.x, y, nsegs);
+  else
+    causal_tc_body<T, kModeDq, EXT, false, false>(mapDO, mapV, mapK, mapQ, mapDQ, norm_const, H, N, prefix, chunks_per_seg, keep, count, nullptr,
+                                                  none, nullptr, blockIdx.x, y - nsegs, nsegs);
 }
 
 inline size_t causal_bwd_kv_smem_bytes() {

@@ -153,6 +153,30 @@ int launch_bwd_dkdv(const void* q, const void* k, const void* v, const float* nc
   return COTT_OK;
 }
 
+// dQ, dK, dV and the gradient of norm_const (zeroed by the caller) in one launch; `prefix` / `suffix`: the states of the
+// segments, null for one segment per sequence.
+template <typename T>
+int launch_bwd_both(const void* q, const void* k, const void* v, const float* nc, const void* dout, void* dq, void* dk, void* dv,
+                    float* dnorm, int B, int H, int N, int dtype, cudaStream_t stream, const float* prefix, const float* suffix, SegPlan plan) {
+  const long BH = (long)B * H;
+  CUtensorMap mq, mk, mv, md, mdq, mdk, mdv;
+  int st;
+  if ((st = tmap(&mq, q, dtype, B, H, N, qk_strides(plan, H, N))) || (st = tmap(&mk, k, dtype, B, H, N, qk_strides(plan, H, N))) ||
+      (st = tmap(&mv, v, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&md, dout, dtype, B, H, N, out_strides(plan, H, N))) ||
+      (st = tmap(&mdq, dq, dtype, B, H, N, in_strides(plan, H, N))) || (st = tmap(&mdk, dk, dtype, B, H, N, in_strides(plan, H, N))) ||
+      (st = tmap(&mdv, dv, dtype, B, H, N, in_strides(plan, H, N))))
+    return st;
+  const bool ext = plan.nseg > 1 || plan.keep;
+  auto kern = ext ? causal_bwd_both_kernel<T, true> : causal_bwd_both_kernel<T, false>;
+  const size_t a = causal_tc_smem_bytes(kModeDq), b = causal_bwd_kv_smem_bytes(), smem = a > b ? a : b;
+  COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (plan.cps == 0) plan.cps = plan_segments(N, 1).cps;
+  COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)BH, 2 * plan.nseg), kTcThreads, smem, stream, mq, mk, mv, md, mdq, mdk, mdv, dnorm, nc, H, N,
+                           prefix, suffix, plan.cps, plan.keep, plan.count));
+  COTT_CUDA_TRY(cudaGetLastError());
+  return COTT_OK;
+}
+
 // The one-pass backward: `saved` holds the forward's 16-bit state before every chunk ([B*H][chunks][64][64]).
 template <typename T>
 int launch_bwd_fused(const void* q, const void* k, const void* v, const float* nc, const void* dout, const void* saved,
@@ -255,21 +279,21 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
     plan.keep = keep;
     plan.count = reinterpret_cast<const int*>(ws + 5 * A);
   }
-  if (plan.nseg == 1) {
-    COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
+  COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
+  if (plan.nseg == 1 && plan.rot.sin) {  // (the rotation inside the kernels has a dK/dV kernel with a group of its own)
     plan.dnorm_zeroed = true;
     int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, nullptr, plan);
     return st ? st : launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
   }
-  // dQ: the forward prefix states (left in the workspace by the forward call), read transposed
-  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, ws + 2 * A, plan);
-  if (st) return st;
-  // dK, dV: reverse states of the segments, their exclusive suffix
+  if (plan.nseg == 1) return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, nullptr, plan);
+  // dQ: the forward prefix states (left in the workspace by the forward call), read transposed.  dK, dV: reverse states of
+  // the segments, their exclusive suffix.
+  int st;
   if ((st = launch_seg_state<T, kSegRevState>(q, dout, qk_strides(plan, H, N), out_strides(plan, H, N), nc, ws, B, H, N, dtype, plan,
                                               seg_parts(plan), stream)) ||
       (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream)))
     return st;
-  return launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, ws + 3 * A, plan);
+  return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 2 * A, ws + 3 * A, plan);
 }
 
 // The time-out path of the tensor-core kernels on its own: one CTA sets up what those kernels set up (an
@@ -765,16 +789,10 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
   DeviceScope scope(q);
   COTT_CUDA_TRY(scope.status());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the gradient of norm_const is zeroed before the dQ launch, so that the two kernels follow each other directly
   COTT_CUDA_TRY(cudaMemsetAsync(dnorm_const, 0, sizeof(float) * H, s));
-  SegPlan plan;
-  plan.dnorm_zeroed = true;
-  if (dtype == COTT_BF16) {
-    st = launch_bwd_dq<__nv_bfloat16>(q, k, v, norm_const, dout, dq, B, H, N, dtype, s, nullptr, plan);
-    return st ? st : launch_bwd_dkdv<__nv_bfloat16>(q, k, v, norm_const, dout, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, plan);
-  }
-  st = launch_bwd_dq<__half>(q, k, v, norm_const, dout, dq, B, H, N, dtype, s, nullptr, plan);
-  return st ? st : launch_bwd_dkdv<__half>(q, k, v, norm_const, dout, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, plan);
+  return dtype == COTT_BF16
+             ? launch_bwd_both<__nv_bfloat16>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, nullptr, SegPlan())
+             : launch_bwd_both<__half>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, nullptr, SegPlan());
 }
 
 int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N, 4); }
