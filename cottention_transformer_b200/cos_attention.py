@@ -61,7 +61,7 @@ class _FusedCausal(torch.autograd.Function):
         with torch.cuda.device(q.device):
             # few (batch, head) pairs and a long sequence: cut every sequence into segments that run on
             # different SMs (the library says how many for this device; 1 = not worth it)
-            nseg = L.cott_cos_attn_seg_count(B, H, N) if segments is None else int(segments)
+            nseg = L.cott_cos_attn_seg_choice(B, H, N) if segments is None else int(segments)
             kp = None if keep is None else keep.to(device=q.device, dtype=torch.uint8).contiguous()
             saved = None
             if one_pass:  # keep the 16-bit chunk states for the one-pass backward (cott_cos_attn_bwd_train)
@@ -137,7 +137,7 @@ class _FusedCausalPacked(torch.autograd.Function):
         code, stream = _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device)
         rqk = qlay = None
         with torch.cuda.device(qkv.device):
-            nseg = 1 if sin is not None else L.cott_cos_attn_seg_count(B, H, N)
+            nseg = 1 if sin is not None else L.cott_cos_attn_seg_choice(B, H, N)
             ws = torch.empty(L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg), dtype=torch.uint8, device=qkv.device)
             if sin is not None:  # rotated copies of q and k, [B, N, 2, H, D]
                 rqk = torch.empty(B, N, 2, H, D, dtype=qkv.dtype, device=qkv.device)
@@ -208,7 +208,7 @@ def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None):
         one_segment = m.seg_count(qkv, B, H, N) == 1
     else:
         with torch.cuda.device(qkv.device):
-            one_segment = _lib.lib().cott_cos_attn_seg_count(B, H, N) == 1
+            one_segment = _lib.lib().cott_cos_attn_seg_choice(B, H, N) == 1
     if (2 * sin.shape[-1]) % 16 or not one_segment:
         qkv = rotary_packed_(qkv.contiguous(), sin, cos)
         return m.causal_packed(qkv, norm_const, keep, None, None) if m is not None else _FusedCausalPacked.apply(qkv, norm_const, keep)

@@ -67,21 +67,23 @@ SegPlan plan_segments(int N, int nseg_requested) {
   return p;
 }
 
-// Segments per sequence for `units` independent sequences of N positions: one CTA per SM, at least two chunks each, and
-// only where it pays.  A pass over c chunks takes about c chunk periods; cut into segments of cps chunks it takes cps of
-// them, about half as long again for the segments' own states, and the launches and the prefix in between, which cost
-// `overhead` chunk periods.  (Measured, forward + backward, head dim 64: B 2, H 16, N 1024 in 4 segments of 2 chunks 75 us
-// against 51 us in one; B 4, H 8, N 2048 in 4 segments of 4 chunks 66 us against 90 us; B 1, H 16, N 8192 in 9 of 8 97 against 310.)
-int seg_count(long units, int N, int overhead) {
+// Segments per sequence that `units` independent sequences of N positions can use: one CTA per SM, at least two chunks each.
+int seg_count(long units, int N) {
   const int total = (N + kTcChunk - 1) / kTcChunk;
   if (units <= 0 || total < 4) return 1;
   int sm = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-  long nseg = sm / units;
+  long nseg = sm / units;  // more sequences than half the SMs: no gain
   if (nseg > total / 2) nseg = total / 2;
-  if (nseg < 2) return 1;
-  const long cps = (total + nseg - 1) / nseg;
-  return 2 * total > 3 * cps + 2 * overhead ? (int)nseg : 1;
+  return nseg < 2 ? 1 : (int)nseg;
+}
+// ... and what pays: a pass over c chunks takes about c chunk periods; cut into segments of cps chunks it takes cps of
+// them, about half as long again for the segments' own states, and the launches and the prefix in between, which cost
+// `overhead` chunk periods.  (Measured, forward + backward, head dim 64, segments against one: B 2, H 16, N 1024 in 4 of 2
+// chunks 51 us against 38; B 4, H 8, N 2048 in 4 of 4 64 against 64; B 1, H 16, N 8192 in 9 of 8 97 against 216.)
+int seg_choice(long units, int N, int overhead) {
+  const int nseg = seg_count(units, N), total = (N + kTcChunk - 1) / kTcChunk, cps = (total + nseg - 1) / nseg;
+  return 2 * total > 3 * cps + 2 * overhead ? nseg : 1;
 }
 
 template <typename T>
@@ -407,7 +409,7 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
 
 size_t wide_ws_floats(int B, int H, int N, int dz, int nseg) { return (size_t)B * H * plan_segments(N, nseg).nseg * (size_t)(kTcChunk * dz); }
 
-int wide_seg_count(int B, int H, int N, int dz) { return seg_count((long)B * H * (dz / wide_width(dz)), N, 3); }
+int wide_seg_count(int B, int H, int N, int dz) { return seg_choice((long)B * H * (dz / wide_width(dz)), N, 3); }
 
 // workspace of the fused head-dim-128 pair: the prefix states of the forward-direction passes and those of the reversed
 // ones (first: they are read as 16-byte words), then four fp32 vectors [B*H*N] (1/|q|, 1/|k|, keep a/|k|, -eps/|k|^2) and
@@ -665,7 +667,7 @@ int launch_scan_tc_wide(const void* q, const void* k, const void* v, void* out, 
   const T *qq = static_cast<const T*>(q), *kk = static_cast<const T*>(k), *vv = static_cast<const T*>(v);
   T* oo = static_cast<T*>(out);
   // few (batch, head) pairs and a long sequence: several CTAs per sequence, as in the fused path
-  const SegPlan plan = plan_segments(N, cott_cos_attn_seg_count(B, H, N));
+  const SegPlan plan = plan_segments(N, cott_cos_attn_seg_choice(B, H, N));
   const size_t ws_bytes = plan.nseg > 1 ? 3 * seg_array_floats(B, H, plan.nseg) * sizeof(float) : 0;
   const size_t tmp_bytes = Dk > kTcD ? sizeof(T) * rows * kTcD : 0;
   char* scratch = nullptr;  // stream-ordered: segment states, then the partial result of the slices I > 0
@@ -795,7 +797,8 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
              : launch_bwd_both<__half>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, nullptr, SegPlan());
 }
 
-int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N, 4); }
+int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N); }
+int cott_cos_attn_seg_choice(int B, int H, int N) { return seg_choice((long)B * H, N, 10); }
 
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;

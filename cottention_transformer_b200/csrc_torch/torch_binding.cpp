@@ -98,7 +98,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> causal_fwd(const at::Tensor& q, c
   at::Tensor nc = nc_f32(norm_const, q, H);
   at::Tensor out = at::empty_like(v);
   const auto bytes = q.options().dtype(at::kByte);
-  if (nseg <= 0) nseg = cott_cos_attn_seg_count(B, H, N);
+  if (nseg <= 0) nseg = cott_cos_attn_seg_choice(B, H, N);
   const bool general = nseg > 1 || (keep.has_value() && keep->defined());
   at::Tensor ws = at::empty({general ? (int64_t)std::max<size_t>(cott_cos_attn_seg_workspace_bytes(B, H, N, (int)nseg), 16) : 0}, bytes);
   at::Tensor saved = at::empty({save_states ? (int64_t)std::max<size_t>(cott_cos_attn_saved_bytes(B, H, N), 16) : 0}, bytes);
@@ -131,7 +131,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> causal_bwd(const at::
   at::Tensor dnc = at::empty({H}, q.options().dtype(at::kFloat));
   const unsigned char* kp = static_cast<const unsigned char*>(ptr_or_null(keep));
   void* wsp = ws.numel() ? ws.data_ptr() : nullptr;
-  if (nseg <= 0) nseg = cott_cos_attn_seg_count(B, H, N);  // the forward's choice for the same sizes on the same device
+  if (nseg <= 0) nseg = cott_cos_attn_seg_choice(B, H, N);  // the forward's choice for the same sizes on the same device
   if (saved.numel())
     check(cott_cos_attn_bwd_train(q.data_ptr(), k.data_ptr(), v.data_ptr(), kp, nc.data_ptr<float>(), dout.data_ptr(), saved.data_ptr(), wsp,
                                   (int)nseg, nullptr, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dnc.data_ptr<float>(), B, H, N, D, D,
@@ -277,7 +277,7 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
     at::Tensor out = at::empty({p.B, p.N, p.H, p.D}, p.qkv.options());
     const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
     const bool rot = has(sin);
-    const int nseg = rot ? 1 : cott_cos_attn_seg_count(B, H, N);
+    const int nseg = rot ? 1 : cott_cos_attn_seg_choice(B, H, N);
     at::Tensor ws = bytes_like(p.qkv, cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
     at::Tensor rqk;  // the rotated q and k, [B, N, 2, H, D]
     if (rot) {
@@ -430,7 +430,7 @@ at::Tensor prefill(const at::Tensor& state, const at::Tensor& q_, const at::Tens
   const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
   const c10::cuda::CUDAGuard guard(q.device());
   const at::Tensor nc = nc_f32(norm_const, q, H);
-  const int nseg = D == 128 ? 1 : cott_cos_attn_seg_count(B, H, N);
+  const int nseg = D == 128 ? 1 : cott_cos_attn_seg_choice(B, H, N);
   at::Tensor out = at::empty_like(v);
   const at::Tensor ws = bytes_like(q, D == 128 ? cott_cos_attn_wide_workspace_bytes(B, H, N) : cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
   check(cott_cos_attn_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), nc.data_ptr<float>(), out.data_ptr(), state.data_ptr<float>(),
@@ -541,7 +541,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("_raise_for_status", [](int status) { check(status, "cottention_b200"); }, py::arg("status"));
   m.def("seg_count", [](const at::Tensor& t, int64_t B, int64_t H, int64_t N) {
     const c10::cuda::CUDAGuard guard(t.device());
-    return cott_cos_attn_seg_count((int)B, (int)H, (int)N);
+    return cott_cos_attn_seg_choice((int)B, (int)H, (int)N);
   });
   m.def("cos_attn_causal", &cos_attn_causal);
   m.def("cos_attn_wide", &cos_attn_wide);

@@ -44,7 +44,7 @@ class CosAttnDecodeState:
             raise RuntimeError(f"norm_const must have one entry per head ({H}), got {nc.numel()}")
         out = torch.empty_like(v)
         with torch.cuda.device(q.device):
-            nseg = 1 if wide else L.cott_cos_attn_seg_count(B, H, T)
+            nseg = 1 if wide else L.cott_cos_attn_seg_choice(B, H, T)
             nbytes = L.cott_cos_attn_wide_workspace_bytes(B, H, T) if wide else L.cott_cos_attn_seg_workspace_bytes(B, H, T, nseg)
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
             st = L.cott_cos_attn_prefill(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(self.state),

@@ -149,6 +149,9 @@ typedef struct cott_layout { /* element strides of [B, H, N, 64] views whose inn
   long long out_b, out_h, out_n; /* out and dout */
 } cott_layout;
 int cott_cos_attn_seg_count(int B, int H, int N);
+/* The count that is worth it for these sizes: the one above for long sequences, 1 where cutting a sequence costs more
+ * than it saves.  The operators of the Python package and cott_scan go by this one. */
+int cott_cos_attn_seg_choice(int B, int H, int N);
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg);
 int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
                           const float* norm_const, void* out, void* workspace, int nseg,
