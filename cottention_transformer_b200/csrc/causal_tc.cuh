@@ -1325,6 +1325,27 @@ causal_bwd_both_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_co
                                                   none, nullptr, blockIdx.x, y - nsegs, nsegs);
 }
 
+// The three scans of CustomAttention's backward (Custom_Kernel.py:106-108) in one launch: gridDim.y = 3,
+//   0: dq = scan(dO, V, K)   1: dk = scan_rev(V, dO, Q)   2: dv = scan_rev(K, Q, dO)
+// They do not depend on each other; as three launches of B*H CTAs each had its own ramp and last wave.
+// Measured, B 8, H 16, N 1024 in bf16: the operator forward and backward 75 -> 70 us a pass (four kernels of 15.5 us before).
+template <typename T>
+__global__ void __launch_bounds__(kTcThreads, 1)
+causal_scan_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
+                       const __grid_constant__ CUtensorMap mapDQ, const __grid_constant__ CUtensorMap mapDK,
+                       const __grid_constant__ CUtensorMap mapDV, int H, int N) {
+  const RotArgs none{nullptr, nullptr, 0, 0};
+  if (blockIdx.y == 0) {
+    causal_tc_body<T, kModeScan, false, false, false>(mapDO, mapV, mapK, mapDO, mapDQ, nullptr, H, N, nullptr, 0, nullptr, nullptr, nullptr, none,
+                                                      nullptr, blockIdx.x, 0, 1);
+  } else {
+    const bool dk = blockIdx.y == 1;
+    causal_tc_body<T, kModeScanRev, false, false, false>(dk ? mapV : mapK, dk ? mapDO : mapQ, dk ? mapQ : mapDO, mapQ, dk ? mapDK : mapDV, nullptr, H,
+                                                         N, nullptr, 0, nullptr, nullptr, nullptr, none, nullptr, blockIdx.x, 0, 1);
+  }
+}
+
 inline size_t causal_bwd_kv_smem_bytes() {
   return static_cast<size_t>(kTcStages * 4 * kTileBytes + 2 * kTcD * 128 + 1024);
 }

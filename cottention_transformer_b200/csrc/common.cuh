@@ -131,6 +131,10 @@ bool bidir_tc_usable(int Dk, int Dv, int dtype, std::initializer_list<const void
 bool scan_tc_usable(int Dk, int Dv, int dtype, const void* q, const void* k, const void* v, const void* out);
 int launch_scan_tc(const void* q, const void* k, const void* v, void* out, int B, int H, int N, int Dk, int Dv, int dtype,
                    int reversed, cudaStream_t stream);
+bool scan_bwd_tc_usable(int B, int H, int N, int Dk, int Dv, int dtype, std::initializer_list<const void*> in,
+                        std::initializer_list<const void*> out);
+int launch_scan_bwd_tc(const void* q, const void* k, const void* v, const void* dout, void* dq, void* dk, void* dv, int B, int H, int N,
+                       int dtype, cudaStream_t stream);
 int launch_bidir_fwd_tc(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc,
                         void* out, int B, int H, int N, int dtype, cudaStream_t stream, const cott_layout* layout = nullptr);
 int launch_bidir_bwd_tc(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc,

@@ -708,6 +708,46 @@ int launch_scan_tc(const void* q, const void* k, const void* v, void* out, int B
                             : launch_scan_tc_wide<__half>(q, k, v, out, B, H, N, Dk, Dv, dtype, reversed, stream);
 }
 
+// The three scans of the backward in one launch (head dim 64, one segment per sequence).
+bool scan_bwd_tc_usable(int B, int H, int N, int Dk, int Dv, int dtype, std::initializer_list<const void*> in,
+                        std::initializer_list<const void*> out) {
+  if (Dk != kTcD || Dv != kTcD || (dtype != COTT_BF16 && dtype != COTT_F16) || 3l * B * H > 0x7fffffffL) return false;
+  for (const void* o : out) {  // (an output over an input, or over another output: one scan after the other)
+    if (reinterpret_cast<uintptr_t>(o) & 15) return false;
+    for (const void* i : in)
+      if (o == i) return false;
+    int same = 0;
+    for (const void* p : out) same += p == o;
+    if (same > 1) return false;
+  }
+  for (const void* i : in)
+    if (reinterpret_cast<uintptr_t>(i) & 15) return false;
+  return cott_cos_attn_seg_choice(B, H, N) == 1;
+}
+
+template <typename T>
+int launch_scan_bwd_tc_t(const void* q, const void* k, const void* v, const void* dout, void* dq, void* dk, void* dv, int B, int H, int N,
+                         int dtype, cudaStream_t stream) {
+  const TileStrides dense = contiguous_bhnd(H, N);
+  CUtensorMap mq, mk, mv, md, mdq, mdk, mdv;
+  int st;
+  if ((st = tmap(&mq, q, dtype, B, H, N, dense)) || (st = tmap(&mk, k, dtype, B, H, N, dense)) || (st = tmap(&mv, v, dtype, B, H, N, dense)) ||
+      (st = tmap(&md, dout, dtype, B, H, N, dense)) || (st = tmap(&mdq, dq, dtype, B, H, N, dense)) ||
+      (st = tmap(&mdk, dk, dtype, B, H, N, dense)) || (st = tmap(&mdv, dv, dtype, B, H, N, dense)))
+    return st;
+  auto kern = causal_scan_bwd_kernel<T>;
+  const size_t smem = causal_tc_smem_bytes(kModeScan);
+  COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)((long)B * H), 3), kTcThreads, smem, stream, mq, mk, mv, md, mdq, mdk, mdv, H, N));
+  COTT_CUDA_TRY(cudaGetLastError());
+  return COTT_OK;
+}
+int launch_scan_bwd_tc(const void* q, const void* k, const void* v, const void* dout, void* dq, void* dk, void* dv, int B, int H, int N,
+                       int dtype, cudaStream_t stream) {
+  return dtype == COTT_BF16 ? launch_scan_bwd_tc_t<__nv_bfloat16>(q, k, v, dout, dq, dk, dv, B, H, N, dtype, stream)
+                            : launch_scan_bwd_tc_t<__half>(q, k, v, dout, dq, dk, dv, B, H, N, dtype, stream);
+}
+
 bool bidir_tc_usable(int Dk, int Dv, int dtype, std::initializer_list<const void*> tensors) {
   if (Dk != kTcD || Dv != kTcD || (dtype != COTT_BF16 && dtype != COTT_F16)) return false;
   for (const void* p : tensors)

@@ -80,6 +80,8 @@ int cott_scan_bwd(const void* q, const void* k, const void* v, const void* dout,
   DeviceScope scope(q);
   COTT_CUDA_TRY(scope.status());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (scan_bwd_tc_usable(B, H, N, Dk, Dv, dtype, {q, k, v, dout}, {dq, dk, dv}))
+    return launch_scan_bwd_tc(q, k, v, dout, dq, dk, dv, B, H, N, dtype, s);
   // dq = scan(dout, v, k): "Q"=dout [Dv], "K"=v [Dv], "V"=k [Dk]
   st = scan_dispatch(dout, v, k, dq, B, H, N, Dv, Dk, dtype, 0, s);
   if (st != COTT_OK) return st;

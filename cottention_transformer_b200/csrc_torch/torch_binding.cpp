@@ -406,6 +406,16 @@ struct CustomAttentionFn : torch::autograd::Function<CustomAttentionFn> {
     const variable_list s = ctx->get_saved_variables();
     const at::Tensor Q = s[0].contiguous(), K = s[1].contiguous(), V = s[2].contiguous(), g = grads[0].contiguous();
     const at::ScalarType t = Q.scalar_type();
+    // one dtype and one shape in 16 bits: the three scans in one C call (autocast only ever concerns fp32 tensors)
+    if ((t == at::kHalf || t == at::kBFloat16) && K.scalar_type() == t && V.scalar_type() == t && g.scalar_type() == t && Q.dim() == 4 &&
+        Q.sizes() == K.sizes() && Q.sizes() == V.sizes() && Q.sizes() == g.sizes() && Q.size(3) == 64) {
+      const c10::cuda::CUDAGuard guard(Q.device());
+      at::Tensor dq = at::empty_like(Q), dk = at::empty_like(K), dv = at::empty_like(V);
+      check(cott_scan_bwd(Q.data_ptr(), K.data_ptr(), V.data_ptr(), g.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (int)Q.size(0),
+                          (int)Q.size(1), (int)Q.size(2), 64, 64, dtype_code(t), stream_of(Q)),
+            "cott_scan_bwd");
+      return {dq, dk, dv};
+    }
     return {scan_by_dtype(t, g, V, K, false), scan_by_dtype(t, V, g, Q, true), scan_by_dtype(t, K, Q, g, true)};
   }
 };
