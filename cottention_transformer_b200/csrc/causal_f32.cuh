@@ -11,8 +11,10 @@
 // chain with other operands:
 //   out: A = q^  B = k^  C = v'  M = S       dq: A = dO  B = v'  C = k^  M = S^T
 //   dk:  A = v'  B = dO  C = q^  M = R^T     dv: A = k^  B = q^  C = dO  M = R
+// All of them are launched with programmatic dependent launch (common.cuh): seven short kernels in a row (113 -> 108 us a step
+// at the sizes below).
 // Bound by the fp32 FMA rate and the staging before it (256 CTAs at B 2, H 8, N 1024: 3 x 64^3 multiply-adds each).
-// Measured there, forward + backward: 158 us a step, 114 us of it in these seven launches (11 + 7 + 22 | 10 + 7 + 54 + 3);
+// Measured there, forward + backward: 108 us a step (11 + 7 + 22 | 10 + 7 + 54 + 3 one by one);
 // four exact scans with one CTA per sequence (16 of 148 SMs busy, 236 us each) between fifty elementwise passes took 1206 us.
 #pragma once
 
@@ -136,6 +138,8 @@ f32_state_kernel(const float* __restrict__ y, const float* __restrict__ z, const
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const long bh = blockIdx.x / nchunks;
   const int c0 = static_cast<int>(blockIdx.x % nchunks) * kF32Chunk, h = static_cast<int>(bh % H);
+  pdl_allow_next();
+  pdl_wait_prior();
   const float sigma = 1.0f / (1.0f + expf(-norm_const[h]));
   f32_rows(rows, keep ? keep + (bh / H) * N : nullptr, c0, N, sigma);
   f32_stage<D, kF32Norm>(sY, y + bh * N * D, rows, c0, N, tx, ty);
@@ -162,6 +166,8 @@ f32_state_kernel(const float* __restrict__ y, const float* __restrict__ z, const
 template <bool REV>
 __global__ void __launch_bounds__(kF32Threads) f32_prefix_kernel(float* __restrict__ state, int nchunks, int elems) {
   float* p = state + static_cast<long>(blockIdx.x) * nchunks * elems + blockIdx.y * kF32Threads + threadIdx.x;
+  pdl_allow_next();
+  pdl_wait_prior();
   float run = 0.f;
   for (int c = 0; c < nchunks; c += 8) {
     float x[8];
@@ -392,6 +398,8 @@ __global__ void __launch_bounds__(kF32Threads, 3) f32_chunk_kernel(const F32Args
   float* sC = sB + kF32Chunk * (D + 4);
   float* sP = sC + kF32Chunk * (D + 4);
   __shared__ F32Rows rows;
+  pdl_allow_next();
+  pdl_wait_prior();
   if constexpr (FWD) {
     f32_chunk<D, kF32Out>(g, sA, sB, sC, sP, rows);
   } else {
@@ -409,6 +417,8 @@ __global__ void __launch_bounds__(kF32Threads)
 f32_dnorm_kernel(const double* __restrict__ gpart, const float* __restrict__ norm_const, float* __restrict__ dnorm, int B, int H, int nchunks) {
   const int h = blockIdx.x;
   __shared__ double part[kF32Threads / 32];
+  pdl_allow_next();
+  pdl_wait_prior();
   double s = 0.0;
   for (int i = threadIdx.x; i < B * nchunks; i += kF32Threads) s += gpart[(static_cast<long>(i / nchunks) * H + h) * nchunks + i % nchunks];
 #pragma unroll

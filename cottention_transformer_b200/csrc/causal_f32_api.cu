@@ -26,10 +26,9 @@ int launch_f32_states(const float* y, const float* z, const unsigned char* keep,
                       cudaStream_t stream) {
   const int nch = f32_chunks(N);
   const unsigned grid = (unsigned)((long)B * H * nch);
-  f32_state_kernel<D, REV><<<grid, kF32Threads, 2 * kF32Chunk * (D + 4) * sizeof(float), stream>>>(y, z, keep, nc, state, H, N, nch);
-  COTT_CUDA_TRY(cudaGetLastError());
-  f32_prefix_kernel<REV><<<dim3((unsigned)((long)B * H), D * D / kF32Threads), kF32Threads, 0, stream>>>(state, nch, D * D);
-  COTT_CUDA_TRY(cudaGetLastError());
+  COTT_CUDA_TRY(launch_pdl(f32_state_kernel<D, REV>, dim3(grid), kF32Threads, 2 * kF32Chunk * (D + 4) * sizeof(float), stream, y, z, keep, nc,
+                           state, H, N, nch));
+  COTT_CUDA_TRY(launch_pdl(f32_prefix_kernel<REV>, dim3((unsigned)((long)B * H), D * D / kF32Threads), kF32Threads, 0, stream, state, nch, D * D));
   return COTT_OK;
 }
 
@@ -38,8 +37,7 @@ int launch_f32_chunks(const F32Args& g, int B, cudaStream_t stream) {
   const size_t smem = (3 * kF32Chunk * (D + 4) + kF32Chunk * (kF32Chunk + 4)) * sizeof(float);
   auto kern = f32_chunk_kernel<D, FWD>;
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3((unsigned)((long)B * g.H * g.nchunks), FWD ? 1 : 3), kF32Threads, smem, stream>>>(g);
-  COTT_CUDA_TRY(cudaGetLastError());
+  COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)((long)B * g.H * g.nchunks), FWD ? 1 : 3), kF32Threads, smem, stream, g));
   return COTT_OK;
 }
 
@@ -60,8 +58,8 @@ int run_f32_bwd(F32Args g, const float* fwd_ws, float* ws, float* dnorm, int B, 
   g.suffix = ws;
   g.gpart = reinterpret_cast<double*>(ws + A);
   if ((st = launch_f32_chunks<D, false>(g, B, stream))) return st;
-  f32_dnorm_kernel<<<(unsigned)g.H, kF32Threads, 0, stream>>>(g.gpart, g.norm_const, dnorm, B, g.H, g.nchunks);
-  COTT_CUDA_TRY(cudaGetLastError());
+  COTT_CUDA_TRY(launch_pdl(f32_dnorm_kernel, dim3((unsigned)g.H), kF32Threads, 0, stream, static_cast<const double*>(g.gpart), g.norm_const, dnorm, B,
+                           g.H, g.nchunks));
   return COTT_OK;
 }
 

@@ -36,6 +36,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
 
+  pdl_allow_next();
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int bh = blockIdx.x, h = bh % H, bb = bh / H, seg = blockIdx.y;
@@ -67,6 +68,7 @@ seg_state_kernel(const __grid_constant__ CUtensorMap mapY, const __grid_constant
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait_prior();  // nothing another kernel may have written has been read so far
   const uint32_t tS = tmem_slot;
   constexpr uint32_t kIdescS = make_idesc(64, 64, BF, true, true);
 
@@ -161,6 +163,8 @@ inline size_t seg_state_smem_bytes() { return static_cast<size_t>(4 * kTileBytes
 // Measured: 16 x 9 matrices of 16 KB in 6 us (one block per sequence, one load at a time and a transposed copy: 31 us).
 template <bool REV>
 __global__ void __launch_bounds__(64) seg_prefix_kernel(const float4* src, float4* dst, int nseg, int parts, int quads) {
+  pdl_allow_next();
+  pdl_wait_prior();
   const int e = blockIdx.y * 64 + threadIdx.x;
   if (e >= quads) return;
   const int n = nseg * parts;
@@ -199,6 +203,8 @@ __global__ void seg_to_decode_state_kernel(const float* __restrict__ seg_state, 
 // count[b][s] = number of kept positions among 0 .. s of batch entry b (inclusive).  grid = B, block = 256.
 __global__ void keep_count_kernel(const unsigned char* __restrict__ keep, int* __restrict__ count, int N) {
   __shared__ int part[256];
+  pdl_allow_next();
+  pdl_wait_prior();
   const unsigned char* kb = keep + static_cast<size_t>(blockIdx.x) * N;
   int* cb = count + static_cast<size_t>(blockIdx.x) * N;
   const int per = (N + blockDim.x - 1) / blockDim.x;

@@ -221,8 +221,8 @@ int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides s
   auto kern = seg_state_kernel<T, MODE>;
   const size_t smem = seg_state_smem_bytes();
   COTT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3((unsigned)BH, plan.nseg * parts), kSegThreads, smem, stream>>>(my, mz, nc, state, H, N, plan.cps, parts, plan.keep, plan.count);
-  COTT_CUDA_TRY(cudaGetLastError());
+  COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)BH, plan.nseg * parts), kSegThreads, smem, stream, my, mz, nc, state, H, N, plan.cps, parts,
+                           plan.keep, plan.count));
   return COTT_OK;
 }
 
@@ -232,9 +232,8 @@ int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides s
 size_t seg_array_floats(int B, int H, int nseg) { return (size_t)B * H * nseg * kTcD * kTcD; }
 int launch_seg_prefix(const float* src, float* dst, long sequences, int nseg, int parts, int elems, bool reverse, cudaStream_t stream) {
   auto kern = reverse ? seg_prefix_kernel<true> : seg_prefix_kernel<false>;
-  kern<<<dim3((unsigned)sequences, (unsigned)((elems / 4 + 63) / 64)), 64, 0, stream>>>(reinterpret_cast<const float4*>(src),
-                                                                                       reinterpret_cast<float4*>(dst), nseg, parts, elems / 4);
-  COTT_CUDA_TRY(cudaGetLastError());
+  COTT_CUDA_TRY(launch_pdl(kern, dim3((unsigned)sequences, (unsigned)((elems / 4 + 63) / 64)), 64, 0, stream, reinterpret_cast<const float4*>(src),
+                           reinterpret_cast<float4*>(dst), nseg, parts, elems / 4));
   return COTT_OK;
 }
 
@@ -256,8 +255,7 @@ int run_fwd_seg(const void* q, const void* k, const void* v, const unsigned char
   const size_t A = seg_array_floats(B, H, plan.nseg);
   if (keep) {  // running count of the kept positions, behind the state arrays
     int* count = reinterpret_cast<int*>(ws + 5 * A);
-    keep_count_kernel<<<(unsigned)B, 256, 0, stream>>>(keep, count, N);
-    COTT_CUDA_TRY(cudaGetLastError());
+    COTT_CUDA_TRY(launch_pdl(keep_count_kernel, dim3((unsigned)B), 256, 0, stream, keep, count, N));
     plan.keep = keep;
     plan.count = count;
   }
@@ -435,8 +433,7 @@ int run_wide_fwd(const void* q, const void* k, const void* v, const unsigned cha
   if (!decode_state) a.rq_out = ws.rq, a.rk_out = ws.rk, a.w_out = ws.w;  // (a prompt has no backward)
   a.decode_state = decode_state;
   if (keep) {
-    keep_count_kernel<<<(unsigned)B, 256, 0, stream>>>(keep, ws.count, N);
-    COTT_CUDA_TRY(cudaGetLastError());
+    COTT_CUDA_TRY(launch_pdl(keep_count_kernel, dim3((unsigned)B), 256, 0, stream, keep, ws.count, N));
     a.keep = keep, a.count = ws.count;
   }
   WideTensors t{q, k, v, nullptr, out, 128};

@@ -42,6 +42,8 @@ template <typename T, typename I>
 __global__ void __launch_bounds__(256)
 rotary_kernel(const T* q, const T* k, T* oq, T* ok, const float* __restrict__ sin_t, const float* __restrict__ cos_t, RotStrides si,
               RotStrides so, int B, I H, I N, I pieces, I all, long long table_batch_stride, float sign, bool h_inner) {
+  pdl_allow_next();  // (the causal kernels that follow set themselves up meanwhile)
+  pdl_wait_prior();
   const I idx = static_cast<I>(blockIdx.x) * 256 + threadIdx.x;
   if (idx >= H * N * all) return;
   const I row = idx / all, p = idx - row * all;
@@ -82,12 +84,12 @@ int launch_rotary(const void* q, const void* k, void* oq, void* ok, const float*
   const T *qt = static_cast<const T*>(q), *kt = static_cast<const T*>(k);
   T *oqt = static_cast<T*>(oq), *okt = static_cast<T*>(ok);
   if (per + 256 < (1ull << 32))
-    rotary_kernel<T, unsigned><<<grid, 256, 0, stream>>>(qt, kt, oqt, okt, sin_t, cos_t, si, so, B, H, N, pieces, all, table_batch_stride,
-                                                         sign, h_inner);
+    COTT_CUDA_TRY(launch_pdl(rotary_kernel<T, unsigned>, grid, 256, 0, stream, qt, kt, oqt, okt, sin_t, cos_t, si, so, B, (unsigned)H, (unsigned)N,
+                             (unsigned)pieces, (unsigned)all, table_batch_stride, sign, h_inner));
   else
-    rotary_kernel<T, unsigned long long><<<grid, 256, 0, stream>>>(qt, kt, oqt, okt, sin_t, cos_t, si, so, B, H, N, pieces, all,
-                                                                   table_batch_stride, sign, h_inner);
-  COTT_CUDA_TRY(cudaGetLastError());
+    COTT_CUDA_TRY(launch_pdl(rotary_kernel<T, unsigned long long>, grid, 256, 0, stream, qt, kt, oqt, okt, sin_t, cos_t, si, so, B,
+                             (unsigned long long)H, (unsigned long long)N, (unsigned long long)pieces, (unsigned long long)all,
+                             table_batch_stride, sign, h_inner));
   return COTT_OK;
 }
 
