@@ -354,30 +354,34 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
       }
     }
   } else {
-    // dv = dv' / div;  the gradient of norm_const collects ln(n) (v' . dv')
+    // dv = dv' / div;  the gradient of norm_const collects ln(n) (v' . dv').  A sum of terms of both signs: its rows are
+    // added up in fp64.
     double gsum = 0.0;
+    double* ln = reinterpret_cast<double*>(sP);  // (the scores have been read)
+    __syncthreads();
+    if (tid < kF32Chunk) ln[tid] = rows.n[tid] > 1.f ? log(static_cast<double>(rows.n[tid])) : 0.0;
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int t = ty + 16 * r;
       const bool in = c0 + t < N;
       const long o = base + static_cast<long>(c0 + t) * D + NB * tx;
       const float d = rows.div[t], n = rows.n[t], take = rows.take[t];
-      float v[NB] = {}, dot = 0.f;
+      float v[NB] = {};
+      double dot = 0.0;
       if (in) f32_load<NB>(v, g.v + o);
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
         acc[r][j] *= take;
-        dot = fmaf(v[j] / d, acc[r][j], dot);
+        dot = fma(static_cast<double>(v[j] / d), static_cast<double>(acc[r][j]), dot);
         acc[r][j] /= d;
       }
-      dot = f32_row_sum(dot);
-      if (in && n > 1.f) gsum += static_cast<double>(logf(n)) * dot;
+      if (in && n > 1.f) gsum += ln[t] * dot;
       if (in) f32_store<NB>(g.dv + o, acc[r]);
     }
-    // rows of a warp: ty = 2 (warp) + (lane / 16); every lane of a row holds the same sum
-    gsum += __shfl_xor_sync(0xffffffffu, gsum, 16);
-    double* part = reinterpret_cast<double*>(sP);  // (the scores have been read: the sync below comes first)
-    __syncthreads();
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, off);
+    double* part = ln + kF32Chunk;
     if ((tid & 31) == 0) part[tid >> 5] = gsum;
     __syncthreads();
     if (tid == 0) {
@@ -428,7 +432,7 @@ f32_dnorm_kernel(const double* __restrict__ gpart, const float* __restrict__ nor
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < kF32Threads / 32; ++w) t += part[w];
-    const double sigma = 1.0f / (1.0f + expf(-norm_const[h]));
+    const double sigma = 1.0 / (1.0 + exp(-static_cast<double>(norm_const[h])));
     dnorm[h] = static_cast<float>(-sigma * (1.0 - sigma) * t);
   }
 }
