@@ -38,9 +38,18 @@ def fused_supported(q, k, v, keep=None) -> bool:
     )
 
 
+def check_bhnd(q, k, v):
+    """``[B, H, N, D]`` tensors of one shape: the C side takes the sizes from q alone."""
+    if q.dim() != 4:
+        raise ValueError(f"[B, H, N, D] tensors expected, got {q.dim()} dimensions")
+    if k.shape != q.shape or v.shape != q.shape:
+        raise RuntimeError(f"q, k and v must have the same shape, got {list(q.shape)}, {list(k.shape)} and {list(v.shape)}")
+
+
 class _FusedCausal(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, norm_const, segments=None, keep=None, one_pass=False):
+        check_bhnd(q, k, v)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         B, H, N, D = q.shape
         ops = _binding.ops()
@@ -273,6 +282,7 @@ class _FusedWide128(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, norm_const, keep):
+        check_bhnd(q, k, v)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         B, H, N, D = q.shape
         L = _lib.lib()

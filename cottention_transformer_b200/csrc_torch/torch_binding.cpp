@@ -206,6 +206,12 @@ at::Tensor nc_grad(const at::Tensor& dnc, at::IntArrayRef shape, at::ScalarType 
   at::Tensor g = dnc.reshape(shape);
   return g.scalar_type() == dtype ? g : g.to(dtype);
 }
+// [B, H, N, D] tensors of one shape: the C side takes the sizes from q alone
+void check_bhnd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v) {
+  if (q.dim() != 4) throw py::value_error("[B, H, N, D] tensors expected, got " + std::to_string(q.dim()) + " dimensions");
+  TORCH_CHECK(k.sizes() == q.sizes() && v.sizes() == q.sizes(), "q, k and v must have the same shape, got ", q.sizes(), ", ", k.sizes(), " and ",
+              v.sizes());
+}
 at::Tensor bytes_like(const at::Tensor& t, size_t n) { return at::empty({(int64_t)std::max<size_t>(n, 16)}, t.options().dtype(at::kByte)); }
 const unsigned char* u8(const OptTensor& t) { return static_cast<const unsigned char*>(ptr_or_null(t)); }
 at::Tensor dense_as(const at::Tensor& t, at::ScalarType dtype) {
@@ -231,6 +237,7 @@ OptTensor load_opt(AutogradContext* ctx, const char* key) {
 struct CausalFn : torch::autograd::Function<CausalFn> {
   static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
                           const OptTensor& keep, int64_t nseg, bool one_pass) {
+    check_bhnd(q_, k_, v_);
     const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
     const OptTensor kp = keep_u8(keep, q);
     auto [out, ws, saved] = causal_fwd(q, k, v, norm_const, kp, nseg, one_pass);
@@ -364,6 +371,7 @@ struct BidirPackedFn : torch::autograd::Function<BidirPackedFn> {
 struct WideFn : torch::autograd::Function<WideFn> {
   static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
                           const OptTensor& keep) {
+    check_bhnd(q_, k_, v_);
     const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
     const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
     const c10::cuda::CUDAGuard guard(q.device());
@@ -425,6 +433,9 @@ at::Tensor decode_steps(const at::Tensor& state, const at::Tensor& q_, const at:
                         int64_t pos) {
   const at::Tensor q = q_.contiguous(), k = dense_as(k_.scalar_type() == q.scalar_type() ? k_ : k_.to(q.scalar_type()), q.scalar_type()),
                    v = dense_as(v_.scalar_type() == q.scalar_type() ? v_ : v_.to(q.scalar_type()), q.scalar_type());
+  TORCH_CHECK(k.numel() == q.numel() && v.numel() == q.size(0) * q.size(1) * q.size(2) * v.size(3) &&
+                  state.numel() >= q.size(0) * q.size(1) * v.size(3) * q.size(3),
+              "q, k, v and the state do not fit each other: ", q.sizes(), ", ", k.sizes(), ", ", v.sizes(), ", ", state.sizes());
   const c10::cuda::CUDAGuard guard(q.device());
   const at::Tensor nc = nc_at_least(norm_const, q, q.size(1));
   at::Tensor out = at::empty({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
@@ -436,8 +447,10 @@ at::Tensor decode_steps(const at::Tensor& state, const at::Tensor& q_, const at:
 
 // a whole prompt: outputs and the decode state it leaves (head dim 64 or 128)
 at::Tensor prefill(const at::Tensor& state, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const) {
+  check_bhnd(q_, k_, v_);
   const at::Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
   const int B = (int)q.size(0), H = (int)q.size(1), N = (int)q.size(2), D = (int)q.size(3);
+  TORCH_CHECK(state.numel() >= q.size(0) * q.size(1) * D * D, "the state is smaller than the prompt's ", B, " x ", H, " sequences need");
   const c10::cuda::CUDAGuard guard(q.device());
   const at::Tensor nc = nc_f32(norm_const, q, H);
   const int nseg = D == 128 ? 1 : cott_cos_attn_seg_choice(B, H, N);

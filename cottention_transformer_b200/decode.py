@@ -27,7 +27,7 @@ class CosAttnDecodeState:
         """Absorb a whole prompt at once (fresh state only): outputs and state come from the fused causal kernels in one
         call (``cott_cos_attn_prefill``) instead of T recurrent steps.  bf16 / fp16, head dim 64 or 128; anything
         else falls back to ``step``.  Returns ``[B, H, T, d_v]``."""
-        from .cos_attention import cos_attn_causal, fused_supported, wide_supported
+        from .cos_attention import check_bhnd, fused_supported, wide_supported
         wide = wide_supported(q, k, v) and q.shape[-1] == 128
         if self.cur_s != 1 or not (wide or fused_supported(q, k, v)):
             return self.step(q, k, v, norm_const)
@@ -36,7 +36,10 @@ class CosAttnDecodeState:
             out = m.prefill(self.state, q, k, v, norm_const)
             self.cur_s += q.shape[2]
             return out
+        check_bhnd(q, k, v)
         B, H, T, D = q.shape
+        if self.state.numel() < B * H * D * D:
+            raise RuntimeError(f"the state is smaller than the prompt's {B} x {H} sequences need")
         q, k, v = q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous()
         L = _lib.lib()
         nc = norm_const.detach().reshape(-1).to(device=q.device, dtype=torch.float32).contiguous()
@@ -67,6 +70,8 @@ class CosAttnDecodeState:
             out = m.decode_steps(self.state, q, k, v, norm_const, self.cur_s)
             self.cur_s += T
             return out
+        if k.numel() != q.numel() or v.numel() != B * H * T * Dv or self.state.numel() < B * H * Dv * Dk:
+            raise RuntimeError(f"q, k, v and the state do not fit each other: {list(q.shape)}, {list(k.shape)}, {list(v.shape)}, {list(self.state.shape)}")
         q, k, v = q.contiguous(), k.to(q.dtype).contiguous(), v.to(q.dtype).contiguous()
         nc = norm_const.detach().reshape(-1).to(device=q.device, dtype=torch.float32).contiguous()
         out = torch.empty(B, H, T, Dv, dtype=q.dtype, device=q.device)

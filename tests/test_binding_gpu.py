@@ -108,6 +108,33 @@ def test_short_norm_const_is_refused():
         CosAttnDecodeState(1, 3, 64).step(tok, tok, tok, nc[:, :2])
 
 
+@pytest.mark.parametrize("compiled", [True, False])
+@pytest.mark.parametrize("D", [64, 128])
+def test_shapes_that_do_not_fit_are_refused(D, compiled, monkeypatch):
+    """Five dimensions (whose fourth happens to be a head dim), and k, v or a state that would be read past their end."""
+    from cottention_transformer_b200 import CosAttnDecodeState, _binding, cos_attn_causal
+    if not compiled:
+        monkeypatch.setattr(_binding, "autograd", lambda: None)
+    nc = torch.zeros(2, device="cuda")
+    x = torch.randn(1, 2, 3, D, D, device="cuda").bfloat16()
+    with pytest.raises(ValueError):
+        cos_attn_causal(x, x, x, nc)
+    with pytest.raises(ValueError):
+        CosAttnDecodeState(1, 2, D).prefill(x, x, x, nc)
+    q = torch.randn(2, 2, 5, D, device="cuda").bfloat16()
+    for k, v in ((q[:1], q), (q, q[:, :1]), (q, q[:, :, :3])):
+        with pytest.raises(RuntimeError, match="same shape"):
+            cos_attn_causal(q, k, v, nc)
+        with pytest.raises(RuntimeError, match="same shape"):
+            CosAttnDecodeState(2, 2, D).prefill(q, k, v, nc)
+        with pytest.raises(RuntimeError, match="do not fit"):
+            CosAttnDecodeState(2, 2, D).step(q, k, v, nc)
+    with pytest.raises(RuntimeError, match="the state"):
+        CosAttnDecodeState(1, 2, D).prefill(q, q, q, nc)
+    with pytest.raises(RuntimeError, match="the state"):
+        CosAttnDecodeState(1, 2, D).step(q, q, q, nc)
+
+
 @pytest.mark.parametrize("N,rot", [(1, 64), (130, 16), (300, 48)])
 @pytest.mark.parametrize("per_batch", [False, True])
 def test_rotation_inside_the_kernels_gives_the_bits_of_the_copying_pass(N, rot, per_batch):
