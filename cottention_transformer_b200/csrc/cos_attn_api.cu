@@ -179,6 +179,27 @@ int launch_bwd_both(const void* q, const void* k, const void* v, const float* nc
   return COTT_OK;
 }
 
+// Whether dQ and dK/dV may run side by side.  A dK/dV CTA stores rows of dk and dv when it has read all four tiles of
+// their chunk, so as a launch of its own, after the dQ launch, it may write over an input; next to a dQ CTA that is still
+// loading that input it may not.  (The same buffer for dq and one of the others: the later launch has the last word.)
+bool bwd_side_by_side(std::initializer_list<const void*> in, const void* dq, const void* dk, const void* dv) {
+  for (const void* p : in)
+    if (dk == p || dv == p) return false;
+  return dq != dk && dq != dv;
+}
+template <typename T>
+int launch_bwd(const void* q, const void* k, const void* v, const float* nc, const void* dout, void* dq, void* dk, void* dv, float* dnorm,
+               int B, int H, int N, int dtype, cudaStream_t stream, const float* prefix = nullptr, const float* suffix = nullptr,
+               SegPlan plan = SegPlan()) {
+  COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
+  // (the rotation inside the kernels has a dK/dV kernel with a warp group of its own)
+  if (!plan.rot.sin && bwd_side_by_side({q, k, v, dout}, dq, dk, dv))
+    return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, prefix, suffix, plan);
+  plan.dnorm_zeroed = true;
+  int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, prefix, plan);
+  return st ? st : launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, suffix, plan);
+}
+
 // The one-pass backward: `saved` holds the forward's 16-bit state before every chunk ([B*H][chunks][64][64]).
 template <typename T>
 int launch_bwd_fused(const void* q, const void* k, const void* v, const float* nc, const void* dout, const void* saved,
@@ -279,13 +300,7 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
     plan.keep = keep;
     plan.count = reinterpret_cast<const int*>(ws + 5 * A);
   }
-  COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
-  if (plan.nseg == 1 && plan.rot.sin) {  // (the rotation inside the kernels has a dK/dV kernel with a group of its own)
-    plan.dnorm_zeroed = true;
-    int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, nullptr, plan);
-    return st ? st : launch_bwd_dkdv<T>(q, k, v, nc, dout, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, plan);
-  }
-  if (plan.nseg == 1) return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, nullptr, plan);
+  if (plan.nseg == 1) return launch_bwd<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, nullptr, nullptr, plan);
   // dQ: the forward prefix states (left in the workspace by the forward call), read transposed.  dK, dV: reverse states of
   // the segments, their exclusive suffix.
   int st;
@@ -293,7 +308,7 @@ int run_bwd_seg(const void* q, const void* k, const void* v, const unsigned char
                                               seg_parts(plan), stream)) ||
       (st = launch_seg_prefix(ws, ws + 3 * A, (long)B * H, plan.nseg, seg_parts(plan), kTcD * kTcD, true, stream)))
     return st;
-  return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 2 * A, ws + 3 * A, plan);
+  return launch_bwd<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, ws + 2 * A, ws + 3 * A, plan);
 }
 
 // The time-out path of the tensor-core kernels on its own: one CTA sets up what those kernels set up (an
@@ -828,10 +843,8 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
   DeviceScope scope(q);
   COTT_CUDA_TRY(scope.status());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  COTT_CUDA_TRY(cudaMemsetAsync(dnorm_const, 0, sizeof(float) * H, s));
-  return dtype == COTT_BF16
-             ? launch_bwd_both<__nv_bfloat16>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, nullptr, SegPlan())
-             : launch_bwd_both<__half>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s, nullptr, nullptr, SegPlan());
+  return dtype == COTT_BF16 ? launch_bwd<__nv_bfloat16>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s)
+                            : launch_bwd<__half>(q, k, v, norm_const, dout, dq, dk, dv, dnorm_const, B, H, N, dtype, s);
 }
 
 int cott_cos_attn_seg_count(int B, int H, int N) { return seg_count((long)B * H, N); }

@@ -101,8 +101,10 @@ int cott_cos_attn_fwd(const void* q, const void* k, const void* v, const float* 
 
 /*
  * Fused backward of cott_cos_attn_fwd: dq, dk, dv (same layout and dtype as the inputs) and
- * dnorm_const (H floats, overwritten).  Two launches: a forward-direction pass for dq and a
- * reverse-direction pass for dk, dv and dnorm_const.
+ * dnorm_const (H floats, overwritten).  One launch: CTAs of a forward-direction pass for dq beside
+ * CTAs of a reverse-direction pass for dk, dv and dnorm_const.  dk and dv may each be one of q, k, v, dout
+ * (the same address and strides; dq may not): the two passes are then two launches, one after the other, as
+ * in the calls below.  The same holds for _bwd_seg and _bwd_split.
  *
  * Replaces CustomAttention.backward (Cuda_Kernel/Custom_Kernel.py:35-141, three kernel calls) plus
  * the autograd of GPTCosAttention.py:229-230 (normalize) and :241 (length-norm; this is where the
@@ -113,7 +115,7 @@ int cott_cos_attn_bwd(const void* q, const void* k, const void* v, const float* 
                       int N, int Dk, int Dv, int dtype, void* stream);
 
 /*
- * The two launches of cott_cos_attn_bwd as separate calls (same arguments, same results), so
+ * The two passes of cott_cos_attn_bwd as separate calls and launches (same arguments, same results), so
  * that a caller can time or schedule them individually:
  *   _dq    forward-direction pass: dq     (role of Custom_Kernel.py:106 + autograd of the q normalize)
  *   _dkdv  reverse-direction pass: dk, dv, dnorm_const   (Custom_Kernel.py:107-108 + autograd of the

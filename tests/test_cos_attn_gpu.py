@@ -432,3 +432,39 @@ def test_rotary_backward_leaves_a_shared_gradient_alone():
     gx = x.grad.view(B, N, 3, H, d)
     assert torch.equal(gx[:, :, 2], w.view(B, N, 3, H, d)[:, :, 2])
     assert not torch.equal(gx[:, 1:, 0], w.view(B, N, 3, H, d)[:, 1:, 0])
+
+
+@pytest.mark.parametrize("nseg", [1, 3])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("B,H,N", [(1, 2, 700), (3, 60, 500)])
+def test_backward_over_its_inputs(B, H, N, masked, nseg):
+    """dk and dv in the place of k and v (or of one another's input), and one buffer for dq and dk: the results of the
+    separate calls, whatever runs side by side otherwise."""
+    from cottention_transformer_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v, do = (torch.randn(B, H, N, 64, device="cuda", generator=g).bfloat16() for _ in range(4))
+    nc = 0.5 + 0.2 * torch.randn(H, device="cuda", generator=g)
+    keep = (torch.rand(B, N, device="cuda", generator=g) < 0.7).to(torch.uint8) if masked else None
+    L, P, st = _lib.lib(), _lib.ptr, _lib.stream_ptr(q.device)
+    ws = torch.empty(L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg), dtype=torch.uint8, device="cuda")
+    out, dnc = torch.empty_like(q), torch.empty(H, device="cuda")
+
+    def run(x, dq, dk, dv):
+        _lib.check(L.cott_cos_attn_fwd_seg(P(x[0]), P(x[1]), P(x[2]), P(keep), P(nc), P(out), P(ws), nseg, None, B, H, N, 64, 64, 3, st), "fwd")
+        _lib.check(L.cott_cos_attn_bwd_seg(P(x[0]), P(x[1]), P(x[2]), P(keep), P(nc), P(x[3]), P(ws), nseg, None, P(dq), P(dk), P(dv), P(dnc), B, H,
+                                           N, 64, 64, 3, st), "bwd")
+        _lib.check_device_status()
+        return dq, dk, dv
+
+    want = run((q, k, v, do), *(torch.empty_like(q) for _ in range(3)))
+    for _ in range(3):  # (a race may go well once)
+        x = [t.clone() for t in (q, k, v, do)]
+        got = run(x, torch.empty_like(q), x[1], x[2])
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        x = [t.clone() for t in (q, k, v, do)]
+        got = run(x, torch.empty_like(q), x[3], x[0])
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        x = [t.clone() for t in (q, k, v, do)]
+        dqk = torch.empty_like(q)
+        got = run(x, dqk, dqk, torch.empty_like(q))
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
