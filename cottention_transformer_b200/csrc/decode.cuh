@@ -25,6 +25,7 @@ namespace cott {
 constexpr int kDecodeThreads = 128;
 constexpr int kDecodeCtasPerSm = 8;
 template <int DK> struct DecodeCfg { static constexpr int kRows = DK == 128 ? 32 : 64; };  // state rows of a CTA
+constexpr int kDecodeMaxDv = 128;
 
 template <typename T>
 __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
@@ -33,14 +34,14 @@ __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
 // positions: optional [B] int64 array of the 1-based position of the FIRST token of this call for
 // each batch entry; if null, `pos0` is used for all.  LPR = lanes per state row = Dk/4.
 // (the kernel is latency-bound on its state loads, so resident CTAs are what hides the HBM latency)
-template <typename T, int DK>
-__global__ void __launch_bounds__(kDecodeThreads, kDecodeCtasPerSm)
+// ROWS: state rows of a CTA.
+template <typename T, int DK, int ROWS>
+__global__ void __launch_bounds__(kDecodeThreads, ROWS <= DecodeCfg<DK>::kRows ? kDecodeCtasPerSm : 2)
 decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
               const float* __restrict__ norm_const, T* __restrict__ out, int H, int Dv, int Tsteps, long long pos0,
               const long long* __restrict__ positions) {
   constexpr int LPR = DK / 4;                    // lanes per row (4, 8, 16 or 32)
   constexpr int ROWS_PER_PASS = kDecodeThreads / LPR;
-  constexpr int ROWS = DecodeCfg<DK>::kRows;
   constexpr int MAXR = (ROWS + ROWS_PER_PASS - 1) / ROWS_PER_PASS;  // state rows held per thread
   __shared__ float sq[DK], sk[DK], sv[ROWS];
   __shared__ float red[2][kDecodeThreads / 32];
@@ -130,15 +131,34 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
   }
 }
 
+template <typename T, int DK, int ROWS>
+int launch_decode_rows(float* state, const T* q, const T* k, const T* v, const float* nc, T* out, unsigned states, int H, int Dv, int T_steps,
+                       long long pos0, const long long* positions, cudaStream_t stream) {
+  COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK, ROWS>, dim3(states, (Dv + ROWS - 1) / ROWS), kDecodeThreads, 0, stream, state, q, k, v, nc, out, H,
+                           Dv, T_steps, pos0, positions));
+  return COTT_OK;
+}
+
 template <typename T>
 int launch_decode(float* state, const void* q, const void* k, const void* v, const float* nc, void* out, int B, int H,
                   int Dk, int Dv, int T_steps, long long pos0, const long long* positions, cudaStream_t stream) {
-  const unsigned grid = static_cast<unsigned>(static_cast<long>(B) * H);
-#define COTT_DECODE_CASE(DK)                                                                                              \
-  case DK:                                                                                                                \
-    COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK>, dim3(grid, (Dv + DecodeCfg<DK>::kRows - 1) / DecodeCfg<DK>::kRows),    \
-                             kDecodeThreads, 0, stream, state, static_cast<const T*>(q), static_cast<const T*>(k),        \
-                             static_cast<const T*>(v), nc, static_cast<T*>(out), H, Dv, T_steps, pos0, positions));       \
+  const unsigned states = static_cast<unsigned>(static_cast<long>(B) * H);
+  // Every CTA of a state reads the whole of q and k (and its own part of v), at its own time.  Tokens that `out` is written
+  // over are therefore read by one CTA per state, which has read a token when it stores the output of it.
+  const size_t tokens = static_cast<size_t>(states) * T_steps * sizeof(T);
+  auto overlaps = [&](const void* p, int d) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), o = reinterpret_cast<uintptr_t>(out);
+    return a < o + tokens * Dv && o < a + tokens * d;
+  };
+  const bool one_cta = overlaps(q, Dk) || overlaps(k, Dk) || (out != v && overlaps(v, Dv));
+  const T *tq = static_cast<const T*>(q), *tk = static_cast<const T*>(k), *tv = static_cast<const T*>(v);
+  T* to = static_cast<T*>(out);
+  int st = COTT_OK;
+#define COTT_DECODE_CASE(DK)                                                                                                        \
+  case DK:                                                                                                                          \
+    st = one_cta ? launch_decode_rows<T, DK, kDecodeMaxDv>(state, tq, tk, tv, nc, to, states, H, Dv, T_steps, pos0, positions, stream) \
+                 : launch_decode_rows<T, DK, DecodeCfg<DK>::kRows>(state, tq, tk, tv, nc, to, states, H, Dv, T_steps, pos0, positions, \
+                                                                   stream);                                                         \
     break;
   switch (Dk) {
     COTT_DECODE_CASE(16)
@@ -148,6 +168,7 @@ int launch_decode(float* state, const void* q, const void* k, const void* v, con
     default: return fail(COTT_ERR_SHAPE, "decode supports D_attn in {16, 32, 64, 128} (got %d)", Dk);
   }
 #undef COTT_DECODE_CASE
+  if (st) return st;
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }

@@ -265,7 +265,7 @@ int cott_cos_attn_prefill_state(const void* k, const void* v, const float* norm_
  * Replaces the fast_inference branch of GPTCosAttention._cos_attn for one token,
  * GPT_Trainer/GPTCosAttention.py:229-230,236,253-272 (state init :76-85; driven token by token by
  * GPT_Trainer/fast_infer.py:111-139).  The reference keeps a float64 [1,H,d,d] state on the CPU;
- * this one is float32, batched, in HBM.  Dk in {16,32,64,128}, 1 <= Dv <= 128.
+ * this one is float32, batched, in HBM.  Dk in {16,32,64,128}, 1 <= Dv <= 128.  `out` may be q, k or v.
  */
 int cott_decode_step(float* state, const void* q, const void* k, const void* v, const float* norm_const,
                      void* out, int B, int H, int Dk, int Dv, int dtype, long long pos,

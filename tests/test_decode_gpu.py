@@ -106,3 +106,45 @@ def test_prefill_hands_the_state_to_decode(dt, shape, d):
     assert (out_fast[:, :, N:].float() - out_ref[:, :, N:].float()).abs().max().item() <= 2e-2 * scale
     s_scale = ref.state.abs().max().item()
     assert (fast.state - ref.state).abs().max().item() <= 1e-2 * s_scale
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Dk,Dv", [(64, 100), (32, 128), (64, 65), (128, 70), (128, 33), (16, 96)])
+def test_states_shared_by_several_ctas(Dk, Dv, dt):
+    """Value dims that leave the last CTA of a state a few rows, or one."""
+    from cottention_transformer_b200 import CosAttnDecodeState
+    B, H, T = 2, 3, 4
+    g = torch.Generator().manual_seed(Dk * Dv)
+    q, k = (torch.randn(B, H, T, Dk, generator=g).to(dt) for _ in range(2))
+    v = torch.randn(B, H, T, Dv, generator=g).to(dt)
+    nc = torch.linspace(-0.5, 1.0, H)
+    state = torch.zeros(B, H, Dv, Dk, dtype=torch.float64)
+    want = torch.stack([O.decode_step(state, t + 1, q[:, :, t], k[:, :, t], v[:, :, t], nc) for t in range(T)], 2)
+    st = CosAttnDecodeState(B, H, Dk, Dv)
+    got = st.step(q.cuda(), k.cuda(), v.cuda(), nc.cuda())
+    tol = 1e-4 if dt == torch.float32 else 2e-2 * want.abs().max().item()
+    assert (got.double().cpu() - want).abs().max().item() <= tol
+    assert (st.state.double().cpu() - state).abs().max().item() <= 1e-4
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,T", [(128, 1), (128, 5), (64, 3), (32, 1)])
+def test_outputs_over_the_tokens(D, T, dt):
+    """The output in the place of q, k or v, with as many states as keep several CTAs of one state apart in time."""
+    from cottention_transformer_b200 import _lib
+    B, H = 512, 8
+    g = torch.Generator(device="cuda").manual_seed(D + T)
+    x = [torch.randn(B, H, T, D, device="cuda", generator=g).to(dt) for _ in range(3)]
+    nc = torch.linspace(-0.5, 1.0, H, device="cuda")
+    L, P = _lib.lib(), _lib.ptr
+
+    def run(over):
+        t = [a.clone() for a in x]
+        state, out = torch.zeros(B, H, D, D, device="cuda"), torch.empty_like(x[0]) if over is None else t[over]
+        _lib.check(L.cott_decode_steps(P(state), P(t[0]), P(t[1]), P(t[2]), P(nc), P(out), B, H, T, D, D, _lib.DTYPE_CODE[dt], 7, None,
+                                       _lib.stream_ptr(state.device)), "decode")
+        return out, state
+
+    want = run(None)
+    for over in (0, 1, 2):
+        assert all(torch.allclose(a.float(), b.float(), rtol=1e-2 if dt != torch.float32 else 1e-5, atol=1e-5) for a, b in zip(run(over), want)), over
