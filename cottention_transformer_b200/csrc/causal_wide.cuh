@@ -524,7 +524,7 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
             if (a.row_mode == kWdRowNorm) {
               float dot = row_dot_acc<T>(dst, row, t);
               if (!pair_sum(dot, c)) break;
-              alpha = -beta * beta * beta * dot;
+              alpha = -beta * beta * (beta * dot);  // (x^ . g first: the cube of 1/|x| underflows from |x| = 5e12 on)
             }
             row_from_acc<T, true>(dst, row, t, beta, alpha);
           }

@@ -72,3 +72,19 @@ def test_prefill_state_128(N):
     vp = v.double() / n ** torch.sigmoid(nc.double())
     want = torch.einsum("bhnj,bhni->bhji", vp, torch.nn.functional.normalize(k.double(), dim=-1))
     assert st.cur_s == N + 1 and _rel(st.state, want) <= REL16[torch.bfloat16]
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1e14, 1e18])
+def test_fused_128_dq_of_long_and_short_rows(scale):
+    """dq through the normalisation for rows whose 1/|q| is far from 1 (bf16 reaches that far): the part of the gradient
+    along q cancels whatever |q| is."""
+    from cottention_transformer_b200 import cos_attn_causal
+    g = torch.Generator().manual_seed(7)
+    q, k, v, do = (torch.randn(1, 2, 300, 128, generator=g).bfloat16() for _ in range(4))
+    q = (q.float() * scale).bfloat16()
+    nc = 0.5 + 0.2 * torch.randn(1, 2, 1, 1, generator=g)
+    leaf = [t.cuda().requires_grad_() for t in (q, k, v, nc)]
+    (dq,) = torch.autograd.grad(cos_attn_causal(*leaf), leaf[0], do.cuda())
+    ref = [t.double().requires_grad_() for t in (q, k, v, nc)]
+    (want,) = torch.autograd.grad(O.cos_attn_causal(*ref), ref[0], do.double())
+    assert _rel(dq.double() * scale, want * scale) <= REL16[torch.bfloat16]
