@@ -263,26 +263,34 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
   }
 
   float acc[4][NB] = {};
-  {  // acc = P C, over the columns that survive for any row of the thread
-    const int s0 = LOWER ? 0 : (ty & ~3), s1 = LOWER ? ((ty + 48) & ~3) + 4 : kF32Chunk;
+  {  // acc = P C by blocks of 16 columns.  A row takes the columns on its side of the diagonal and no other: a masked score
+     // times an infinity is a NaN, so what a row may not see is not multiplied by zero but left out.  Row ty + 16 r has the
+     // blocks before (after) block r whole, block r up to (from) itself.
+#pragma unroll
+    for (int blk = 0; blk < 4; ++blk) {
 #pragma unroll 2
-    for (int s = s0; s < s1; s += 4) {
-      float p[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) f32_load<4>(p[r], sP + (ty + 16 * r) * LP + s);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float b[NB];
-        if constexpr (MT) {
-#pragma unroll
-          for (int j = 0; j < NB; ++j) b[j] = sC[(s + e) * LD + tx + 16 * j];
-        } else {
-          f32_load<NB>(b, sC + (s + e) * LD + NB * tx);
-        }
+      for (int s = 16 * blk; s < 16 * blk + 16; s += 4) {
+        float p[4][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
+          if (LOWER ? r >= blk : r <= blk) f32_load<4>(p[r], sP + (ty + 16 * r) * LP + s);
 #pragma unroll
-          for (int j = 0; j < NB; ++j) acc[r][j] = fmaf(p[r][e], b[j], acc[r][j]);
+        for (int e = 0; e < 4; ++e) {
+          float b[NB];
+          if constexpr (MT) {
+#pragma unroll
+            for (int j = 0; j < NB; ++j) b[j] = sC[(s + e) * LD + tx + 16 * j];
+          } else {
+            f32_load<NB>(b, sC + (s + e) * LD + NB * tx);
+          }
+          const bool own = LOWER ? s + e <= ty + 16 * blk : s + e >= ty + 16 * blk;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if ((LOWER ? r > blk : r < blk) || (r == blk && own)) {
+#pragma unroll
+              for (int j = 0; j < NB; ++j) acc[r][j] = fmaf(p[r][e], b[j], acc[r][j]);
+            }
+        }
       }
     }
   }
@@ -376,7 +384,7 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
         dot = fma(static_cast<double>(v[j] / d), static_cast<double>(acc[r][j]), dot);
         acc[r][j] /= d;
       }
-      if (in && n > 1.f) gsum += ln[t] * dot;
+      if (in && n >= 1.f) gsum += ln[t] * dot;  // (ln 1 = 0 times an infinity is a NaN, here as in the module math)
       if (in) f32_store<NB>(g.dv + o, acc[r]);
     }
 #pragma unroll

@@ -97,3 +97,31 @@ def test_f32_forms_that_stay_with_the_unfused_path():
     assert not f32_supported(q[:, :, :0], q[:, :, :0], q[:, :, :0], nc)
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert not f32_supported(q, q, q, nc)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("N,pos", [(150, 70), (150, 64), (150, 127), (64, 0), (200, 199), (130, 129)])
+@pytest.mark.parametrize("D", [32, 64])
+def test_non_finite_rows_reach_what_the_sums_contain(D, N, pos, bad):
+    """A non-finite value of v or of the incoming gradient enters the sums it is a term of and no other: the causal mask
+    leaves a term out, it does not multiply it by zero."""
+    from cottention_transformer_b200 import cos_attn_causal
+    q, k, v, do, nc, _ = (None if t is None else t.cuda() for t in _inputs(1, 2, N, D, False, seed=N + pos))
+    t = torch.arange(N, device="cuda").view(N, 1)
+    col = torch.arange(D, device="cuda").view(1, D) == 5
+    vb, dob = v.clone(), do.clone()
+    vb[0, 1, pos, 5] = bad
+    out, dq, dk, dv, dnc = _run(cos_attn_causal, q, k, vb, do, nc, None)
+    assert torch.equal(~out[0, 1].isfinite(), (t >= pos) & col)             # out_t = sum_{s <= t} (q^_t . k^_s) v'_s
+    assert torch.equal(~dq[0, 1].isfinite(), (t >= pos).expand(N, D))       # dq^_t = sum_{s <= t} (dO_t . v'_s) k^_s
+    assert torch.equal(~dk[0, 1].isfinite(), (t == pos).expand(N, D))       # dk^_s = sum_{t >= s} (v'_s . dO_t) q^_t
+    assert dv.isfinite().all()                                              # dv'_s = sum_{t >= s} (q^_t . k^_s) dO_t
+    assert not dnc[0, 1].isfinite().any()                                   # (also at position 1, whose ln n is zero)
+    assert all(x[0, 0].isfinite().all() for x in (out, dq, dk, dv, dnc))
+    dob[0, 1, pos, 5] = bad
+    out, dq, dk, dv, dnc = _run(cos_attn_causal, q, k, v, dob, nc, None)
+    assert out.isfinite().all()
+    assert torch.equal(~dq[0, 1].isfinite(), (t == pos).expand(N, D))
+    assert torch.equal(~dk[0, 1].isfinite(), (t <= pos).expand(N, D))
+    assert torch.equal(~dv[0, 1].isfinite(), (t <= pos) & col)
+    assert all(x[0, 0].isfinite().all() for x in (out, dq, dk, dv, dnc))
