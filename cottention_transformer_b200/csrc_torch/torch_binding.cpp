@@ -404,29 +404,39 @@ struct WideFn : torch::autograd::Function<WideFn> {
 at::Tensor scan_by_dtype(at::ScalarType t, at::Tensor Q, at::Tensor K, at::Tensor V, bool reversed) {
   return t == at::kHalf ? forward_<at::kHalf>(Q, K, V, 1, false, reversed) : forward_<at::kBFloat16>(Q, K, V, 1, false, reversed);
 }
-struct CustomAttentionFn : torch::autograd::Function<CustomAttentionFn> {
-  static Variable forward(AutogradContext* ctx, const at::Tensor& Q_, const at::Tensor& K_, const at::Tensor& V_) {
-    const at::Tensor Q = Q_.contiguous(), K = K_.contiguous(), V = V_.contiguous();
+struct ScanFn : torch::autograd::Function<ScanFn> {
+  // `entry`: the dtype whose entry point the scans go through
+  static Variable forward(AutogradContext* ctx, const at::Tensor& Q, const at::Tensor& K, const at::Tensor& V, int64_t entry, bool reversed) {
     ctx->save_for_backward({Q, K, V});
-    return scan_by_dtype(Q.scalar_type(), Q, K, V, false);
+    ctx->saved_data["entry"] = entry;
+    ctx->saved_data["reversed"] = reversed;
+    return scan_by_dtype((at::ScalarType)entry, Q, K, V, reversed);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
-    const at::Tensor Q = s[0].contiguous(), K = s[1].contiguous(), V = s[2].contiguous(), g = grads[0].contiguous();
-    const at::ScalarType t = Q.scalar_type();
+    const at::Tensor &Q = s[0], &K = s[1], &V = s[2], g = grads[0].contiguous();
+    const int64_t entry = ctx->saved_data["entry"].toInt();
+    const at::ScalarType t = (at::ScalarType)entry;
+    const bool rev = ctx->saved_data["reversed"].toBool();
+    if (at::GradMode::is_enabled())  // create_graph: the gradients are scans themselves, with nodes of their own
+      return {apply(g, V, K, entry, rev), apply(V, g, Q, entry, !rev), apply(K, Q, g, entry, !rev), Variable(), Variable()};
     // one dtype and one shape in 16 bits: the three scans in one C call (autocast only ever concerns fp32 tensors)
-    if ((t == at::kHalf || t == at::kBFloat16) && K.scalar_type() == t && V.scalar_type() == t && g.scalar_type() == t && Q.dim() == 4 &&
-        Q.sizes() == K.sizes() && Q.sizes() == V.sizes() && Q.sizes() == g.sizes() && Q.size(3) == 64) {
+    if (!rev && (t == at::kHalf || t == at::kBFloat16) && Q.scalar_type() == t && K.scalar_type() == t && V.scalar_type() == t && g.scalar_type() == t &&
+        Q.dim() == 4 && Q.sizes() == K.sizes() && Q.sizes() == V.sizes() && Q.sizes() == g.sizes() && Q.size(3) == 64) {
       const c10::cuda::CUDAGuard guard(Q.device());
       at::Tensor dq = at::empty_like(Q), dk = at::empty_like(K), dv = at::empty_like(V);
       check(cott_scan_bwd(Q.data_ptr(), K.data_ptr(), V.data_ptr(), g.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (int)Q.size(0),
                           (int)Q.size(1), (int)Q.size(2), 64, 64, dtype_code(t), stream_of(Q)),
             "cott_scan_bwd");
-      return {dq, dk, dv};
+      return {dq, dk, dv, Variable(), Variable()};
     }
-    return {scan_by_dtype(t, g, V, K, false), scan_by_dtype(t, V, g, Q, true), scan_by_dtype(t, K, Q, g, true)};
+    return {scan_by_dtype(t, g, V, K, rev), scan_by_dtype(t, V, g, Q, !rev), scan_by_dtype(t, K, Q, g, !rev), Variable(), Variable()};
   }
 };
+// (dense before the node, so that what it saves is still connected to the caller's tensors)
+at::Tensor custom_attention(const at::Tensor& Q, const at::Tensor& K, const at::Tensor& V) {
+  return ScanFn::apply(Q.contiguous(), K.contiguous(), V.contiguous(), (int64_t)Q.scalar_type(), false);
+}
 
 // one decode call on a [B, H, Dv, Dk] state
 at::Tensor decode_steps(const at::Tensor& state, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
@@ -478,7 +488,7 @@ at::Tensor exact_causal(const at::Tensor& q, const at::Tensor& k, const at::Tens
     const at::Tensor m = keep->view({B, 1, N, 1}).to(q.scalar_type());
     qh = qh * m, kh = kh * m, vp = vp * m;
   }
-  return CustomAttentionFn::apply(qh, kh, vp);
+  return custom_attention(qh, kh, vp);
 }
 struct F32Fn : torch::autograd::Function<F32Fn> {
   static Variable forward(AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_, const at::Tensor& v_, const at::Tensor& norm_const,
@@ -540,7 +550,6 @@ at::Tensor causal_packed(const at::Tensor& qkv, const at::Tensor& norm_const, co
 at::Tensor bidir_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep) {
   return BidirPackedFn::apply(qkv, norm_const, keep);
 }
-at::Tensor custom_attention(const at::Tensor& Q, const at::Tensor& K, const at::Tensor& V) { return CustomAttentionFn::apply(Q, K, V); }
 
 }  // namespace
 

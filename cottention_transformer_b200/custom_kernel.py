@@ -10,7 +10,9 @@ False)`` (``:9-32``); ``backward`` runs the three permuted scans (``:106-108``)
 
 each through the same name-dispatch, so the autocast rules of the entry points apply to the
 backward exactly as they do in the reference.  Passes ``torch.autograd.gradcheck`` in float64, the
-reference's only correctness check (``:184-188``).
+reference's only correctness check (``:184-188``), and ``gradgradcheck``: under ``create_graph`` the three
+scans are differentiable themselves (the reference's kernel calls are not, and drop out of a second
+derivative without a word).
 """
 from __future__ import annotations
 
@@ -26,6 +28,32 @@ _BY_DTYPE = {
 }
 
 
+def _scans(fn, g, Q, K, V, reversed):
+    """The gradients of ``fn(Q, K, V, 1, False, reversed)``: three more scans."""
+    return fn(g, V, K, 1, False, reversed), fn(V, g, Q, 1, False, not reversed), fn(K, Q, g, 1, False, not reversed)
+
+
+class _Scan(torch.autograd.Function):
+    """One scan in either direction through the entry point ``fn``, as often differentiable as one likes: its gradients are
+    scans again."""
+
+    @staticmethod
+    def forward(ctx, Q, K, V, fn, reversed):
+        ctx.save_for_backward(Q, K, V)
+        ctx.fn, ctx.reversed = fn, reversed
+        return fn(Q, K, V, 1, False, reversed)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return *_differentiable_scans(ctx.fn, grad_output.contiguous(), *ctx.saved_tensors, ctx.reversed), None, None
+
+
+def _differentiable_scans(fn, g, Q, K, V, reversed):
+    if not torch.is_grad_enabled():
+        return _scans(fn, g, Q, K, V, reversed)
+    return _scans(lambda q, k, v, _block, _inplace, rev: _Scan.apply(q, k, v, fn, rev), g, Q, K, V, reversed)
+
+
 class CustomAttention(torch.autograd.Function):
     @classmethod
     def apply(cls, *args):
@@ -34,6 +62,7 @@ class CustomAttention(torch.autograd.Function):
             m = _binding.autograd()
             if m is not None:
                 return m.custom_attention(*args)
+            args = [t.contiguous() for t in args]  # (dense before the node: what it saves stays connected to the caller's tensors)
         return super().apply(*args)
 
     @staticmethod
@@ -57,7 +86,4 @@ class CustomAttention(torch.autograd.Function):
         fn = _BY_DTYPE.get(Q.dtype)
         if fn is None:
             raise ValueError("Only float32, float64, float16, and bfloat16 are supported")
-        grad_Q = fn(grad_output, V, K, 1, False, False)
-        grad_K = fn(V, grad_output, Q, 1, False, True)
-        grad_V = fn(K, Q, grad_output, 1, False, True)
-        return grad_Q, grad_K, grad_V
+        return _differentiable_scans(fn, grad_output, Q, K, V, False)

@@ -125,3 +125,37 @@ def test_non_finite_rows_reach_what_the_sums_contain(D, N, pos, bad):
     assert torch.equal(~dk[0, 1].isfinite(), (t <= pos).expand(N, D))
     assert torch.equal(~dv[0, 1].isfinite(), (t <= pos) & col)
     assert all(x[0, 0].isfinite().all() for x in (out, dq, dk, dv, dnc))
+
+
+@pytest.mark.parametrize("compiled", [True, False])
+@pytest.mark.parametrize("masked", [False, True])
+def test_second_derivatives(masked, compiled, monkeypatch):
+    """create_graph: the gradients' gradients with respect to every input against fp64 autograd of the oracle."""
+    from cottention_transformer_b200 import _binding, cos_attn_causal
+    if not compiled:
+        monkeypatch.setattr(_binding, "autograd", lambda: None)
+    q, k, v, do, nc, keep = _inputs(2, 2, 70, 32, masked, seed=11)
+    w = [torch.randn(t.shape, generator=torch.Generator().manual_seed(i)) for i, t in enumerate((q, k, v, nc))]
+
+    def second(fn, dtype, dev):
+        x = [t.to(dev, dtype).requires_grad_() for t in (q, k, v, nc, do)]
+        out = fn(*x[:4], None if keep is None else keep.to(dev))
+        first = torch.autograd.grad(out, x[:4], x[4], create_graph=True)
+        return torch.autograd.grad(sum((g * u.to(dev, dtype)).sum() for g, u in zip(first, w)), x)
+
+    want = second(lambda q, k, v, n, kp: O.cos_attn_causal(q, k, v, n, keep=kp), torch.float64, "cpu")
+    got = second(lambda q, k, v, n, kp: cos_attn_causal(q.transpose(1, 2).contiguous().transpose(1, 2), k, v, n, kp), torch.float32, "cuda")
+    for name, a, b in zip(("q", "k", "v", "norm_const", "dout"), got, want):
+        # two passes of fp32 sums one after the other, and for norm_const signed sums over the sequence
+        assert _rel(a, b) <= (20 if name == "norm_const" else 5) * REL32, (name, _rel(a, b))
+
+
+@pytest.mark.parametrize("compiled", [True, False])
+def test_the_operator_itself_twice(compiled, monkeypatch):
+    from cottention_transformer_b200 import CustomAttention, _binding
+    if not compiled:
+        monkeypatch.setattr(_binding, "autograd", lambda: None)
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(1, 2, 5, 32, generator=g, dtype=torch.float64).cuda().requires_grad_() for _ in range(3))
+    assert torch.autograd.gradcheck(CustomAttention.apply, (q, k, v), fast_mode=True)
+    assert torch.autograd.gradgradcheck(CustomAttention.apply, (q, k.transpose(1, 2).contiguous().transpose(1, 2), v), fast_mode=True)
