@@ -30,14 +30,20 @@ def module():
     return _mod
 
 
+def transformed() -> bool:
+    """Whether something looks at a Python function and its operators, or refuses them by name, and would not see the nodes
+    of the compiled module: tracing, compilation, functorch transforms, forward-mode differentiation, dispatch modes (which
+    count, record or choose operators, as selective checkpointing does)."""
+    import torch
+    C = torch._C
+    return (torch.compiler.is_compiling() or C._get_tracing_state() is not None or C._functorch.peek_interpreter_stack() is not None
+            or C._len_torch_dispatch_stack() > 0 or torch.autograd.forward_ad._current_level >= 0)
+
+
 def autograd():
     """The module whose functions carry their own autograd nodes, or None where the Python autograd functions are needed:
-    without the binding, and under tracing, compilation and functorch transforms, which look at a Python function and its
-    operators (or refuse them by name) and would not see these."""
-    import torch
-    if torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None or torch._C._functorch.peek_interpreter_stack() is not None:
-        return None
-    return module()
+    without the binding, and where the call is ``transformed()``."""
+    return None if transformed() else module()
 
 
 def ops():

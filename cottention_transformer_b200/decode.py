@@ -27,7 +27,7 @@ class CosAttnDecodeState:
         """Absorb a whole prompt at once (fresh state only): outputs and state come from the fused causal kernels in one
         call (``cott_cos_attn_prefill``) instead of T recurrent steps.  bf16 / fp16, head dim 64 or 128; anything
         else falls back to ``step``.  Returns ``[B, H, T, d_v]``."""
-        from .cos_attention import check_bhnd, fused_supported, wide_supported
+        from .cos_attention import check_bhnd, cos_attn_causal, fused_supported, wide_supported
         wide = wide_supported(q, k, v) and q.shape[-1] == 128
         if self.cur_s != 1 or not (wide or fused_supported(q, k, v)):
             return self.step(q, k, v, norm_const)
@@ -40,18 +40,29 @@ class CosAttnDecodeState:
         B, H, T, D = q.shape
         if self.state.numel() < B * H * D * D:
             raise RuntimeError(f"the state is smaller than the prompt's {B} x {H} sequences need")
-        q, k, v = q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous()
+        k, v = k.contiguous(), v.contiguous()
         L = _lib.lib()
         nc = norm_const.detach().reshape(-1).to(device=q.device, dtype=torch.float32).contiguous()
         if nc.numel() != H:
             raise RuntimeError(f"norm_const must have one entry per head ({H}), got {nc.numel()}")
-        out = torch.empty_like(v)
+        # (transformed: the outputs from the operator that the transform knows, or that refuses it, and the state by itself)
+        by_operator = _binding.transformed()
+        if by_operator:
+            with torch.no_grad():
+                out = cos_attn_causal(q, k, v, norm_const)
+        else:
+            q = q.contiguous()
+            out = torch.empty_like(v)
         with torch.cuda.device(q.device):
             nseg = 1 if wide else L.cott_cos_attn_seg_choice(B, H, T)
             nbytes = L.cott_cos_attn_wide_workspace_bytes(B, H, T) if wide else L.cott_cos_attn_seg_workspace_bytes(B, H, T, nseg)
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-            st = L.cott_cos_attn_prefill(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(self.state),
-                                         _lib.ptr(ws), nseg, B, H, T, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
+            if by_operator:
+                st = L.cott_cos_attn_prefill_state(_lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(self.state), _lib.ptr(ws), nseg,
+                                                   0, B, H, T, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
+            else:
+                st = L.cott_cos_attn_prefill(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(self.state),
+                                             _lib.ptr(ws), nseg, B, H, T, D, D, _lib.DTYPE_CODE[q.dtype], _lib.stream_ptr(q.device))
         _lib.check(st, "cott_cos_attn_prefill")
         self.cur_s += T
         return out

@@ -97,6 +97,48 @@ def test_transforms_are_refused_as_before():
         torch.func.jvp(lambda q: cos_attn_causal(q, x[1], x[2], nc), (x[0],), (x[0],))
 
 
+def test_dispatch_modes_see_the_operators():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from cottention_transformer_b200 import cos_attn_causal
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    x, nc, _, do, _ = _args("causal", torch.bfloat16)
+    names = []
+    leaf = [t.clone().requires_grad_() for t in x]
+    with Seen():
+        out = cos_attn_causal(*leaf, nc)
+    assert any("causal_fwd" in n for n in names)
+    assert torch.equal(out, cos_attn_causal(*leaf, nc))
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, leaf, do), torch.autograd.grad(cos_attn_causal(*leaf, nc), leaf, do)))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_transformed_prefill(D):
+    """Forward-mode differentiation is refused, not dropped; a trace runs the operator and does not return an empty buffer."""
+    import torch.autograd.forward_ad as fw
+
+    from cottention_transformer_b200 import CosAttnDecodeState
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v, q2 = (torch.randn(1, 2, 200, D, device="cuda", generator=g).bfloat16() for _ in range(4))
+    nc = torch.full((2,), 0.5, device="cuda")
+    with fw.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        CosAttnDecodeState(1, 2, D).prefill(fw.make_dual(q, q), k, v, nc)
+    with fw.dual_level():
+        st = CosAttnDecodeState(1, 2, D)
+        out = st.prefill(q, k, v, nc)
+    ref = CosAttnDecodeState(1, 2, D)
+    assert torch.equal(out, ref.prefill(q, k, v, nc))
+    # the state: another kernel, the same sums of 16-bit products in fp32
+    assert (st.state - ref.state).norm() <= 1e-3 * ref.state.norm() and st.cur_s == ref.cur_s
+    traced = torch.jit.trace(lambda a: CosAttnDecodeState(1, 2, D).prefill(a, k, v, nc), (q,), check_trace=False)
+    assert torch.equal(traced(q2), CosAttnDecodeState(1, 2, D).prefill(q2, k, v, nc))
+
+
 def test_short_norm_const_is_refused():
     from cottention_transformer_b200 import CosAttnDecodeState, cos_attn_bidirectional_packed, cos_attn_causal_packed
     x, nc, _, _, _ = _args("packed", torch.bfloat16)
