@@ -571,18 +571,21 @@ TORCH_LIBRARY_IMPL(cottention_b200, CUDA, m) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // how a non-zero status of the C ABI surfaces in Python: RuntimeError carrying the status text and the library's message
   m.def("_raise_for_status", [](int status) { check(status, "cottention_b200"); }, py::arg("status"));
+  // Without the interpreter lock, as calls through ctypes and torch.ops run: a launch may wait for room in the stream's
+  // queue, and what the queue waits for may be another Python thread.
+  using Unlocked = py::call_guard<py::gil_scoped_release>;
   m.def("seg_count", [](const at::Tensor& t, int64_t B, int64_t H, int64_t N) {
     const c10::cuda::CUDAGuard guard(t.device());
     return cott_cos_attn_seg_choice((int)B, (int)H, (int)N);
   });
-  m.def("cos_attn_causal", &cos_attn_causal);
-  m.def("cos_attn_wide", &cos_attn_wide);
-  m.def("cos_attn_f32", &cos_attn_f32);
-  m.def("causal_packed", &causal_packed);
-  m.def("bidir_packed", &bidir_packed);
-  m.def("custom_attention", &custom_attention);
-  m.def("decode_steps", &decode_steps);
-  m.def("prefill", &prefill);
+  m.def("cos_attn_causal", &cos_attn_causal, Unlocked());
+  m.def("cos_attn_wide", &cos_attn_wide, Unlocked());
+  m.def("cos_attn_f32", &cos_attn_f32, Unlocked());
+  m.def("causal_packed", &causal_packed, Unlocked());
+  m.def("bidir_packed", &bidir_packed, Unlocked());
+  m.def("custom_attention", &custom_attention, Unlocked());
+  m.def("decode_steps", &decode_steps, Unlocked());
+  m.def("prefill", &prefill, Unlocked());
   m.def("float32", &forward_<at::kBFloat16>, "FastAttention forward (float32 entry point)", py::arg("Q"), py::arg("K"), py::arg("V"),
         py::arg("block_size"), py::arg("inplace") = false, py::arg("reversed") = false);
   m.def("float64", &forward_<at::kBFloat16>, "FastAttention forward (float64 entry point)", py::arg("Q"), py::arg("K"), py::arg("V"),

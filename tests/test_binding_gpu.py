@@ -139,6 +139,41 @@ def test_transformed_prefill(D):
     assert torch.equal(traced(q2), CosAttnDecodeState(1, 2, D).prefill(q2, k, v, nc))
 
 
+def test_other_python_threads_run_while_a_launch_waits():
+    """A call that waits for room in the launch queue (behind a kernel of about half a second) does not hold the
+    interpreter lock meanwhile."""
+    import threading
+    import time
+
+    from cottention_transformer_b200 import CosAttnDecodeState
+    tok = torch.randn(1, 1, 1, 64, device="cuda").bfloat16()
+    nc, st = torch.zeros(1, device="cuda"), CosAttnDecodeState(1, 1, 64)
+    st.step(tok, tok, tok, nc)
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    other = threading.Thread(target=tick)
+    other.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(1_000_000_000)
+    for _ in range(3000):
+        st.step(tok, tok, tok, nc)
+    waited = time.perf_counter() - t0
+    stop.set()
+    other.join()
+    torch.cuda.synchronize()
+    assert waited > 0.2, "the queue took all launches: nothing was tested"
+    assert max(gaps) < 0.5 * waited
+
+
 def test_short_norm_const_is_refused():
     from cottention_transformer_b200 import CosAttnDecodeState, cos_attn_bidirectional_packed, cos_attn_causal_packed
     x, nc, _, _, _ = _args("packed", torch.bfloat16)
