@@ -128,13 +128,25 @@ def _table_stride(sin, N):
     return N * sin.shape[-1] if sin.dim() == 3 and sin.shape[0] > 1 else 0
 
 
+def _rotated_copy(qkv, sin, cos, lay):
+    """The q and k of a packed ``[B, N, 3, H, D]`` tensor, rotated: ``[B, N, 2, H, D]`` and its layout."""
+    B, N, _, H, D = qkv.shape
+    rqk = torch.empty(B, N, 2, H, D, dtype=qkv.dtype, device=qkv.device)
+    qlay = _lib.CottLayout(N * 2 * H * D, D, 2 * H * D, 0, 0, 0)
+    st = _lib.lib().cott_rotary_copy(_lib.ptr(qkv[:, :, 0]), _lib.ptr(qkv[:, :, 1]), _lib.ptr(rqk[:, :, 0]), _lib.ptr(rqk[:, :, 1]), _lib.ptr(sin),
+                                     _lib.ptr(cos), ctypes.byref(lay), ctypes.byref(qlay), B, H, N, D, 2 * sin.shape[-1], _table_stride(sin, N),
+                                     _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device))
+    _lib.check(st, "cott_rotary_copy")
+    return rqk, qlay
+
+
 class _FusedCausalPacked(torch.autograd.Function):
     """The fused causal op on the packed output of a QKV projection: ``qkv`` is ``[B, N, 3, H, 64]`` and the result
     ``[B, N, H, 64]``; q, k, v, the output and all gradients are read and written in place through strided tensor
     maps, so the head split / merge permutes (GPTCosAttention.py:447-449,478-479,500) cost no copy."""
 
     @staticmethod
-    def forward(ctx, qkv, norm_const, keep=None, sin=None, cos=None):
+    def forward(ctx, qkv, norm_const, keep=None, sin=None, cos=None, keep_rotated=True):
         qkv = qkv.contiguous()
         B, N, three, H, D = qkv.shape
         nc = norm_const.detach().reshape(-1).to(device=qkv.device, dtype=torch.float32).contiguous()
@@ -146,19 +158,15 @@ class _FusedCausalPacked(torch.autograd.Function):
         code, stream = _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device)
         rqk = qlay = None
         with torch.cuda.device(qkv.device):
-            nseg = 1 if sin is not None else L.cott_cos_attn_seg_choice(B, H, N)
+            nseg = L.cott_cos_attn_seg_choice(B, H, N)
             ws = torch.empty(L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg), dtype=torch.uint8, device=qkv.device)
-            if sin is not None:  # rotated copies of q and k, [B, N, 2, H, D]
-                rqk = torch.empty(B, N, 2, H, D, dtype=qkv.dtype, device=qkv.device)
-                qlay = _lib.CottLayout(N * 2 * H * D, D, 2 * H * D, 0, 0, 0)
-                st = L.cott_rotary_copy(_lib.ptr(q), _lib.ptr(k), _lib.ptr(rqk[:, :, 0]), _lib.ptr(rqk[:, :, 1]), _lib.ptr(sin), _lib.ptr(cos),
-                                        ctypes.byref(lay), ctypes.byref(qlay), B, H, N, D, 2 * sin.shape[-1], _table_stride(sin, N), code, stream)
-                _lib.check(st, "cott_rotary_copy")
+            if sin is not None:
+                rqk, qlay = _rotated_copy(qkv, sin, cos, lay)
                 q, k = rqk[:, :, 0], rqk[:, :, 1]
             st = L.cott_cos_attn_fwd_split(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kp), _lib.ptr(nc), _lib.ptr(out), _lib.ptr(ws), nseg,
                                            ctypes.byref(lay), None if qlay is None else ctypes.byref(qlay), B, H, N, D, D, code, stream)
         _lib.check(st, "cott_cos_attn_fwd_split")
-        ctx.save_for_backward(qkv, nc, sin, cos, rqk)
+        ctx.save_for_backward(qkv, nc, sin, cos, rqk if keep_rotated else None)
         ctx.ws, ctx.nseg, ctx.kp, ctx.lay, ctx.qlay = ws, nseg, kp, lay, qlay
         ctx.nc_shape, ctx.nc_dtype = norm_const.shape, norm_const.dtype
         return out
@@ -172,8 +180,10 @@ class _FusedCausalPacked(torch.autograd.Function):
         dnc = torch.empty(H, dtype=torch.float32, device=qkv.device)
         L = _lib.lib()
         code, stream = _lib.DTYPE_CODE[qkv.dtype], _lib.stream_ptr(qkv.device)
-        q, k = (qkv[:, :, 0], qkv[:, :, 1]) if rqk is None else (rqk[:, :, 0], rqk[:, :, 1])
         with torch.cuda.device(qkv.device):
+            if sin is not None and rqk is None:
+                rqk, _ = _rotated_copy(qkv, sin, cos, ctx.lay)
+            q, k = (qkv[:, :, 0], qkv[:, :, 1]) if rqk is None else (rqk[:, :, 0], rqk[:, :, 1])
             st = L.cott_cos_attn_bwd_split(
                 _lib.ptr(q), _lib.ptr(k), _lib.ptr(qkv[:, :, 2]), _lib.ptr(ctx.kp), _lib.ptr(nc), _lib.ptr(dout), _lib.ptr(ctx.ws), ctx.nseg,
                 ctypes.byref(ctx.lay), None if rqk is None else ctypes.byref(ctx.qlay), _lib.ptr(dqkv[:, :, 0]), _lib.ptr(dqkv[:, :, 1]),
@@ -183,10 +193,10 @@ class _FusedCausalPacked(torch.autograd.Function):
                 st = L.cott_rotary(_lib.ptr(dqkv[:, :, 0]), _lib.ptr(dqkv[:, :, 1]), _lib.ptr(sin), _lib.ptr(cos), ctypes.byref(ctx.lay), B, H, N, D,
                                    2 * sin.shape[-1], _table_stride(sin, N), 1, code, stream)
                 _lib.check(st, "cott_rotary")
-        return dqkv, dnc.reshape(ctx.nc_shape).to(ctx.nc_dtype), None, None, None
+        return dqkv, dnc.reshape(ctx.nc_shape).to(ctx.nc_dtype), None, None, None, None
 
 
-def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None):
+def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None, keep_rotated=True):
     """Causal cosine attention on a packed ``[B, N, 3, H, 64]`` bf16 / fp16 tensor (the reshaped output of one QKV
     projection); returns ``[B, N, H, 64]`` (reshape to ``[B, N, H*64]`` for the output projection).  Same function
     as ``cos_attn_causal`` on the permuted tensors, without the permute copies in either direction.
@@ -194,36 +204,25 @@ def cos_attn_causal_packed(qkv, norm_const, keep=None, rotary=None):
     ``rotary=(sin, cos)`` -- fp32 ``[N, rot/2]`` or ``[B, N, rot/2]``, the two halves of the module's
     ``embed_positions`` gathered at ``position_ids`` (GPTCosAttention.py:458-476) -- applies the rotary embedding to
     q and k: the same bits as ``rotary_packed_`` followed by this op, and ``qkv`` itself is left as the projection wrote
-    it.  The rotated q and k go to a buffer that is kept for the backward (two thirds of ``qkv``), and dq and dk are
-    rotated back in place.  (Inside the kernels, ``cott_cos_attn_fwd_rotary`` / ``_bwd_rotary``, the rotation needs neither
-    buffer nor passes but sits on the chunk chain of all three kernels: 109 us for B 8, H 16, N 1024 forward and backward against 78 us with
-    the passes.)
-    The rotary dim must be a multiple of 16; sequences that this op would cut into segments (few heads, very long N) are
-    rotated in ``qkv`` itself instead."""
+    it.  The rotary dim must be a multiple of 8.  The rotated q and k are a copy, two thirds of ``qkv``, and dq and dk are
+    rotated back in place.  ``keep_rotated`` holds that copy for the backward; without it nothing beyond ``qkv`` is held
+    and the backward makes the copy again (one more pass over q and k, 10.6 us for B 8, H 16, N 1024).
+    (Inside the kernels, ``cott_cos_attn_fwd_rotary`` / ``_bwd_rotary``, the rotation needs neither copy nor passes but sits on
+    the chunk chain of all three kernels: 109 us for these sizes forward and backward against 78 us with the passes.)"""
     if not qkv.is_cuda:
         raise RuntimeError("cos_attn_causal_packed needs a CUDA tensor (there is no CPU path)")
     if qkv.dim() != 5 or qkv.shape[2] != 3 or qkv.shape[-1] != 64 or qkv.dtype not in FUSED_DTYPES:
         raise RuntimeError("cos_attn_causal_packed takes a [B, N, 3, H, 64] bfloat16 / float16 tensor")
+    sin = cos = None
+    if rotary is not None:
+        sin, cos = (t.to(device=qkv.device, dtype=torch.float32).contiguous() for t in rotary)
+        B, N = qkv.shape[:2]
+        if sin.shape != cos.shape or sin.shape[-2] != N or (sin.dim() == 3 and sin.shape[0] not in (1, B)):
+            raise RuntimeError("sin / cos must be [N, rot/2] or [B, N, rot/2]")
     m = _binding.autograd()
-    if rotary is None:
-        return m.causal_packed(qkv, norm_const, keep, None, None) if m is not None else _FusedCausalPacked.apply(qkv, norm_const, keep)
-    sin, cos = rotary
-    sin = sin.to(device=qkv.device, dtype=torch.float32).contiguous()
-    cos = cos.to(device=qkv.device, dtype=torch.float32).contiguous()
-    B, N, _, H, _ = qkv.shape
-    if sin.shape != cos.shape or sin.shape[-2] != N or (sin.dim() == 3 and sin.shape[0] not in (1, B)):
-        raise RuntimeError("sin / cos must be [N, rot/2] or [B, N, rot/2]")
     if m is not None:
-        one_segment = m.seg_count(qkv, B, H, N) == 1
-    else:
-        with torch.cuda.device(qkv.device):
-            one_segment = _lib.lib().cott_cos_attn_seg_choice(B, H, N) == 1
-    if (2 * sin.shape[-1]) % 16 or not one_segment:
-        qkv = rotary_packed_(qkv.contiguous(), sin, cos)
-        return m.causal_packed(qkv, norm_const, keep, None, None) if m is not None else _FusedCausalPacked.apply(qkv, norm_const, keep)
-    if m is not None:
-        return m.causal_packed(qkv, norm_const, keep, sin, cos)
-    return _FusedCausalPacked.apply(qkv, norm_const, keep, sin, cos)
+        return m.causal_packed(qkv, norm_const, keep, sin, cos, bool(keep_rotated))
+    return _FusedCausalPacked.apply(qkv, norm_const, keep, sin, cos, bool(keep_rotated))
 
 
 class _RotaryPacked(torch.autograd.Function):

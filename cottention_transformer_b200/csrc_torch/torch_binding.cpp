@@ -276,7 +276,7 @@ struct Packed {
 };
 struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
   static Variable forward(AutogradContext* ctx, const at::Tensor& qkv_, const at::Tensor& norm_const, const OptTensor& keep,
-                          const OptTensor& sin, const OptTensor& cos) {
+                          const OptTensor& sin, const OptTensor& cos, bool keep_rotated) {
     const Packed p(qkv_.contiguous());
     const c10::cuda::CUDAGuard guard(p.qkv.device());
     const at::Tensor nc = nc_at_least(norm_const, p.qkv, p.H);
@@ -284,18 +284,14 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
     at::Tensor out = at::empty({p.B, p.N, p.H, p.D}, p.qkv.options());
     const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
     const bool rot = has(sin);
-    const int nseg = rot ? 1 : cott_cos_attn_seg_choice(B, H, N);
+    const int nseg = cott_cos_attn_seg_choice(B, H, N);
     at::Tensor ws = bytes_like(p.qkv, cott_cos_attn_seg_workspace_bytes(B, H, N, nseg));
-    at::Tensor rqk;  // the rotated q and k, [B, N, 2, H, D]
-    if (rot) {
-      rqk = at::empty({p.B, p.N, 2, p.H, p.D}, p.qkv.options());
-      rotate(p, rqk, *sin, *cos, false);
-    }
+    const at::Tensor rqk = rot ? rotated(p, *sin, *cos) : at::Tensor();
     const cott_layout ql = qk_layout(p);
     check(cott_cos_attn_fwd_split(rot ? rqk.data_ptr() : p.part(0), rot ? k_of(rqk, p) : p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(),
                                   out.data_ptr(), ws.data_ptr(), nseg, &p.lay, rot ? &ql : nullptr, B, H, N, D, D, code, stream_of(p.qkv)),
           "cott_cos_attn_fwd_split");
-    ctx->save_for_backward({p.qkv, nc, rot ? *sin : at::Tensor(), rot ? *cos : at::Tensor(), rqk});
+    ctx->save_for_backward({p.qkv, nc, rot ? *sin : at::Tensor(), rot ? *cos : at::Tensor(), keep_rotated ? rqk : at::Tensor()});
     ctx->saved_data["ws"] = ws;
     ctx->saved_data["nseg"] = (int64_t)nseg;
     save_opt(ctx, "keep", kp);
@@ -304,21 +300,22 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
   }
   static cott_layout qk_layout(const Packed& p) { return cott_layout{p.N * 2 * p.H * p.D, p.D, 2 * p.H * p.D, 0, 0, 0}; }
   static void* k_of(const at::Tensor& rqk, const Packed& p) { return static_cast<char*>(rqk.data_ptr()) + p.H * p.D * p.e; }
-  // q and k of `p` rotated into rqk, or (inverse) the gradients in `p` rotated back in place
-  static void rotate(const Packed& p, const at::Tensor& rqk, const at::Tensor& sin, const at::Tensor& cos, bool inverse) {
-    const int64_t half = sin.size(-1);
-    const long long stride = sin.dim() == 3 && sin.size(0) > 1 ? (long long)(p.N * half) : 0;
-    const int B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D, code = dtype_code(p.qkv.scalar_type());
-    if (inverse) {
-      check(cott_rotary(p.part(0), p.part(1), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, B, H, N, D, (int)(2 * half), stride, 1, code,
-                        stream_of(p.qkv)),
-            "cott_rotary");
-      return;
-    }
+  static long long table_stride(const Packed& p, const at::Tensor& sin) { return sin.dim() == 3 && sin.size(0) > 1 ? (long long)(p.N * sin.size(-1)) : 0; }
+  // q and k of `p`, rotated: [B, N, 2, H, D]
+  static at::Tensor rotated(const Packed& p, const at::Tensor& sin, const at::Tensor& cos) {
+    at::Tensor rqk = at::empty({p.B, p.N, 2, p.H, p.D}, p.qkv.options());
     const cott_layout ql = qk_layout(p);
-    check(cott_rotary_copy(p.part(0), p.part(1), rqk.data_ptr(), k_of(rqk, p), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, &ql, B, H, N, D,
-                           (int)(2 * half), stride, code, stream_of(p.qkv)),
+    check(cott_rotary_copy(p.part(0), p.part(1), rqk.data_ptr(), k_of(rqk, p), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, &ql, (int)p.B,
+                           (int)p.H, (int)p.N, (int)p.D, (int)(2 * sin.size(-1)), table_stride(p, sin), dtype_code(p.qkv.scalar_type()),
+                           stream_of(p.qkv)),
           "cott_rotary_copy");
+    return rqk;
+  }
+  // the gradients of the rotated q and k in `p`, back through the rotation in place
+  static void rotate_back(const Packed& p, const at::Tensor& sin, const at::Tensor& cos) {
+    check(cott_rotary(p.part(0), p.part(1), sin.data_ptr<float>(), cos.data_ptr<float>(), &p.lay, (int)p.B, (int)p.H, (int)p.N, (int)p.D,
+                      (int)(2 * sin.size(-1)), table_stride(p, sin), 1, dtype_code(p.qkv.scalar_type()), stream_of(p.qkv)),
+          "cott_rotary");
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
@@ -329,13 +326,14 @@ struct CausalPackedFn : torch::autograd::Function<CausalPackedFn> {
     at::Tensor dnc = at::empty({p.H}, p.qkv.options().dtype(at::kFloat));
     const int code = dtype_code(p.qkv.scalar_type()), B = (int)p.B, H = (int)p.H, N = (int)p.N, D = (int)p.D;
     const bool rot = s[2].defined();
+    const at::Tensor rqk = !rot || s[4].defined() ? s[4] : rotated(p, s[2], s[3]);
     const cott_layout ql = qk_layout(p);
-    check(cott_cos_attn_bwd_split(rot ? s[4].data_ptr() : p.part(0), rot ? k_of(s[4], p) : p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(),
+    check(cott_cos_attn_bwd_split(rot ? rqk.data_ptr() : p.part(0), rot ? k_of(rqk, p) : p.part(1), p.part(2), u8(kp), nc.data_ptr<float>(),
                                   dout.data_ptr(), ws.data_ptr(), (int)ctx->saved_data["nseg"].toInt(), &p.lay, rot ? &ql : nullptr, d.part(0),
                                   d.part(1), d.part(2), dnc.data_ptr<float>(), B, H, N, D, D, code, stream_of(p.qkv)),
           "cott_cos_attn_bwd_split");
-    if (rot) rotate(d, at::Tensor(), s[2], s[3], true);
-    return {d.qkv, nc_grad(ctx, dnc), Variable(), Variable(), Variable()};
+    if (rot) rotate_back(d, s[2], s[3]);
+    return {d.qkv, nc_grad(ctx, dnc), Variable(), Variable(), Variable(), Variable()};
   }
 };
 struct BidirPackedFn : torch::autograd::Function<BidirPackedFn> {
@@ -544,8 +542,9 @@ at::Tensor cos_attn_wide(const at::Tensor& q, const at::Tensor& k, const at::Ten
 at::Tensor cos_attn_f32(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& norm_const, const OptTensor& keep) {
   return F32Fn::apply(q, k, v, norm_const.clone(), has(keep) ? OptTensor(keep->clone(at::MemoryFormat::Contiguous)) : OptTensor());
 }
-at::Tensor causal_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep, const OptTensor& sin, const OptTensor& cos) {
-  return CausalPackedFn::apply(qkv, norm_const, keep, sin, cos);
+at::Tensor causal_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep, const OptTensor& sin, const OptTensor& cos,
+                         bool keep_rotated) {
+  return CausalPackedFn::apply(qkv, norm_const, keep, sin, cos, keep_rotated);
 }
 at::Tensor bidir_packed(const at::Tensor& qkv, const at::Tensor& norm_const, const OptTensor& keep) {
   return BidirPackedFn::apply(qkv, norm_const, keep);
@@ -574,10 +573,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // Without the interpreter lock, as calls through ctypes and torch.ops run: a launch may wait for room in the stream's
   // queue, and what the queue waits for may be another Python thread.
   using Unlocked = py::call_guard<py::gil_scoped_release>;
-  m.def("seg_count", [](const at::Tensor& t, int64_t B, int64_t H, int64_t N) {
-    const c10::cuda::CUDAGuard guard(t.device());
-    return cott_cos_attn_seg_choice((int)B, (int)H, (int)N);
-  });
   m.def("cos_attn_causal", &cos_attn_causal, Unlocked());
   m.def("cos_attn_wide", &cos_attn_wide, Unlocked());
   m.def("cos_attn_f32", &cos_attn_f32, Unlocked());

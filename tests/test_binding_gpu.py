@@ -53,8 +53,7 @@ def test_same_bits_as_the_python_functions(name, dt, masked, monkeypatch):
         leaf = [t.clone().requires_grad_() for t in x]
         ncl = nc.clone().requires_grad_()
         k = keep.clone() if masked else None
-        src = [t * 1 for t in leaf] if name == "rotary" else leaf  # (few heads: the rotary embedding works in place)
-        out = _call(name, src, ncl, k, rot_args)
+        out = _call(name, leaf, ncl, k, rot_args)
         if masked:
             k.fill_(True)  # what the caller does to its mask afterwards is not the backward's business
         wrt = leaf if name == "dropin" else [*leaf, ncl]
@@ -183,6 +182,31 @@ def test_short_norm_const_is_refused():
     tok = torch.randn(1, 3, 1, 64, device="cuda").bfloat16()
     with pytest.raises(RuntimeError, match="one entry per head"):
         CosAttnDecodeState(1, 3, 64).step(tok, tok, tok, nc[:, :2])
+
+
+@pytest.mark.parametrize("compiled", [True, False])
+@pytest.mark.parametrize("keep_rotated", [True, False])
+@pytest.mark.parametrize("B,H,N,rot,segments", [(2, 3, 150, 32, 1), (1, 2, 4100, 64, 2), (1, 3, 5000, 24, 2), (1, 8, 300, 8, 1)])
+def test_rotary_leaves_the_projection_alone(B, H, N, rot, segments, keep_rotated, compiled, monkeypatch):
+    """Whatever the sizes: cut into segments or not, rotary dims that are no multiple of 16 included."""
+    from cottention_transformer_b200 import _binding, _lib, cos_attn_causal_packed, rotary_packed_
+    if not compiled:
+        monkeypatch.setattr(_binding, "autograd", lambda: None)
+    assert (_lib.lib().cott_cos_attn_seg_choice(B, H, N) > 1) == (segments > 1)
+    g = torch.Generator(device="cuda").manual_seed(N + rot)
+    qkv = torch.randn(B, N, 3, H, 64, device="cuda", generator=g).bfloat16()
+    do = torch.randn(B, N, H, 64, device="cuda", generator=g).bfloat16()
+    nc = torch.full((H,), 0.5, device="cuda")
+    ang = torch.rand(N, rot // 2, device="cuda", generator=g) * 6
+    sc = (torch.sin(ang), torch.cos(ang))
+    leaf = qkv.clone().requires_grad_()
+    out = cos_attn_causal_packed(leaf, nc, rotary=sc, keep_rotated=keep_rotated)
+    (dx,) = torch.autograd.grad(out, leaf, do)
+    assert torch.equal(leaf, qkv)
+    other = qkv.clone().requires_grad_()
+    want = cos_attn_causal_packed(rotary_packed_(other * 1, *sc), nc)
+    (dw,) = torch.autograd.grad(want, other, do)
+    assert torch.equal(out, want) and torch.equal(dx, dw)
 
 
 @pytest.mark.parametrize("compiled", [True, False])
