@@ -58,6 +58,7 @@ struct SegPlan {
 TileStrides in_strides(const SegPlan& p, long H, long N) { return p.in.n ? p.in : contiguous_bhnd(H, N); }
 TileStrides qk_strides(const SegPlan& p, long H, long N) { return p.qk.n ? p.qk : in_strides(p, H, N); }
 TileStrides out_strides(const SegPlan& p, long H, long N) { return p.out.n ? p.out : contiguous_bhnd(H, N); }
+constexpr long kMaxGridY = 65535;  // (segments that a caller asks for may be that many: N of 4 million positions and more)
 SegPlan plan_segments(int N, int nseg_requested) {
   const int total = (N + kTcChunk - 1) / kTcChunk;
   SegPlan p;
@@ -193,7 +194,7 @@ int launch_bwd(const void* q, const void* k, const void* v, const float* nc, con
                SegPlan plan = SegPlan()) {
   COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
   // (the rotation inside the kernels has a dK/dV kernel with a warp group of its own)
-  if (!plan.rot.sin && bwd_side_by_side({q, k, v, dout}, dq, dk, dv))
+  if (!plan.rot.sin && 2l * plan.nseg <= kMaxGridY && bwd_side_by_side({q, k, v, dout}, dq, dk, dv))
     return launch_bwd_both<T>(q, k, v, nc, dout, dq, dk, dv, dnorm, B, H, N, dtype, stream, prefix, suffix, plan);
   plan.dnorm_zeroed = true;
   int st = launch_bwd_dq<T>(q, k, v, nc, dout, dq, B, H, N, dtype, stream, prefix, plan);
@@ -231,7 +232,7 @@ int launch_bwd_fused(const void* q, const void* k, const void* v, const float* n
 // state[bh][seg] of every segment: Y^T Z with one operand row-scaled (see seg_state_kernel)
 // Two CTAs per segment where it has the chunks for them: the kernel only streams (two stages of 32 KB and an M = 64 MMA),
 // two of its CTAs fit an SM, and one per SM left the memory half idle (B 1, H 16, N 65536: 66 -> 48 us).
-int seg_parts(const SegPlan& plan) { return plan.cps >= 4 ? 2 : 1; }
+int seg_parts(const SegPlan& plan) { return plan.cps >= 4 && 2l * plan.nseg <= kMaxGridY ? 2 : 1; }
 template <typename T, int MODE>
 int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides sz, const float* nc, float* state, int B,
                      int H, int N, int dtype, SegPlan plan, int parts, cudaStream_t stream) {

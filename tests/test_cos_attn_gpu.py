@@ -468,3 +468,20 @@ def test_backward_over_its_inputs(B, H, N, masked, nseg):
         dqk = torch.empty_like(q)
         got = run(x, dqk, dqk, torch.empty_like(q))
         assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+
+
+def test_more_segments_than_half_a_grid_dimension():
+    """33000 segments of one chunk: forward and backward launch, with the result of the library's own choice."""
+    from cottention_transformer_b200 import _lib, cos_attn_causal
+    N = 33000 * 128
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v, do = (torch.randn(1, 1, N, 64, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(4))
+    nc = torch.full((1,), 0.5, device="cuda")
+    res = []
+    for segments in (33000, None):
+        leaf = [t.detach().requires_grad_() for t in (q, k, v)]
+        out = cos_attn_causal(*leaf, nc, segments=segments)
+        res.append((out.detach(), *torch.autograd.grad(out, leaf, do)))
+    _lib.check_device_status()
+    for a, b in zip(*res):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= REL16
