@@ -245,13 +245,13 @@ int cott_cos_attn_f32_bwd(const float* q, const float* k, const float* v, const 
  * 128 (a state-only pass of the 128-wide kernel; `nseg` is ignored, `workspace` is
  * cott_cos_attn_wide_workspace_bytes(B, H, N) bytes, the outputs come from cott_cos_attn_wide_fwd).
  */
+int cott_cos_attn_prefill_state(const void* k, const void* v, const float* norm_const, float* state,
+                                void* workspace, int nseg, int accumulate, int B, int H, int N, int Dk, int Dv,
+                                int dtype, void* stream);
 /* The same with the prompt's outputs in the same call (cott_cos_attn_fwd(_seg) / cott_cos_attn_wide_fwd and the state, which
  * the last CTA of every sequence stores): `state` is overwritten.  `nseg`, `workspace`: as in cott_cos_attn_prefill_state. */
 int cott_cos_attn_prefill(const void* q, const void* k, const void* v, const float* norm_const, void* out, float* state,
                           void* workspace, int nseg, int B, int H, int N, int Dk, int Dv, int dtype, void* stream);
-int cott_cos_attn_prefill_state(const void* k, const void* v, const float* norm_const, float* state,
-                                void* workspace, int nseg, int accumulate, int B, int H, int N, int Dk, int Dv,
-                                int dtype, void* stream);
 
 /*
  * Recurrent decode.  Per (batch, head) a float32 state[b,h,j,i] ([B,H,Dv,Dk], updated in place) is

@@ -122,6 +122,12 @@ def test_segment_plan_is_host_arithmetic(lib):
     assert L.cott_cos_attn_seg_count(1, 16, 262144) == 9        # 16 heads -> 9 segments each (144 CTAs)
     assert L.cott_cos_attn_seg_count(1, 1, 256) == 1            # two chunks: nothing to cut
     assert L.cott_cos_attn_seg_count(1, 1, 1024) == 4           # at least two chunks per segment
+    # what the operators go by: all of them where the cut pays, one where its set-up costs more
+    assert L.cott_cos_attn_seg_choice(1, 16, 262144) == 9
+    assert L.cott_cos_attn_seg_choice(1, 16, 8192) == 9
+    assert L.cott_cos_attn_seg_choice(2, 16, 1024) == 1
+    assert L.cott_cos_attn_seg_choice(8, 16, 4096) == 1
+    assert L.cott_cos_attn_seg_choice(0, 16, 4096) == L.cott_cos_attn_seg_choice(1, 1, 0) == 1
     n = L.cott_cos_attn_seg_workspace_bytes(1, 16, 262144, 9)
     assert n == 5 * 16 * 9 * 64 * 64 * 4 + 262144 * 4
     # a segment count the sequence cannot use is clamped (1000 tokens = 8 chunks -> at most 8 segments)

@@ -37,3 +37,29 @@ def test_prefill_outputs_and_state(B, H, N, D):
                                                                torch.nn.functional.normalize(kn[:, :, 0].double(), dim=-1))
     want = torch.einsum("bhji,bhi->bhj", S, torch.nn.functional.normalize(qn[:, :, 0].double(), dim=-1))
     assert _rel(nxt[:, :, 0], want) <= REL16
+
+
+@pytest.mark.parametrize("accumulate", [0, 1])
+@pytest.mark.parametrize("D,B,H,N,nseg", [(64, 2, 3, 1, 1), (64, 1, 2, 777, 1), (64, 2, 2, 1300, 3), (64, 1, 3, 5000, 20), (128, 2, 3, 130, 1),
+                                          (128, 1, 2, 1, 1), (128, 1, 1, 1001, 0), (128, 1, 3, 5000, 0)])
+def test_state_of_a_prompt_by_itself(D, B, H, N, nseg, accumulate):
+    """``cott_cos_attn_prefill_state``: one and several segments, the last one ragged, over a state and added to it.  (Head
+    dim 128 chooses its segments itself.)"""
+    from cottention_transformer_b200 import _lib
+    L, P = _lib.lib(), _lib.ptr
+    g = torch.Generator().manual_seed(N + D)
+    k, v = (torch.randn(B, H, N, D, generator=g).bfloat16() for _ in range(2))
+    nc = 0.5 + 0.2 * torch.randn(H, generator=g)
+    before = torch.randn(B, H, D, D, generator=g)
+    state, kd, vd, ncd = before.cuda(), k.cuda(), v.cuda(), nc.cuda()
+    nbytes = L.cott_cos_attn_wide_workspace_bytes(B, H, N) if D == 128 else L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    _lib.check(L.cott_cos_attn_prefill_state(P(kd), P(vd), P(ncd), P(state), P(ws), nseg, accumulate, B, H, N, D, D, 3,
+                                             _lib.stream_ptr(state.device)), "prefill_state")
+    _lib.check_device_status()
+    n = torch.arange(1, N + 1).double().view(1, 1, N, 1)
+    vp = v.double() / n ** torch.sigmoid(nc.double()).view(1, H, 1, 1)
+    want = torch.einsum("bhnj,bhni->bhji", vp, torch.nn.functional.normalize(k.double(), dim=-1))
+    # (what was there before enters with 1, exactly: the tolerance is that of the products)
+    got = state.double().cpu() - (before.double() if accumulate else 0)
+    assert ((got - want).norm() / want.norm()).item() <= REL16
