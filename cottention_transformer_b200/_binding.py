@@ -14,6 +14,7 @@ import os
 _PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cott_torch_binding.so")
 _mod = None
 _tried = False
+_looks = None
 
 
 def module():
@@ -34,10 +35,14 @@ def transformed() -> bool:
     """Whether something looks at a Python function and its operators, or refuses them by name, and would not see the nodes
     of the compiled module: tracing, compilation, functorch transforms, forward-mode differentiation, dispatch modes (which
     count, record or choose operators, as selective checkpointing does)."""
-    import torch
-    C = torch._C
-    return (torch.compiler.is_compiling() or C._get_tracing_state() is not None or C._functorch.peek_interpreter_stack() is not None
-            or C._len_torch_dispatch_stack() > 0 or torch.autograd.forward_ad._current_level >= 0)
+    global _looks
+    if _looks is None:  # (bound once: this runs before every call)
+        import torch
+        from torch.autograd import forward_ad
+        C = torch._C
+        _looks = torch.compiler.is_compiling, C._get_tracing_state, C._functorch.peek_interpreter_stack, C._len_torch_dispatch_stack, forward_ad
+    compiling, tracing, functorch, modes, fw = _looks
+    return compiling() or tracing() is not None or functorch() is not None or modes() > 0 or fw._current_level >= 0
 
 
 def autograd():
