@@ -11,10 +11,15 @@ from __future__ import annotations
 import importlib.util
 import os
 
+import torch
+from torch.autograd import forward_ad as _fw
+
 _PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cott_torch_binding.so")
 _mod = None
 _tried = False
-_looks = None
+# (bound here: transformed() runs before every call)
+_compiling, _tracing, _functorch, _modes = (torch.compiler.is_compiling, torch._C._get_tracing_state, torch._C._functorch.peek_interpreter_stack,
+                                            torch._C._len_torch_dispatch_stack)
 
 
 def module():
@@ -23,7 +28,6 @@ def module():
     if not _tried:
         _tried = True
         if os.path.exists(_PATH) and os.environ.get("COTT_NO_TORCH_BINDING", "") != "1":
-            import torch  # noqa: F401  (libtorch must be loaded first)
             spec = importlib.util.spec_from_file_location("cott_torch_binding", _PATH)
             mod = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(mod)  # also registers torch.ops.cottention_b200.*
@@ -35,14 +39,7 @@ def transformed() -> bool:
     """Whether something looks at a Python function and its operators, or refuses them by name, and would not see the nodes
     of the compiled module: tracing, compilation, functorch transforms, forward-mode differentiation, dispatch modes (which
     count, record or choose operators, as selective checkpointing does)."""
-    global _looks
-    if _looks is None:  # (bound once: this runs before every call)
-        import torch
-        from torch.autograd import forward_ad
-        C = torch._C
-        _looks = torch.compiler.is_compiling, C._get_tracing_state, C._functorch.peek_interpreter_stack, C._len_torch_dispatch_stack, forward_ad
-    compiling, tracing, functorch, modes, fw = _looks
-    return compiling() or tracing() is not None or functorch() is not None or modes() > 0 or fw._current_level >= 0
+    return _compiling() or _tracing() is not None or _functorch() is not None or _modes() > 0 or _fw._current_level >= 0
 
 
 def autograd():
@@ -55,5 +52,4 @@ def ops():
     """``torch.ops.cottention_b200`` when the binding is loaded, else None."""
     if module() is None:
         return None
-    import torch
     return torch.ops.cottention_b200
