@@ -236,7 +236,7 @@ def bench_long_context(N, B=1, H=16, d=64, iters=5):
     nc, dnc = 0.5 * torch.ones(H, device=dev), torch.empty(H, device=dev)
     st = _lib.stream_ptr(dev)
     P = lambda t: t.data_ptr()  # noqa: E731
-    nseg = L.cott_cos_attn_seg_count(B, H, N)
+    nseg = L.cott_cos_attn_seg_choice(B, H, N)
     ws = torch.empty(max(L.cott_cos_attn_seg_workspace_bytes(B, H, N, nseg), 16), dtype=torch.uint8, device=dev)
 
     def step(n):
@@ -256,8 +256,8 @@ def bench_long_context(N, B=1, H=16, d=64, iters=5):
 
 
 def bench_long_context_d128(N, B=1, H=16, d=128, iters=5):
-    """Head dim 128 has no fused kernel: ``cos_attn_causal`` keeps the row factors in fp32 outside four tensor-core
-    scans that run as 64-wide launches (``_WideCausal``)."""
+    """The same at head dim 128, through ``cos_attn_causal`` with its autograd step (the fused 128-wide kernels, which choose
+    their segments themselves)."""
     from .cos_attention import cos_attn_causal
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(1234)
@@ -310,7 +310,7 @@ def bench_prefill_sharded(N, d, world=1, rank=0, iters=3, H=16):
 
 def bench_one_pass(B=8, H=16, N=4096, d=64, iters=20):
     """The two backward routes at the headline shape, kernels only through the C ABI: forward / forward that also keeps
-    its chunk states, and the two-kernel backward / the one-pass backward that reads those states."""
+    its chunk states, and the two-pass backward / the one-pass backward that reads those states."""
     L = _lib.lib()
     dev = torch.device("cuda", torch.cuda.current_device())
     g = torch.Generator(device=dev).manual_seed(1234)

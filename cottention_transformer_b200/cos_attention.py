@@ -8,8 +8,8 @@ differentiable w.r.t. q, k, v and ``norm_const``.
 
 Two modes, chosen by dtype (not a fallback chain -- each mode is a CUDA path of this library):
 
-* float16 / bfloat16, head dim 64, no padding mask: ONE fused tensor-core kernel for the forward
-  (``cott_cos_attn_fwd``) and two for the backward (``cott_cos_attn_bwd``), fp32 accumulation;
+* float16 / bfloat16, head dim 64 (with a padding mask the running count of kept positions is a launch more): ONE fused tensor-core kernel for the forward
+  (``cott_cos_attn_fwd``) and one launch for the backward (``cott_cos_attn_bwd``), fp32 accumulation;
 * float16 / bfloat16, head dim 128: the fused head-dim-128 kernels (``cott_cos_attn_wide_fwd`` / ``_bwd``);
 * float16 / bfloat16, head dim 192 / 256: the row factors pulled out of the scan, tensor-core scans on
   64-wide slices of the head dimension, closed-form backward (``_WideCausal``);
@@ -474,7 +474,7 @@ def cos_attn_causal(q, k, v, norm_const, keep=None, segments=None, one_pass_back
     same results); ``None`` lets the library choose -- more than one only for few (batch, head) pairs.
     ``one_pass_backward`` (fused path only): the forward also keeps its 16-bit chunk states (half the size of q) and
     the backward is one kernel that reads every tensor once (``cott_cos_attn_fwd_train`` / ``_bwd_train``) instead
-    of two kernels that each read all four: 7.5 instead of 11 tensor passes of HBM traffic at about the same run
+    of two passes that each read all four: 7.5 instead of 11 tensor passes of HBM traffic at about the same run
     time on an otherwise idle B200.
     """
     if not (q.is_cuda and k.is_cuda and v.is_cuda):

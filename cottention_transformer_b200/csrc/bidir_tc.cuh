@@ -16,7 +16,7 @@
 //   S = K^T Zw,  D = Qw^T dO;   out = (Q S) keep/|q|;
 //   AccQ = dO S^T,  AccK = Zw D^T = dk^/|k|,  AccV = K D = |k| dv'
 //   dq = keep/|q| (AccQ - q^ (q^.AccQ)),  dk = AccK - k^ (k^.AccK),  dv = w AccV,  v'.dv' = w (v . AccV)
-// Roles: warp 0 lane 0 = TMA loads and stores, warp 1 lane 0 = MMA issue, warps 2-5 = the per-row work
+// Roles: one thread of warp 0 = TMA loads and stores, one of warp 1 = MMA issue, warps 2-5 = the per-row work
 // (row norms, operand scaling in place, state conversion, output rows staged in place over an input
 // tile and stored by TMA).  Every wait is bounded (see causal_tc.cuh).
 #pragma once
@@ -235,7 +235,7 @@ bidir_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
 // bit per stage.
 // TMEM (512 columns): S 64 | D 64 | 2 x (AccQ 64 | AccK 64 | AccV 64) -- the accumulators are double-buffered, so the
 // MMAs of the next chunk run while the rows of this one are written (the second pass is a chain MMAs -> rows otherwise)
-// Warps: 0 = TMA (lane 0), 1 = MMA issue (lane 0), three groups of four (each warp works on the tile rows /
+// Warps: 0 = TMA (one thread), 1 = MMA issue (one thread), three groups of four (each warp works on the tile rows /
 // TMEM lanes 32 (w % 4) ..).  First pass: group 0 (warps 2-5) builds Qw, group 1 (6-9) Zw, in place, and both leave
 // their row factors.  Second pass: group 0 writes the dv rows (and, for a reloaded chunk, the row factors first),
 // group 1 the dq rows, group 2 (10-13) the dk rows.

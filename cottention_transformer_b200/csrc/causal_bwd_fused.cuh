@@ -2,7 +2,7 @@
 // the length-norm parameter from a single read of q, k, v, dO (tcgen05 + TMEM + TMA).
 //
 // The reference's backward is three scans (Cuda_Kernel/Custom_Kernel.py:106-108): dQ needs the state of
-// everything BEFORE a position, dK and dV the state of everything AFTER it, which is why two kernels walking in
+// everything BEFORE a position, dK and dV the state of everything AFTER it, which is why two passes walking in
 // opposite directions each had to read all four tensors.  Here the forward pass leaves its 16-bit state operand
 // of every chunk in HBM (8 KB per 128 positions: half a tensor pass, `saved`), so the prefix state is a TMA load
 // away and one reverse walk does everything (the reference's own unused sketch of a merged backward,
@@ -184,12 +184,12 @@ causal_bwd_fused_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
   auto has_s = [&](int ci) { return last_chunk - ci > 0; };
 
   // Roles:
-  //   warp 0, lane 0:   score tiles E, F of item ci+1; state R += Qw^T dO (ci)
-  //   warp 1, lane 0:   accumulators AccQ, AccK, AccV of item ci
+  //   warp 0, one thread:  score tiles E, F of item ci+1; state R += Qw^T dO (ci)
+  //   warp 1, one thread:  accumulators AccQ, AccK, AccV of item ci
   //   warps 2-5:        score group: mask + convert E into shared memory; Vw of the next item
   //   warps 6-9:        dK/dV group: output rows of dV and dK, the norm_const gradient
   //   warps 10-13:      operand group: mask + convert F in TMEM; fp32 R -> 16-bit operand; Qw of the next item
-  //   warp 14, lane 0:  TMA loads and stores
+  //   warp 14, one thread: TMA loads and stores
   //   warps 15-18:      dQ group: output rows of dQ
   constexpr uint32_t kIdescP = make_idesc(128, 128, BF, false, false);
   constexpr uint32_t kIdescKK = make_idesc(128, 64, BF, false, false);  // A K-major, B K-major

@@ -628,13 +628,13 @@ __device__ __forceinline__ void causal_tc_body(const CUtensorMap& mapX, const CU
   // through the mbarriers.  The per-row work is spread over six groups of four warps (warp w of a group
   // owns TMEM lanes / tile rows 32 (w % 4) ..): each group's work per chunk is serial and latency-bound,
   // so the chunk period is set by the busiest group.
-  //   warp 0, lane 0:   scores P(c+1) = X Y^T
-  //   warp 19, lane 0:  state S += Y^T Zw (c)
-  //   warp 1, lane 0:   accumulators Acc(c) = X S + P Zw
+  //   warp 0, one thread:  scores P(c+1) = X Y^T
+  //   warp 19, one thread: state S += Y^T Zw (c)
+  //   warp 1, one thread:  accumulators Acc(c) = X S + P Zw
   //   warps 2-5:        score group: mask + convert P
   //   warps 6-9, 20-23: output groups (even / odd chunks): row norm of q, accumulator -> output rows
   //   warps 10-13:      state group: fp32 state -> 16-bit operand
-  //   warp 14, lane 0:  TMA loads and stores
+  //   warp 14, one thread: TMA loads and stores
   //   warps 15-18, 24-27: operand groups (even / odd chunks): Zw in place
   constexpr uint32_t kIdescP = make_idesc(128, 128, BF, false, false);
   constexpr uint32_t kIdescAcc = make_idesc(128, 64, BF, false, true);
@@ -1029,8 +1029,8 @@ __device__ __forceinline__ void causal_bwd_kv_body(const CUtensorMap& mapQ, cons
 
   // iteration ci handles chunk nchunks-1-ci (the sequence is walked backwards)
   // Two issuing threads (see causal_tc_kernel):
-  //   warp 0, lane 0:  TMA loads, score tiles E, F of chunk ci+1, state R += Qw^T dO (ci)
-  //   warp 1, lane 0:  accumulators AccK, AccV of chunk ci
+  //   warp 0, one thread: TMA loads, score tiles E, F of chunk ci+1, state R += Qw^T dO (ci)
+  //   warp 1, one thread: accumulators AccK, AccV of chunk ci
   constexpr uint32_t kIdescP = make_idesc(128, 128, BF, false, false);
   constexpr uint32_t kIdescAccKK = make_idesc(128, 64, BF, false, false);  // B K-major (V R^T)
   constexpr uint32_t kIdescAccMN = make_idesc(128, 64, BF, false, true);   // B MN-major

@@ -174,13 +174,13 @@ wide_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
   const uint32_t tP0 = tmem, tAcc = tmem + 256, tS = tmem + 384;  // P 2 x 128 | Acc W | S W
 
   // Roles:
-  //   warp 0, lane 0:   scores P(c+1) = X Y^T
-  //   warp 1, lane 0:   accumulators Acc(c) = X S + P Zs
-  //   warp 19, lane 0:  state S += Y^T Zs (c)
+  //   warp 0, one thread:  scores P(c+1) = X Y^T
+  //   warp 1, one thread:  accumulators Acc(c) = X S + P Zs
+  //   warp 19, one thread: state S += Y^T Zs (c)
   //   warps 2-5:        mask group: mask + convert P in TMEM
   //   warps 6-9, 20-23: output groups (panel 0 / panel 1 of the slice): accumulator -> output rows
   //   warps 10-13:      state group: fp32 state -> 16-bit operand
-  //   warp 14, lane 0:  TMA loads and stores
+  //   warp 14, one thread: TMA loads and stores
   //   warps 15-18:      operand group: row norms / row scalings of Y and Z in place
   constexpr uint32_t kIdescP = make_idesc(128, 128, BF, false, false);
   constexpr uint32_t kIdescAcc = make_idesc(128, W, BF, false, true);

@@ -250,7 +250,7 @@ int launch_seg_state(const void* y, const void* z, TileStrides sy, TileStrides s
 
 // workspace of the segment-parallel path: five arrays of B*H*nseg fp32 [64 x 64] matrices, then the running keep count
 //   0, 1 the (half) segments' own states, of the pass that is running | 2 exclusive prefix of the forward ones |
-//   3 exclusive suffix of the reverse ones
+//   3 exclusive suffix of the reverse ones | 4 unused (callers know the size)
 size_t seg_array_floats(int B, int H, int nseg) { return (size_t)B * H * nseg * kTcD * kTcD; }
 int launch_seg_prefix(const float* src, float* dst, long sequences, int nseg, int parts, int elems, bool reverse, cudaStream_t stream) {
   auto kern = reverse ? seg_prefix_kernel<true> : seg_prefix_kernel<false>;

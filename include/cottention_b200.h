@@ -66,7 +66,7 @@ const char* cott_status_string(int status);
  * Memory: unlike the reference's kernel call, which needs no workspace, the tensor-core paths take stream-ordered
  * scratch from a memory pool that the LIBRARY owns and keeps for the life of the process (cudaMallocFromPoolAsync /
  * cudaFreeAsync on `stream`, release threshold = unlimited) in two cases: few (batch, head) pairs with a long sequence
- * (fp32 segment states, 2 x B*H*ceil(Dv/64)*nseg*32 KB) and D_attn = 192 / 256 (one [B,H,N,64] partial result).  The
+ * (fp32 segment states: 3 x B*H*ceil(Dv/64)*nseg*16 KB at D_attn = 64, B*H*nseg*Dv*512 bytes at 128) and D_attn = 192 / 256 (one [B,H,N,64] partial result).  The
  * allocation is visible under stream capture.  Callers that must control every byte use the fused entry points below,
  * which take their workspace from the caller.
  */
@@ -134,7 +134,8 @@ int cott_cos_attn_bwd_dkdv(const void* q, const void* k, const void* v, const fl
  * SMs.  The results are those of cott_cos_attn_fwd / cott_cos_attn_bwd (the state is carried across
  * segment boundaries in fp32; summation order differs).  No counterpart in the reference, whose kernel
  * (combined_kernel_general.cu:96-251) is sequential in N with one block per (batch, head, output column).
- *   cott_cos_attn_seg_count            suggested nseg for this device (1 = use the plain calls)
+ *   cott_cos_attn_seg_count            nseg that the SMs of this device have room for (1 = use the plain calls)
+ *   cott_cos_attn_seg_choice           nseg that pays on this device
  *   cott_cos_attn_seg_workspace_bytes  size of `workspace` (device memory, 16-byte aligned) for that nseg
  *   _fwd_seg writes the segment states into `workspace`; pass the same buffer and nseg, untouched, to _bwd_seg.
  * These two calls also take the padding mask of GPTCosAttention.py:232-248: `keep` ([B, N] bytes, non-zero =
@@ -151,8 +152,8 @@ typedef struct cott_layout { /* element strides of [B, H, N, 64] views whose inn
   long long out_b, out_h, out_n; /* out and dout */
 } cott_layout;
 int cott_cos_attn_seg_count(int B, int H, int N);
-/* The count that is worth it for these sizes: the one above for long sequences, 1 where cutting a sequence costs more
- * than it saves.  The operators of the Python package and cott_scan go by this one. */
+/* seg_count for long sequences, 1 where cutting a sequence costs more than it saves.  The operators of the Python package
+ * and cott_scan go by this one. */
 int cott_cos_attn_seg_choice(int B, int H, int N);
 size_t cott_cos_attn_seg_workspace_bytes(int B, int H, int N, int nseg);
 int cott_cos_attn_fwd_seg(const void* q, const void* k, const void* v, const unsigned char* keep,
@@ -181,7 +182,7 @@ int cott_cos_attn_bwd_split(const void* q, const void* k, const void* v, const u
  * tensor-core products consume it ([B*H][ceil(N/128)][64][64] elements of `dtype`, cott_cos_attn_saved_bytes(B, H, N)
  * bytes = half the size of q; device memory, 16-byte aligned).  cott_cos_attn_bwd_train takes q, k, v, dout and
  * `saved`, untouched, and produces dq, dk, dv, dnorm_const in a single reverse walk over the sequence: every input
- * tensor is read once (7.5 tensor passes against the 11 of cott_cos_attn_bwd, whose two kernels walk in opposite
+ * tensor is read once (7.5 tensor passes against the 11 of cott_cos_attn_bwd, whose two passes walk in opposite
  * directions and each read q, k, v, dout).  Same results as cott_cos_attn_bwd up to rounding.
  * `workspace` is only needed (and only touched) when nseg > 1 or keep != NULL; pass the same buffer to both calls.
  *
