@@ -6,8 +6,7 @@
 //     state[j][i] += v'[j] * k^[i]                                          (:264, layout [d_v, d_k])
 //     out[j]       = sum_i q^[i] * state[j][i]                              (:267)
 // The reference runs this on the CPU in float64 for batch 1; here the state is fp32 in HBM,
-// [B, H, d_v, d_k], updated in place.  One CTA per 16 KB of a (b,h) state (64 rows, at d_k = 128 32 of them: the
-// rows are independent of each other); a row of the state is spread over d_k/4 lanes that each own one float4, so
+// [B, H, d_v, d_k], updated in place.  A CTA owns some rows of a (b,h) state (they are independent of each other); a row of the state is spread over d_k/4 lanes that each own one float4, so
 // every state access is a coalesced 128-bit access and the row dot product is a shuffle reduction.
 //
 // cott_decode_steps runs T consecutive positions in one launch with the state held in registers
@@ -18,14 +17,22 @@
 
 namespace cott {
 
-// Bound by HBM: the state is read and written once.  128 threads with 16 KB of state in registers and eight CTAs per SM:
-// the CTAs of an SM are at different points of load -> products -> store, and the last wave is short.  (The 1024
-// (b,h) states of a batch-64, 16-head step are one wave at d = 64.  At d = 128 one CTA per state, 64 KB and two per SM, was
-// three and a half waves that loaded and stored in turn: 28.1 us for 64 x 16 states, now 24.5.)
-constexpr int kDecodeThreads = 128;
-constexpr int kDecodeCtasPerSm = 8;
-template <int DK> struct DecodeCfg { static constexpr int kRows = DK == 128 ? 32 : 64; };  // state rows of a CTA
-constexpr int kDecodeMaxDv = 128;
+// How a state is spread: state rows (held in registers) and threads of a CTA, CTAs per SM (the register budget), and whether a
+// state may be more than one CTA.  Bound by HBM for one token a call, by the token loop's latency for several.
+// Measured, us a call (device time, launches back to back, state in fp32):
+//   d = 64, 64 rows x 128 threads.  Eight CTAs per SM leave 64 registers and spill in the token loop, seven do not, and the 1024
+//     states of a batch-64, 16-head step are still one wave: one token 7.2 -> 6.2, 16 tokens 49.9 -> 40.8 (fp32 tokens 48.2 ->
+//     40.2).  The first row and the row count of a split state, as run-time values, cost the same loop 3-8 % (52.3, 52.1).
+//   d = 128, 32 rows x 128 threads x 7, a state in four CTAs: their loads, products and stores are at different points and the
+//     last wave is short.  A whole state per CTA (256 threads x 2): one token 27.6 -> 26.5 for 1024 states, 5.0 -> 3.6 for 32; 16
+//     tokens 202 -> 171, 47.0 -> 32.9 for 128.  (With eight per SM 128 states took 48.7.)
+//   d = 128, one token and 1024 states or more: 64 rows x 128 threads x 4, which load q and k half as often.  1024 states 26.5 ->
+//     25.8, 4096 states 96.3 -> 88.8, 8192 with fp32 tokens 190.5 -> 172.4; below, and for more tokens, it is the slower one
+//     (512 states 14.9 -> 15.3, 1024 states with four tokens 52.6 -> 58.1).
+template <int ROWS, int THREADS, int CTAS, bool SPLIT> struct DecodeCfg {
+  static constexpr int kRows = ROWS, kThreads = THREADS, kCtas = CTAS;
+  static constexpr bool kSplit = SPLIT;
+};
 
 template <typename T>
 __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
@@ -34,17 +41,17 @@ __device__ __forceinline__ float ld_as_float(const T* p) { return to_acc(*p); }
 // positions: optional [B] int64 array of the 1-based position of the FIRST token of this call for
 // each batch entry; if null, `pos0` is used for all.  LPR = lanes per state row = Dk/4.
 // (the kernel is latency-bound on its state loads, so resident CTAs are what hides the HBM latency)
-// ROWS: state rows of a CTA.
-template <typename T, int DK, int ROWS>
-__global__ void __launch_bounds__(kDecodeThreads, ROWS <= DecodeCfg<DK>::kRows ? kDecodeCtasPerSm : 2)
+template <typename T, int DK, typename CFG>
+__global__ void __launch_bounds__(CFG::kThreads, CFG::kCtas)
 decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
               const float* __restrict__ norm_const, T* __restrict__ out, int H, int Dv, int Tsteps, long long pos0,
               const long long* __restrict__ positions) {
+  constexpr int ROWS = CFG::kRows;
   constexpr int LPR = DK / 4;                    // lanes per row (4, 8, 16 or 32)
-  constexpr int ROWS_PER_PASS = kDecodeThreads / LPR;
+  constexpr int ROWS_PER_PASS = CFG::kThreads / LPR;
   constexpr int MAXR = (ROWS + ROWS_PER_PASS - 1) / ROWS_PER_PASS;  // state rows held per thread
   __shared__ float sq[DK], sk[DK], sv[ROWS];
-  __shared__ float red[2][kDecodeThreads / 32];
+  __shared__ float red[2][CFG::kThreads / 32];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long bh = blockIdx.x;
@@ -58,8 +65,8 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
   const float sigma = 1.0f / (1.0f + __expf(-norm_const[h]));
   const long long p0 = positions ? positions[b] : pos0;
   const int piece = tid % LPR;        // which float4 of the row
-  const int j0 = static_cast<int>(blockIdx.y) * ROWS;  // first row of this CTA
-  const int rows = min(ROWS, Dv - j0);
+  const int j0 = CFG::kSplit ? static_cast<int>(blockIdx.y) * ROWS : 0;  // first row of this CTA
+  const int rows = CFG::kSplit ? min(ROWS, Dv - j0) : Dv;
   const int row0 = tid / LPR;         // first row of this thread, in the CTA; then += ROWS_PER_PASS
 
   float* st = state + (bh * static_cast<long>(Dv) + j0) * DK;
@@ -97,7 +104,7 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
     __syncthreads();
     float nq = 0.f, nk = 0.f;
 #pragma unroll
-    for (int w = 0; w < kDecodeThreads / 32; ++w) {
+    for (int w = 0; w < CFG::kThreads / 32; ++w) {
       nq += red[0][w];
       nk += red[1][w];
     }
@@ -131,12 +138,36 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
   }
 }
 
-template <typename T, int DK, int ROWS>
-int launch_decode_rows(float* state, const T* q, const T* k, const T* v, const float* nc, T* out, unsigned states, int H, int Dv, int T_steps,
-                       long long pos0, const long long* positions, cudaStream_t stream) {
-  COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK, ROWS>, dim3(states, (Dv + ROWS - 1) / ROWS), kDecodeThreads, 0, stream, state, q, k, v, nc, out, H,
-                           Dv, T_steps, pos0, positions));
+template <typename T> struct DecodeCall {
+  float* state;
+  const T *q, *k, *v;
+  const float* nc;
+  T* out;
+  unsigned states;
+  int H, Dv, T_steps;
+  long long pos0;
+  const long long* positions;
+  cudaStream_t stream;
+};
+template <typename T, int DK, typename CFG>
+int launch_decode_as(const DecodeCall<T>& c) {
+  COTT_CUDA_TRY(launch_pdl(decode_kernel<T, DK, CFG>, dim3(c.states, (c.Dv + CFG::kRows - 1) / CFG::kRows), CFG::kThreads, 0, c.stream, c.state, c.q,
+                           c.k, c.v, c.nc, c.out, c.H, c.Dv, c.T_steps, c.pos0, c.positions));
   return COTT_OK;
+}
+// `whole`: every state by one CTA
+template <typename T, int DK>
+int launch_decode_dk(const DecodeCall<T>& c, bool whole) {
+  if constexpr (DK == 128) {
+    if (whole) return launch_decode_as<T, DK, DecodeCfg<128, 256, 2, false>>(c);
+    if (c.T_steps == 1 && c.states >= 1024) return launch_decode_as<T, DK, DecodeCfg<64, 128, 4, true>>(c);
+    return launch_decode_as<T, DK, DecodeCfg<32, 128, 7, true>>(c);
+  } else {
+    constexpr int kCtas = DK == 64 ? 7 : 8;
+    if (c.Dv <= 64) return launch_decode_as<T, DK, DecodeCfg<64, 128, kCtas, false>>(c);
+    if (whole) return launch_decode_as<T, DK, DecodeCfg<128, 256, 4, false>>(c);
+    return launch_decode_as<T, DK, DecodeCfg<64, 128, kCtas, true>>(c);
+  }
 }
 
 template <typename T>
@@ -150,24 +181,17 @@ int launch_decode(float* state, const void* q, const void* k, const void* v, con
     const uintptr_t a = reinterpret_cast<uintptr_t>(p), o = reinterpret_cast<uintptr_t>(out);
     return a < o + tokens * Dv && o < a + tokens * d;
   };
-  const bool one_cta = overlaps(q, Dk) || overlaps(k, Dk) || (out != v && overlaps(v, Dv));
-  const T *tq = static_cast<const T*>(q), *tk = static_cast<const T*>(k), *tv = static_cast<const T*>(v);
-  T* to = static_cast<T*>(out);
+  const bool whole = overlaps(q, Dk) || overlaps(k, Dk) || (out != v && overlaps(v, Dv));
+  const DecodeCall<T> c = {state, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), nc, static_cast<T*>(out), states, H,
+                           Dv, T_steps, pos0, positions, stream};
   int st = COTT_OK;
-#define COTT_DECODE_CASE(DK)                                                                                                        \
-  case DK:                                                                                                                          \
-    st = one_cta ? launch_decode_rows<T, DK, kDecodeMaxDv>(state, tq, tk, tv, nc, to, states, H, Dv, T_steps, pos0, positions, stream) \
-                 : launch_decode_rows<T, DK, DecodeCfg<DK>::kRows>(state, tq, tk, tv, nc, to, states, H, Dv, T_steps, pos0, positions, \
-                                                                   stream);                                                         \
-    break;
   switch (Dk) {
-    COTT_DECODE_CASE(16)
-    COTT_DECODE_CASE(32)
-    COTT_DECODE_CASE(64)
-    COTT_DECODE_CASE(128)
+    case 16: st = launch_decode_dk<T, 16>(c, whole); break;
+    case 32: st = launch_decode_dk<T, 32>(c, whole); break;
+    case 64: st = launch_decode_dk<T, 64>(c, whole); break;
+    case 128: st = launch_decode_dk<T, 128>(c, whole); break;
     default: return fail(COTT_ERR_SHAPE, "decode supports D_attn in {16, 32, 64, 128} (got %d)", Dk);
   }
-#undef COTT_DECODE_CASE
   if (st) return st;
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;

@@ -148,3 +148,25 @@ def test_outputs_over_the_tokens(D, T, dt):
     want = run(None)
     for over in (0, 1, 2):
         assert all(torch.allclose(a.float(), b.float(), rtol=1e-2 if dt != torch.float32 else 1e-5, atol=1e-5) for a, b in zip(run(over), want)), over
+
+
+@pytest.mark.parametrize("Dv", [33, 70, 128])
+def test_many_states_at_once(Dv):
+    """Head dim 128, one token: 1100 states take another split than 550 of them; same sums, same results."""
+    from cottention_transformer_b200 import CosAttnDecodeState
+    B, H, D = 11, 100, 128
+    g = torch.Generator(device="cuda").manual_seed(Dv)
+    q, k = (torch.randn(B, H, 1, D, device="cuda", generator=g) for _ in range(2))
+    v = torch.randn(B, H, 1, Dv, device="cuda", generator=g)
+    nc = torch.linspace(-0.5, 1.0, H, device="cuda")
+    before = torch.randn(B, H, Dv, D, device="cuda", generator=g)
+
+    def run(sel):
+        st = CosAttnDecodeState(q[sel].shape[0], H, D, Dv)
+        st.state.copy_(before[sel])
+        st.cur_s = 9
+        return st.step(q[sel], k[sel], v[sel], nc), st.state
+
+    whole, parts = run(slice(None)), [run(slice(0, 5)), run(slice(5, 10)), run(slice(10, 11))]
+    for i in range(2):
+        assert torch.allclose(whole[i], torch.cat([x[i] for x in parts]), rtol=1e-5, atol=1e-5)
