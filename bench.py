@@ -12,7 +12,7 @@ Keys beyond the basic contract:
   e2e        the same through the public host-buffer call (``CausalHostStep``) with pinned HOST buffers: every
              step copies q, k, v, dO host->device and out, dq, dk, dv, dnorm device->host inside the timed
              region, pipelined over the batch on three streams (the PCIe link is full duplex)
-  roofline   the dominant kernel (reverse-direction dK/dV pass): algorithmic bytes per launch /
+  roofline   the dominant kernel (the backward, dQ and dK/dV CTAs in one launch): algorithmic bytes per launch /
              average launch duration (CUDA events on the launching stream, inside the timed region)
              against the measured HBM copy bandwidth
   cpu_baseline  the reference's PyTorch CPU formulation (cumsum form + autograd) restated in oracle/,
@@ -48,9 +48,9 @@ import torch  # noqa: E402
 B_PER_GPU, H, N, D = 8, 16, 4096, 64
 WORKLOAD = "causal cosine attention fwd+bwd, B=8/GPU H=16 N=4096 d=64 bf16 (Q,K L2-normalised N(0,1), norm_const=0.5)"
 ELEM = 2  # bf16
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of causal_bwd_kv_kernel at the bench shape, RECORDED from an
-# ncu capture of this kernel (268.5 MB read + 98.2 MB write): a run of this file does not measure it.
-RECORDED_TRAFFIC_BYTES_PER_LAUNCH = 366_749_952
+# dram__bytes_read.sum + dram__bytes_write.sum per launch of causal_bwd_both_kernel at the bench shape, RECORDED from an
+# ncu capture of this kernel (496.2 MB read + 178.4 MB write): a run of this file does not measure it.
+RECORDED_TRAFFIC_BYTES_PER_LAUNCH = 674_652_160
 
 
 def _peaks():
@@ -371,12 +371,8 @@ def main():
     def fwd():
         _lib.check(L.cott_cos_attn_fwd(P(q), P(k), P(v), P(nc), P(out), B_PER_GPU, H, N, D, D, code, stream), "fwd")
 
-    def bwd_dq():
-        _lib.check(L.cott_cos_attn_bwd_dq(P(q), P(k), P(v), P(nc), P(do), P(dq), B_PER_GPU, H, N, D, D, code, stream), "dq")
-
-    def bwd_dkdv():
-        _lib.check(L.cott_cos_attn_bwd_dkdv(P(q), P(k), P(v), P(nc), P(do), P(dk), P(dv), P(dnc), B_PER_GPU, H, N, D, D,
-                                            code, stream), "dkdv")
+    def bwd():
+        _lib.check(L.cott_cos_attn_bwd(P(q), P(k), P(v), P(nc), P(do), P(dq), P(dk), P(dv), P(dnc), B_PER_GPU, H, N, D, D, code, stream), "bwd")
 
     def barrier():
         if world > 1:
@@ -385,8 +381,8 @@ def main():
 
     # ---- device-resident timing --------------------------------------------------------------------
     for _ in range(args.warmup):
-        fwd(), bwd_dq(), bwd_dkdv()
-    ev = [[torch.cuda.Event(enable_timing=True) for _ in range(4)] for _ in range(args.steps)]
+        fwd(), bwd()
+    ev = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(args.steps)]
     sampler = ClockSampler(local_rank)
     sampler.start()
     sampler.ready.wait(timeout=10)
@@ -396,18 +392,15 @@ def main():
         ev[i][0].record()
         fwd()
         ev[i][1].record()
-        bwd_dq()
+        bwd()
         ev[i][2].record()
-        bwd_dkdv()
-        ev[i][3].record()
     barrier()
     sampler.armed = False
     clocks = sampler.stop()
     _lib.check_device_status()
-    total_ms = ev[0][0].elapsed_time(ev[-1][3])
+    total_ms = ev[0][0].elapsed_time(ev[-1][2])
     t_fwd = sum(e[0].elapsed_time(e[1]) for e in ev) / args.steps
-    t_dq = sum(e[1].elapsed_time(e[2]) for e in ev) / args.steps
-    t_kv = sum(e[2].elapsed_time(e[3]) for e in ev) / args.steps
+    t_bwd = sum(e[1].elapsed_time(e[2]) for e in ev) / args.steps
     if world > 1:
         t = torch.tensor([total_ms], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
@@ -473,10 +466,10 @@ def main():
     if rank == 0:
         peak, peak_kind = _peaks()
         per_launch = lambda passes: passes * B_PER_GPU * H * N * D * ELEM  # noqa: E731
-        kv_bytes = per_launch(6)  # read q, k, v, dO; write dk, dv
-        achieved = kv_bytes / (t_kv * 1e-3) / 1e9
+        bwd_bytes = per_launch(7)  # read q, k, v, dO; write dq, dk, dv
+        achieved = bwd_bytes / (t_bwd * 1e-3) / 1e9
         step_bytes = per_launch(11)  # 4 (fwd) + 7 (bwd) tensor passes
-        step_gbs = step_bytes / ((t_fwd + t_dq + t_kv) * 1e-3) / 1e9
+        step_gbs = step_bytes / ((t_fwd + t_bwd) * 1e-3) / 1e9
         line = {
             "metric": "causal cosine-attention fwd+bwd tokens/s", "value": value, "unit": "tokens/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
@@ -487,14 +480,13 @@ def main():
             "clocks": clocks,
             "e2e": {"value": e2e_value, "unit": "tokens/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "copy_ceiling": copy_ceiling},
-            "gpu_launches": 3 * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "causal_bwd_kv_kernel", "achieved": achieved, "peak": peak,
+            "gpu_launches": 2 * args.steps,
+            "roofline": {"bound": "hbm", "kernel": "causal_bwd_both_kernel", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": RECORDED_TRAFFIC_BYTES_PER_LAUNCH,
                          "traffic_source": "recorded: one ncu capture of this kernel at this shape (dram bytes read + "
                                            "written per launch), not measured by this run",
-                         "peak_source": peak_kind, "algorithmic_bytes_per_launch": kv_bytes,
-                         "kernel_us": {"causal_tc_kernel<fwd>": t_fwd * 1e3, "causal_tc_kernel<dq>": t_dq * 1e3,
-                                       "causal_bwd_kv_kernel": t_kv * 1e3},
+                         "peak_source": peak_kind, "algorithmic_bytes_per_launch": bwd_bytes,
+                         "kernel_us": {"causal_tc_kernel<fwd>": t_fwd * 1e3, "causal_bwd_both_kernel": t_bwd * 1e3},
                          "step": {"algorithmic_bytes": step_bytes, "achieved": step_gbs, "frac": step_gbs / peak}},
         }
         if world == 1 and not args.no_cpu_baseline:

@@ -18,7 +18,7 @@ _PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cott_torch_bin
 _mod = None
 _tried = False
 # (bound here: transformed() runs before every call)
-_compiling, _tracing, _functorch, _modes = (torch.compiler.is_compiling, torch._C._get_tracing_state, torch._C._functorch.peek_interpreter_stack,
+_compiling, _tracing, _functorch, _modes = (torch.compiler.is_compiling, torch._C._is_tracing, torch._C._functorch.peek_interpreter_stack,
                                             torch._C._len_torch_dispatch_stack)
 
 
@@ -39,7 +39,7 @@ def transformed() -> bool:
     """Whether something looks at a Python function and its operators, or refuses them by name, and would not see the nodes
     of the compiled module: tracing, compilation, functorch transforms, forward-mode differentiation, dispatch modes (which
     count, record or choose operators, as selective checkpointing does)."""
-    return _compiling() or _tracing() is not None or _functorch() is not None or _modes() > 0 or _fw._current_level >= 0
+    return _compiling() or _tracing() or _functorch() is not None or _modes() > 0 or _fw._current_level >= 0
 
 
 def autograd():

@@ -80,8 +80,15 @@ int seg_count(long units, int N) {
 }
 // ... and what pays: a pass over c chunks takes about c chunk periods; cut into segments of cps chunks it takes cps of
 // them, about half as long again for the segments' own states, and the launches and the prefix in between, which cost
-// `overhead` chunk periods.  (Measured, forward + backward, head dim 64, segments against one: B 2, H 16, N 1024 in 4 of 2
-// chunks 51 us against 38; B 4, H 8, N 2048 in 4 of 4 64 against 64; B 1, H 16, N 8192 in 9 of 8 97 against 216.)
+// `overhead` chunk periods.  The line is drawn for a training step; one rule for all calls, so that a forward pass, a prompt
+// and a scan of the same sizes agree.  Measured, one segment per sequence against all that there is room for, us:
+//   head dim 64, overhead 10.  Forward + backward, kernels: B 2, H 16, N 1024 (4 of 2 chunks) 38 / 51, B 4, H 8, N 2048 (4 of
+//     4) 64 / 64, B 1, H 16, N 8192 (9 of 8) 216 / 97.  Forward alone (a prompt): B 1, H 16, N 1536 16.3 / 16.6, N 2048 20.5 / 17.4,
+//     N 4096 37.2 / 21.6; B 4, H 16, N 4096 38.9 / 45.3 (one is taken).  The bare scan: B 1, H 16, N 1536 12.6 / 14.4, N 2048
+//     15.7 / 14.8; B 3, H 16, N 8192 54.2 / 57.6.
+//   head dim 128, overhead 3.  Forward + backward: B 1, H 16, N 1024 111 / 104, B 4, H 16, N 2048 218 / 203; N 1024 119 / 123 (one
+//     is taken).  Forward alone: 27.0 / 27.0, 49.4 / 59.8, 27.1 / 39.3; the scan: 20.8 / 24.7, 40.9 / 50.7, 21.9 / 33.1 -- close to
+//     the line a pass by itself would rather not be cut.
 int seg_choice(long units, int N, int overhead) {
   const int nseg = seg_count(units, N), total = (N + kTcChunk - 1) / kTcChunk, cps = (total + nseg - 1) / nseg;
   return 2 * total > 3 * cps + 2 * overhead ? nseg : 1;

@@ -406,16 +406,15 @@ struct ScanFn : torch::autograd::Function<ScanFn> {
   // `entry`: the dtype whose entry point the scans go through
   static Variable forward(AutogradContext* ctx, const at::Tensor& Q, const at::Tensor& K, const at::Tensor& V, int64_t entry, bool reversed) {
     ctx->save_for_backward({Q, K, V});
-    ctx->saved_data["entry"] = entry;
-    ctx->saved_data["reversed"] = reversed;
+    ctx->saved_data["scan"] = 2 * entry + (reversed ? 1 : 0);
     return scan_by_dtype((at::ScalarType)entry, Q, K, V, reversed);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
     const at::Tensor &Q = s[0], &K = s[1], &V = s[2], g = grads[0].contiguous();
-    const int64_t entry = ctx->saved_data["entry"].toInt();
+    const int64_t scan = ctx->saved_data["scan"].toInt(), entry = scan / 2;
     const at::ScalarType t = (at::ScalarType)entry;
-    const bool rev = ctx->saved_data["reversed"].toBool();
+    const bool rev = scan % 2;
     if (at::GradMode::is_enabled())  // create_graph: the gradients are scans themselves, with nodes of their own
       return {apply(g, V, K, entry, rev), apply(V, g, Q, entry, !rev), apply(K, Q, g, entry, !rev), Variable(), Variable()};
     // one dtype and one shape in 16 bits: the three scans in one C call (autocast only ever concerns fp32 tensors)
