@@ -68,27 +68,29 @@ SegPlan plan_segments(int N, int nseg_requested) {
   return p;
 }
 
+int sm_count() {
+  int sm = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  return sm;
+}
 // Segments per sequence that `units` independent sequences of N positions can use: one CTA per SM, at least two chunks each.
 int seg_count(long units, int N) {
   const int total = (N + kTcChunk - 1) / kTcChunk;
   if (units <= 0 || total < 4) return 1;
-  int sm = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-  long nseg = sm / units;  // more sequences than half the SMs: no gain
+  long nseg = sm_count() / units;  // more sequences than half the SMs: no gain
   if (nseg > total / 2) nseg = total / 2;
   return nseg < 2 ? 1 : (int)nseg;
 }
 // ... and what pays: a pass over c chunks takes about c chunk periods; cut into segments of cps chunks it takes cps of
 // them, about half as long again for the segments' own states, and the launches and the prefix in between, which cost
-// `overhead` chunk periods.  The line is drawn for a training step; one rule for all calls, so that a forward pass, a prompt
-// and a scan of the same sizes agree.  Measured, one segment per sequence against all that there is room for, us:
+// `overhead` chunk periods.  The line is drawn for a training step; one rule for all calls, so that a forward pass and
+// a prompt of the same sizes agree.  Measured, one segment per sequence against all that there is room for, us:
 //   head dim 64, overhead 10.  Forward + backward, kernels: B 2, H 16, N 1024 (4 of 2 chunks) 38 / 51, B 4, H 8, N 2048 (4 of
 //     4) 64 / 64, B 1, H 16, N 8192 (9 of 8) 216 / 97.  Forward alone (a prompt): B 1, H 16, N 1536 16.3 / 16.6, N 2048 20.5 / 17.4,
 //     N 4096 37.2 / 21.6; B 4, H 16, N 4096 38.9 / 45.3 (one is taken).  The bare scan: B 1, H 16, N 1536 12.6 / 14.4, N 2048
 //     15.7 / 14.8; B 3, H 16, N 8192 54.2 / 57.6.
 //   head dim 128, overhead 3.  Forward + backward: B 1, H 16, N 1024 111 / 104, B 4, H 16, N 2048 218 / 203; N 1024 119 / 123 (one
-//     is taken).  Forward alone: 27.0 / 27.0, 49.4 / 59.8, 27.1 / 39.3; the scan: 20.8 / 24.7, 40.9 / 50.7, 21.9 / 33.1 -- close to
-//     the line a pass by itself would rather not be cut.
+//     is taken).  Forward alone: 27.0 / 27.0, 49.4 / 59.8, 27.1 / 39.3: close to the line a prompt would rather not be cut.
 int seg_choice(long units, int N, int overhead) {
   const int nseg = seg_count(units, N), total = (N + kTcChunk - 1) / kTcChunk, cps = (total + nseg - 1) / nseg;
   return 2 * total > 3 * cps + 2 * overhead ? nseg : 1;
@@ -364,6 +366,7 @@ struct WideTensors {  // X, Y: [B,H,N,128]; Z, C, out: [B,H,N,dz] (dz a multiple
   const void *x, *y, *z, *c;
   void* out;
   int dz;
+  int width;  // columns of Z (and of the state) that one CTA owns: 64, or 128 where dz is a multiple of it
 };
 inline TileStrides dense_rows(long H, long N, long D) { return TileStrides{H * N * D, N * D, D}; }
 
@@ -389,11 +392,9 @@ int launch_wide_w(const WideTensors& t, WideArgs a, int B, int H, int N, int dty
   COTT_CUDA_TRY(cudaGetLastError());
   return COTT_OK;
 }
-// columns of V (and of the state) that one CTA owns: the whole head where the value dimension allows it
-inline int wide_width(int dz) { return dz % 128 == 0 ? 128 : 64; }
 template <typename T, bool REV, bool NORMS, bool STATE_ONLY>
 int launch_wide_t(const WideTensors& t, const WideArgs& a, int B, int H, int N, int dtype, int nseg, cudaStream_t stream) {
-  if (wide_width(t.dz) == 128) return launch_wide_w<T, 128, REV, NORMS, STATE_ONLY>(t, a, B, H, N, dtype, nseg, stream);
+  if (t.width == 128) return launch_wide_w<T, 128, REV, NORMS, STATE_ONLY>(t, a, B, H, N, dtype, nseg, stream);
   if constexpr (!NORMS) return launch_wide_w<T, 64, REV, false, STATE_ONLY>(t, a, B, H, N, dtype, nseg, stream);
   return fail(COTT_ERR_UNSUPPORTED, "the fused head-dim-128 path takes a value dim of 128 (got %d)", t.dz);
 }
@@ -414,7 +415,6 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
     a.init_state = given_prefix;
     a.init_transposed = 1;
   } else if (plan.nseg > 1) {
-    const int W = wide_width(t.dz);
     WideArgs sa = a;
     sa.state_out = ws;
     sa.rq_out = sa.rk_out = sa.w_out = sa.decode_state = nullptr;
@@ -422,7 +422,7 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
     st.x = nullptr, st.c = nullptr, st.out = nullptr;
     int r = launch_wide_t<T, REV, NORMS, true>(st, sa, B, H, N, dtype, plan.nseg, stream);
     if (r) return r;
-    if ((r = launch_seg_prefix(ws, ws, (long)B * H * (t.dz / W), plan.nseg, 1, kTcChunk * W, false, stream))) return r;
+    if ((r = launch_seg_prefix(ws, ws, (long)B * H * (t.dz / t.width), plan.nseg, 1, kTcChunk * t.width, false, stream))) return r;
     a.init_state = ws;
   }
   return launch_wide_t<T, REV, NORMS, false>(t, a, B, H, N, dtype, plan.nseg, stream);
@@ -430,7 +430,8 @@ int run_wide(const WideTensors& t, WideArgs a, int B, int H, int N, int dtype, i
 
 size_t wide_ws_floats(int B, int H, int N, int dz, int nseg) { return (size_t)B * H * plan_segments(N, nseg).nseg * (size_t)(kTcChunk * dz); }
 
-int wide_seg_count(int B, int H, int N, int dz) { return seg_choice((long)B * H * (dz / wide_width(dz)), N, 3); }
+// the fused pair: a CTA owns the whole head
+int wide_seg_count(int B, int H, int N) { return seg_choice((long)B * H, N, 3); }
 
 // workspace of the fused head-dim-128 pair: the prefix states of the forward-direction passes and those of the reversed
 // ones (first: they are read as 16-byte words), then four fp32 vectors [B*H*N] (1/|q|, 1/|k|, keep a/|k|, -eps/|k|^2) and
@@ -441,7 +442,7 @@ struct WideWs {
   int* count;
 };
 WideWs wide_ws(void* workspace, int B, int H, int N) {
-  const size_t V = (size_t)B * H * N, A = wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128));
+  const size_t V = (size_t)B * H * N, A = wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N));
   float* f = static_cast<float*>(workspace);
   float* v = f + 2 * A;
   return WideWs{f, f + A, v, v + V, v + 2 * V, v + 3 * V, reinterpret_cast<int*>(v + 4 * V)};
@@ -459,20 +460,20 @@ int run_wide_fwd(const void* q, const void* k, const void* v, const unsigned cha
     COTT_CUDA_TRY(launch_pdl(keep_count_kernel, dim3((unsigned)B), 256, 0, stream, keep, ws.count, N));
     a.keep = keep, a.count = ws.count;
   }
-  WideTensors t{q, k, v, nullptr, out, 128};
-  return run_wide<T, false, true>(t, a, B, H, N, dtype, wide_seg_count(B, H, N, 128), ws.seg_fwd, stream);
+  WideTensors t{q, k, v, nullptr, out, 128, 128};
+  return run_wide<T, false, true>(t, a, B, H, N, dtype, wide_seg_count(B, H, N), ws.seg_fwd, stream);
 }
 
 template <typename T>
 int run_wide_bwd(const void* q, const void* k, const void* v, const unsigned char* keep, const float* nc, const void* dout,
                  void* workspace, void* dq, void* dk, void* dv, float* dnorm, int B, int H, int N, int dtype, cudaStream_t stream) {
   WideWs ws = wide_ws(workspace, B, H, N);
-  const int nseg = wide_seg_count(B, H, N, 128);
+  const int nseg = wide_seg_count(B, H, N);
   int st;
   {  // dq = rq scan(dO, V, diag(w) K), through the normalisation      (Custom_Kernel.py:106 with the module math around it)
     WideArgs a = {};
     a.zscale = ws.w, a.oscale = ws.rq, a.row_mode = kWdRowNorm;
-    WideTensors t{dout, v, k, q, dq, 128};
+    WideTensors t{dout, v, k, q, dq, 128, 128};
     if ((st = run_wide<T, false, false>(t, a, B, H, N, dtype, nseg, nullptr, stream, ws.seg_fwd))) return st;
   }
   COTT_CUDA_TRY(cudaMemsetAsync(dnorm, 0, sizeof(float) * H, stream));
@@ -480,13 +481,13 @@ int run_wide_bwd(const void* q, const void* k, const void* v, const unsigned cha
     WideArgs a = {};
     a.yscale = ws.rq, a.oscale = ws.w, a.row_mode = kWdRowEps;
     a.rk = ws.rk, a.ck_out = ws.ck, a.dnorm = dnorm, a.norm_const = nc, a.count = keep ? ws.count : nullptr;
-    WideTensors t{k, q, dout, v, dv, 128};
+    WideTensors t{k, q, dout, v, dv, 128, 128};
     if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, ws.seg_rev, stream))) return st;
   }
   {  // dk = w scan_rev(V, dO, diag(rq) Q) + ck k                    (:107)
     WideArgs a = {};
     a.zscale = ws.rq, a.oscale = ws.w, a.row_mode = kWdRowAdd, a.ccoef = ws.ck;
-    WideTensors t{v, dout, q, k, dk, 128};
+    WideTensors t{v, dout, q, k, dk, 128, 128};
     if ((st = run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, nullptr, stream, ws.seg_rev))) return st;
   }
   return COTT_OK;
@@ -656,12 +657,27 @@ cudaError_t scratch_pool(cudaMemPool_t* pool) {
   return cudaSuccess;
 }
 
+// Columns of V that one CTA of the bare scan owns at head dim 128.  With 64 a sequence is two CTAs for every 128 columns, which
+// compute the same scores: as long as all of them run at once that costs nothing, their chunks are shorter, and fewer sequences
+// need to be cut into segments.  With 128 there are half as many of them, and twice as many segments where there is room.
+// Measured, us a scan (bf16, one 128-wide CTA / two 64-wide ones / segments as chosen for either width):
+//   more than one wave of 64-wide CTAs: B 5, H 16, N 1024 22.9 / 33.4; B 8 29.5 / 40.2
+//   one wave, not cut: B 4, H 16, N 4096 73 / 60 (cut in two at 128: 89); B 4, H 12, N 2048 41.1 / 35.2; B 2, H 16, N 1024 21.0 / 18.3
+//   cut at 64 too: B 1, H 4, N 2048 in 8 segments either way 23.9 / 20.0; B 1, H 16, N 8192 in 9 / 4 51.2 / 56.0; N 32768 152 / 169
+int scan128_width(int B, int H, int N, int Dv) {
+  if (Dv % 128) return 64;
+  const long units = (long)B * H * (Dv / 64);
+  if (units > sm_count()) return 128;
+  const int total = (N + kTcChunk - 1) / kTcChunk, n64 = seg_choice(units, N, 3), n128 = seg_choice(units / 2, N, 3);
+  return n64 > 1 && 2 * ((total + n64 - 1) / n64) > 3 * ((total + n128 - 1) / n128) ? 128 : 64;
+}
+
 // Head dim 128 for Q and K: the native kernel (both halves of q, k go into the same score and state accumulators);
 // scratch only for the segment states of long sequences with few (batch, head) pairs.
 template <typename T>
 int launch_scan_tc_128(const void* q, const void* k, const void* v, void* out, int B, int H, int N, int Dv, int dtype,
                        int reversed, cudaStream_t stream) {
-  const int nseg = wide_seg_count(B, H, N, Dv);
+  const int W = scan128_width(B, H, N, Dv), nseg = seg_choice((long)B * H * (Dv / W), N, 3);
   const size_t ws_bytes = nseg > 1 ? wide_ws_floats(B, H, N, Dv, nseg) * sizeof(float) : 0;
   float* ws = nullptr;
   if (ws_bytes) {
@@ -669,7 +685,7 @@ int launch_scan_tc_128(const void* q, const void* k, const void* v, void* out, i
     COTT_CUDA_TRY(scratch_pool(&pool));
     COTT_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), ws_bytes, pool, stream));
   }
-  WideTensors t{q, k, v, nullptr, out, Dv};
+  WideTensors t{q, k, v, nullptr, out, Dv, W};
   WideArgs a = {};
   const int st = reversed ? run_wide<T, true, false>(t, a, B, H, N, dtype, nseg, ws, stream)
                           : run_wide<T, false, false>(t, a, B, H, N, dtype, nseg, ws, stream);
@@ -1030,7 +1046,7 @@ int cott_cos_attn_bwd_train(const void* q, const void* k, const void* v, const u
 size_t cott_cos_attn_wide_workspace_bytes(int B, int H, int N) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
   const size_t V = (size_t)B * H * N, cnt = ((size_t)B * N + 3) & ~(size_t)3;
-  return (4 * V + cnt + 2 * wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N, 128))) * sizeof(float);
+  return (4 * V + cnt + 2 * wide_ws_floats(B, H, N, 128, wide_seg_count(B, H, N))) * sizeof(float);
 }
 
 static int check_wide_args(int B, int H, int N, int Dk, int Dv, int dtype) {
@@ -1087,12 +1103,12 @@ template <typename T>
 int run_wide_prefill_state(const void* k, const void* v, const float* nc, float* state, void* workspace, int accumulate, int B,
                            int H, int N, int dtype, cudaStream_t stream) {
   WideWs ws = wide_ws(workspace, B, H, N);
-  const SegPlan plan = plan_segments(N, wide_seg_count(B, H, N, 128));
+  const SegPlan plan = plan_segments(N, wide_seg_count(B, H, N));
   WideArgs a = {};
   a.norm_const = nc;
   a.chunks_per_seg = plan.cps;
   a.state_out = ws.seg_fwd;
-  WideTensors t{nullptr, k, v, nullptr, nullptr, 128};
+  WideTensors t{nullptr, k, v, nullptr, nullptr, 128, 128};
   int st = launch_wide_t<T, false, true, true>(t, a, B, H, N, dtype, plan.nseg, stream);
   if (st) return st;
   wide_seg_to_decode_state_kernel<<<dim3((unsigned)((long)B * H), 16), 256, 0, stream>>>(ws.seg_fwd, state, plan.nseg, accumulate != 0);

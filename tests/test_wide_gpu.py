@@ -88,3 +88,17 @@ def test_fused_128_dq_of_long_and_short_rows(scale):
     ref = [t.double().requires_grad_() for t in (q, k, v, nc)]
     (want,) = torch.autograd.grad(O.cos_attn_causal(*ref), ref[0], do.double())
     assert _rel(dq.double() * scale, want * scale) <= REL16[torch.bfloat16]
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("H,N,Dv", [(80, 300, 128), (74, 130, 128), (16, 4200, 128), (4, 4200, 256), (40, 260, 256)])
+def test_scan_128_choice_of_width(H, N, Dv, reverse):
+    """Either side of the rule for the columns of a CTA: more CTAs than one wave holds, one wave, and segments."""
+    from cottention_transformer_b200 import kernel, _lib
+    g = torch.Generator().manual_seed(Dv + N)
+    q, k = (torch.nn.functional.normalize(torch.randn(1, H, N, 128, generator=g), dim=-1).bfloat16() for _ in range(2))
+    v = torch.randn(1, H, N, Dv, generator=g).bfloat16()
+    got = kernel.bfloat16(q.cuda(), k.cuda(), v.cuda(), 1, False, reverse)
+    _lib.check_device_status()
+    few = [0, H - 1]
+    assert _rel(got[:, few], O.scan_recurrent(q[:, few].double(), k[:, few].double(), v[:, few].double(), reverse, "f64")) <= REL16[torch.bfloat16]
