@@ -138,6 +138,11 @@ decode_kernel(float* __restrict__ state, const T* __restrict__ q, const T* __res
   }
 }
 
+inline int decode_sms() {
+  int sm = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  return sm;
+}
 template <typename T> struct DecodeCall {
   float* state;
   const T *q, *k, *v;
@@ -155,18 +160,28 @@ int launch_decode_as(const DecodeCall<T>& c) {
                            c.k, c.v, c.nc, c.out, c.H, c.Dv, c.T_steps, c.pos0, c.positions));
   return COTT_OK;
 }
+// Seven CTAs per SM or eight, for the splits that have the choice: a CTA takes about 8/7 as long with eight, but where they save a
+// wave they are the better ones (d = 64, eight tokens: 1036 states 22.2 us in one wave of seven, 1040 26.6 in one of eight, 1200 31.2 in two).
+template <typename T, int DK, int ROWS, bool SPLIT>
+int launch_decode_waves(const DecodeCall<T>& c) {
+  const long n = static_cast<long>(c.states) * ((c.Dv + ROWS - 1) / ROWS), s7 = 7l * decode_sms(), s8 = 8l * decode_sms();
+  return 8 * ((n + s8 - 1) / s8) < 7 * ((n + s7 - 1) / s7) ? launch_decode_as<T, DK, DecodeCfg<ROWS, 128, 8, SPLIT>>(c)
+                                                          : launch_decode_as<T, DK, DecodeCfg<ROWS, 128, 7, SPLIT>>(c);
+}
 // `whole`: every state by one CTA
 template <typename T, int DK>
 int launch_decode_dk(const DecodeCall<T>& c, bool whole) {
   if constexpr (DK == 128) {
+    // (several tokens, and states that are one wave by themselves but not in four CTAs of seven per SM: 272 states, eight fp32
+    // tokens 25.6 us against 27.0 in four CTAs of eight)
+    if (c.T_steps > 1 && c.states <= 2u * decode_sms() && 4l * c.states > 7l * decode_sms()) whole = true;
     if (whole) return launch_decode_as<T, DK, DecodeCfg<128, 256, 2, false>>(c);
     if (c.T_steps == 1 && c.states >= 1024) return launch_decode_as<T, DK, DecodeCfg<64, 128, 4, true>>(c);
-    return launch_decode_as<T, DK, DecodeCfg<32, 128, 7, true>>(c);
+    return launch_decode_waves<T, DK, 32, true>(c);
   } else {
-    constexpr int kCtas = DK == 64 ? 7 : 8;
-    if (c.Dv <= 64) return launch_decode_as<T, DK, DecodeCfg<64, 128, kCtas, false>>(c);
-    if (whole) return launch_decode_as<T, DK, DecodeCfg<128, 256, 4, false>>(c);
-    return launch_decode_as<T, DK, DecodeCfg<64, 128, kCtas, true>>(c);
+    if (whole && c.Dv > 64) return launch_decode_as<T, DK, DecodeCfg<128, 256, 4, false>>(c);
+    if constexpr (DK == 64) return c.Dv <= 64 ? launch_decode_waves<T, DK, 64, false>(c) : launch_decode_waves<T, DK, 64, true>(c);
+    return c.Dv <= 64 ? launch_decode_as<T, DK, DecodeCfg<64, 128, 8, false>>(c) : launch_decode_as<T, DK, DecodeCfg<64, 128, 8, true>>(c);
   }
 }
 
