@@ -3,7 +3,10 @@
 // Math (GPT_Trainer/GPTCosAttention.py:229-248,282 and its backward, see causal_tc.cuh), with every product and sum in
 // fp32 and the module's own roundings: q^ = q / max(|q|, 1e-12), k^ likewise, v' = v / max(n_s^sigma, 1), masked rows zero.
 //
-// The sequence is cut into chunks of 64 positions and EVERY chunk of EVERY (batch, head) is a CTA of its own:
+// The sequence is cut into chunks of 64 positions, from its start for the passes that run forward and from its end for those that
+// run backward (a sum that starts with a whole chunk needs the state for fewer rows: the error of dk and dv against 64 bits over
+// sequences of 64 to 1024 is 2.2e-7, with one grid for both directions it was 2.3e-7), and EVERY chunk of EVERY (batch, head)
+// is a CTA of its own:
 //   1. f32_state_kernel    the chunk's own state  sum_s y_s (x) z_s   (forward: k^, v'; reverse: q^, dO)
 //   2. f32_prefix_kernel   exclusive prefix (suffix) over the chunks of a sequence, in place
 //   3. f32_chunk_kernel    the rows of the chunk: mask(A B^T) C + A M with M the state before (after) the chunk
@@ -14,7 +17,7 @@
 // All of them are launched with programmatic dependent launch (common.cuh): seven short kernels in a row (113 -> 108 us a step
 // at the sizes below).
 // Bound by the fp32 FMA rate and the staging before it (256 CTAs at B 2, H 8, N 1024: 3 x 64^3 multiply-adds each).
-// Measured there, forward + backward: 108 us a step (11 + 7 + 22 | 10 + 7 + 54 + 3 one by one);
+// Measured there, forward + backward: 104 us a step (11 + 7 + 20 | 10 + 6 + 52 + 3 one by one); B 8, H 16, N 1024 521 us;
 // four exact scans with one CTA per sequence (16 of 148 SMs busy, 236 us each) between fifty elementwise passes took 1206 us.
 #pragma once
 
@@ -54,6 +57,13 @@ __device__ __forceinline__ float f32_row_sum(float x) {
 // max(x, lo) that lets a NaN through, as torch.clamp does
 __device__ __forceinline__ float f32_clamp_min(float x, float lo) { return x < lo ? lo : x; }
 
+// first position of a chunk; cut from the end, the first chunk of a sequence may begin before it
+template <bool REV>
+__device__ __forceinline__ int f32_chunk_start(int chunk, int nchunks, int N) {
+  return REV ? N - kF32Chunk * (nchunks - chunk) : kF32Chunk * chunk;
+}
+__device__ __forceinline__ bool f32_inside(int pos, int N) { return static_cast<unsigned>(pos) < static_cast<unsigned>(N); }
+
 // The row factors of a chunk: div[r] = max(n^sigma, 1), n[r] = the running count n_s, take[r] = un-masked.
 struct F32Rows {
   float div[kF32Chunk], n[kF32Chunk], take[kF32Chunk];
@@ -75,15 +85,15 @@ __device__ __forceinline__ void f32_rows(F32Rows& rows, const unsigned char* kee
     for (int w = 0; w < kF32Threads / 32; ++w) before += rows.part[w];
   }
   if (tid < kF32Chunk) {
-    int n = before + tid + 1;
-    float take = c0 + tid < N ? 1.f : 0.f;
+    int n = max(before + tid + 1, 0);
+    float take = f32_inside(c0 + tid, N) ? 1.f : 0.f;
     if (keep_b) {
       // inclusive count inside the chunk: the flags before this thread's 32-row half, then the ballot of its own half
-      const bool kp = c0 + tid < N && keep_b[c0 + tid];
+      const bool kp = f32_inside(c0 + tid, N) && keep_b[c0 + tid];
       const unsigned mine = __ballot_sync(0xffffffffu, kp);
       n = before + __popc(mine & (0xffffffffu >> (31 - (tid & 31))));
       if (tid >= 32)
-        for (int s = 0; s < 32; ++s) n += (c0 + s < N && keep_b[c0 + s]) ? 1 : 0;
+        for (int s = 0; s < 32; ++s) n += (f32_inside(c0 + s, N) && keep_b[c0 + s]) ? 1 : 0;
       take = kp ? 1.f : 0.f;
     }
     rows.n[tid] = static_cast<float>(n);
@@ -104,7 +114,7 @@ __device__ __forceinline__ void f32_stage(float* dst, const float* __restrict__ 
     const int r = ty + 16 * a;
 #pragma unroll
     for (int e = 0; e < NB; ++e) x[a][e] = 0.f;
-    if (c0 + r < N) f32_load<NB>(x[a], src + static_cast<long>(c0 + r) * D + NB * tx);
+    if (f32_inside(c0 + r, N)) f32_load<NB>(x[a], src + static_cast<long>(c0 + r) * D + NB * tx);
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
@@ -137,7 +147,7 @@ f32_state_kernel(const float* __restrict__ y, const float* __restrict__ z, const
   __shared__ F32Rows rows;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const long bh = blockIdx.x / nchunks;
-  const int c0 = static_cast<int>(blockIdx.x % nchunks) * kF32Chunk, h = static_cast<int>(bh % H);
+  const int c0 = f32_chunk_start<REV>(static_cast<int>(blockIdx.x % nchunks), nchunks, N), h = static_cast<int>(bh % H);
   pdl_allow_next();
   pdl_wait_prior();
   const float sigma = 1.0f / (1.0f + expf(-norm_const[h]));
@@ -200,7 +210,7 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
   constexpr bool MT = PASS == kF32Dq || PASS == kF32Dk;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const long bh = blockIdx.x / g.nchunks;
-  const int chunk = static_cast<int>(blockIdx.x % g.nchunks), c0 = chunk * kF32Chunk, h = static_cast<int>(bh % g.H), N = g.N;
+  const int N = g.N, chunk = static_cast<int>(blockIdx.x % g.nchunks), c0 = f32_chunk_start<!LOWER>(chunk, g.nchunks, N), h = static_cast<int>(bh % g.H);
   const long base = bh * N * D;
   const float sigma = 1.0f / (1.0f + expf(-g.norm_const[h]));
   const bool with_state = LOWER ? chunk > 0 : chunk + 1 < g.nchunks;  // the first (last) chunk has nothing before (after) it
@@ -329,7 +339,7 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
   if constexpr (PASS == kF32Out) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
-      if (c0 + ty + 16 * r < N) f32_store<NB>(g.out + base + static_cast<long>(c0 + ty + 16 * r) * D + NB * tx, acc[r]);
+      if (f32_inside(c0 + ty + 16 * r, N)) f32_store<NB>(g.out + base + static_cast<long>(c0 + ty + 16 * r) * D + NB * tx, acc[r]);
   } else if constexpr (MT) {
     // through the normalisation: dx = (g - x^ (x^ . g)) / max(|x|, eps) with g the masked row and x^ = x / max(|x|, eps);
     // a row shorter than eps is divided by eps alone (its norm was clamped: no gradient through it)
@@ -338,7 +348,7 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int t = ty + 16 * r;
-      const bool in = c0 + t < N;
+      const bool in = f32_inside(c0 + t, N);
       const long o = static_cast<long>(c0 + t) * D + tx;
       float x[NB], s = 0.f;
 #pragma unroll
@@ -372,7 +382,7 @@ __device__ __forceinline__ void f32_chunk(const F32Args& g, float* sA, float* sB
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int t = ty + 16 * r;
-      const bool in = c0 + t < N;
+      const bool in = f32_inside(c0 + t, N);
       const long o = base + static_cast<long>(c0 + t) * D + NB * tx;
       const float d = rows.div[t], n = rows.n[t], take = rows.take[t];
       float v[NB] = {};

@@ -161,3 +161,20 @@ def test_the_operator_itself_twice(compiled, monkeypatch):
     q, k, v = (torch.randn(1, 2, 5, 32, generator=g, dtype=torch.float64).cuda().requires_grad_() for _ in range(3))
     assert torch.autograd.gradcheck(CustomAttention.apply, (q, k, v), fast_mode=True)
     assert torch.autograd.gradgradcheck(CustomAttention.apply, (q, k.transpose(1, 2).contiguous().transpose(1, 2), v), fast_mode=True)
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("N", [65, 100, 150])
+def test_sums_begin_with_a_whole_chunk_in_their_own_direction(N, D):
+    """Forward sums are cut from the first position, reversed ones from the last: the 64 rows where either begins are those
+    of the 64 positions by themselves, bit for bit.  (With a norm_const of -200 the length factor is 1 everywhere.)"""
+    from cottention_transformer_b200 import cos_attn_causal
+    q, k, v, do, nc, _ = (None if t is None else t.cuda() for t in _inputs(2, 2, N, D, False, seed=N))
+    nc = torch.full_like(nc, -200.0)
+    whole = _run(cos_attn_causal, q, k, v, do, nc, None)
+    first = _run(cos_attn_causal, *(t[:, :, :64].contiguous() for t in (q, k, v, do)), nc, None)
+    last = _run(cos_attn_causal, *(t[:, :, -64:].contiguous() for t in (q, k, v, do)), nc, None)
+    for i in (0, 1):
+        assert torch.equal(whole[i][:, :, :64], first[i])
+    for i in (2, 3):
+        assert torch.equal(whole[i][:, :, -64:], last[i])
