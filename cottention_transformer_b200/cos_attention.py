@@ -8,8 +8,8 @@ differentiable w.r.t. q, k, v and ``norm_const``.
 
 Two modes, chosen by dtype (not a fallback chain -- each mode is a CUDA path of this library):
 
-* float16 / bfloat16, head dim 64 (with a padding mask the running count of kept positions is a launch more): ONE fused tensor-core kernel for the forward
-  (``cott_cos_attn_fwd``) and one launch for the backward (``cott_cos_attn_bwd``), fp32 accumulation;
+* float16 / bfloat16, head dim 64: ONE fused tensor-core kernel for the forward (``cott_cos_attn_fwd``) and one for the
+  backward (``cott_cos_attn_bwd``), fp32 accumulation; with a padding mask, one more that counts the kept positions;
 * float16 / bfloat16, head dim 128: the fused head-dim-128 kernels (``cott_cos_attn_wide_fwd`` / ``_bwd``);
 * float16 / bfloat16, head dim 192 / 256: the row factors pulled out of the scan, tensor-core scans on
   64-wide slices of the head dimension, closed-form backward (``_WideCausal``);
